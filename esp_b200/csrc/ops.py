@@ -91,7 +91,7 @@ _SIGNATURES = {
                       c_int, c_int, c_float, c_float, c_float, P, P],
     "esp_wait_probe": [c_int, P, P],
     "esp_moe_combine": [P, P, P, P, P, P, c_int, c_int, c_int, P, P, c_int, P],
-    "esp_pick_tokens": [P, c_int, c_int, P, P, P, P, P, P],
+    "esp_pick_tokens": [P, c_int, c_int, P, P, P, P, P, P, P],
     "esp_moe_combine_add_rmsnorm": [P, P, P, P, P, P, P, P, P, P, c_int, P, c_int, c_int, c_int, c_float, c_int, P, P, c_int, P, c_float,
                                     P],
     "esp_gemm_skinny": [P, c_longlong, P, P, c_longlong, P, P, c_int, c_longlong, P, c_int, c_int, c_int, c_int, c_int,
@@ -517,14 +517,16 @@ def moe_combine_add_rmsnorm(expert_out, topk_ids, inverse, gate, shared, x, gamm
         float(eps_y), _stream()), "moe_combine_add_rmsnorm")
 
 
-def pick_tokens(logits, temperature, top_p, rng_state, row_slot, tokens):
+def pick_tokens(logits, temperature, top_p, rng_state, row_slot, tokens, status=None):
     """tokens[r] = arg-max of row r when temperature[r] == 0 (or temperature is
     None), else a draw from the row's own splitmix64 stream rng_state[row_slot[r]]
-    (int64 storage read as unsigned)."""
+    (int64 storage read as unsigned).  ``status`` (int32): gets the bit of
+    non-finite logits, as ``finite_check`` sets it, from the same pass."""
     n, vocab = logits.shape
     _check(_fn("core", "esp_pick_tokens")(
         _ptr(logits, torch.float32, "logits"), n, vocab, _ptr(temperature, torch.float32), _ptr(top_p, torch.float32),
-        _ptr(rng_state, torch.int64), _ptr(row_slot, torch.int32), _ptr(tokens, torch.int32), _stream()), "pick_tokens")
+        _ptr(rng_state, torch.int64), _ptr(row_slot, torch.int32), _ptr(tokens, torch.int32),
+        _ptr(status, torch.int32), _stream()), "pick_tokens")
 
 
 # ---------------------------------------------------------------------------

@@ -407,9 +407,8 @@ class Engine:
             return logits, None
         b = ctx.n_seqs
         out = self.rt.ws.get("picked_tokens", (b + 1,), torch.int32)
-        ops.finite_check(logits, self.rt.status)
         ops.pick_tokens(logits, extra[0].view(torch.float32), extra[1].view(torch.float32),
-                        self.cache.engine_state.view(-1), extra[2], out)
+                        self.cache.engine_state.view(-1), extra[2], out, status=self.rt.status)
         out[b:].copy_(self.rt.status)
         return logits, out
 

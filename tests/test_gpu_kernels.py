@@ -428,6 +428,47 @@ def test_sampling_at_a_large_flat_vocabulary_picks_the_token_under_the_draw():
             f"row {r}: draw {thr:.6f} is outside [{cum[rank - 1] if rank else 0:.6f}, {cum[rank]:.6f}]")
 
 
+@pytest.mark.parametrize("vocab", [1, 255, 8192, 8193, 32770, 151936, 230001, (1 << 21) + 5])
+def test_sampling_of_equal_weights_takes_the_exact_place(vocab):
+    """A block alone (to 8,192 ids), a cluster with its weights in shared memory, one that reads them anew, and one whose
+    blocks have 2^18 ids and more.  The logits are 0 at a random subset and -inf elsewhere, so every weight is exactly 1
+    or 0 and the place of the chosen id follows from whole numbers: no tolerance."""
+    one = 1 << 40
+    rng = np.random.default_rng(vocab)
+    shares, tops, temps = [1.0, 0.5, 0.001, 0.0], [None, 0.0, 0.37, 1.0, 5.0], [0.7, 1.0, 3.0]
+    lists = [np.nonzero(rng.random(vocab) < s)[0] if s else np.array([vocab - 1]) for s in shares]
+    lists = [ids if ids.size else np.array([0]) for ids in lists]
+    cases = [(ids, tp, temps[(i + j) % 3]) for i, ids in enumerate(lists) for j, tp in enumerate(tops)]
+    logits = torch.full((len(cases), vocab), -float("inf"), device=DEV)
+    for r, (ids, _tp, _t) in enumerate(cases):
+        logits[r, torch.from_numpy(ids).to(DEV)] = 0.25 * r
+    seeds = [77 + 13 * r for r in range(len(cases))]
+    state, tokens = torch.tensor(seeds, dtype=torch.int64, device=DEV), torch.empty(len(cases), dtype=torch.int32, device=DEV)
+    st = status()
+    ops.pick_tokens(logits, torch.tensor([t for _i, _p, t in cases], device=DEV),
+                    torch.tensor([-1.0 if p is None else p for _i, p, _t in cases], device=DEV), state,
+                    torch.arange(len(cases), dtype=torch.int32, device=DEV), tokens, status=st)
+    assert st.item() == (2 if bool(torch.isinf(logits).any()) else 0)
+    for r, ((ids, tp, _t), got) in enumerate(zip(cases, tokens.tolist())):
+        stream = plain.SplitMix64(seeds[r])
+        u = float(np.float32(stream.next_f64()))
+        kept = len(ids) * one
+        if tp is not None:
+            target = int(float(kept) * float(np.float32(min(max(tp, 0.0), 1.0))))
+            kept = min(kept, max(1, -(-target // one)) * one)
+        place = max(1, -(-min(kept, int(u * float(kept))) // one))
+        assert got == ids[place - 1], f"row {r}"
+        assert (state[r].item() & ((1 << 64) - 1)) == stream.state
+
+
+def test_sampling_at_a_temperature_without_an_inverse_takes_the_arg_max():
+    logits = rnd(2, 9000)
+    tokens = torch.empty(2, dtype=torch.int32, device=DEV)
+    ops.pick_tokens(logits, torch.tensor([1e-39, 1e-40], device=DEV), torch.tensor([-1.0, 0.9], device=DEV),
+                    torch.zeros(2, dtype=torch.int64, device=DEV), torch.arange(2, dtype=torch.int32, device=DEV), tokens)
+    assert tokens.tolist() == logits.argmax(1).tolist()
+
+
 def test_sampling_follows_the_distribution():
     logits = torch.tensor([[0.0, 1.0, 2.0, -1.0, 0.5]], device=DEV).repeat(4096, 1).contiguous()
     state = torch.arange(4096, dtype=torch.int64, device=DEV) * 7919 + 3
