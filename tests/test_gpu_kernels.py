@@ -120,6 +120,42 @@ def test_gemm_simt_grouped_with_gather_and_empty_groups():
     assert torch.all(c[total:] == 7.0), "rows beyond the groups were written"
 
 
+@pytest.mark.parametrize("a_dt, w_dt", [(torch.float32, torch.float32), (torch.float32, torch.bfloat16)])
+@pytest.mark.parametrize("rows, groups, n, k", [
+    (8, 0, 65, 72),           # few rows, two by one outputs a thread, the last columns and the last k short
+    (17, 0, 37900, 40),       # few rows, four by two outputs a thread, three runs of rows
+    (25, 0, 66, 128),         # the first row count that takes tiles: the small ones
+    (131, 0, 19000, 20),      # large tiles, the last one with three rows
+    (30, 0, 130, 33),         # rows that do not start on 16 bytes
+    (300, 30, 70, 40),        # groups of few rows, some with more than eight
+    (150, 9, 66, 36),         # tiles of 32 rows
+    (1500, 20, 130, 24),      # large tiles of groups
+    (300, 40, 33, 9),         # groups, unaligned rows
+])
+def test_gemm_simt_routes_give_the_same_bits(a_dt, w_dt, rows, groups, n, k):
+    """Every kernel and tile adds the products in the order of k: the rows of any call have the bits of a chain of
+    multiply-adds over k, here made by a call with one row (its own route), and lie within rounding of the 64-bit product."""
+    rng = np.random.default_rng(rows)
+    a = rnd(rows, k, dtype=a_dt)
+    w = rnd(max(1, groups), n, k, dtype=w_dt, seed=1)
+    c = torch.full((rows + 1, n), 7.0, device=DEV)
+    if groups:
+        group_of = np.sort(np.concatenate([rng.integers(0, groups, rows - 20), np.full(20, 3)]))
+        offsets = torch.tensor(np.searchsorted(group_of, np.arange(groups + 1)), dtype=torch.int32, device=DEV)
+        ops.gemm_simt(a, w, c, group_offsets=offsets, rows=rows)
+    else:
+        group_of = np.zeros(rows, dtype=np.int64)
+        ops.gemm_simt(a, w[0], c, rows=rows)
+    assert torch.all(c[rows:] == 7.0)
+    one = torch.empty(1, n, device=DEV)
+    for r in sorted(set([0, 7, rows // 2, rows - 1] + rng.integers(0, rows, 6).tolist())):
+        ops.gemm_simt(a[r:r + 1], w[group_of[r]], one)
+        assert torch.equal(one[0], c[r]), f"row {r}"
+        exact = w[group_of[r]].double() @ a[r].double()
+        bound = k * 2.0 ** -24 * (w[group_of[r]].double().abs() @ a[r].double().abs())     # k roundings of partial sums
+        assert torch.all((c[r].double() - exact).abs() <= bound), f"row {r}"
+
+
 @pytest.mark.parametrize("dtype", [torch.float32, torch.bfloat16])
 @pytest.mark.parametrize("hd, rot", [(24, 24), (128, 128), (40, 16)])
 def test_rope_kvwrite(dtype, hd, rot):
