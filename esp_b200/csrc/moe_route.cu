@@ -16,6 +16,18 @@ enum : int {
     ROUTE_CHOSEN = 4,     // scores are the logits themselves; the weights are a softmax over the chosen experts' logits alone
 };
 
+constexpr int LANE_EXPERTS = 4;     // experts that a lane keeps in registers while its warp routes a token: up to 128 in all
+
+// A float as an unsigned number of the same order, -0 taken as 0; zero for what is never chosen (NaN, -infinity).
+__device__ __forceinline__ unsigned order_key(float v) {
+    if (!(v > -INFINITY)) return 0u;
+    const unsigned u = __float_as_uint(v + 0.f);
+    return (u & 0x80000000u) ? ~u : u | 0x80000000u;
+}
+__device__ __forceinline__ float key_value(unsigned k) {
+    return k == 0u ? -INFINITY : __uint_as_float((k & 0x80000000u) ? k & 0x7fffffffu : ~k);
+}
+
 // A token's scores from its logits, by one warp: with z = lg + bias (null: no bias) ps[e] = softmax(z)[e], sigmoid(z[e])
 // or z[e] itself (``flags``).  lg and ps may be the same array.  ``probs`` (may be null) receives a copy.
 __device__ __forceinline__ void scores_from_logits(const float* lg, float* ps, int n_experts, int lane, int flags,
@@ -24,6 +36,34 @@ __device__ __forceinline__ void scores_from_logits(const float* lg, float* ps, i
         for (int e = lane; e < n_experts; e += 32) {
             const float z = lg[e] + (bias ? bias[e] : 0.f);
             const float p = (flags & ROUTE_CHOSEN) ? z : 1.0f / (1.0f + expf(-z));
+            ps[e] = p;
+            if (probs) probs[e] = p;
+        }
+        return;
+    }
+    if (n_experts <= LANE_EXPERTS * 32) {
+        // a lane's experts stay in registers: one read of the logits, their latency taken once
+        float z[LANE_EXPERTS], mx = -INFINITY, sum = 0.f;
+#pragma unroll
+        for (int i = 0; i < LANE_EXPERTS; i++) {
+            const int e = lane + 32 * i;
+            z[i] = e < n_experts ? lg[e] + (bias ? bias[e] : 0.f) : -INFINITY;
+        }
+#pragma unroll
+        for (int i = 0; i < LANE_EXPERTS; i++) mx = fmaxf(mx, z[i]);
+        mx = warp_max(mx);
+#pragma unroll
+        for (int i = 0; i < LANE_EXPERTS; i++) {
+            if (lane + 32 * i >= n_experts) continue;
+            z[i] = expf(z[i] - mx);
+            sum += z[i];
+        }
+        sum = warp_sum(sum);
+#pragma unroll
+        for (int i = 0; i < LANE_EXPERTS; i++) {
+            const int e = lane + 32 * i;
+            if (e >= n_experts) continue;
+            const float p = z[i] / sum;
             ps[e] = p;
             if (probs) probs[e] = p;
         }
@@ -108,6 +148,37 @@ __device__ __forceinline__ float choose_topk(float* ps, float* cs, int n_experts
         }
     }
     float mass = 0.f;
+    if (n_experts <= LANE_EXPERTS * 32) {
+        // the scores as ordered integers in registers: a rank is two warp reductions of integers (redux) in place of ten
+        // shuffles and a trip through shared memory
+        unsigned key[LANE_EXPERTS];
+#pragma unroll
+        for (int i = 0; i < LANE_EXPERTS; i++) {
+            const int e = lane + 32 * i;
+            const float p = e < n_experts ? sel[e] : -INFINITY;
+            if (!(p == p) || p == INFINITY) bad = true;
+            key[i] = order_key(p);
+        }
+        for (int r = 0; r < top_k; r++) {
+            unsigned mine = key[0];
+#pragma unroll
+            for (int i = 1; i < LANE_EXPERTS; i++) mine = max(mine, key[i]);
+            const unsigned best = __reduce_max_sync(0xffffffffu, mine);
+            unsigned at = 0x7fffffffu;                        // this lane's lowest expert with that score
+#pragma unroll
+            for (int i = LANE_EXPERTS - 1; i >= 0; i--)
+                if (key[i] == best && lane + 32 * i < n_experts) at = lane + 32 * i;
+            int best_e = (int)__reduce_min_sync(0xffffffffu, at);
+            if (best == 0u) best_e = 0, bad = true;           // nothing is left to choose
+            const float score = sel == ps ? key_value(best) : ps[best_e];
+#pragma unroll
+            for (int i = 0; i < LANE_EXPERTS; i++)
+                if (lane + 32 * i == best_e) key[i] = 0u;     // taken out of the running
+            if (lane == r) { my_p = score; my_e = best_e; }   // top_k <= 32: rank r is kept by lane r
+            mass += score;
+        }
+        return mass;
+    }
     for (int r = 0; r < top_k; r++) {
         float best = -INFINITY;
         int best_e = 0x7fffffff;
@@ -425,7 +496,10 @@ router_logits_kernel(const TH* __restrict__ h, const TW* __restrict__ w_router, 
 
 // One block: a warp per token turns its logits into probabilities, picks the top k (ties to the lower
 // id) and the routing weights; then the whole block builds the permutation as moe_permute_kernel does.
-__global__ void __launch_bounds__(256)
+// Bound by the latency of one token's chain, times the tokens a warp has in turn: up to 32 warps.  With the logits' kernel, 60
+// experts, 4 chosen, eight warps and top-k by shuffles -> this: 64 tokens 37.5 -> 15.2 us, 19 tokens 15.9 -> 7.8, 8 tokens
+// 8.0 -> 7.0, 1 token 7.7 -> 6.6.
+__global__ void __launch_bounds__(1024)
 route_small_kernel(const float* __restrict__ logits, int* __restrict__ topk_ids, float* __restrict__ topk_w,
                    float* __restrict__ gate, float* __restrict__ probs_out, int n_tokens, int n_experts, int top_k,
                    int norm_topk, int has_gate, RouteChoice choice, int n_real, int* __restrict__ offsets, int* __restrict__ perm_token,
@@ -436,16 +510,17 @@ route_small_kernel(const float* __restrict__ logits, int* __restrict__ topk_ids,
     pdl_wait();
     logits = behind_wait(logits);
     extern __shared__ float sm_f[];
-    float* ps_all = sm_f;                                      // [8 warps][2 * n_experts]: scores, corrected scores
-    int* counts = reinterpret_cast<int*>(sm_f + 16 * n_experts); // [n_experts]
+    const int threads = blockDim.x, warps = threads >> 5;
+    float* ps_all = sm_f;                                      // [warps][2 * n_experts]: scores, corrected scores
+    int* counts = reinterpret_cast<int*>(sm_f + 2 * warps * n_experts); // [n_experts]
     int* cursor = counts + n_experts;                           // [n_experts + 1]
     int* pair_e = cursor + n_experts + 1;                       // [n_tokens * top_k]
     float* pair_w = reinterpret_cast<float*>(pair_e + n_tokens * top_k);   // [n_tokens * top_k]
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
-    for (int e = tid; e < n_experts; e += 256) counts[e] = 0;
+    for (int e = tid; e < n_experts; e += threads) counts[e] = 0;
     __syncthreads();
     float* ps = ps_all + warp * 2 * n_experts;
-    for (int n = warp; n < n_tokens; n += 8) {
+    for (int n = warp; n < n_tokens; n += warps) {
         const float* lg = logits + (size_t)n * (n_experts + 1);
         scores_from_logits(lg, ps, n_experts, lane, norm_topk, choice.bias, probs_out ? probs_out + (size_t)n * n_experts : nullptr);
         if (lane == 0 && has_gate) gate[n] = 1.0f / (1.0f + expf(-lg[n_experts]));
@@ -506,7 +581,7 @@ route_small_kernel(const float* __restrict__ logits, int* __restrict__ topk_ids,
     }
     __syncthreads();
     const int n_pairs = n_tokens * top_k;
-    for (int i = tid; i < n_pairs; i += 256) {
+    for (int i = tid; i < n_pairs; i += threads) {
         const int e = pair_e[i];
         if (e >= n_real) { inverse[i] = -1; continue; }
         const int row = atomicAdd(&cursor[e], 1);
@@ -958,8 +1033,13 @@ ESP_API int esp_route_small(const void* h, int h_is_bf16, const void* w_router, 
     if (tile_group && (!tile_row0 || !tile_count || !n_tiles || max_tiles < (n_real < n_tokens * top_k ? n_real : n_tokens * top_k)))
         return (int)cudaErrorInvalidValue;
     const size_t smem_a = (size_t)width * sizeof(float);
-    const size_t smem_b = (size_t)(16 * n_experts) * sizeof(float) + (size_t)(2 * n_experts + 1) * sizeof(int) +
-                          (size_t)n_tokens * top_k * (sizeof(int) + sizeof(float));
+    auto route_smem = [&](int warps) {
+        return (size_t)(2 * warps * n_experts) * sizeof(float) + (size_t)(2 * n_experts + 1) * sizeof(int) +
+               (size_t)n_tokens * top_k * (sizeof(int) + sizeof(float));
+    };
+    int warps = n_tokens <= 8 ? 8 : n_tokens <= 16 ? 16 : 32;
+    while (warps > 8 && route_smem(warps) > 48 * 1024) warps /= 2;
+    const size_t smem_b = route_smem(warps);
     if (smem_a > 48 * 1024 || smem_b > 48 * 1024) return (int)cudaErrorInvalidValue;
     const dim3 grid(n_tokens, (n_experts + 1 + 7) / 8);
 #define ESP_LOGITS(TH, TW)                                                                                        \
@@ -970,7 +1050,7 @@ ESP_API int esp_route_small(const void* h, int h_is_bf16, const void* w_router, 
     else if (w_is_bf16) ESP_LOGITS(float, bf16);
     else ESP_LOGITS(float, float);
 #undef ESP_LOGITS
-    esp_launch_pdl(ESP_PDL_SMALL, route_small_kernel, dim3(1), dim3(256), smem_b, stream, logits, topk_ids, topk_w, gate, probs_out, n_tokens, n_experts, top_k,
+    esp_launch_pdl(ESP_PDL_SMALL, route_small_kernel, dim3(1), dim3(32 * warps), smem_b, stream, logits, topk_ids, topk_w, gate, probs_out, n_tokens, n_experts, top_k,
                                                    norm_topk, w_gate ? 1 : 0, choice, n_real, offsets, perm_token, perm_weight, inverse,
                                                    status, distinct, tile_group, tile_row0, tile_count, n_tiles);
     return esp_launch_status();

@@ -440,7 +440,7 @@ ROUTE_SMALL_TOKENS = 64
 
 
 def route_small_fits(width: int, n_experts: int) -> bool:
-    # the second kernel's shared memory: probabilities of eight tokens, counts and cursors, and the step's pairs
+    # the second kernel's shared memory: probabilities of at least eight tokens at a time, counts and cursors, and the step's pairs
     return width * 4 <= 48 * 1024 and (16 * n_experts) * 4 + (2 * n_experts + 1) * 4 + ROUTE_SMALL_TOKENS * 32 * 8 <= 48 * 1024
 
 

@@ -330,6 +330,32 @@ def test_route_small_equals_router_and_permutation(w_dt, n, e, k, norm):
             assert off[ids_np[t, r]] <= row < off[ids_np[t, r] + 1] and pt[row] == t and pw[row] == w_b[t, r].item()
 
 
+@pytest.mark.parametrize("e, k", [(1, 1), (31, 4), (32, 32), (33, 8), (128, 32), (129, 7)])
+@pytest.mark.parametrize("n", [5, 8, 9, 64])
+def test_route_small_chooses_in_order_with_ties_and_masked_scores(n, e, k):
+    """The raw logits as scores (chosen_softmax): negative ones, both zeros, many ties and -infinity, chosen in the order of
+    a stable sort; sizes around a warp's width and the limit of the experts that a warp keeps in registers."""
+    rng = np.random.default_rng(n * 1000 + e)
+    want = rng.choice([-3.5, -1.0, -0.0, 0.0, 0.5, 2.0], (n, e)).astype(np.float32)
+    if e > k + 1:
+        want[1, rng.integers(0, e)] = -np.inf
+    lg = torch.tensor(want, device=DEV)
+    h = torch.eye(n, 64, device=DEV)
+    w = torch.zeros(e, 64, device=DEV)
+    w[:, :n] = torch.where(torch.isinf(lg), torch.full_like(lg, -3e38), lg).t()
+    bias = torch.zeros(e, device=DEV)
+    i32, f32 = lambda *sh: torch.empty(*sh, dtype=torch.int32, device=DEV), lambda *sh: torch.empty(*sh, device=DEV)
+    ids, wt, st = i32(n, k), f32(n, k), status()
+    ops.route_small(h, w, None, f32(n, e + 1), ids, wt, None, k, False, i32(e + 1), i32(n * k), f32(n * k), i32(n, k), st,
+                    bias=bias, chosen_softmax=True)
+    order = np.argsort(-np.where(np.isinf(want), -3e38, want) + 0.0, axis=1, kind="stable")[:, :k]
+    assert st.item() == 0
+    assert np.array_equal(ids.cpu().numpy(), order)
+    chosen = np.take_along_axis(want.astype(np.float64), order, 1)
+    ref = np.exp(chosen - chosen[:, :1])
+    close(wt, torch.tensor(ref / ref.sum(1, keepdims=True), device=DEV), torch.float32, "routing weights")
+
+
 def test_moe_permute_and_combine():
     n, k, e, width = 37, 3, 6, 50
     rng = np.random.default_rng(0)
