@@ -97,43 +97,124 @@ __global__ void latent_q_rotate_kernel(const float* __restrict__ q, const float*
 // ---------------------------------------------------------------------------------------------- per-head products
 // out[n, h, j] = sum_i a[n, h, i] * w[h, j, i]   (i < kin, j < nout); a's and out's heads may be parts of wider rows:
 // a[n, h, i] = a[n * lda + h * a_head + i], out[n, h, j] = out[n * ldo + h * o_head + j].
-// A block takes ROWS rows of one head; a warp takes output channels in turn, its lanes the input channels, so a
-// weight row is read once per ROWS rows; sums run lane-wise in index order and then over a fixed butterfly.
+// A block takes PH_ROWS rows and PH_OUTS output channels of one head, a warp PH_WARP of the channels at once.  Lane l has the
+// input channels 4 l .. 4 l + 3 of every 128, adds its products in index order, and the lanes' sums meet in a fixed
+// butterfly that brings row r of channel c to lane 8 c + r: the order of a sum depends on kin alone.
+// Few rows are bound by latency: the weights (4 values a load) of the first 512 input channels are asked for before the
+// kernel waits for its predecessor, all of them at once.  Eight rows, 16 heads, 512 -> 128 and 128 -> 512 channels, inside
+// a step: 35 and 19 us with a channel at a time and 2-byte loads, 7 and 3 here.
 constexpr int PH_ROWS = 8;
 constexpr int PH_OUTS = 16;       // output channels of a block
+constexpr int PH_WARP = 4;        // of a warp
+constexpr int PH_PIECES = 4;      // runs of 128 input channels whose weights a warp has in registers at a time
+
+// four consecutive weights as they lie in memory
+template <typename TW> struct Four;
+template <> struct Four<float> {
+    float4 v;
+    __device__ __forceinline__ void load(const float* p) { v = *reinterpret_cast<const float4*>(p); }
+    __device__ __forceinline__ void set(int i, float x) { (&v.x)[i] = x; }
+    __device__ __forceinline__ float4 get() const { return v; }
+};
+template <> struct Four<bf16> {
+    uint2 v;
+    __device__ __forceinline__ void load(const bf16* p) { v = *reinterpret_cast<const uint2*>(p); }
+    __device__ __forceinline__ void set(int i, bf16 x) {
+        const unsigned b = __bfloat16_as_ushort(x);
+        unsigned& w = i < 2 ? v.x : v.y;
+        w = (i & 1) ? (w & 0xffffu) | (b << 16) : (w & 0xffff0000u) | b;
+    }
+    __device__ __forceinline__ float4 get() const {
+        return make_float4(__uint_as_float(v.x << 16), __uint_as_float(v.x & 0xffff0000u), __uint_as_float(v.y << 16),
+                           __uint_as_float(v.y & 0xffff0000u));
+    }
+};
+
 template <typename TA, typename TW, typename TO>
 __global__ void __launch_bounds__(128)
 per_head_linear_kernel(const TA* __restrict__ a, long long lda, int a_head, const TW* __restrict__ w, TO* __restrict__ out,
                        long long ldo, int o_head, int n_rows, int kin, int nout) {
+    static_assert(PH_WARP * PH_ROWS == 32 && PH_OUTS == 4 * PH_WARP, "a lane ends up with one result");
     pdl_trigger();
-    pdl_wait();
-    extern __shared__ float as[];                  // [PH_ROWS][kin]
-    const int n0 = blockIdx.x * PH_ROWS, h = blockIdx.y;
+    extern __shared__ float4 as4[];                // [PH_ROWS][quads]
+    const int n0 = blockIdx.x * PH_ROWS, h = blockIdx.y, quads = (kin + 3) / 4;
     const int rows = min(PH_ROWS, n_rows - n0);
-    for (int idx = threadIdx.x; idx < PH_ROWS * kin; idx += blockDim.x) {
-        const int r = idx / kin, i = idx - r * kin;
-        as[idx] = r < rows ? to_f32(a[(size_t)(n0 + r) * lda + (size_t)h * a_head + i]) : 0.f;
+    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    const int j0 = blockIdx.z * PH_OUTS + warp * PH_WARP;
+    const TW* wh = w + ((size_t)h * nout + j0) * kin;
+    const bool wide = kin % 4 == 0 && (reinterpret_cast<uintptr_t>(w) & 15) == 0;
+    Four<TW> wt[PH_PIECES][PH_WARP];
+    auto load_weights = [&](int q0) {              // q0: the first quad of the pieces
+#pragma unroll
+        for (int s = 0; s < PH_PIECES; s++)
+#pragma unroll
+            for (int c = 0; c < PH_WARP; c++) {
+                const int q = q0 + s * 32 + lane;
+                wt[s][c].v = {};
+                if (j0 + c >= nout || q >= quads) continue;
+                const TW* src = wh + (size_t)c * kin + 4 * q;
+                if (wide) {
+                    wt[s][c].load(src);
+                } else {
+#pragma unroll
+                    for (int i = 0; i < 4; i++)
+                        if (4 * q + i < kin) wt[s][c].set(i, src[i]);
+                }
+            }
+    };
+    load_weights(0);
+    pdl_wait();
+    a = behind_wait(a);
+    const bool wide_a = kin % 4 == 0 && lda % 4 == 0 && a_head % 4 == 0 && (reinterpret_cast<uintptr_t>(a) & (4 * sizeof(TA) - 1)) == 0;
+    for (int idx = threadIdx.x; idx < rows * quads; idx += 128) {
+        const int r = idx / quads, i = (idx - r * quads) * 4;
+        const TA* src = a + (size_t)(n0 + r) * lda + (size_t)h * a_head + i;
+        if (wide_a) {
+            Four<TA> v;
+            v.load(src);
+            as4[idx] = v.get();
+        } else {
+            as4[idx] = make_float4(to_f32(src[0]), i + 1 < kin ? to_f32(src[1]) : 0.f, i + 2 < kin ? to_f32(src[2]) : 0.f,
+                                   i + 3 < kin ? to_f32(src[3]) : 0.f);
+        }
     }
     __syncthreads();
-    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-    const TW* wh = w + (size_t)h * nout * kin;
-    const int j_end = min(nout, ((int)blockIdx.z + 1) * PH_OUTS);
-    for (int j = blockIdx.z * PH_OUTS + warp; j < j_end; j += 4) {
-        float acc[PH_ROWS];
+    float acc[PH_WARP * PH_ROWS];
 #pragma unroll
-        for (int r = 0; r < PH_ROWS; r++) acc[r] = 0.f;
-        for (int i = lane; i < kin; i += 32) {
-            const float wv = to_f32(wh[(size_t)j * kin + i]);
+    for (int i = 0; i < PH_WARP * PH_ROWS; i++) acc[i] = 0.f;
+    for (int q0 = 0; q0 < quads; q0 += 32 * PH_PIECES) {
+        if (q0 > 0) load_weights(q0);
 #pragma unroll
-            for (int r = 0; r < PH_ROWS; r++) acc[r] = fmaf(as[r * kin + i], wv, acc[r]);
-        }
+        for (int s = 0; s < PH_PIECES; s++) {
+            const int q = q0 + s * 32 + lane;
+            if (q >= quads) continue;
+            float4 f[PH_WARP];
 #pragma unroll
-        for (int r = 0; r < PH_ROWS; r++) {
-            if (r >= rows) break;                   // the same for every lane
-            const float s = warp_sum(acc[r]);
-            if (lane == 0) out[(size_t)(n0 + r) * ldo + (size_t)h * o_head + j] = from_f32<TO>(s);
+            for (int c = 0; c < PH_WARP; c++) f[c] = wt[s][c].get();
+#pragma unroll
+            for (int r = 0; r < PH_ROWS; r++) {
+                if (r >= rows) break;               // the same for every lane
+                const float4 x = as4[r * quads + q];
+#pragma unroll
+                for (int c = 0; c < PH_WARP; c++) {
+                    float& t = acc[c * PH_ROWS + r];
+                    t = fmaf(x.w, f[c].w, fmaf(x.z, f[c].z, fmaf(x.y, f[c].y, fmaf(x.x, f[c].x, t))));
+                }
+            }
         }
     }
+    // 32 sums over 32 lanes: at every step a lane hands half of its sums to its partner and takes the other half's
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) {
+        const bool upper = (lane & o) != 0;
+#pragma unroll
+        for (int i = 0; i < o; i++) {
+            const float give = upper ? acc[i] : acc[i + o], keep = upper ? acc[i + o] : acc[i];
+            acc[i] = keep + __shfl_xor_sync(0xffffffffu, give, o);
+        }
+    }
+    const int r = lane % PH_ROWS, j = j0 + lane / PH_ROWS;
+    if (r < rows && j < nout) out[(size_t)(n0 + r) * ldo + (size_t)h * o_head + j] = from_f32<TO>(acc[0]);
 }
 
 // The same product on the tensor cores for many rows and bfloat16 weights: a block takes 64 rows x 64 output channels
@@ -506,7 +587,7 @@ ESP_API int esp_per_head_linear(const void* a, int a_dtype, long long lda, int a
     if (w_dtype == 1 && n_rows >= PHM_MIN_ROWS)
         return launch_per_head_mma(a, a_dtype, lda, a_head, w, out, o_dtype, ldo, o_head, n_rows, H, kin, nout, stream);
     dim3 grid((n_rows + PH_ROWS - 1) / PH_ROWS, H, (nout + PH_OUTS - 1) / PH_OUTS);
-    const size_t smem = (size_t)PH_ROWS * kin * sizeof(float);
+    const size_t smem = (size_t)PH_ROWS * ((kin + 3) / 4) * sizeof(float4);
 #define ESP_CASE(code_, TA, TW, TO)                                                                                          \
     case code_:                                                                                                             \
         esp_launch_pdl(ESP_PDL_SMALL, per_head_linear_kernel<TA, TW, TO>, grid, dim3(128), smem, stream, (const TA*)a, lda,   \

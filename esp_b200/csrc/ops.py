@@ -31,7 +31,7 @@ _SIGNATURES = {
     "esp_token_shift_keep": [P, c_int, P, c_longlong, P, P, c_int, c_int, P],
     "esp_gate_prepare": [c_int, P, c_longlong, P, c_longlong, P, P, P, P, P, c_longlong, c_int, P],
     "esp_gated_scan": [c_int, c_int, P, c_longlong, P, c_longlong, P, c_longlong, P, c_longlong, P, P, P, P, c_longlong, P, P, P,
-                       c_int, c_int, c_int, c_int, P],
+                       c_int, c_longlong, c_int, c_int, c_int, P],
     "esp_linear_attn_chunks": [P, P, P, c_longlong, P, P, P, P, P, P, P, c_int, P, c_longlong, P, c_int, c_int, c_int, c_int, c_int,
                                P],
     "esp_linear_attn_steps": [P, P, P, c_longlong, P, P, P, c_longlong, P, P, P, c_int, c_int, c_int, c_int, P],
@@ -973,8 +973,8 @@ def gated_scan(mode, q, k, g, v, gate_bias, lower, bonus, state, seq_start, seq_
     _check(_fn("mixers", "esp_gated_scan")(
         int(mode), 1 if ready else 0, pq, ldq, pk, ldk, pg, ldg, pv, ldv, _ptr(gate_bias, torch.float32, "gate_bias"),
         _ptr(lower, torch.float32, "lower"), _ptr(bonus, torch.float32, "bonus"), state.data_ptr(), state.stride(0),
-        _ptr(seq_start, torch.int32), _ptr(seq_slot, torch.int32), _ptr(out, torch.float32, "out"), int(n_seqs), heads,
-        key_dim, value_dim, _stream()), "gated_scan")
+        _ptr(seq_start, torch.int32), _ptr(seq_slot, torch.int32), _ptr(out, torch.float32, "out"), int(n_seqs), q.shape[0],
+        heads, key_dim, value_dim, _stream()), "gated_scan")
 
 
 LINEAR_CHUNK = 64            # tokens of a chunk of linear_attn_chunks

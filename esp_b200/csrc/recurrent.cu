@@ -109,7 +109,9 @@ constexpr int SCAN_UNROLL = ESP_SCAN_UNROLL;
 constexpr int CPT = ESP_SCAN_CPT;   // value columns a thread keeps: a token's q, k, d are read once for all of them
 constexpr int KT = 16;          // key channels a thread keeps
 constexpr int KTP = KT + 4;     // a slice's stride in shared memory: slices 80 bytes apart fall into different banks
-constexpr int CHUNK = 16;       // tokens staged at a time
+// Tokens staged at a time: 16, or 2 where the sequences bring one or two each.  Sixteen take 63 KB a block (K = V = 128), three
+// blocks an SM, and zeroing them was most of a decode step's time (8 sequences, 16 heads of 128 x 128, inside a step: 21 -> 7 us).
+constexpr int CHUNK_LONG = 16, CHUNK_SHORT = 2;
 constexpr int MAX_K = 16 * KT;  // key channels of a head that the kernel takes
 
 enum : int {
@@ -142,7 +144,7 @@ __device__ __forceinline__ void cp_async_wait_all() { asm volatile("cp.async.wai
 // q, k, g: [rows, ld*] float (k may be null in GATE_LOWER_SIGMOID); v: [rows, ldv]; head h reads columns
 // [h*K, (h+1)*K) (v: [h*V, (h+1)*V)).  state: [slots, state_stride] floats, the head's block at h*V*K laid out
 // [V][K] (a thread's key slice is contiguous).  out: [rows, H*V] float.
-template <int MODE, bool READY>
+template <int MODE, bool READY, int CHUNK>
 __global__ void __launch_bounds__(SCAN_THREADS)
 gated_scan_kernel(const float* __restrict__ q, long long ldq, const float* __restrict__ k, long long ldk,
                   const float* __restrict__ g, long long ldg, const float* __restrict__ v, long long ldv,
@@ -180,11 +182,22 @@ gated_scan_kernel(const float* __restrict__ q, long long ldq, const float* __res
     __syncthreads();
 
     pdl_wait();
+    // a thread's slice of the state in pieces of 16 bytes where they are aligned
+    const bool quads = K % 4 == 0 && state_stride % 4 == 0 && ((size_t)state & 15) == 0;
     float S[CPT][KT];
 #pragma unroll
     for (int j = 0; j < CPT; j++)
 #pragma unroll
-        for (int i = 0; i < KT; i++) S[j][i] = (live[j] && part * KT + i < K) ? srow[(size_t)j * K + i] : 0.f;
+        for (int i = 0; i < KT; i += 4) {
+            const bool in = live[j] && part * KT + i < K;
+            if (quads) {
+                const float4 s4 = in ? *reinterpret_cast<const float4*>(srow + (size_t)j * K + i) : make_float4(0.f, 0.f, 0.f, 0.f);
+                S[j][i] = s4.x, S[j][i + 1] = s4.y, S[j][i + 2] = s4.z, S[j][i + 3] = s4.w;
+            } else {
+#pragma unroll
+                for (int e = 0; e < 4; e++) S[j][i + e] = (live[j] && part * KT + i + e < K) ? srow[(size_t)j * K + i + e] : 0.f;
+            }
+        }
 
     // 16-byte copies where every row piece is aligned (the usual case: K, V and the row strides multiples of 4)
     const bool wide = (K % 4 == 0) && (V % 4 == 0) && (vt % 4 == 0) && (ldq % 4 == 0) && (!LOADS_D || ldg % 4 == 0) &&
@@ -304,8 +317,16 @@ gated_scan_kernel(const float* __restrict__ q, long long ldq, const float* __res
     for (int j = 0; j < CPT; j++) {
         if (!live[j]) continue;
 #pragma unroll
-        for (int i = 0; i < KT; i++)
-            if (part * KT + i < K) srow[(size_t)j * K + i] = S[j][i];
+        for (int i = 0; i < KT; i += 4) {
+            if (quads) {
+                if (part * KT + i < K)
+                    *reinterpret_cast<float4*>(srow + (size_t)j * K + i) = make_float4(S[j][i], S[j][i + 1], S[j][i + 2], S[j][i + 3]);
+            } else {
+#pragma unroll
+                for (int e = 0; e < 4; e++)
+                    if (part * KT + i + e < K) srow[(size_t)j * K + i + e] = S[j][i + e];
+            }
+        }
     }
 }
 
@@ -740,11 +761,12 @@ ESP_API int esp_gate_prepare(int mode, const float* q, long long ldq, const floa
 // mode: 0 = decay exp(-exp(.)) with an extra weight on the token being read, 1 = lower-bounded sigmoid gate that also writes,
 // 2 (with ready) = one ready-made decay per head and token, g being [rows, H]; q and k as given, the output reads S_t.
 // 3 = one decay per head, g and lower being [H] (see GATE_FIXED).
+// rows: how many rows the sequences bring in all.
 // ready: q, k and g already hold the query, the written key and the decay (esp_gate_prepare made them).
 ESP_API int esp_gated_scan(int mode, int ready, const float* q, long long ldq, const float* k, long long ldk, const float* g,
                            long long ldg, const float* v, long long ldv, const float* gate_bias, const float* lower,
                            const float* bonus, float* state, long long state_stride, const int* seq_start,
-                           const int* seq_slot, float* out, int n_seqs, int H, int K, int V, cudaStream_t stream) {
+                           const int* seq_slot, float* out, int n_seqs, long long rows, int H, int K, int V, cudaStream_t stream) {
     if (n_seqs <= 0) return 0;
     if (K <= 0 || V <= 0 || K > MAX_K || H > 65535) return (int)cudaErrorInvalidValue;
     int ks = 1;
@@ -755,14 +777,15 @@ ESP_API int esp_gated_scan(int mode, int ready, const float* q, long long ldq, c
     if ((long long)n_seqs * H * ((V + (threads / ks) * CPT - 1) / ((threads / ks) * CPT)) < 148 && ks <= 32 && V > (64 / ks) * CPT) threads = ESP_SCAN_SMALL_THREADS;
     const int vt = (threads / ks) * CPT;
     const int vtiles = (V + vt - 1) / vt;
-    const size_t smem = 2 * (size_t)CHUNK * (3 * ks * KTP + vt) * sizeof(float);
+    const bool few = rows <= (long long)CHUNK_SHORT * n_seqs;      // a longer run among them still passes, two tokens at a time
+    const size_t smem = 2 * (size_t)(few ? CHUNK_SHORT : CHUNK_LONG) * (3 * ks * KTP + vt) * sizeof(float);
     dim3 grid(n_seqs, H, vtiles);
     if ((mode == GATE_EXP_EXP || mode == GATE_FIXED || ready) && !k) return (int)cudaErrorInvalidValue;
 #define ESP_SCAN(MODE_, READY_)                                                                                              \
     {                                                                                                                       \
-        auto kernel = gated_scan_kernel<MODE_, READY_>;                                                                     \
+        auto kernel = few ? gated_scan_kernel<MODE_, READY_, CHUNK_SHORT> : gated_scan_kernel<MODE_, READY_, CHUNK_LONG>;    \
         static bool set = false;                                                                                            \
-        if (!set) { cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, 160 * 1024); set = true; }     \
+        if (!set && !few) { cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, 160 * 1024); set = true; } \
         /* a step of many rows runs long and holds its shared memory: no early start beside its predecessor */             \
         esp_launch_pdl(READY_ ? 0 : ESP_PDL_SMALL, kernel, grid, dim3(threads), smem, stream, q, ldq, k, ldk, g, ldg, v, ldv, \
                        gate_bias, lower, bonus, state, state_stride, seq_start, seq_slot, out, H, K, V, ks, vt);            \

@@ -224,6 +224,49 @@ def test_per_head_product(a_dtype, w_dtype, o_dtype):
     assert float(got[..., nout:].abs().max()) == 0.0
 
 
+@pytest.mark.parametrize("N, kin, nout", [(1, 128, 17), (8, 130, 16), (9, 512, 33), (7, 516, 5), (16, 1000, 3), (3, 1, 1)])
+@pytest.mark.parametrize("w_dtype", [torch.float32, torch.bfloat16])
+def test_per_head_product_of_few_rows(N, kin, nout, w_dtype):
+    """Sizes around the kernel's pieces (128 channels a piece, four pieces at a time, four outputs a warp, eight rows), rows on
+    any alignment; a row's sum does not depend on the others."""
+    torch.manual_seed(kin)
+    H = 3
+    a = torch.randn(N, H * kin, device=DEV)
+    w = torch.randn(H, nout, kin, device=DEV).to(w_dtype)
+    out = torch.full((N, H * (nout + 1)), 5.0, device=DEV)
+    ops.per_head_linear(a, H * kin, kin, w, out, H * (nout + 1), nout + 1, N, H, kin, nout)
+    a64, w64 = a.double().view(N, H, kin), w.double()
+    got = out.view(N, H, nout + 1)
+    bound = (kin + 8) * 2.0 ** -24 * torch.einsum("nhi,hji->nhj", a64.abs(), w64.abs())        # a rounding per addition
+    assert torch.all((got[..., :nout].double() - torch.einsum("nhi,hji->nhj", a64, w64)).abs() <= bound)
+    assert torch.all(got[..., nout:] == 5.0)
+    one = torch.zeros(1, H * nout, device=DEV)
+    ops.per_head_linear(a[N - 1:], H * kin, kin, w, one, H * nout, nout, 1, H, kin, nout)
+    assert torch.equal(one.view(H, nout), got[N - 1, :, :nout])
+
+
+@pytest.mark.parametrize("mode", [ops.SCAN_DECAY_BONUS, ops.SCAN_LOWER_SIGMOID])
+@pytest.mark.parametrize("K, V", [(128, 128), (30, 7), (16, 20)])
+def test_gated_scan_of_few_rows_equals_the_staging_of_many(mode, K, V):
+    """Runs of one to three rows (two tokens staged at a time) give the bits that they give beside a long run (sixteen)."""
+    torch.manual_seed(K)
+    H, runs = 2, [1, 3, 2, 1]
+    T, more = sum(runs), 40
+    q, k, g = (torch.randn(T + more, H * K, device=DEV) for _ in range(3))
+    v = torch.randn(T + more, H * V, device=DEV)
+    first, bonus, low = torch.randn(6, H * K * V, device=DEV), torch.randn(H * K, device=DEV), torch.rand(H * K, device=DEV)
+    results = []
+    for lens in (runs, runs + [more]):
+        starts = np.concatenate([[0], np.cumsum(lens)])
+        n = int(starts[-1])
+        state, out = first.clone(), torch.zeros(n, H * V, device=DEV)
+        ops.gated_scan(mode, q[:n], k[:n] if mode == ops.SCAN_DECAY_BONUS else None, g[:n], v[:n], None,
+                       low if mode == ops.SCAN_LOWER_SIGMOID else None, bonus if mode == ops.SCAN_DECAY_BONUS else None, state,
+                       i32(starts.tolist()), i32([4, 0, 3, 1, 5][:len(lens)]), out, len(lens), H, K, V)
+        results.append((out[:T], state[:5]))
+    assert torch.equal(results[0][0], results[1][0]) and torch.equal(results[0][1], results[1][1])
+
+
 def attention_reference(qx, rows, pos, window, scale, hdv):
     """qx [H, hdk], rows [pos + 1, hdk] (float64): the query at ``pos`` over its visible rows."""
     lo = max(0, pos - window + 1) if window else 0
