@@ -25,8 +25,8 @@
 namespace {
 constexpr int WARPS = 8;
 // 16-byte pieces of each of its two weight rows that a lane has in flight, and blocks per SM.  Measured on the
-// 24-layer decode step: 4 pieces and 3 blocks beat 8 and 2, 6 and 2, 2 and 4 at batch 1 and at batch 8.
-constexpr int UNROLL = 4;
+// 24-layer decode step: 4 pieces and 3 blocks beat 8 and 2, 6 and 2, 2 and 4 at batch 1 and at batch 8, each for every
+// product; dense products of few blocks take 8 and 2 (launch_variant).
 #define ESP_SKINNY_BLOCKS 3
 
 struct SkinnyParams {
@@ -132,8 +132,8 @@ __device__ __forceinline__ uint4 load_stream(const bf16* p) {
 // KS: how many of the block's 8 warps share one tile of weight rows, each with its own slice of K (8 / KS
 // tiles per block).  Few tiles: KS = 8, so that every SM still gets work; many tiles: KS = 1, each warp
 // walks all of K of its own tile (longer streams per warp, no reduction between warps); 2 and 4 lie between.
-template <int NBLK, int MODE, typename TC, int KS>
-__global__ void __launch_bounds__(WARPS * 32, ESP_SKINNY_BLOCKS)
+template <int NBLK, int MODE, typename TC, int KS, int UNROLL>
+__global__ void __launch_bounds__(WARPS * 32, UNROLL > 4 ? 2 : ESP_SKINNY_BLOCKS)
 gemm_skinny_kernel(SkinnyParams p) {
     constexpr bool SWIGLU = MODE == MODE_SWIGLU, ROPE = MODE == MODE_ROPE, PAIRS = SWIGLU || ROPE;
     extern __shared__ __align__(16) unsigned char smem_raw[];
@@ -353,13 +353,13 @@ gemm_skinny_kernel(SkinnyParams p) {
     }
 }
 
-template <int NBLK, int MODE, typename TC, int KS>
-int launch_variant(const SkinnyParams& p, int groups, int tiles, cudaStream_t stream) {
+template <int NBLK, int MODE, typename TC, int KS, int UNROLL>
+int launch_unrolled(const SkinnyParams& p, int groups, int tiles, cudaStream_t stream) {
     const size_t smem = (size_t)8 * NBLK * (p.K + 32) * sizeof(bf16) + (size_t)WARPS * NBLK * 32 * 4 * sizeof(float);
     if (smem > 227 * 1024) return (int)cudaErrorInvalidValue;
     static bool raised = false;        // per instantiation
     if (smem > 48 * 1024 && !raised) {
-        cudaError_t e = cudaFuncSetAttribute(gemm_skinny_kernel<NBLK, MODE, TC, KS>,
+        cudaError_t e = cudaFuncSetAttribute(gemm_skinny_kernel<NBLK, MODE, TC, KS, UNROLL>,
                                              cudaFuncAttributeMaxDynamicSharedMemorySize, 227 * 1024);
         if (e != cudaSuccess) return (int)e;
         raised = true;
@@ -374,8 +374,21 @@ int launch_variant(const SkinnyParams& p, int groups, int tiles, cudaStream_t st
     const bool fits = p.M <= 8 && (long long)grid.x * grid.y <= 148 * ESP_SKINNY_BLOCKS && weight_bytes <= (128ll << 20);
     const int kind = !p.group_offsets ? ESP_PDL_DENSE : p.offsets_ready ? ESP_PDL_GROUPED_AFTER
                      : fits && esp_pdl_enabled(ESP_PDL_GROUPED_FITS) ? ESP_PDL_GROUPED_FITS : ESP_PDL_GROUPED;
-    esp_launch_pdl(kind, gemm_skinny_kernel<NBLK, MODE, TC, KS>, grid, dim3(WARPS * 32), smem, stream, p);
+    esp_launch_pdl(kind, gemm_skinny_kernel<NBLK, MODE, TC, KS, UNROLL>, grid, dim3(WARPS * 32), smem, stream, p);
     return esp_launch_status();
+}
+
+template <int NBLK, int MODE, typename TC, int KS>
+int launch_variant(const SkinnyParams& p, int groups, int tiles, cudaStream_t stream) {
+    // A dense product of at most two blocks per SM: eight pieces of each row in flight instead of four, for which two blocks
+    // leave the registers.  A warp's slice of a row then is one or two trips to memory (eight rows, K = 5,632, N = 2,048: 20.5 ->
+    // 18.4 us; 2,048 x 768 10.2 -> 8.2; 3,584 x 4,608 18.6 -> 16.7; one row the same or 1 us less).  Larger grids keep four
+    // pieces and three blocks.
+    constexpr int TILES = WARPS / KS;
+    if constexpr (KS >= 4) {
+        if (!p.group_offsets && (tiles + TILES - 1) / TILES <= 2 * 148) return launch_unrolled<NBLK, MODE, TC, KS, 8>(p, groups, tiles, stream);
+    }
+    return launch_unrolled<NBLK, MODE, TC, KS, 4>(p, groups, tiles, stream);
 }
 
 template <int NBLK, int MODE, typename TC>
