@@ -259,6 +259,57 @@ def test_attention_finds_the_key_that_matters(dtype, nh, nkv, hd, window):
         close(out[i].view(nh, hd), ref, dtype, f"query {i} (sequence {s}, position {p}, target key {target})")
 
 
+@pytest.mark.parametrize("hd, vd, page", [(128, 128, 64), (40, 24, 64), (4, 128, 16)])
+@pytest.mark.parametrize("opts", [dict(window=None), dict(window=70), dict(window=70, keep=5), dict(window=None, chunk=48),
+                                  dict(window=None, sink=True, softcap=5.0), dict(window=1)])
+def test_attention_in_32_bit_of_runs_of_tokens(hd, vd, page, opts):
+    """Runs of tokens that begin and end on any position, cut by the 16 tokens a block takes, beside single ones: the 64-bit
+    result over the visible keys, the bits of the same token in a call by itself, and nothing of a value that a token
+    does not see although a later token of its run does."""
+    torch.manual_seed(hd)
+    nh, nkv, lens = 4, 2, [150, 130, 40]
+    per = -(-max(lens) // page)
+    table = torch.tensor([[3 * i + s for i in range(per)] for s in range(3)], dtype=torch.int32, device=DEV)
+    kc, vc = torch.randn(3 * per, nkv, page, hd, device=DEV), torch.randn(3 * per, nkv, page, vd, device=DEV)
+    where = lambda s, p: (int(table[s, p // page]), slice(None), p % page)
+    vc[where(0, 149)] = float("nan")                         # seen by the last token of sequence 0 alone
+    toks = [(0, p) for p in range(91, 150)] + [(1, 129), (2, 0), (2, 1), (2, 2), (2, 39)] + [(1, p) for p in range(0, 33)]
+    q = torch.randn(len(toks), nh * hd, device=DEV)
+    opts = dict(opts)
+    window, chunk, keep, softcap = (opts.get(k) for k in ("window", "chunk", "keep", "softcap"))
+    i32 = lambda v: torch.tensor(v, dtype=torch.int32, device=DEV)
+    st = status()
+
+    def run(idx):
+        out = torch.full((len(idx), nh * vd), 3.0, device=DEV)
+        ops.attn_simt(q[idx].contiguous(), kc, vc, out, i32([toks[i][0] for i in idx]), i32([toks[i][1] for i in idx]), table, page, nh,
+                      nkv, hd, opts.get("window"), st, vd=vd, **{k: v for k, v in opts.items() if k != "window"})
+        return out.view(len(idx), nh, vd)
+
+    got = run(list(range(len(toks))))
+    for i, (s, pos) in enumerate(toks):
+        lo = pos - pos % chunk if chunk else max(0, pos - window + 1) if window else 0
+        keys = [j for j in range(pos + 1) if j >= lo or j < (keep or 0)]
+        k = torch.stack([kc[where(s, j)] for j in keys]).double()
+        v = torch.stack([vc[where(s, j)] for j in keys]).double()
+        x = torch.einsum("hd,khd->hk", q[i].double().view(nh, hd), k.repeat_interleave(nh // nkv, 1)) / np.sqrt(hd)
+        if softcap:
+            x = softcap * torch.tanh(x / softcap)
+        if opts.get("sink"):
+            x = torch.cat([x, torch.zeros(nh, 1, device=DEV, dtype=torch.float64)], 1)
+        ref = torch.einsum("hk,khd->hd", torch.softmax(x, 1)[:, :len(keys)], v.repeat_interleave(nh // nkv, 1))
+        if (s, pos) == (0, 149):
+            assert torch.isnan(got[i]).all()
+            continue
+        close(got[i], ref, torch.float32, f"token {i} (sequence {s}, position {pos})")
+        if i % 7 == 0 or i == len(toks) - 1:
+            assert torch.equal(run([i])[0], got[i])
+    assert st.item() == 0
+    table[1, 32 // page] = 3 * per                           # a page that does not exist
+    run([i for i, t in enumerate(toks) if t == (1, 32)])
+    assert st.item() == 8
+
+
 @pytest.mark.parametrize("h_dt, w_dt", [(torch.float32, torch.float32), (torch.float32, torch.bfloat16)])
 @pytest.mark.parametrize("norm", [False, True])
 def test_router_topk(h_dt, w_dt, norm):
