@@ -86,12 +86,13 @@ __device__ __forceinline__ float block_max(float v, float* scratch) {
     return scratch[32];
 }
 
-// A row that a block holds in registers, up to four pieces of four channels a thread (piece threadIdx.x + i * blockDim.x of
+// A row that a block holds in registers, up to PIECES pieces of four channels a thread (piece threadIdx.x + i * blockDim.x of
 // ``pieces``): takes ``mean`` off every channel and returns the sum of the squares of what is left.
-__device__ __forceinline__ float take_mean(float4 (&v)[4], int pieces, float mean, float* scratch) {
+template <int PIECES>
+__device__ __forceinline__ float take_mean(float4 (&v)[PIECES], int pieces, float mean, float* scratch) {
     float ss = 0.f;
 #pragma unroll
-    for (int i = 0; i < 4; i++) {
+    for (int i = 0; i < PIECES; i++) {
         if (threadIdx.x + i * blockDim.x >= pieces) continue;
         v[i].x -= mean, v[i].y -= mean, v[i].z -= mean, v[i].w -= mean;
         ss = fmaf(v[i].w, v[i].w, fmaf(v[i].z, v[i].z, fmaf(v[i].y, v[i].y, fmaf(v[i].x, v[i].x, ss))));

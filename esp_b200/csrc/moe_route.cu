@@ -749,6 +749,57 @@ moe_permute_kernel(const int* __restrict__ topk_ids, const float* __restrict__ t
     }
 }
 
+// A token's chosen experts in ascending id, by the first warp of a block: src[j] is the row of expert_out that stands at
+// place j of the order, or -1; weight[j] is what it counts: 1 for such a row; for an id from n_real on (``ident`` given) the
+// routing weight of the token's own input; 0 where there is nothing to add.  A lane ranks its own id among the others'.
+__device__ __forceinline__ void order_by_expert(const int* ids, const int* inverse, const float* weights, bool passing, int n_real,
+                                                int top_k, int* src, float* weight) {
+    const int lane = threadIdx.x;
+    if (lane >= 32) return;
+    const int id = lane < top_k ? ids[lane] : 0x7fffffff, row = lane < top_k ? inverse[lane] : -1;
+    const float w = passing && lane < top_k && id >= n_real ? weights[lane] : 0.f;
+    int place = 0;
+    for (int k = 0; k < top_k; k++) {
+        const int other = __shfl_sync(0xffffffffu, id, k);
+        place += other < id || (other == id && k < lane);
+    }
+    if (lane < top_k) src[place] = row, weight[place] = row >= 0 ? 1.0f : w;
+}
+
+// acc[i] += the token's terms in their order, for the block's pieces q = threadIdx.x + i * blockDim.x.  AHEAD terms of all
+// pieces are asked for before the first is added: with one load after the other a row of 2,048 channels and four experts
+// took sixteen trips to memory, one after the other (2,048 rows 33.6 -> 25.7 us, of which the bytes take 21; 4,096 rows of
+// 3,584 channels and eight experts 188 -> 127 us).
+template <int PIECES, int AHEAD>
+__device__ __forceinline__ void add_terms(float4 (&acc)[PIECES], const float* expert_out, const float* ident_row, const int* src,
+                                          const float* weight, int top_k, int width, int pieces) {
+    for (int j0 = 0; j0 < top_k; j0 += AHEAD) {
+        float4 e[AHEAD][PIECES];
+#pragma unroll
+        for (int a = 0; a < AHEAD; a++) {
+            if (j0 + a >= top_k || weight[j0 + a] == 0.f) continue;      // the same for the whole block
+            const int row = src[j0 + a];
+            const float4* from = reinterpret_cast<const float4*>(row >= 0 ? expert_out + (size_t)row * width : ident_row);
+#pragma unroll
+            for (int i = 0; i < PIECES; i++) {
+                const int q = threadIdx.x + i * blockDim.x;
+                if (q < pieces) e[a][i] = __ldg(from + q);
+            }
+        }
+#pragma unroll
+        for (int a = 0; a < AHEAD; a++) {
+            if (j0 + a >= top_k || weight[j0 + a] == 0.f) continue;
+            const float w = weight[j0 + a];                               // 1 for an expert's row: the product is the row itself
+#pragma unroll
+            for (int i = 0; i < PIECES; i++) {
+                if (threadIdx.x + i * blockDim.x >= pieces) continue;
+                acc[i].x = fmaf(w, e[a][i].x, acc[i].x), acc[i].y = fmaf(w, e[a][i].y, acc[i].y);
+                acc[i].z = fmaf(w, e[a][i].z, acc[i].z), acc[i].w = fmaf(w, e[a][i].w, acc[i].w);
+            }
+        }
+    }
+}
+
 // y[t, :] = sum over the token's chosen experts, in ascending expert id, of
 // expert_out[inverse[t, r], :] (already scaled by the routing weight), then
 // + gate[t] * shared[t, :].  With ``ident`` (float [tokens, width]): a chosen id from n_real on is an expert without
@@ -761,58 +812,38 @@ __global__ void moe_combine_kernel(const float* __restrict__ expert_out, const i
     pdl_wait();
     expert_out = behind_wait(expert_out);
     shared = behind_wait(shared);
-    __shared__ int order[MAX_TOPK];
-    __shared__ float pass_w[MAX_TOPK];
-    const int t = blockIdx.x;
-    if (threadIdx.x == 0) {
-        int ids[MAX_TOPK];
-        for (int r = 0; r < top_k; r++) { ids[r] = topk_ids[(size_t)t * top_k + r]; order[r] = r; }
-        for (int a = 1; a < top_k; a++) {          // insertion sort of ranks by expert id
-            const int oa = order[a], ia = ids[oa];
-            int b = a - 1;
-            while (b >= 0 && ids[order[b]] > ia) { order[b + 1] = order[b]; b--; }
-            order[b + 1] = oa;
-        }
-        for (int r = 0; r < top_k; r++) {
-            const int o = order[r];
-            pass_w[r] = (ident && ids[o] >= n_real) ? topk_w[(size_t)t * top_k + o] : 0.f;
-            order[r] = inverse[(size_t)t * top_k + o];
-        }
-    }
+    __shared__ int src[MAX_TOPK];
+    __shared__ float weight[MAX_TOPK];
+    const size_t t = blockIdx.x;
+    order_by_expert(topk_ids + t * top_k, inverse + t * top_k, topk_w ? topk_w + t * top_k : nullptr, ident != nullptr, n_real, top_k,
+                    src, weight);
     __syncthreads();
     const float g = gate ? gate[t] : 1.0f;       // no gate: the shared rows are added as they are
     if ((width & 3) == 0) {
         // four columns per thread; each column still adds its terms in the same order
-        for (int i = threadIdx.x * 4; i < width; i += blockDim.x * 4) {
-            float4 acc = make_float4(0.f, 0.f, 0.f, 0.f);
-            for (int r = 0; r < top_k; r++) {
-                const int row = order[r];
-                if (row >= 0) {
-                    const float4 v = __ldg(reinterpret_cast<const float4*>(expert_out + (size_t)row * width + i));
-                    acc.x += v.x; acc.y += v.y; acc.z += v.z; acc.w += v.w;
-                } else if (pass_w[r] != 0.f) {
-                    const float4 v = *reinterpret_cast<const float4*>(ident + (size_t)t * width + i);
-                    const float pw = pass_w[r];
-                    acc.x += pw * v.x; acc.y += pw * v.y; acc.z += pw * v.z; acc.w += pw * v.w;
-                }
-            }
+        const int pieces = width / 4;
+        for (int q0 = 0; q0 < pieces; q0 += blockDim.x) {
+            const int q = q0 + threadIdx.x;
+            float4 acc[1] = {make_float4(0.f, 0.f, 0.f, 0.f)}, own = acc[0];
+            if (shared && q < pieces) own = __ldg(reinterpret_cast<const float4*>(shared + t * width) + q);
+            add_terms<1, 4>(acc, expert_out + 4 * q0, ident ? ident + t * width + 4 * q0 : nullptr, src, weight, top_k, width, pieces - q0);
+            if (q >= pieces) continue;
             if (shared) {
-                const float4 v = __ldg(reinterpret_cast<const float4*>(shared + (size_t)t * width + i));
-                acc.x += g * v.x; acc.y += g * v.y; acc.z += g * v.z; acc.w += g * v.w;
+                acc[0].x += g * own.x; acc[0].y += g * own.y; acc[0].z += g * own.z; acc[0].w += g * own.w;
             }
-            *reinterpret_cast<float4*>(y + (size_t)t * width + i) = acc;
+            reinterpret_cast<float4*>(y + t * width)[q] = acc[0];
         }
         return;
     }
     for (int i = threadIdx.x; i < width; i += blockDim.x) {
         float acc = 0.f;
-        for (int r = 0; r < top_k; r++) {
-            const int row = order[r];
-            if (row >= 0) acc += expert_out[(size_t)row * width + i];
-            else if (pass_w[r] != 0.f) acc += pass_w[r] * ident[(size_t)t * width + i];
+        for (int j = 0; j < top_k; j++) {
+            if (weight[j] == 0.f) continue;
+            const float* from = src[j] >= 0 ? expert_out + (size_t)src[j] * width : ident + t * width;
+            acc = fmaf(weight[j], from[i], acc);
         }
-        if (shared) acc += g * shared[(size_t)t * width + i];
-        y[(size_t)t * width + i] = acc;
+        if (shared) acc += g * shared[t * width + i];
+        y[t * width + i] = acc;
     }
 }
 // The combine above fused with what follows it in a pre-norm block: the residual add and the next RMSNorm.
@@ -822,8 +853,9 @@ __global__ void moe_combine_kernel(const float* __restrict__ expert_out, const i
 // results are the same bits.  Width a multiple of 4, at most 16384.  With gamma_y the combined row is normalised before it
 // is added: y <- y / sqrt(mean(y^2) + eps_y) * gamma_y (POST), and then gamma null: h[r] = v as it is; h null: the add alone.
 // LAYER: the norm behind the add is the layer norm, (v - mean(v)) * rsqrt(mean((v - mean(v))^2) + eps) * gamma + beta.
-template <typename TH, bool POST, bool LAYER>
-__global__ void __launch_bounds__(1024)
+// A thread has PIECES runs of four channels.
+template <typename TH, bool POST, bool LAYER, int PIECES, int MAX_THREADS, int MIN_BLOCKS, int AHEAD>
+__global__ void __launch_bounds__(MAX_THREADS, MIN_BLOCKS)
 moe_combine_add_rmsnorm_kernel(const float* __restrict__ expert_out, const int* __restrict__ topk_ids,
                                const int* __restrict__ inverse, const float* __restrict__ gate,
                                const float* __restrict__ shared, float* __restrict__ x, const float* __restrict__ gamma,
@@ -836,31 +868,18 @@ moe_combine_add_rmsnorm_kernel(const float* __restrict__ expert_out, const int* 
     // the kernels before it have ended: the routing, the gate and the residual row are complete and are read before
     // the wait, while that kernel finishes.  ``early`` 0 (every grouped product a dependent launch): everything waits.
     if (!early) pdl_wait();
-    __shared__ int order[MAX_TOPK];
-    __shared__ float pass_w[MAX_TOPK];          // weight of a chosen expert without weights (its output is its input), else 0
+    __shared__ int src[MAX_TOPK];
+    __shared__ float weight[MAX_TOPK];
     __shared__ float scratch[33];
     const int r = blockIdx.x;
     const size_t t = rows ? (size_t)rows[r] : (size_t)r;
-    if (threadIdx.x == 0) {
-        int ids[MAX_TOPK];
-        for (int j = 0; j < top_k; j++) { ids[j] = topk_ids[t * top_k + j]; order[j] = j; }
-        for (int a = 1; a < top_k; a++) {
-            const int oa = order[a], ia = ids[oa];
-            int b = a - 1;
-            while (b >= 0 && ids[order[b]] > ia) { order[b + 1] = order[b]; b--; }
-            order[b + 1] = oa;
-        }
-        for (int j = 0; j < top_k; j++) {
-            const int o = order[j];
-            pass_w[j] = (ident && ids[o] >= n_real) ? topk_w[t * top_k + o] : 0.f;
-            order[j] = inverse[t * top_k + o];
-        }
-    }
+    order_by_expert(topk_ids + t * top_k, inverse + t * top_k, topk_w ? topk_w + t * top_k : nullptr, ident != nullptr, n_real, top_k,
+                    src, weight);
     const float g = gate ? gate[t] : 1.0f;       // no gate: the shared rows are added as they are
     const int pieces = width / 4;
-    float4 v[4];
+    float4 v[PIECES];
 #pragma unroll
-    for (int i = 0; i < 4; i++) {
+    for (int i = 0; i < PIECES; i++) {
         const int q = threadIdx.x + i * blockDim.x;
         if (q < pieces) v[i] = reinterpret_cast<float4*>(x + t * width)[q];
     }
@@ -868,36 +887,30 @@ moe_combine_add_rmsnorm_kernel(const float* __restrict__ expert_out, const int* 
     pdl_wait();
     expert_out = behind_wait(expert_out);
     shared = behind_wait(shared);
-    float4 y[4];
+    float4 y[PIECES], own[PIECES];
     float ssy = 0.f;
 #pragma unroll
-    for (int i = 0; i < 4; i++) {
+    for (int i = 0; i < PIECES; i++) {
         const int q = threadIdx.x + i * blockDim.x;
-        if (q < pieces) {
-            float4 acc = make_float4(0.f, 0.f, 0.f, 0.f);
-            for (int j = 0; j < top_k; j++) {
-                const int row = order[j];
-                if (row >= 0) {
-                    const float4 e = __ldg(reinterpret_cast<const float4*>(expert_out + (size_t)row * width) + q);
-                    acc.x += e.x; acc.y += e.y; acc.z += e.z; acc.w += e.w;
-                } else if (pass_w[j] != 0.f) {
-                    const float4 e = reinterpret_cast<const float4*>(ident + t * width)[q];
-                    const float pw = pass_w[j];
-                    acc.x += pw * e.x; acc.y += pw * e.y; acc.z += pw * e.z; acc.w += pw * e.w;
-                }
-            }
-            if (shared) {
-                const float4 e = __ldg(reinterpret_cast<const float4*>(shared + t * width) + q);
-                acc.x += g * e.x; acc.y += g * e.y; acc.z += g * e.z; acc.w += g * e.w;
-            }
-            y[i] = acc;
-            if (POST) ssy = fmaf(acc.w, acc.w, fmaf(acc.z, acc.z, fmaf(acc.y, acc.y, fmaf(acc.x, acc.x, ssy))));
+        y[i] = make_float4(0.f, 0.f, 0.f, 0.f);
+        if (AHEAD > 1 && shared && q < pieces) own[i] = __ldg(reinterpret_cast<const float4*>(shared + t * width) + q);
+    }
+    add_terms<PIECES, AHEAD>(y, expert_out, ident ? ident + t * width : nullptr, src, weight, top_k, width, pieces);
+#pragma unroll
+    for (int i = 0; i < PIECES; i++) {
+        if (threadIdx.x + i * blockDim.x >= pieces) continue;
+        float4 acc = y[i];
+        if (shared) {
+            if (AHEAD == 1) own[i] = __ldg(reinterpret_cast<const float4*>(shared + t * width) + threadIdx.x + i * blockDim.x);
+            acc.x += g * own[i].x; acc.y += g * own[i].y; acc.z += g * own[i].z; acc.w += g * own[i].w;
         }
+        y[i] = acc;
+        if (POST) ssy = fmaf(acc.w, acc.w, fmaf(acc.z, acc.z, fmaf(acc.y, acc.y, fmaf(acc.x, acc.x, ssy))));
     }
     const float inv_y = POST ? 1.0f / sqrtf(block_sum(ssy, scratch) / (float)width + eps_y) : 1.0f;
     float ss = 0.f;
 #pragma unroll
-    for (int i = 0; i < 4; i++) {
+    for (int i = 0; i < PIECES; i++) {
         const int q = threadIdx.x + i * blockDim.x;
         if (q < pieces) {
             float4 acc = y[i];
@@ -923,7 +936,7 @@ moe_combine_add_rmsnorm_kernel(const float* __restrict__ expert_out, const int* 
     if (POST && !h) return;
     if (POST && !gamma) {
 #pragma unroll
-        for (int i = 0; i < 4; i++) {
+        for (int i = 0; i < PIECES; i++) {
             const int q = threadIdx.x + i * blockDim.x;
             if (q < pieces) Vec4<TH>::store(h + (size_t)r * width + 4 * q, v[i].x, v[i].y, v[i].z, v[i].w);
         }
@@ -933,7 +946,7 @@ moe_combine_add_rmsnorm_kernel(const float* __restrict__ expert_out, const int* 
     if (LAYER) total = take_mean(v, pieces, total / (float)width, scratch);
     const float inv = 1.0f / sqrtf(total / (float)width + eps);
 #pragma unroll
-    for (int i = 0; i < 4; i++) {
+    for (int i = 0; i < PIECES; i++) {
         const int q = threadIdx.x + i * blockDim.x;
         if (q < pieces) {
             const float4 gm = reinterpret_cast<const float4*>(gamma)[q];
@@ -1106,10 +1119,17 @@ ESP_API int esp_moe_combine_add_rmsnorm(const float* expert_out, const int* topk
     // more rows in flight per SM.
     if (width / 4 <= 1024 && !(h_is_bf16 && n_rows >= 256)) threads = (width / 4 + 31) / 32 * 32;
     const int early = esp_pdl_enabled(ESP_PDL_GROUPED) ? 0 : 1;
+#define ESP_COMBINE_AS(TH, POST, LAYER, ...)                                                                                      \
+    esp_launch_pdl(ESP_PDL_SMALL, moe_combine_add_rmsnorm_kernel<TH, POST, LAYER, __VA_ARGS__>, dim3(n_rows), dim3(threads), 0, stream, \
+                   expert_out, topk_ids, inverse, gate, shared, x, gamma, beta, rows, (TH*)h, h32, width, top_k, eps, write_x, early,  \
+                   topk_w, ident, n_real, gamma_y, eps_y)
+    // registers for the loads in flight: one piece a thread in blocks of up to 1,024, four pieces in blocks of up to 256 or 1,024
 #define ESP_COMBINE(TH, POST, LAYER)                                                                                              \
-    esp_launch_pdl(ESP_PDL_SMALL, moe_combine_add_rmsnorm_kernel<TH, POST, LAYER>, dim3(n_rows), dim3(threads), 0, stream, expert_out,  \
-                   topk_ids, inverse, gate, shared, x, gamma, beta, rows, (TH*)h, h32, width, top_k, eps, write_x, early, topk_w,      \
-                   ident, n_real, gamma_y, eps_y)
+    do {                                                                                                                         \
+        if (threads * 4 >= width) ESP_COMBINE_AS(TH, POST, LAYER, 1, 1024, 1, 4);                                                  \
+        else if (threads <= 256) ESP_COMBINE_AS(TH, POST, LAYER, 4, 256, 2, 2);                                                    \
+        else ESP_COMBINE_AS(TH, POST, LAYER, 4, 1024, 1, 1);                                                                      \
+    } while (0)
     if (h_is_bf16) {
         if (gamma_y) ESP_COMBINE(bf16, true, false);
         else if (beta) ESP_COMBINE(bf16, false, true);
@@ -1120,5 +1140,6 @@ ESP_API int esp_moe_combine_add_rmsnorm(const float* expert_out, const int* topk
         else ESP_COMBINE(float, false, false);
     }
 #undef ESP_COMBINE
+#undef ESP_COMBINE_AS
     return esp_launch_status();
 }
