@@ -128,6 +128,7 @@ def _fn(library: str, name: str):
 
 
 _device_index = None
+_raw_stream = getattr(torch._C, "_cuda_getCurrentRawStream", None)
 
 
 def _stream() -> int:
@@ -136,9 +137,8 @@ def _stream() -> int:
     global _device_index
     if _device_index is None:
         _device_index = torch.cuda.current_device()
-    raw = getattr(torch._C, "_cuda_getCurrentRawStream", None)
-    if raw is not None:
-        return raw(_device_index)
+    if _raw_stream is not None:
+        return _raw_stream(_device_index)
     return torch.cuda.current_stream().cuda_stream
 
 
@@ -213,6 +213,11 @@ def _check(code: int, what: str) -> None:
 def _ptr(t, dtype=None, what="tensor"):
     if t is None:
         return None
+    # a launch asks for six of these on average: what is in order leaves by the short way
+    if t.is_cuda and t.is_contiguous():
+        have = t.dtype
+        if have is dtype or dtype is None or (dtype is FLOATS and (have is _F32 or have is _BF16)):
+            return t.data_ptr()
     if not t.is_cuda:
         raise Backend(f"{what} must live on the GPU; this library has no CPU path")
     if not t.is_contiguous():
@@ -222,7 +227,8 @@ def _ptr(t, dtype=None, what="tensor"):
     return t.data_ptr()
 
 
-FLOATS = (torch.float32, torch.bfloat16)
+_F32, _BF16 = torch.float32, torch.bfloat16
+FLOATS = (_F32, _BF16)
 
 
 def _is_bf16(t) -> int:

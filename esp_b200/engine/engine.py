@@ -23,7 +23,7 @@ from ..sampling import as_signed64
 from ..config import config_from_json
 from ..errors import Backend, InvalidRequest, NonFiniteScores
 from ..parts import Runtime, StepContext
-from ..parts.base import StepHost
+from ..parts.base import SideStream, StepHost
 from ..weights import FolderSource, InitSpec, RandomSource, load_into
 from .model import DecoderModel
 
@@ -106,8 +106,11 @@ class Engine:
         self.poison_logits_row: Optional[int] = None
         self.poison_steps: Optional[int] = None
         self._pinned = None
-        self._pinned_event = None
-        self._copy_stream = None
+        self._pinned_event = torch.cuda.Event()
+        self._copies = SideStream(self.rt.device)      # tokens on their way to the host
+        # results of steps launched and not yet read: a buffer and its event each, used in turn
+        self._fetch_ring: list = []
+        self._fetch_turn = 0
         self.staged_bytes = 0
         self._meta_dev = None
         self.steps_run = 0
@@ -196,16 +199,14 @@ class Engine:
             cap = max(total, 1 << 16)
             self._pinned = torch.empty(cap, dtype=torch.int32, pin_memory=True)
             self._meta_dev = torch.empty(cap, dtype=torch.int32, device=self.rt.device)
-            self._pinned_event = None
-        if self._pinned_event is not None:
+        else:
             self._pinned_event.synchronize()         # the last copy out of the pinned buffer is done
         host = self._pinned.numpy()
         for a, off in zip(arrays, offsets):
             host[off:off + a.size] = a.reshape(-1)
         self._meta_dev[:total].copy_(self._pinned[:total], non_blocking=True)
         self.staged_bytes = 4 * total                # what the last step copied to the device
-        self._pinned_event = torch.cuda.Event()
-        self._pinned_event.record()
+        self._pinned_event.record(self._copies.current())
         return [self._meta_dev[off:off + a.size].view(a.shape) for a, off in zip(arrays, offsets)]
 
     def plan_step(self, entries: list):
@@ -280,21 +281,16 @@ class Engine:
         and returns at once; ``result()`` waits for that copy only, not for
         steps launched since."""
         with torch.cuda.device(self.rt.device):
-            if self._copy_stream is None:
-                self._copy_stream = torch.cuda.Stream()
-                self._fetch_ring = [torch.empty(self.cache.book.slots.n + 1, dtype=torch.int32, pin_memory=True)
+            if not self._fetch_ring:
+                self._fetch_ring = [(torch.empty(self.cache.book.slots.n + 1, dtype=torch.int32, pin_memory=True), torch.cuda.Event())
                                     for _ in range(4)]
-                self._fetch_turn = 0
             kept = tokens.clone()                     # a replayed graph writes its tokens into the same buffer every time
-            done = torch.cuda.Event()
-            done.record()
-            host = self._fetch_ring[self._fetch_turn % len(self._fetch_ring)][:kept.shape[0]]
+            buffer, landed = self._fetch_ring[self._fetch_turn % len(self._fetch_ring)]
+            host = buffer[:kept.shape[0]]
             self._fetch_turn += 1
-            self._copy_stream.wait_event(done)
-            with torch.cuda.stream(self._copy_stream):
+            with self._copies:
                 host.copy_(kept, non_blocking=True)
-                landed = torch.cuda.Event()
-                landed.record()
+            landed.record(self._copies.stream)
             return PendingTokens(kept, host, landed)
 
     def seed_slot(self, slot: int, seed: int) -> None:

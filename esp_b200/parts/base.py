@@ -184,6 +184,50 @@ class Workspace:
         return sum(b.numel() * b.element_size() for b in self._bufs.values())
 
 
+class SideStream:
+    """A second stream for work that may run beside the current one: ``with side:`` makes it the current stream, behind
+    everything launched so far; ``side.join()`` lets the then current stream wait for it.  The two events are made once and
+    recorded again at every use (a wait takes the event as it stands when the wait is made), and streams are looked up and set
+    by their numbers: with new events and ``torch.cuda.stream`` a fork and a join took 30 us of host time, 0.7 of the 4.9 ms
+    of a prompt of 19 tokens over 24 layers."""
+
+    def __init__(self, device):
+        self.stream = torch.cuda.Stream(device=device)
+        self._index = self.stream.device_index
+        self._forked, self._joined = torch.cuda.Event(), torch.cuda.Event()
+        self._left: list = []                # streams to go back to
+        self._known: dict = {}               # a stream's numbers -> its object
+
+    def current(self):
+        ids = torch._C._cuda_getCurrentStream(self._index)
+        found = self._known.get(ids)
+        if found is None:
+            if len(self._known) >= 64:
+                self._known.clear()
+            found = torch.cuda.Stream(stream_id=ids[0], device_index=ids[1], device_type=ids[2])
+            self._known[ids] = found
+        return found
+
+    @staticmethod
+    def _set(stream) -> None:
+        torch._C._cuda_setStream(stream_id=stream.stream_id, device_index=stream.device_index, device_type=stream.device_type)
+
+    def __enter__(self):
+        main = self.current()
+        self._forked.record(main)
+        self.stream.wait_event(self._forked)
+        self._left.append(main)
+        self._set(self.stream)
+        return self
+
+    def __exit__(self, *exc):
+        self._set(self._left.pop())
+
+    def join(self) -> None:
+        self._joined.record(self.stream)
+        self.current().wait_event(self._joined)
+
+
 class Runtime:
     """Device, activation dtype, scratch and the device status word."""
 
@@ -202,7 +246,7 @@ class Runtime:
                 raise Backend("esp_b200 runs on a CUDA device only; there is no CPU path")
             self.ws = Workspace(self.device)
             self.status = torch.zeros(1, dtype=torch.int32, device=self.device)
-            self.side_stream = torch.cuda.Stream(device=self.device)     # for work that may run beside the main stream
+            self.side_stream = SideStream(self.device)     # for work that may run beside the main stream
             self.sm_count = torch.cuda.get_device_properties(self.device).multi_processor_count
         self.ffn_chunk_tokens = ffn_chunk_tokens
         self.record_routing = False       # debugging aid: MoE parts put their choices into ctx.aux

@@ -245,15 +245,13 @@ class ParallelResidualBlock(Part):
             n = x.shape[0]
             side = rt.side_stream if n <= BESIDE_ROWS or n * x.shape[1] >= BESIDE_WORK else None
             if side is not None:
-                main = torch.cuda.current_stream()
-                side.wait_stream(main)
-                with torch.cuda.stream(side):
+                with side:
                     mixed = plain_delta(None, self.mixer.forward(h, ctx, layer))
             else:
                 mixed = plain_delta(None, self.mixer.forward(h, ctx, layer))
             pending = self.ffn.forward(h, ctx, h32=h32)
             if side is not None:
-                main.wait_stream(side)
+                side.join()
             if not getattr(pending, "take_along", lambda rows: False)(mixed):
                 pending = plain_delta(None, pending).add_(mixed)
         if "residual_trace" in ctx.aux:

@@ -319,18 +319,14 @@ class MoeSwiGluShared(Part):
         beside = has_shared and n <= SIDE_STREAM_ROWS and rt.side_stream is not None
         ahead = has_shared and not beside and n >= AHEAD_ROWS and rt.side_stream is not None and rt.dtype == torch.bfloat16
         if ahead:
-            main = torch.cuda.current_stream()
-            rt.side_stream.wait_stream(main)
             act_s = ws.get("moe_shared_act", (n, s.shared_intermediate), rt.dtype)
-            with torch.cuda.stream(rt.side_stream):
+            with rt.side_stream:
                 swiglu_linear(rt, h, self.w_shared_gate_up, act_s, "moe_shared", max_ctas=max(2, rt.sm_count - ROUTING_SMS),
                               glu=s.shared_glu)
         if beside:
             # few rows: the shared expert depends neither on the router nor on the routing, so it runs beside
             # them and the routed experts on a second stream (in a captured step: a parallel branch of the graph)
-            main = torch.cuda.current_stream()
-            rt.side_stream.wait_stream(main)
-            with torch.cuda.stream(rt.side_stream):
+            with rt.side_stream:
                 _swiglu_mlp(rt, h, self.w_shared_gate_up, self.w_shared_down, shared, "moe_shared", glu=s.shared_glu)
         uses_tc05 = grouped_uses_tc05(h, self.w_gate_up, n * k, n) and Im % 8 == 0
         if uses_tc05 and R > E:
@@ -357,10 +353,10 @@ class MoeSwiGluShared(Part):
         if rt.record_routing:
             ctx.aux.setdefault("routing", []).append((s.prefix, row0, ids.clone(), wts.clone(), probs))
         if ahead:
-            main.wait_stream(rt.side_stream)
+            rt.side_stream.join()
         expert_out = self.experts(h, offsets, perm_token, perm_weight, n * k, n, tiles)
         if beside:
-            main.wait_stream(rt.side_stream)
+            rt.side_stream.join()
         elif ahead:
             linear(rt, act_s, self.w_shared_down, shared)
         elif has_shared:
@@ -508,9 +504,7 @@ class ScaledInputMoe(Part):
         if beside:
             # few rows: the shared expert needs nothing of the routing and runs beside it on a second stream
             shared = ws.get("moe_shared_out", (n, H), torch.float32)
-            main = torch.cuda.current_stream()
-            rt.side_stream.wait_stream(main)
-            with torch.cuda.stream(rt.side_stream):
+            with rt.side_stream:
                 _relu2_mlp(rt, h, self.w_shared_up, self.w_shared_down, shared, "moe_shared")
         if n <= ops.ROUTE_SMALL_TOKENS and ops.route_small_fits(H, E):
             logits = ws.get("moe_logits", (n, E + 1), torch.float32)
@@ -545,7 +539,7 @@ class ScaledInputMoe(Part):
             ops.gemm_simt(act, self.w_down, out, group_offsets=offsets, rows=rows)
         if self.w_shared_up is not None:
             if beside:
-                main.wait_stream(rt.side_stream)
+                rt.side_stream.join()
             else:
                 shared = ws.get("moe_shared_out", (n, H), torch.float32)
                 _relu2_mlp(rt, h, self.w_shared_up, self.w_shared_down, shared, "moe_shared")
