@@ -259,6 +259,39 @@ def test_attention_finds_the_key_that_matters(dtype, nh, nkv, hd, window):
         close(out[i].view(nh, hd), ref, dtype, f"query {i} (sequence {s}, position {p}, target key {target})")
 
 
+@pytest.mark.parametrize("nh, nkv, hd, window", [(4, 4, 128, None), (20, 1, 64, None), (6, 2, 40, 30)])
+@pytest.mark.parametrize("sink", [False, True])
+def test_decode_attention_of_rows_with_one_split(nh, nkv, hd, window, sink):
+    """Rows whose keys lie in one split are written from the registers: nothing of the scratch is read or written for them, the
+    counters stay zero, and rows of two splits stand beside them."""
+    torch.manual_seed(nh)
+    lens, split = [1, 63, 64, 65, 128, 129, 100], 128
+    ks = [torch.randn(n, nkv, hd) for n in lens]
+    vs = [torch.randn(n, nkv, hd) for n in lens]
+    tables = [[3 * s + i for i in range(3)] for s in range(len(lens))]
+    kc, vc = paged(ks, vs, tables, 3 * len(lens), nkv, hd, torch.bfloat16)
+    q = torch.randn(len(lens), nh, hd).to(torch.bfloat16)
+    i32 = lambda v: torch.tensor(v, dtype=torch.int32, device=DEV)
+    tile = ops.attn_decode_tile(hd, hd)
+    part_o = torch.full((len(lens), nh, 2, tile), float("nan"), device=DEV)
+    part_ml = torch.full((len(lens), nh, 2, 2), float("nan"), device=DEV)
+    counters = torch.zeros(ops.ATTN_DECODE_COUNTERS, dtype=torch.int32, device=DEV)
+    out, st = torch.empty(len(lens), nh * hd, dtype=torch.bfloat16, device=DEV), status()
+    ops.attn_decode(q.reshape(len(lens), -1).to(DEV), kc, vc, out, part_o, part_ml, counters, i32(list(range(len(lens)))),
+                    i32([n - 1 for n in lens]), i32(tables), 64, nh, nkv, hd, window, split, 2, st, sink=sink)
+    assert st.item() == 0 and counters.abs().max().item() == 0
+    for r, n in enumerate(lens):
+        if n <= split:
+            assert torch.isnan(part_o[r]).all() and torch.isnan(part_ml[r]).all()
+        lo = max(0, n - (window or n))
+        k, v = (t[r][lo:].to(torch.bfloat16).double().repeat_interleave(nh // nkv, 1) for t in (ks, vs))
+        x = torch.einsum("hd,khd->hk", q[r].double(), k) / np.sqrt(hd)
+        if sink:
+            x = torch.cat([x, torch.zeros(nh, 1, dtype=torch.float64)], 1)
+        ref = torch.einsum("hk,khd->hd", torch.softmax(x, 1)[:, :n - lo], v)
+        close(out[r].view(nh, hd), ref, torch.bfloat16, f"row {r}")
+
+
 @pytest.mark.parametrize("hd, vd, page", [(128, 128, 64), (40, 24, 64), (4, 128, 16)])
 @pytest.mark.parametrize("opts", [dict(window=None), dict(window=70), dict(window=70, keep=5), dict(window=None, chunk=48),
                                   dict(window=None, sink=True, softcap=5.0), dict(window=1)])
