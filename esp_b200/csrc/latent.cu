@@ -98,37 +98,29 @@ __global__ void latent_q_rotate_kernel(const float* __restrict__ q, const float*
 // out[n, h, j] = sum_i a[n, h, i] * w[h, j, i]   (i < kin, j < nout); a's and out's heads may be parts of wider rows:
 // a[n, h, i] = a[n * lda + h * a_head + i], out[n, h, j] = out[n * ldo + h * o_head + j].
 // A block takes PH_ROWS rows and PH_OUTS output channels of one head, a warp PH_WARP of the channels at once.  Lane l has the
-// input channels 4 l .. 4 l + 3 of every 128, adds its products in index order, and the lanes' sums meet in a fixed
-// butterfly that brings row r of channel c to lane 8 c + r: the order of a sum depends on kin alone.
-// Few rows are bound by latency: the weights (4 values a load) of the first 512 input channels are asked for before the
-// kernel waits for its predecessor, all of them at once.  Eight rows, 16 heads, 512 -> 128 and 128 -> 512 channels, inside
-// a step: 35 and 19 us with a channel at a time and 2-byte loads, 7 and 3 here.
+// input channels l, l + 32, l + 64, ... and adds its products in that order; the lanes' sums meet in the butterfly of
+// warp_sum (partners 16, 8, 4, 2, 1 lanes away), cut so that row r of channel c ends in lane 8 c + r.  The order of a sum depends on
+// kin alone, and results travel through 16-bit activations, so it is part of what this kernel promises.
+// The inputs lie in shared memory so that the channels l, l + 32, l + 64 and l + 96 of a piece of 128 are 16 bytes (PH slots).
+// Few rows are bound by latency: the weights of the first 512 input channels are asked for before the kernel waits for its
+// predecessor, all of them at once.  Eight rows, 16 heads, cold: 512 -> 128
+// channels 33.7 -> 12.3 us, 128 -> 512 18.4 -> 10.2, against a channel at a time.
 constexpr int PH_ROWS = 8;
 constexpr int PH_OUTS = 16;       // output channels of a block
 constexpr int PH_WARP = 4;        // of a warp
 constexpr int PH_PIECES = 4;      // runs of 128 input channels whose weights a warp has in registers at a time
 
-// four consecutive weights as they lie in memory
-template <typename TW> struct Four;
-template <> struct Four<float> {
-    float4 v;
-    __device__ __forceinline__ void load(const float* p) { v = *reinterpret_cast<const float4*>(p); }
-    __device__ __forceinline__ void set(int i, float x) { (&v.x)[i] = x; }
-    __device__ __forceinline__ float4 get() const { return v; }
-};
-template <> struct Four<bf16> {
-    uint2 v;
-    __device__ __forceinline__ void load(const bf16* p) { v = *reinterpret_cast<const uint2*>(p); }
-    __device__ __forceinline__ void set(int i, bf16 x) {
-        const unsigned b = __bfloat16_as_ushort(x);
-        unsigned& w = i < 2 ? v.x : v.y;
-        w = (i & 1) ? (w & 0xffffu) | (b << 16) : (w & 0xffff0000u) | b;
-    }
-    __device__ __forceinline__ float4 get() const {
-        return make_float4(__uint_as_float(v.x << 16), __uint_as_float(v.x & 0xffff0000u), __uint_as_float(v.y << 16),
-                           __uint_as_float(v.y & 0xffff0000u));
-    }
-};
+// the place of channel i among a row's inputs; within 8 lanes the places are turned, so that the four channels that a thread
+// stages go to banks of their own
+__device__ __forceinline__ int ph_slot(int lane) { return lane ^ (lane >> 3); }
+__device__ __forceinline__ int ph_place(int i) { return i / 128 * 128 + ph_slot(i % 32) * 4 + i % 128 / 32; }
+
+__device__ __forceinline__ float4 four_values(const float* p) { return *reinterpret_cast<const float4*>(p); }
+__device__ __forceinline__ float4 four_values(const bf16* p) {
+    const uint2 v = *reinterpret_cast<const uint2*>(p);
+    return make_float4(__uint_as_float(v.x << 16), __uint_as_float(v.x & 0xffff0000u), __uint_as_float(v.y << 16),
+                       __uint_as_float(v.y & 0xffff0000u));
+}
 
 template <typename TA, typename TW, typename TO>
 __global__ void __launch_bounds__(128)
@@ -136,71 +128,77 @@ per_head_linear_kernel(const TA* __restrict__ a, long long lda, int a_head, cons
                        long long ldo, int o_head, int n_rows, int kin, int nout) {
     static_assert(PH_WARP * PH_ROWS == 32 && PH_OUTS == 4 * PH_WARP, "a lane ends up with one result");
     pdl_trigger();
-    extern __shared__ float4 as4[];                // [PH_ROWS][quads]
-    const int n0 = blockIdx.x * PH_ROWS, h = blockIdx.y, quads = (kin + 3) / 4;
+    extern __shared__ __align__(16) float as[];    // [PH_ROWS][width]
+    const int n0 = blockIdx.x * PH_ROWS, h = blockIdx.y;
     const int rows = min(PH_ROWS, n_rows - n0);
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     const int j0 = blockIdx.z * PH_OUTS + warp * PH_WARP;
     const TW* wh = w + ((size_t)h * nout + j0) * kin;
-    const bool wide = kin % 4 == 0 && (reinterpret_cast<uintptr_t>(w) & 15) == 0;
-    Four<TW> wt[PH_PIECES][PH_WARP];
-    auto load_weights = [&](int q0) {              // q0: the first quad of the pieces
+    TW wt[PH_PIECES][4][PH_WARP];
+    auto load_weights = [&](int i0) {
 #pragma unroll
-        for (int s = 0; s < PH_PIECES; s++)
+        for (int p = 0; p < PH_PIECES; p++) {
+            if (i0 + p * 128 >= kin) break;         // the same for every lane
 #pragma unroll
-            for (int c = 0; c < PH_WARP; c++) {
-                const int q = q0 + s * 32 + lane;
-                wt[s][c].v = {};
-                if (j0 + c >= nout || q >= quads) continue;
-                const TW* src = wh + (size_t)c * kin + 4 * q;
-                if (wide) {
-                    wt[s][c].load(src);
-                } else {
+            for (int e = 0; e < 4; e++)
 #pragma unroll
-                    for (int i = 0; i < 4; i++)
-                        if (4 * q + i < kin) wt[s][c].set(i, src[i]);
+                for (int c = 0; c < PH_WARP; c++) {
+                    const int i = i0 + p * 128 + e * 32 + lane;
+                    wt[p][e][c] = i < kin && j0 + c < nout ? wh[(size_t)c * kin + i] : from_f32<TW>(0.f);
                 }
-            }
+        }
     };
     load_weights(0);
     pdl_wait();
     a = behind_wait(a);
-    const bool wide_a = kin % 4 == 0 && lda % 4 == 0 && a_head % 4 == 0 && (reinterpret_cast<uintptr_t>(a) & (4 * sizeof(TA) - 1)) == 0;
-    for (int idx = threadIdx.x; idx < rows * quads; idx += 128) {
-        const int r = idx / quads, i = (idx - r * quads) * 4;
-        const TA* src = a + (size_t)(n0 + r) * lda + (size_t)h * a_head + i;
-        if (wide_a) {
-            Four<TA> v;
-            v.load(src);
-            as4[idx] = v.get();
-        } else {
-            as4[idx] = make_float4(to_f32(src[0]), i + 1 < kin ? to_f32(src[1]) : 0.f, i + 2 < kin ? to_f32(src[2]) : 0.f,
-                                   i + 3 < kin ? to_f32(src[3]) : 0.f);
+    const int width = (kin + 127) / 128 * 128;
+    const TA* src = a + (size_t)n0 * lda + (size_t)h * a_head;
+    if (kin % 4 == 0 && lda % 4 == 0 && a_head % 4 == 0 && (reinterpret_cast<uintptr_t>(a) & (4 * sizeof(TA) - 1)) == 0) {
+        const int quads = kin / 4;
+#pragma unroll 4
+        for (int idx = threadIdx.x; idx < rows * quads; idx += 128) {
+            const int r = idx / quads, i = (idx - r * quads) * 4;
+            const float4 v = four_values(src + r * lda + i);
+            float* to = as + r * width;
+            to[ph_place(i)] = v.x, to[ph_place(i + 1)] = v.y, to[ph_place(i + 2)] = v.z, to[ph_place(i + 3)] = v.w;
+        }
+    } else {
+        for (int idx = threadIdx.x; idx < rows * kin; idx += 128) {
+            const int r = idx / kin, i = idx - r * kin;
+            as[r * width + ph_place(i)] = to_f32(src[r * lda + i]);
         }
     }
     __syncthreads();
     float acc[PH_WARP * PH_ROWS];
 #pragma unroll
     for (int i = 0; i < PH_WARP * PH_ROWS; i++) acc[i] = 0.f;
-    for (int q0 = 0; q0 < quads; q0 += 32 * PH_PIECES) {
-        if (q0 > 0) load_weights(q0);
+    for (int i0 = 0; i0 < kin; i0 += 128 * PH_PIECES) {
+        if (i0 > 0) load_weights(i0);
 #pragma unroll
-        for (int s = 0; s < PH_PIECES; s++) {
-            const int q = q0 + s * 32 + lane;
-            if (q >= quads) continue;
-            float4 f[PH_WARP];
+        for (int p = 0; p < PH_PIECES; p++) {
+            const int left = kin - i0 - p * 128;
+            if (left <= 0) break;                   // the same for every lane
+            float f[4][PH_WARP];
 #pragma unroll
-            for (int c = 0; c < PH_WARP; c++) f[c] = wt[s][c].get();
+            for (int e = 0; e < 4; e++)
 #pragma unroll
-            for (int r = 0; r < PH_ROWS; r++) {
-                if (r >= rows) break;               // the same for every lane
-                const float4 x = as4[r * quads + q];
+                for (int c = 0; c < PH_WARP; c++) f[e][c] = to_f32(wt[p][e][c]);
+            auto add_rows = [&](int steps) {        // of 32 channels that this lane has
 #pragma unroll
-                for (int c = 0; c < PH_WARP; c++) {
-                    float& t = acc[c * PH_ROWS + r];
-                    t = fmaf(x.w, f[c].w, fmaf(x.z, f[c].z, fmaf(x.y, f[c].y, fmaf(x.x, f[c].x, t))));
+                for (int r = 0; r < PH_ROWS; r++) {
+                    if (r >= rows) break;           // the same for every lane
+                    const float4 v = *reinterpret_cast<const float4*>(as + r * width + i0 + p * 128 + ph_slot(lane) * 4);
+                    const float x[4] = {v.x, v.y, v.z, v.w};
+#pragma unroll
+                    for (int e = 0; e < 4; e++) {
+                        if (e >= steps) continue;
+#pragma unroll
+                        for (int c = 0; c < PH_WARP; c++) acc[c * PH_ROWS + r] = fmaf(x[e], f[e][c], acc[c * PH_ROWS + r]);
+                    }
                 }
-            }
+            };
+            if (left >= 128) add_rows(4);
+            else add_rows((left - lane + 31) / 32); // places behind the last channel hold whatever is there
         }
     }
     // 32 sums over 32 lanes: at every step a lane hands half of its sums to its partner and takes the other half's
@@ -587,7 +585,7 @@ ESP_API int esp_per_head_linear(const void* a, int a_dtype, long long lda, int a
     if (w_dtype == 1 && n_rows >= PHM_MIN_ROWS)
         return launch_per_head_mma(a, a_dtype, lda, a_head, w, out, o_dtype, ldo, o_head, n_rows, H, kin, nout, stream);
     dim3 grid((n_rows + PH_ROWS - 1) / PH_ROWS, H, (nout + PH_OUTS - 1) / PH_OUTS);
-    const size_t smem = (size_t)PH_ROWS * ((kin + 3) / 4) * sizeof(float4);
+    const size_t smem = (size_t)PH_ROWS * ((kin + 127) / 128 * 128) * sizeof(float);       // 48 KB at most, as the limit above is a multiple of 128
 #define ESP_CASE(code_, TA, TW, TO)                                                                                          \
     case code_:                                                                                                             \
         esp_launch_pdl(ESP_PDL_SMALL, per_head_linear_kernel<TA, TW, TO>, grid, dim3(128), smem, stream, (const TA*)a, lda,   \

@@ -227,7 +227,7 @@ def test_per_head_product(a_dtype, w_dtype, o_dtype):
 @pytest.mark.parametrize("N, kin, nout", [(1, 128, 17), (8, 130, 16), (9, 512, 33), (7, 516, 5), (16, 1000, 3), (3, 1, 1)])
 @pytest.mark.parametrize("w_dtype", [torch.float32, torch.bfloat16])
 def test_per_head_product_of_few_rows(N, kin, nout, w_dtype):
-    """Sizes around the kernel's pieces (128 channels a piece, four pieces at a time, four outputs a warp, eight rows), rows on
+    """Sizes around the kernel's pieces (32 channels a step, sixteen steps at a time, four outputs a warp, eight rows), rows on
     any alignment; a row's sum does not depend on the others."""
     torch.manual_seed(kin)
     H = 3
@@ -243,6 +243,25 @@ def test_per_head_product_of_few_rows(N, kin, nout, w_dtype):
     one = torch.zeros(1, H * nout, device=DEV)
     ops.per_head_linear(a[N - 1:], H * kin, kin, w, one, H * nout, nout, 1, H, kin, nout)
     assert torch.equal(one.view(H, nout), got[N - 1, :, :nout])
+
+
+@pytest.mark.parametrize("kin", [1, 40, 128, 130, 512, 516, 1000])
+@pytest.mark.parametrize("w_dtype", [torch.float32, torch.bfloat16])
+def test_per_head_product_keeps_the_order_of_its_sums(kin, w_dtype):
+    """Lane l of 32 adds the products of the channels l, l + 32, ...; then partners 16, 8, 4, 2 and 1 lanes away add up.  Whole
+    numbers with products up to 2^25, exact in 64 bits, so that one rounding to 32 bits is the multiply-add's own: no tolerance."""
+    rng = np.random.default_rng(kin)
+    N, H, nout = 9, 2, 5
+    a, w = rng.integers(-2 ** 17, 2 ** 17, (N, H, kin)).astype(np.float64), rng.integers(-256, 257, (H, nout, kin)).astype(np.float64)
+    sums = np.zeros((N, H, nout, 32))
+    for i in range(kin):
+        sums[..., i % 32] = (a[:, :, None, i] * w[None, :, :, i] + sums[..., i % 32]).astype(np.float32)
+    for step in (16, 8, 4, 2, 1):
+        sums = (sums + sums[..., np.arange(32) ^ step]).astype(np.float32).astype(np.float64)
+    out = torch.zeros(N, H * nout, device=DEV)
+    ops.per_head_linear(torch.tensor(a, dtype=torch.float32, device=DEV).view(N, -1), H * kin, kin, torch.tensor(w, device=DEV).to(w_dtype),
+                        out, H * nout, nout, N, H, kin, nout)
+    assert np.array_equal(out.view(N, H, nout).cpu().numpy(), sums[..., 0].astype(np.float32))
 
 
 @pytest.mark.parametrize("mode", [ops.SCAN_DECAY_BONUS, ops.SCAN_LOWER_SIGMOID])
