@@ -66,6 +66,7 @@ struct PickShared {
     int found_bin[2];
     float best_v[CS];
     int best_i[CS];
+    int heaviest, first[CS];                         // lowest id of weight 1: this block's, every block's
     u64 warp_u64[PICK_WARPS];
     float warp_v[PICK_WARPS];
     int warp_i[PICK_WARPS];
@@ -156,7 +157,10 @@ struct Picker {
         }
         if (tid == PICK_THREADS - 1) {
 #pragma unroll
-            for (int c = 0; c < CS; c++) (first_level ? of(c)->total1 : of(c)->totalx)[rank] = at;
+            for (int c = 0; c < CS; c++) {
+                (first_level ? of(c)->total1 : of(c)->totalx)[rank] = at;
+                if (first_level) of(c)->first[rank] = s.heaviest;
+            }
         }
         sync();
     }
@@ -267,7 +271,10 @@ pick_tokens_kernel(const float* __restrict__ logits, int vocab, int per_block, i
     if (rank == 0 && tid == 0) rng_state[row_slot[r]] = state;
     const float inv_t = 1.0f / temp;
 
-    // first level, shared by both searches; the weights take the logits' place in shared memory
+    // first level, shared by both searches; the weights take the logits' place in shared memory.  The first rank is the
+    // lowest id whose weight is 1: logits that differ can have that weight alike, so it need not be the arg-max.
+    int heaviest = 0x7fffffff;
+    if (tid == 0) s.heaviest = heaviest;
     pick.clear(L1_BINS);
     for (int at = 0; at < n; at += PICK_THREADS) {
         const int i = at + tid;
@@ -277,12 +284,15 @@ pick_tokens_kernel(const float* __restrict__ logits, int vocab, int per_block, i
             if (keep) weights[i] = w;
         }
         const u64 m = mass_of(w);
+        if (w == 1.f) heaviest = min(heaviest, i0 + i);
         pick.add((ONE_BITS - __float_as_uint(w)) >> 18 & (L1_BINS - 1), m);
     }
+    if (heaviest != 0x7fffffff) atomicMin(&s.heaviest, heaviest);
     pick.template merge<L1_BINS>(s.cum1, true);
     u64 kept = 0;
+    int first = 0x7fffffff;
 #pragma unroll
-    for (int c = 0; c < CS; c++) kept += s.total1[c];
+    for (int c = 0; c < CS; c++) kept += s.total1[c], first = min(first, s.first[c]);
     if (kept < FIRST_MASS) {                 // no weight is a number (a temperature whose inverse overflows): the arg-max
         if (rank == 0 && tid == 0) tokens[r] = bi;
         return;
@@ -329,7 +339,7 @@ pick_tokens_kernel(const float* __restrict__ logits, int vocab, int per_block, i
     u64 threshold = (u64)((double)u * (double)kept);
     if (threshold > kept) threshold = kept;
     if (threshold <= FIRST_MASS) {
-        if (rank == 0 && tid == 0) tokens[r] = bi;
+        if (rank == 0 && tid == 0) tokens[r] = first;
         return;
     }
     u64 before;
@@ -346,7 +356,7 @@ pick_tokens_kernel(const float* __restrict__ logits, int vocab, int per_block, i
     }
     pick.sync();                             // no block leaves while another reads its histogram
     if (!mine) {
-        if (m == 0 && rank == 0 && tid == 0) tokens[r] = bi;
+        if (m == 0 && rank == 0 && tid == 0) tokens[r] = first;
         return;
     }
     for (int at = 0; at < n; at += PICK_THREADS) {

@@ -607,6 +607,36 @@ def test_sampling_of_equal_weights_takes_the_exact_place(vocab):
         assert (state[r].item() & ((1 << 64) - 1)) == stream.state
 
 
+@pytest.mark.parametrize("vocab", [300, 8192, 8193, 32770, 230001])
+@pytest.mark.parametrize("temperature", [2.0, 100.0, 1e9])
+def test_sampling_ranks_by_weight_where_logits_differ(vocab, temperature):
+    """Logits a few steps of 32 bits apart have the same weight, 1: the first rank is the lowest of their ids, not the arg-max, and
+    each is drawn by its own share.  All other weights are 0 (at 1e9: all are 1), so the places are whole numbers: no tolerance."""
+    one, rows = 1 << 40, 48
+    rng = np.random.default_rng(vocab)
+    ids = np.sort(rng.choice(vocab, 5, replace=False))
+    top = np.float32(1.0)
+    logits = torch.full((rows, vocab), -1000.0 * temperature if temperature < 1e9 else 0.5)
+    for j, i in enumerate(ids):
+        logits[:, i] = float(np.nextafter(top, np.float32(0))) if j != 3 else float(top)        # the arg-max is the fourth
+    heaviest = ids if temperature < 1e9 else np.arange(vocab)
+    tops = [None, 0.0, 0.3, 0.7]
+    cases = [(1000 + 7 * r, tops[r % 4]) for r in range(rows)]
+    state, tokens = torch.tensor([s for s, _p in cases], dtype=torch.int64, device=DEV), torch.empty(rows, dtype=torch.int32, device=DEV)
+    ops.pick_tokens(logits.to(DEV), torch.full((rows,), temperature, device=DEV),
+                    torch.tensor([-1.0 if p is None else p for _s, p in cases], device=DEV), state,
+                    torch.arange(rows, dtype=torch.int32, device=DEV), tokens)
+    want = []
+    for seed, tp in cases:
+        u = float(np.float32(plain.SplitMix64(seed).next_f64()))
+        kept = len(heaviest) * one
+        if tp is not None:
+            kept = min(kept, max(1, -(-int(float(kept) * float(np.float32(tp))) // one)) * one)
+        want.append(int(heaviest[max(1, -(-min(kept, int(u * float(kept))) // one)) - 1]))
+    assert tokens.tolist() == want
+    assert heaviest[0] in want
+
+
 def test_sampling_at_a_temperature_without_an_inverse_takes_the_arg_max():
     logits = rnd(2, 9000)
     tokens = torch.empty(2, dtype=torch.int32, device=DEV)
