@@ -11,8 +11,8 @@
 // [group_offsets[g], group_offsets[g+1]) and its own [N, K] slice of W.
 //
 // Two kernels share that order.  ``gemm_simt_kernel`` cuts the output into tiles and is bound by the multiply-add
-// units; ``gemm_simt_few_kernel`` streams the weights past at most eight rows at a time and is bound by memory or, for
-// few columns, by the chain of K dependent additions.
+// units; ``gemm_simt_few_kernel`` streams the weights past eight rows a block and is bound by memory or, for few columns, by
+// the chain of K dependent additions.
 #include "common.cuh"
 
 namespace {
@@ -67,31 +67,42 @@ struct SimtParams {
 // Every warp finds it by itself.  Returns false past the last tile.
 template <int BM>
 __device__ __forceinline__ bool group_tile(const SimtParams& p, int tile, int& group, int& m0, int& m_end) {
+    constexpr int ROUNDS = 4;                                        // of 32 groups whose offsets are asked for at once
     const int lane = threadIdx.x & 31;
     int before = 0;
-    for (int g0 = 0; g0 < p.groups; g0 += 32) {
-        const int g = g0 + lane;
-        const int begin = g < p.groups ? p.group_offsets[g] : 0, end = g < p.groups ? p.group_offsets[g + 1] : 0;
-        const int tiles = end > begin ? (end - begin + BM - 1) / BM : 0;
-        int upto = tiles;                                            // tiles of the lanes up to this one
+    bool found = false;
+    for (int g0 = 0; g0 < p.groups; g0 += 32 * ROUNDS) {
+        int begin[ROUNDS], end[ROUNDS];
 #pragma unroll
-        for (int o = 1; o < 32; o <<= 1) {
-            const int v = __shfl_up_sync(0xffffffffu, upto, o);
-            if (lane >= o) upto += v;
+        for (int r = 0; r < ROUNDS; r++) {
+            const int g = g0 + 32 * r + lane;
+            begin[r] = g < p.groups ? p.group_offsets[g] : 0;
+            end[r] = g < p.groups ? p.group_offsets[g + 1] : 0;
         }
-        const bool mine = tile >= before + upto - tiles && tile < before + upto;
-        const unsigned hit = __ballot_sync(0xffffffffu, mine);
-        if (hit) {
-            const int src = __ffs(hit) - 1;
-            const int first = begin + (tile - (before + upto - tiles)) * BM;
-            group = g0 + src;
-            m0 = __shfl_sync(0xffffffffu, first, src);
-            m_end = __shfl_sync(0xffffffffu, end, src);
-            return true;
+#pragma unroll
+        for (int r = 0; r < ROUNDS; r++) {
+            const int tiles = end[r] > begin[r] ? (end[r] - begin[r] + BM - 1) / BM : 0;
+            int upto = tiles;                                        // tiles of the lanes up to this one
+#pragma unroll
+            for (int o = 1; o < 32; o <<= 1) {
+                const int v = __shfl_up_sync(0xffffffffu, upto, o);
+                if (lane >= o) upto += v;
+            }
+            const bool mine = tile >= before + upto - tiles && tile < before + upto;
+            const unsigned hit = __ballot_sync(0xffffffffu, mine);
+            if (hit) {                                               // of one round at most
+                const int src = __ffs(hit) - 1;
+                const int first = begin[r] + (tile - (before + upto - tiles)) * BM;
+                group = g0 + 32 * r + src;
+                m0 = __shfl_sync(0xffffffffu, first, src);
+                m_end = __shfl_sync(0xffffffffu, end[r], src);
+                found = true;
+            }
+            before += __shfl_sync(0xffffffffu, upto, 31);
         }
-        before += __shfl_sync(0xffffffffu, upto, 31);
+        if (found) break;
     }
-    return false;
+    return found;
 }
 
 template <typename TC>
@@ -243,7 +254,8 @@ __device__ __forceinline__ void copy16(void* dst, const void* src, bool valid) {
 __device__ __forceinline__ float4 read4(const float* p) { return *reinterpret_cast<const float4*>(p); }
 __device__ __forceinline__ float4 read4(const bf16* p) { return widen4(*reinterpret_cast<const uint2*>(p)); }
 
-// BN columns against up to eight rows at a time; a thread has RT rows of CT columns.  The weights (and the rows) pass
+// BN columns against up to eight rows; a thread has RT rows of CT columns.  Further rows are further blocks', which find the
+// weights in L2: a block that took a group's rows eight by eight made 90 passes over them where 720 rows fell to one group.  The weights (and the rows) pass
 // through a ring of FEW_STAGES pieces of FEW_K k in shared memory, filled by cp.async, so that the loads run ahead of the
 // chains of additions.  The ring's size is known to the compiler (no dynamic shared memory): it then spends the registers
 // that the ring leaves on reading several k ahead; without, 6 x 2,048 x 2,048 takes 28 us instead of 20.  Wants rows of A
@@ -252,94 +264,107 @@ __device__ __forceinline__ float4 read4(const bf16* p) { return widen4(*reinterp
 // additions is 4.3 of them).
 template <typename TA, typename TW, typename TC, int BN, int RT, int CT, int FEW_K, int FEW_STAGES>
 __global__ void __launch_bounds__(BN / CT * (FEW_ROWS / RT))
-gemm_simt_few_kernel(SimtParams p) {
+gemm_simt_few_kernel(SimtParams p, int chunks) {
     constexpr int TX = BN / CT, THREADS = TX * (FEW_ROWS / RT);
     constexpr int A_PIECE = 16 / sizeof(TA), W_PIECE = 16 / sizeof(TW);
     constexpr int A_LD = FEW_K + A_PIECE, W_LD = FEW_K + W_PIECE;      // 16 bytes apart in the banks from row to row
     __shared__ __align__(16) TA As[FEW_STAGES][FEW_ROWS][A_LD];
     __shared__ __align__(16) TW Ws[FEW_STAGES][BN][W_LD];
-    int m_begin = 0, m_end = p.M;
-    const TW* Wg = reinterpret_cast<const TW*>(p.W);
+    // Dense: the eights of rows vary fastest, so that they share a read of their weights.  Groups: the columns do, as the
+    // blocks behind the last eight have nothing to do and would leave the others unevenly spread over the SMs.
+    int m0, m_end = p.M, group = 0, n0;
     if (p.group_offsets) {
-        m_begin = p.group_offsets[blockIdx.y];
-        m_end = p.group_offsets[blockIdx.y + 1];
-        Wg += (size_t)blockIdx.y * p.N * p.K;
+        const int n_tiles = (p.N + BN - 1) / BN;
+        n0 = blockIdx.x % n_tiles * BN;
+        if (!group_tile<FEW_ROWS>(p, blockIdx.x / n_tiles, group, m0, m_end)) return;
+    } else {
+        n0 = blockIdx.x / chunks * BN;
+        m0 = blockIdx.x % chunks * FEW_ROWS;
     }
-    const int n0 = blockIdx.x * BN, tid = threadIdx.x, col = tid % TX, r0 = tid / TX * RT;
-    const int steps = (p.K + FEW_K - 1) / FEW_K;
-    for (int m0 = m_begin; m0 < m_end; m0 += FEW_ROWS) {
-        const int rows = min(FEW_ROWS, m_end - m0);
-        auto fill = [&](int step) {
-            if (step < steps) {
-                const int k0 = step * FEW_K, s = step % FEW_STAGES;
+    const int tid = threadIdx.x, col = tid % TX, r0 = tid / TX * RT;
+    const int steps = (p.K + FEW_K - 1) / FEW_K, rows = min(FEW_ROWS, m_end - m0);
+    // this thread's places in a stage: of the weights rows wr + j * W_ROWS at wk, of A rows ar + j * A_ROWS at ak
+    constexpr int W_LINE = FEW_K / W_PIECE, W_ROWS = THREADS / W_LINE, W_COPIES = BN / W_ROWS;
+    constexpr int A_LINE = FEW_K / A_PIECE, A_ROWS = THREADS / A_LINE, A_COPIES = (FEW_ROWS + A_ROWS - 1) / A_ROWS;
+    static_assert(W_ROWS * W_LINE == THREADS && W_COPIES * W_ROWS == BN && A_ROWS * A_LINE == THREADS, "whole lines");
+    const int wr = tid / W_LINE, wk = tid % W_LINE * W_PIECE, ar = tid / A_LINE, ak = tid % A_LINE * A_PIECE;
+    const TW* const Wg = reinterpret_cast<const TW*>(p.W) + (size_t)group * p.N * p.K;
+    const TW* const w_src = Wg + (size_t)(n0 + wr) * p.K + wk;
+    const TA* a_src[A_COPIES];
 #pragma unroll
-                for (int i = tid; i < BN * (FEW_K / W_PIECE); i += THREADS) {
-                    const int r = i / (FEW_K / W_PIECE), k = i % (FEW_K / W_PIECE) * W_PIECE;
-                    const bool valid = n0 + r < p.N && k0 + k < p.K;
-                    copy16(&Ws[s][r][k], valid ? Wg + (size_t)(n0 + r) * p.K + k0 + k : Wg, valid);
-                }
-                for (int i = tid; i < rows * (FEW_K / A_PIECE); i += THREADS) {
-                    const int r = i / (FEW_K / A_PIECE), k = i % (FEW_K / A_PIECE) * A_PIECE;
-                    if (k0 + k < p.K) {
-                        const int m = m0 + r;
-                        copy16(&As[s][r][k], reinterpret_cast<const TA*>(p.A) + (size_t)(p.a_rows ? p.a_rows[m] : m) * p.lda + k0 + k, true);
-                    }
-                }
+    for (int j = 0; j < A_COPIES; j++) {
+        const int r = ar + j * A_ROWS;
+        a_src[j] = r < rows ? reinterpret_cast<const TA*>(p.A) + (size_t)(p.a_rows ? p.a_rows[m0 + r] : m0 + r) * p.lda + ak : nullptr;
+    }
+    auto fill = [&](int step) {
+        if (step < steps) {
+            const int k0 = step * FEW_K, s = step % FEW_STAGES;
+#pragma unroll
+            for (int j = 0; j < W_COPIES; j++) {
+                const bool valid = n0 + wr + j * W_ROWS < p.N && k0 + wk < p.K;
+                copy16(&Ws[s][wr + j * W_ROWS][wk], valid ? w_src + (size_t)j * W_ROWS * p.K + k0 : Wg, valid);
             }
-            asm volatile("cp.async.commit_group;\n" ::: "memory");
+#pragma unroll
+            for (int j = 0; j < A_COPIES; j++)
+                if (a_src[j] && k0 + ak < p.K) copy16(&As[s][ar + j * A_ROWS][ak], a_src[j] + k0, true);
+        }
+        asm volatile("cp.async.commit_group;\n" ::: "memory");
+    };
+    for (int s = 0; s < FEW_STAGES - 1; s++) fill(s);
+    float acc[RT][CT];
+#pragma unroll
+    for (int i = 0; i < RT; i++)
+#pragma unroll
+        for (int j = 0; j < CT; j++) acc[i][j] = 0.f;
+    const bool busy = r0 < rows;
+    for (int step = 0; step < steps; step++) {
+        asm volatile("cp.async.wait_group %0;\n" ::"n"(FEW_STAGES - 2) : "memory");
+        __syncthreads();                                          // the stage is whole, and the one filled next is read out
+        fill(step + FEW_STAGES - 1);
+        if (!busy) continue;
+        const int s = step % FEW_STAGES, left = p.K - step * FEW_K;
+        auto four = [&](int k) {
+            float4 av[RT], wv[CT];
+#pragma unroll
+            for (int j = 0; j < CT; j++) wv[j] = read4(&Ws[s][j * TX + col][k]);
+#pragma unroll
+            for (int i = 0; i < RT; i++) av[i] = read4(&As[s][r0 + i][k]);        // rows behind the last one: whatever is there, never stored
+#pragma unroll
+            for (int i = 0; i < RT; i++)
+#pragma unroll
+                for (int j = 0; j < CT; j++)
+                    acc[i][j] = fmaf(av[i].w, wv[j].w, fmaf(av[i].z, wv[j].z, fmaf(av[i].y, wv[j].y, fmaf(av[i].x, wv[j].x, acc[i][j]))));
         };
-        for (int s = 0; s < FEW_STAGES - 1; s++) fill(s);
-        float acc[RT][CT];
+        if (left >= FEW_K) {
 #pragma unroll
-        for (int i = 0; i < RT; i++)
-#pragma unroll
-            for (int j = 0; j < CT; j++) acc[i][j] = 0.f;
-        const bool busy = r0 < rows;
-        for (int step = 0; step < steps; step++) {
-            asm volatile("cp.async.wait_group %0;\n" ::"n"(FEW_STAGES - 2) : "memory");
-            __syncthreads();                                          // the stage is whole, and the one filled next is read out
-            fill(step + FEW_STAGES - 1);
-            if (!busy) continue;
-            const int s = step % FEW_STAGES, left = p.K - step * FEW_K;
-            auto four = [&](int k) {
-                float4 av[RT], wv[CT];
-#pragma unroll
-                for (int j = 0; j < CT; j++) wv[j] = read4(&Ws[s][j * TX + col][k]);
-#pragma unroll
-                for (int i = 0; i < RT; i++) av[i] = read4(&As[s][r0 + i][k]);        // rows behind the last one: whatever is there, never stored
-#pragma unroll
-                for (int i = 0; i < RT; i++)
-#pragma unroll
-                    for (int j = 0; j < CT; j++)
-                        acc[i][j] = fmaf(av[i].w, wv[j].w, fmaf(av[i].z, wv[j].z, fmaf(av[i].y, wv[j].y, fmaf(av[i].x, wv[j].x, acc[i][j]))));
-            };
-            if (left >= FEW_K) {
-#pragma unroll
-                for (int k = 0; k < FEW_K; k += 4) four(k);
-            } else {
-                for (int k = 0; k < left; k += 4) four(k);
-            }
+            for (int k = 0; k < FEW_K; k += 4) four(k);
+        } else {
+            for (int k = 0; k < left; k += 4) four(k);
         }
-        asm volatile("cp.async.wait_group 0;\n" ::: "memory");
+    }
+    asm volatile("cp.async.wait_group 0;\n" ::: "memory");
 #pragma unroll
-        for (int i = 0; i < RT; i++) {
-            if (r0 + i >= rows) continue;
-            const int m = m0 + r0 + i;
-            const float scale = p.row_scale ? p.row_scale[m] : 1.0f;
+    for (int i = 0; i < RT; i++) {
+        if (r0 + i >= rows) continue;
+        const int m = m0 + r0 + i;
+        const float scale = p.row_scale ? p.row_scale[m] : 1.0f;
 #pragma unroll
-            for (int j = 0; j < CT; j++) {
-                const int n = n0 + j * TX + col;
-                if (n < p.N) store_out<TC>(p, m, n, acc[i][j], scale);
-            }
+        for (int j = 0; j < CT; j++) {
+            const int n = n0 + j * TX + col;
+            if (n < p.N) store_out<TC>(p, m, n, acc[i][j], scale);
         }
-        __syncthreads();                                              // the ring is free for the next eight rows
     }
 }
 
 template <typename TA, typename TW, typename TC, int BN, int RT, int CT, int FEW_K, int FEW_STAGES>
-int launch_few(const SimtParams& p, int groups, cudaStream_t stream) {
+int launch_few(const SimtParams& p, cudaStream_t stream) {
+    // Eights of rows: of groups an upper bound, as a group that has rows has one and another for every eight behind its first
+    const long long first = p.group_offsets ? min(p.M, p.groups) : 0;
+    const long long chunks = first + (p.group_offsets ? (p.M - first) / FEW_ROWS : (p.M + FEW_ROWS - 1) / FEW_ROWS);
+    const long long blocks = chunks * ((p.N + BN - 1) / BN);
+    if (blocks > 0x7fffffffll) return (int)cudaErrorInvalidValue;
     gemm_simt_few_kernel<TA, TW, TC, BN, RT, CT, FEW_K, FEW_STAGES>
-        <<<dim3((p.N + BN - 1) / BN, groups), BN / CT * (FEW_ROWS / RT), 0, stream>>>(p);
+        <<<(unsigned)blocks, BN / CT * (FEW_ROWS / RT), 0, stream>>>(p, (int)chunks);
     return esp_launch_status();
 }
 
@@ -361,13 +386,13 @@ int launch(SimtParams p, cudaStream_t stream) {
     p.wide_w = wide(p.W, p.K, sizeof(TW), 4);
     const bool grouped = p.group_offsets != nullptr;
     const long long groups = grouped ? p.groups : 1;
-    // Few rows: up to 24 pass the weights in eights, faster than a tile (N = 2,048: 16 rows 44 us against 103, 32 rows 73
-    // against 103; N = 6,144: 32 rows 114 against 106); of a group about 12 (60 groups, N = 2,816: 400 rows in all 345 us against 388,
-    // 800 rows 549 against 543).  Four by two outputs a thread read shared memory least; they want as many blocks
+    // Few rows: up to 24 pass the weights in eights, faster than a tile (N = 2,048: 24 rows 31 us against 110; N = 151,936: 24 rows
+    // 533 against 711); of a group about 12 on average, however they are spread (60 groups, N = 2,816, 400 rows in all: even 254 us
+    // against 388, all in one group 182 against 375 with the tiles of 64 x 64 of before; 720 rows 402 and 318 against 1,553 and 595).  Four by two outputs a thread read shared memory least; they want as many blocks
     // as the SMs hold at once (four each), below that two by one have the more warps (6 rows, N = 2,048: 21 us against 37).
     if (p.M <= (grouped ? 12 * groups : 24) && wide(p.A, p.lda, sizeof(TA), 16 / sizeof(TA)) && wide(p.W, p.K, sizeof(TW), 16 / sizeof(TW))) {
-        if ((p.N + 63) / 64 * groups >= 592) return launch_few<TA, TW, TC, 64, 4, 2, 64, 2>(p, (int)groups, stream);
-        return launch_few<TA, TW, TC, 32, 2, 1, 64, 4>(p, (int)groups, stream);
+        if ((p.N + 63) / 64 * groups >= 592) return launch_few<TA, TW, TC, 64, 4, 2, 64, 2>(p, stream);
+        return launch_few<TA, TW, TC, 32, 2, 1, 64, 4>(p, stream);
     }
     // Tiles: the larger one multiplies faster, the smaller one leaves less of the last wave (and of a group's end) empty.
     // Dense: what the busiest SM multiplies, with the smaller tile's outputs at 0.87 of the larger one's rate, tells them apart

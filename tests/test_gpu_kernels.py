@@ -156,6 +156,39 @@ def test_gemm_simt_routes_give_the_same_bits(a_dt, w_dt, rows, groups, n, k):
         assert torch.all((c[r].double() - exact).abs() <= bound), f"row {r}"
 
 
+def device_time(call, runs=5):
+    """The shortest of a few runs, in microseconds."""
+    times = []
+    for _ in range(runs + 1):
+        first, last = (torch.cuda.Event(enable_timing=True) for _ in range(2))
+        first.record()
+        call()
+        last.record()
+        last.synchronize()
+        times.append(first.elapsed_time(last) * 1e3)
+    return min(times[1:])
+
+
+@pytest.mark.parametrize("w_dt", [torch.float32, torch.bfloat16])
+@pytest.mark.parametrize("rows, groups", [(720, 60), (100, 300), (17, 2)])
+def test_gemm_simt_rows_that_all_fall_to_one_group(w_dt, rows, groups):
+    """As many rows on average as the kernel of few rows takes, but all of one group: the bits of a call for each row, and no
+    more than twice the time that even groups take (a block that walked its group's rows took nearly seven times as long)."""
+    n, k, one = 2048, 520, groups - 1
+    a, w = rnd(rows, k), rnd(groups, n, k, dtype=w_dt, seed=1)
+    uneven = torch.tensor([0] * groups + [rows], dtype=torch.int32, device=DEV)
+    even = torch.tensor(np.linspace(0, rows, groups + 1).astype(int), dtype=torch.int32, device=DEV)
+    c, want = torch.full((rows + 1, n), 7.0, device=DEV), torch.empty(1, n, device=DEV)
+    ops.gemm_simt(a, w, c, group_offsets=uneven, rows=rows)
+    assert torch.all(c[rows] == 7.0)
+    for r in (0, 7, 8, rows // 2, rows - 1):
+        ops.gemm_simt(a[r:r + 1], w[one], want)
+        assert torch.equal(want[0], c[r]), f"row {r}"
+    if rows == 720:
+        times = [device_time(lambda: ops.gemm_simt(a, w, c, group_offsets=off, rows=rows)) for off in (uneven, even)]
+        assert times[0] <= 2 * times[1], times
+
+
 @pytest.mark.parametrize("dtype", [torch.float32, torch.bfloat16])
 @pytest.mark.parametrize("hd, rot", [(24, 24), (128, 128), (40, 16)])
 def test_rope_kvwrite(dtype, hd, rot):
