@@ -387,10 +387,13 @@ int launch(SimtParams p, cudaStream_t stream) {
     const bool grouped = p.group_offsets != nullptr;
     const long long groups = grouped ? p.groups : 1;
     // Few rows: up to 24 pass the weights in eights, faster than a tile (N = 2,048: 24 rows 31 us against 110; N = 151,936: 24 rows
-    // 533 against 711); of a group about 12 on average, however they are spread (60 groups, N = 2,816, 400 rows in all: even 254 us
+    // 533 against 711), and more of them while the eights' outputs of a row are at most 46,000 in all, a few waves of blocks
+    // (N = 2,048: 64 rows 50 us against 113; N = 11,264: 32 rows 108 against 124, 40 rows 128 against 125; K = 5,632, N = 6,144: 64 rows
+    // 311 against 297).  Of a group about 12 on average, however they are spread (60 groups, N = 2,816, 400 rows in all: even 254 us
     // against 388, all in one group 182 against 375 with the tiles of 64 x 64 of before; 720 rows 402 and 318 against 1,553 and 595).  Four by two outputs a thread read shared memory least; they want as many blocks
     // as the SMs hold at once (four each), below that two by one have the more warps (6 rows, N = 2,048: 21 us against 37).
-    if (p.M <= (grouped ? 12 * groups : 24) && wide(p.A, p.lda, sizeof(TA), 16 / sizeof(TA)) && wide(p.W, p.K, sizeof(TW), 16 / sizeof(TW))) {
+    const bool few = grouped ? p.M <= 12 * groups : p.M <= 24 || (p.M + 7ll) / 8 * p.N <= 46000;
+    if (few && wide(p.A, p.lda, sizeof(TA), 16 / sizeof(TA)) && wide(p.W, p.K, sizeof(TW), 16 / sizeof(TW))) {
         if ((p.N + 63) / 64 * groups >= 592) return launch_few<TA, TW, TC, 64, 4, 2, 64, 2>(p, stream);
         return launch_few<TA, TW, TC, 32, 2, 1, 64, 4>(p, stream);
     }

@@ -124,7 +124,9 @@ def test_gemm_simt_grouped_with_gather_and_empty_groups():
 @pytest.mark.parametrize("rows, groups, n, k", [
     (8, 0, 65, 72),           # few rows, two by one outputs a thread, the last columns and the last k short
     (17, 0, 37900, 40),       # few rows, four by two outputs a thread, three runs of rows
-    (25, 0, 66, 128),         # the first row count that takes tiles: the small ones
+    (25, 0, 66, 128),         # more rows, in eights as long as they are few blocks
+    (25, 0, 11500, 36),       # the most columns of that
+    (25, 0, 11501, 36),       # the small tiles
     (131, 0, 19000, 20),      # large tiles, the last one with three rows
     (30, 0, 130, 33),         # rows that do not start on 16 bytes
     (300, 30, 70, 40),        # groups of few rows, some with more than eight
