@@ -31,24 +31,52 @@ __device__ __forceinline__ float2 unpack2(unsigned long long v) {
     return r;
 }
 
-// four values from p[k], in float; those at K and beyond are zero.  ``wide``: p + k is aligned to four values and K a
-// multiple of four.
-__device__ __forceinline__ float4 load4(const float* p, int k, int K, bool wide) {
-    if (!p) return make_float4(0.f, 0.f, 0.f, 0.f);
-    if (wide) return k < K ? __ldg(reinterpret_cast<const float4*>(p + k)) : make_float4(0.f, 0.f, 0.f, 0.f);
-    return make_float4(k < K ? p[k] : 0.f, k + 1 < K ? p[k + 1] : 0.f, k + 2 < K ? p[k + 2] : 0.f, k + 3 < K ? p[k + 3] : 0.f);
-}
 __device__ __forceinline__ float4 widen4(uint2 v) {
     const __nv_bfloat162 lo = *reinterpret_cast<const __nv_bfloat162*>(&v.x), hi = *reinterpret_cast<const __nv_bfloat162*>(&v.y);
     const float2 a = __bfloat1622float2(lo), b = __bfloat1622float2(hi);
     return make_float4(a.x, a.y, b.x, b.y);
 }
-__device__ __forceinline__ float4 load4(const bf16* p, int k, int K, bool wide) {
-    if (!p) return make_float4(0.f, 0.f, 0.f, 0.f);
-    if (wide) return k < K ? widen4(__ldg(reinterpret_cast<const uint2*>(p + k))) : make_float4(0.f, 0.f, 0.f, 0.f);
-    return make_float4(k < K ? to_f32(p[k]) : 0.f, k + 1 < K ? to_f32(p[k + 1]) : 0.f, k + 2 < K ? to_f32(p[k + 2]) : 0.f,
-                       k + 3 < K ? to_f32(p[k + 3]) : 0.f);
-}
+// Four values from p[k] as they lie in memory; those at K and beyond are zero.  ``wide``: p + k is aligned to four values
+// and K a multiple of four.  They become floats only when they are asked for: a conversion beside the load would wait for it.
+template <typename T> struct Loaded4;
+template <> struct Loaded4<float> {
+    float4 v;
+    __device__ __forceinline__ void load(const float* p, int k, int K, bool wide) {
+        v = make_float4(0.f, 0.f, 0.f, 0.f);
+        if (!p) return;
+        if (wide) {
+            if (k < K) v = __ldg(reinterpret_cast<const float4*>(p + k));
+        } else {
+            if (k < K) v.x = p[k];
+            if (k + 1 < K) v.y = p[k + 1];
+            if (k + 2 < K) v.z = p[k + 2];
+            if (k + 3 < K) v.w = p[k + 3];
+        }
+    }
+    __device__ __forceinline__ float4 get(bool) const { return v; }
+};
+template <> struct Loaded4<bf16> {
+    uint2 pairs;                         // wide
+    unsigned short one[4];               // else
+    __device__ __forceinline__ void load(const bf16* p, int k, int K, bool wide) {
+        pairs = make_uint2(0u, 0u);
+#pragma unroll
+        for (int i = 0; i < 4; i++) one[i] = 0;
+        if (!p) return;
+        if (wide) {
+            if (k < K) pairs = __ldg(reinterpret_cast<const uint2*>(p + k));
+        } else {
+#pragma unroll
+            for (int i = 0; i < 4; i++)
+                if (k + i < K) one[i] = __ldg(reinterpret_cast<const unsigned short*>(p) + k + i);
+        }
+    }
+    __device__ __forceinline__ float4 get(bool wide) const {
+        if (wide) return widen4(pairs);
+        return make_float4(__uint_as_float((unsigned)one[0] << 16), __uint_as_float((unsigned)one[1] << 16),
+                           __uint_as_float((unsigned)one[2] << 16), __uint_as_float((unsigned)one[3] << 16));
+    }
+};
 
 struct SimtParams {
     const void* A;
@@ -158,23 +186,26 @@ gemm_simt_kernel(SimtParams p, int m_tiles) {
         const int n = n0 + lrow + i * (THREADS / 4);
         w_src[i] = n < p.N ? Wg + (size_t)n * p.K : nullptr;
     }
-    float4 a_next[A_LOADS], w_next[W_LOADS];
+    Loaded4<TA> a_next[A_LOADS];
+    Loaded4<TW> w_next[W_LOADS];
     auto fetch = [&](int k0) {
 #pragma unroll
-        for (int i = 0; i < A_LOADS; i++) a_next[i] = load4(a_src[i], k0 + lk, p.K, p.wide_a);
+        for (int i = 0; i < A_LOADS; i++) a_next[i].load(a_src[i], k0 + lk, p.K, p.wide_a);
 #pragma unroll
-        for (int i = 0; i < W_LOADS; i++) w_next[i] = load4(w_src[i], k0 + lk, p.K, p.wide_w);
+        for (int i = 0; i < W_LOADS; i++) w_next[i].load(w_src[i], k0 + lk, p.K, p.wide_w);
     };
     auto put = [&](int buf) {
 #pragma unroll
         for (int i = 0; i < A_LOADS; i++) {
             float* d = &As[buf][lk][lrow + i * (THREADS / 4)];
-            d[0] = a_next[i].x, d[A_LD] = a_next[i].y, d[2 * A_LD] = a_next[i].z, d[3 * A_LD] = a_next[i].w;
+            const float4 v = a_next[i].get(p.wide_a);
+            d[0] = v.x, d[A_LD] = v.y, d[2 * A_LD] = v.z, d[3 * A_LD] = v.w;
         }
 #pragma unroll
         for (int i = 0; i < W_LOADS; i++) {
             float* d = &Ws[buf][lk][lrow + i * (THREADS / 4)];
-            d[0] = w_next[i].x, d[W_LD] = w_next[i].y, d[2 * W_LD] = w_next[i].z, d[3 * W_LD] = w_next[i].w;
+            const float4 v = w_next[i].get(p.wide_w);
+            d[0] = v.x, d[W_LD] = v.y, d[2 * W_LD] = v.z, d[3 * W_LD] = v.w;
         }
     };
 

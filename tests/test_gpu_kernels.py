@@ -120,7 +120,7 @@ def test_gemm_simt_grouped_with_gather_and_empty_groups():
     assert torch.all(c[total:] == 7.0), "rows beyond the groups were written"
 
 
-@pytest.mark.parametrize("a_dt, w_dt", [(torch.float32, torch.float32), (torch.float32, torch.bfloat16)])
+@pytest.mark.parametrize("a_dt, w_dt", [(torch.float32, torch.float32), (torch.float32, torch.bfloat16), (torch.bfloat16, torch.bfloat16)])
 @pytest.mark.parametrize("rows, groups, n, k", [
     (8, 0, 65, 72),           # few rows, two by one outputs a thread, the last columns and the last k short
     (17, 0, 37900, 40),       # few rows, four by two outputs a thread, three runs of rows
@@ -169,6 +169,14 @@ def device_time(call, runs=5):
         last.synchronize()
         times.append(first.elapsed_time(last) * 1e3)
     return min(times[1:])
+
+
+def test_gemm_simt_tiles_of_16_bit_weights_take_no_longer():
+    """Half the bytes: a conversion that waits for its load inside the k loop made them take 1.6 times as long as 32-bit weights."""
+    a, w, c = rnd(200, 5632), rnd(2048, 5632), torch.empty(200, 2048, device=DEV)
+    narrow = w.bfloat16()
+    times = [device_time(lambda: ops.gemm_simt(a, x, c)) for x in (narrow, w)]
+    assert times[0] <= 1.25 * times[1], times
 
 
 @pytest.mark.parametrize("w_dt", [torch.float32, torch.bfloat16])
