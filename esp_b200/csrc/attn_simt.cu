@@ -115,14 +115,19 @@ attn_simt_kernel(const T* __restrict__ q, const T* __restrict__ k_cache, const T
 }
 
 // The same for the 32-bit cache with one key per value and heads of up to 128 channels (multiples of 4), with up to 16
-// queries of a sequence at once.  A block has ``span`` tokens, which it takes run by run (tokens of one sequence at
-// consecutive positions).  Keys and values pass through shared memory 64 at a time, from absolute multiples of 64 on, each
-// read once for all queries of the run; a thread makes 2 x 4 scores, each a chain over the channels, and then 4 queries x 4
-// channels of the output, each a chain over the keys.  A key that a query does not see has the score -infinity, adds an exact
-// zero to the sum of weights and is left out of the output, so a row depends on its own position alone.
-// The kernel above takes a block per query, each thread a key of its own: every load of a warp touches 32 lines, and
-// the queries of a prompt read the same keys again and again.  Six prompts of about 1,400 tokens in all, then three steps of
-// one token each, 16 heads of 128, four layers: 11.3 ms with it, 2.2 ms with this.
+// queries of a sequence at once.  The tokens are cut into windows of 16; a run (tokens of one sequence at consecutive positions)
+// within a window is worked on by one block, run i of a window by the block with blockIdx.z = i modulo gridDim.z.  Keys and
+// values pass through shared memory 64 at a time, from absolute multiples of 64 on, each read once for all queries of the run; the
+// places of a chunk's keys in the cache are looked up once, while the chunk before it is worked on.  A thread makes 2 x 4
+// scores, each a chain over the channels, and then 4 queries x 4 channels of the output, each a chain over the keys; runs of
+// one or two tokens give a thread one score and one channel (the same chains, on all warps and not on one).  A key that a
+// query does not see has the score -infinity, adds an exact zero to the sum of weights and is left out of the output, so a row
+// depends on its own position alone: not on its run, nor on which of the two ways the run takes.
+// The softmax takes 64 keys at a time where the kernel above takes 256, so the two differ in the order of their sums.
+// Bound by the latency of a chunk's steps, two blocks an SM.  The kernel above takes a block per query, each thread a key of
+// its own: every load of a warp touches 32 lines, and the queries of a prompt read the same keys again and again.
+// 16 heads of 128, that kernel -> this: a prompt of 1,400 tokens 8,960 -> 558 us; a token each of sequences of about 3,000:
+// one 1,936 -> 255, 65 2,850 -> 1,100, 256 8,670 -> 4,340.
 constexpr int TQ = 16, TK = 64, P_LD = TQ + 4;
 
 __device__ __forceinline__ void copy16(float* dst, const float* src, bool valid) {
@@ -130,34 +135,44 @@ __device__ __forceinline__ void copy16(float* dst, const float* src, bool valid)
     asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;\n" ::"r"(d), "l"(src), "r"(valid ? 16 : 0) : "memory");
 }
 
-__global__ void __launch_bounds__(THREADS)
+__global__ void __launch_bounds__(THREADS, 2)
 attn_simt_tile_kernel(const float* __restrict__ q, const float* __restrict__ k_cache, const float* __restrict__ v_cache,
                       float* __restrict__ out, const int* __restrict__ tok_seq, const int* __restrict__ tok_pos,
                       const int* __restrict__ block_table, int table_stride, int n_pages, int page, int n_tokens, int nh, int nkv, int hd,
                       int vd, float scale, int sink, const float* __restrict__ sink_vals, int window, int chunk, int keep,
-                      float softcap, int span, int* __restrict__ status) {
+                      float softcap, int* __restrict__ status) {
     extern __shared__ __align__(16) float tile_smem[];
+    __shared__ long long places[2][TK];                        // cache rows of a chunk's keys for this head, or -1, for two chunks in turn
     const int k_ld = hd + 4;                                   // rows 16 bytes apart in the banks
     float* ks = tile_smem;                                     // [TK][k_ld]
     float* vs = ks + TK * k_ld;                                // [TK][vd]
     float* qs = vs + TK * vd;                                  // [TQ][hd]
     float* ps = qs + TQ * hd;                                  // [TK][P_LD]: scores, then weights, of key x query
     float* factor = ps + TK * P_LD;                            // [TQ]: what the sums so far are multiplied with; at the end 1 / l
-    int* bad = reinterpret_cast<int*>(factor + TQ);            // [TK]: the key's page is not to be had
-    const int h = blockIdx.y, tid = threadIdx.x, n_end = min(n_tokens, (int)(blockIdx.x + 1) * span);
-    int rows;
-    for (int n = blockIdx.x * span; n < n_end; n += rows) {
-        const int seq = tok_seq[n], pos = tok_pos[n];
-        rows = 1;
-        while (n + rows < n_end && tok_seq[n + rows] == seq && tok_pos[n + rows] == pos + rows) rows++;
+    const int h = blockIdx.y, tid = threadIdx.x, lane = tid % 32, kvh = h / (nh / nkv);
+    const int n0 = blockIdx.x * TQ, n_here = min(TQ, n_tokens - n0);
+    // the window's tokens, a lane each, and where its runs begin: every warp finds them by itself
+    const int tok_s = lane < n_here ? tok_seq[n0 + lane] : 0, tok_p = lane < n_here ? tok_pos[n0 + lane] : 0;
+    const int before_s = __shfl_up_sync(0xffffffffu, tok_s, 1), before_p = __shfl_up_sync(0xffffffffu, tok_p, 1);
+    unsigned starts = __ballot_sync(0xffffffffu, lane < n_here && (lane == 0 || tok_s != before_s || tok_p != before_p + 1));
+    // this thread's part of a chunk's copy: 16 bytes of the keys first, first + step, ... (threads beyond whole rows rest)
+    const int k_quads = hd / 4, k_first = tid / k_quads, k_step = THREADS / k_quads, k_at = tid % k_quads * 4;
+    const int v_quads = vd / 4, v_first = tid / v_quads, v_step = THREADS / v_quads, v_at = tid % v_quads * 4;
+    const float root = sqrtf((float)hd);
+    for (int run = 0; starts; run++) {
+        const int at = __ffs(starts) - 1;
+        starts &= starts - 1;
+        if (run % gridDim.z != blockIdx.z) continue;
+        const int rows = (starts ? __ffs(starts) - 1 : n_here) - at, n = n0 + at;
+        const int seq = __shfl_sync(0xffffffffu, tok_s, at), pos = __shfl_sync(0xffffffffu, tok_p, at);
+        const bool few = rows <= 2;
         const int last = pos + rows - 1;
-        const int kvh = h / (nh / nkv);
         const int lo = visible_keys(pos, window, chunk, keep).lo;
         const int lo_last = visible_keys(last, window, chunk, keep).lo, kept = visible_keys(last, window, chunk, keep).kept;
         auto next_chunk = [&](int c) { return c * TK >= kept && c < lo / TK ? lo / TK : c; };   // nothing between the kept keys and the window
 
-        for (int i = tid; i < TQ * hd / 4; i += THREADS) {
-            const int r = i / (hd / 4), d = i % (hd / 4) * 4;
+        for (int i = tid; i < TQ * k_quads; i += THREADS) {
+            const int r = i / k_quads, d = i % k_quads * 4;
             *reinterpret_cast<float4*>(qs + r * hd + d) =
                 r < rows ? *reinterpret_cast<const float4*>(q + ((size_t)(n + r) * nh + h) * hd + d) : make_float4(0.f, 0.f, 0.f, 0.f);
         }
@@ -165,8 +180,8 @@ attn_simt_tile_kernel(const float* __restrict__ q, const float* __restrict__ k_c
         const int my_q = tid / 8, my_l = tid % 8;
         const VisibleKeys seen = visible_keys(pos + my_q, window, chunk, keep);
         float m_run = sink ? (sink_vals ? sink_vals[h] : 0.f) : -INFINITY, l_run = sink ? 1.f : 0.f;
-        const float root = sqrtf((float)hd);
-        // scores: queries 2 sq, 2 sq + 1 and keys sk + 16 i; output: queries 4 oq .. 4 oq + 3, channels 4 od .. 4 od + 3
+        // scores: queries 2 sq, 2 sq + 1 and keys sk + 16 i; output: queries 4 oq .. 4 oq + 3, channels 4 od .. 4 od + 3.
+        // few: scores of query tid / 64 and key tid % 64; output of both queries, channel tid, in acc[0][0] and acc[1][0]
         const int sq = tid / 16, sk = tid % 16, oq = tid / 32, od = tid % 32;
         float acc[4][4];
 #pragma unroll
@@ -174,28 +189,53 @@ attn_simt_tile_kernel(const float* __restrict__ q, const float* __restrict__ k_c
 #pragma unroll
             for (int j = 0; j < 4; j++) acc[i][j] = 0.f;
 
-        auto row_of = [&](int j) {                                 // the cache row of key j of this sequence and head, or -1
-            const int pg = block_table[(size_t)seq * table_stride + j / page];
-            return pg < 0 || pg >= n_pages ? -1ll : ((long long)pg * nkv + kvh) * page + j % page;
+        // key tid of chunk c (the first 64 threads): its page, and from that its place
+        auto page_of = [&](int c) {
+            const int j = c * TK + tid;
+            return tid < TK && j <= last ? block_table[(size_t)seq * table_stride + j / page] : -1;
         };
-        auto fetch = [&](const float* cache, float* dst, int ld, int width, int c, bool keys) {
-            for (int i = tid; i < TK * (width / 4); i += THREADS) {
-                const int t = i / (width / 4), d = i % (width / 4) * 4, j = c * TK + t;
-                const long long row = j <= last ? row_of(j) : -1;
-                copy16(dst + t * ld + d, row >= 0 ? cache + row * width + d : cache, row >= 0);
-                if (keys && d == 0) bad[t] = row < 0;
+        auto put_place = [&](int c, int pg, int buf) {
+            if (tid < TK) places[buf][tid] = pg < 0 || pg >= n_pages ? -1ll : ((long long)pg * nkv + kvh) * page + (c * TK + tid) % page;
+        };
+        auto fetch = [&](const float* cache, float* dst, int ld, int width, int first, int step, int d, int buf) {
+            if (first < step) {
+#pragma unroll 4
+                for (int t = first; t < TK; t += step) {
+                    const long long row = places[buf][t];
+                    copy16(dst + t * ld + d, row >= 0 ? cache + row * width + d : cache, row >= 0);
+                }
             }
             asm volatile("cp.async.commit_group;\n" ::: "memory");
         };
         const int c_end = last / TK;
-        int c = next_chunk(kept > 0 ? 0 : lo / TK);
-        fetch(k_cache, ks, k_ld, hd, c, true);
-        fetch(v_cache, vs, vd, vd, c, false);
+        int c = next_chunk(kept > 0 ? 0 : lo / TK), buf = 0;
+        put_place(c, page_of(c), buf);
+        __syncthreads();
+        fetch(k_cache, ks, k_ld, hd, k_first, k_step, k_at, buf);
+        fetch(v_cache, vs, vd, vd, v_first, v_step, v_at, buf);
         while (c <= c_end) {
             const int c_next = next_chunk(c + 1);
+            const int page_next = c_next <= c_end ? page_of(c_next) : -1;      // arrives while the scores are made
             asm volatile("cp.async.wait_group 1;\n" ::: "memory");
             __syncthreads();                                       // the keys are there, and the queries
-            if (2 * sq < rows) {
+            auto put_score = [&](int t, int r, float dot) {
+                float v = scale > 0.f ? dot * scale : dot / root;
+                if (softcap > 0.f) v = softcap * tanhf(v / softcap);
+                ps[t * P_LD + r] = v;
+            };
+            if (few) {
+                if (tid / TK < rows) {
+                    const float* a_row = qs + tid / TK * hd;
+                    const float* b_row = ks + tid % TK * k_ld;
+                    float s = 0.f;
+#pragma unroll 8
+                    for (int d = 0; d < hd; d += 4) {
+                        const float4 a = *reinterpret_cast<const float4*>(a_row + d), b = *reinterpret_cast<const float4*>(b_row + d);
+                        s = fmaf(a.w, b.w, fmaf(a.z, b.z, fmaf(a.y, b.y, fmaf(a.x, b.x, s))));
+                    }
+                    put_score(tid % TK, tid / TK, s);
+                }
+            } else if (2 * sq < rows) {
                 float s[2][4];
 #pragma unroll
                 for (int i = 0; i < 2; i++)
@@ -217,21 +257,18 @@ attn_simt_tile_kernel(const float* __restrict__ q, const float* __restrict__ k_c
 #pragma unroll
                 for (int i = 0; i < 2; i++)
 #pragma unroll
-                    for (int j = 0; j < 4; j++) {
-                        float v = scale > 0.f ? s[i][j] * scale : s[i][j] / root;
-                        if (softcap > 0.f) v = softcap * tanhf(v / softcap);
-                        ps[(sk + 16 * j) * P_LD + 2 * sq + i] = v;
-                    }
+                    for (int j = 0; j < 4; j++) put_score(sk + 16 * j, 2 * sq + i, s[i][j]);
             }
-            __syncthreads();                                       // the scores are there, and the keys read
+            put_place(c_next, page_next, buf ^ 1);
+            __syncthreads();                                       // the scores and the next places are there, and the keys read
             if (my_q < rows) {
                 float p[TK / 8], best = -INFINITY;
 #pragma unroll
                 for (int i = 0; i < TK / 8; i++) {
                     const int t = my_l + 8 * i, j = c * TK + t;
-                    const bool sees = j <= pos + my_q && seen.sees(j);
-                    if (sees && bad[t]) atomicOr(status, ESP_STATUS_BAD_INDEX);
-                    p[i] = sees && !bad[t] ? ps[t * P_LD + my_q] : -INFINITY;
+                    const bool sees = j <= pos + my_q && seen.sees(j), bad = places[buf][t] < 0;
+                    if (sees && bad) atomicOr(status, ESP_STATUS_BAD_INDEX);
+                    p[i] = sees && !bad ? ps[t * P_LD + my_q] : -INFINITY;
                     best = fmaxf(best, p[i]);
                 }
 #pragma unroll
@@ -257,15 +294,32 @@ attn_simt_tile_kernel(const float* __restrict__ q, const float* __restrict__ k_c
                 if (my_l == 0) factor[my_q] = 0.f;
             }
             asm volatile("cp.async.wait_group 0;\n" ::: "memory");
-            __syncthreads();                                       // the values are there, the weights too, and ``bad`` is read
-            if (c_next <= c_end) fetch(k_cache, ks, k_ld, hd, c_next, true);
+            __syncthreads();                                       // the values are there, the weights too, and this chunk's places are read
+            if (c_next <= c_end) fetch(k_cache, ks, k_ld, hd, k_first, k_step, k_at, buf ^ 1);
             else asm volatile("cp.async.commit_group;\n" ::: "memory");
-            if (4 * oq < rows && 4 * od < vd) {
+            const int count = min(TK, last - c * TK + 1);
+            // a chunk that every query of the run sees whole, or (the same choice for a warp) key by key: a value that is not
+            // finite must not reach the queries that do not see it
+            const bool whole = c * TK + count - 1 <= pos && (c * TK >= lo_last || c * TK + TK <= kept);
+            if (few) {
+                if (tid < vd) {
+                    float first = acc[0][0] * factor[0], second = acc[1][0] * factor[1];
+                    const VisibleKeys of_first = visible_keys(pos, window, chunk, keep), of_second = visible_keys(pos + 1, window, chunk, keep);
+#pragma unroll 8
+                    for (int t = 0; t < count; t++) {
+                        const float2 w = *reinterpret_cast<const float2*>(ps + t * P_LD);
+                        const float v = vs[t * vd + tid];
+                        const int j = c * TK + t;
+                        if (whole || (j <= pos && of_first.sees(j))) first = fmaf(w.x, v, first);
+                        if (whole || (j <= pos + 1 && of_second.sees(j))) second = fmaf(w.y, v, second);
+                    }
+                    acc[0][0] = first, acc[1][0] = second;
+                }
+            } else if (4 * oq < rows && 4 * od < vd) {
 #pragma unroll
                 for (int i = 0; i < 4; i++)
 #pragma unroll
                     for (int j = 0; j < 4; j++) acc[i][j] *= factor[4 * oq + i];
-                const int count = min(TK, last - c * TK + 1);
                 auto add_key = [&](int t, auto seen_by) {
                     const float4 w = *reinterpret_cast<const float4*>(ps + t * P_LD + 4 * oq);
                     const float4 v = *reinterpret_cast<const float4*>(vs + t * vd + 4 * od);
@@ -277,9 +331,7 @@ attn_simt_tile_kernel(const float* __restrict__ q, const float* __restrict__ k_c
                         for (int j = 0; j < 4; j++) acc[i][j] = fmaf(we[i], ve[j], acc[i][j]);
                     }
                 };
-                // a chunk that every query of the run sees whole, or (the same choice for a warp) key by key: a value that is not
-                // finite must not reach the queries that do not see it
-                if (c * TK + count - 1 <= pos && (c * TK >= lo_last || c * TK + TK <= kept)) {
+                if (whole) {
 #pragma unroll 4
                     for (int t = 0; t < count; t++) add_key(t, [](int) { return true; });
                 } else {
@@ -291,22 +343,32 @@ attn_simt_tile_kernel(const float* __restrict__ q, const float* __restrict__ k_c
                 }
             }
             __syncthreads();                                       // the values and weights are read
-            if (c_next <= c_end) fetch(v_cache, vs, vd, vd, c_next, false);
+            if (c_next <= c_end) fetch(v_cache, vs, vd, vd, v_first, v_step, v_at, buf ^ 1);
             else asm volatile("cp.async.commit_group;\n" ::: "memory");
             c = c_next;
+            buf ^= 1;
         }
         if (my_l == 0) factor[my_q] = l_run;
         __syncthreads();
+        if (few) {
 #pragma unroll
-        for (int i = 0; i < 4; i++) {
-            const int r = 4 * oq + i;
-            if (r >= rows || 4 * od >= vd) continue;
-            const float l = factor[r];
-            float* orow = out + ((size_t)(n + r) * nh + h) * vd + 4 * od;
-            *reinterpret_cast<float4*>(orow) = l > 0.f ? make_float4(acc[i][0] / l, acc[i][1] / l, acc[i][2] / l, acc[i][3] / l)
-                                                       : make_float4(0.f, 0.f, 0.f, 0.f);
+            for (int r = 0; r < 2; r++) {
+                if (r >= rows || tid >= vd) continue;
+                const float l = factor[r];
+                out[((size_t)(n + r) * nh + h) * vd + tid] = l > 0.f ? acc[r][0] / l : 0.f;
+            }
+        } else {
+#pragma unroll
+            for (int i = 0; i < 4; i++) {
+                const int r = 4 * oq + i;
+                if (r >= rows || 4 * od >= vd) continue;
+                const float l = factor[r];
+                float* orow = out + ((size_t)(n + r) * nh + h) * vd + 4 * od;
+                *reinterpret_cast<float4*>(orow) = l > 0.f ? make_float4(acc[i][0] / l, acc[i][1] / l, acc[i][2] / l, acc[i][3] / l)
+                                                           : make_float4(0.f, 0.f, 0.f, 0.f);
+            }
         }
-        __syncthreads();                                           // ``factor`` is read before the next run begins
+        __syncthreads();                                           // ``factor`` and the places are read before the next run begins
     }
 }
 }  // namespace
@@ -324,13 +386,17 @@ ESP_API int esp_attn_simt(const void* q, const void* k_cache, const void* v_cach
     // by sizes and alignment alone, never by the number of tokens: a row has the same bits in a prompt and by itself
     const uintptr_t ends = (uintptr_t)q | (uintptr_t)k_cache | (uintptr_t)v_cache | (uintptr_t)out;
     if (!is_bf16 && !out_is_bf16 && maps == 1 && hd % 4 == 0 && vd % 4 == 0 && hd <= 128 && vd <= 128 && ends % 16 == 0) {
-        const int bytes = (TK * (hd + 4) + TK * vd + TQ * hd + TK * P_LD + TQ + TK) * (int)sizeof(float);
+        const int bytes = (TK * (hd + 4) + TK * vd + TQ * hd + TK * P_LD + TQ) * (int)sizeof(float);
         static const cudaError_t raised = cudaFuncSetAttribute(attn_simt_tile_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, 96 * 1024);
         if (raised != cudaSuccess) return (int)raised;
-        const int span = n_tokens <= 64 ? 1 : TQ;      // few tokens are mostly one of each sequence: a block for each of them
-        attn_simt_tile_kernel<<<dim3((n_tokens + span - 1) / span, nh), THREADS, bytes, stream>>>((const float*)q, (const float*)k_cache, (const float*)v_cache, (float*)out,
-                                                                tok_seq, tok_pos, block_table, table_stride, n_pages, page, n_tokens, nh,
-                                                                nkv, hd, vd, scale, sink, sink_vals, window, chunk, keep, softcap, span, status);
+        // How many blocks share a window of 16 tokens: its runs are between one (a prompt) and 16 (a token of each sequence), which the
+        // host does not know.  As many as it takes to fill the device four times over with two blocks an SM; those without a run
+        // leave at once, and come last, as blockIdx.z varies slowest.
+        const long long windows = (n_tokens + TQ - 1) / TQ * (long long)nh;
+        const int sharing = (int)(windows >= 4 * 2 * 148 ? 1 : (4 * 2 * 148 + windows - 1) / windows);
+        attn_simt_tile_kernel<<<dim3((n_tokens + TQ - 1) / TQ, nh, sharing < TQ ? sharing : TQ), THREADS, bytes, stream>>>(
+            (const float*)q, (const float*)k_cache, (const float*)v_cache, (float*)out, tok_seq, tok_pos, block_table, table_stride, n_pages,
+            page, n_tokens, nh, nkv, hd, vd, scale, sink, sink_vals, window, chunk, keep, softcap, status);
         return esp_launch_status();
     }
 #define ESP_SIMT(T, TO)                                                                                                    \

@@ -386,6 +386,38 @@ def test_attention_in_32_bit_of_runs_of_tokens(hd, vd, page, opts):
     assert st.item() == 8
 
 
+@pytest.mark.parametrize("nh, nkv, hd, vd, window", [(16, 16, 128, 128, None), (2, 1, 40, 24, None), (4, 2, 4, 64, 100)])
+def test_attention_in_32_bit_of_many_sequences(nh, nkv, hd, vd, window):
+    """More than 64 tokens of which most are one of each sequence, between runs of two to seventeen: the bits of each token in a
+    call by itself.  One token more than 64 costs about what it adds (blocks that took 16 contexts one after the other made
+    65 take nearly four times as long as 64)."""
+    torch.manual_seed(hd)
+    lens = [1, 2, 1, 3, 17] + [1] * 60
+    pasts = [int(p) for p in np.random.default_rng(hd).integers(0, 260, len(lens))]
+    page, per = 64, 5
+    table = torch.randperm(per * len(lens)).to(torch.int32).to(DEV).view(-1, per)
+    kc, vc = torch.randn(table.numel(), nkv, page, hd, device=DEV), torch.randn(table.numel(), nkv, page, vd, device=DEV)
+    toks = [(s, p + i) for s, (n, p) in enumerate(zip(lens, pasts)) for i in range(n)]
+    i32 = lambda v: torch.tensor(v, dtype=torch.int32, device=DEV)
+    st = status()
+
+    def call(picked):
+        q, out = x[i32([i for i, _t in picked]).long()], torch.full((len(picked), nh * vd), 3.0, device=DEV)
+        seq, pos = i32([t[0] for _i, t in picked]), i32([t[1] for _i, t in picked])
+        return lambda: ops.attn_simt(q, kc, vc, out, seq, pos, table, page, nh, nkv, hd, window, st, vd=vd) or out
+
+    x = torch.randn(len(toks), nh * hd, device=DEV)
+    toks = list(enumerate(toks))
+    got = call(toks)()
+    for i in (0, 1, 2, 3, 6, 7, 22, 23, 24, 25, len(toks) - 1):
+        assert torch.equal(call([toks[i]])()[0], got[i]), f"token {i}"
+    assert st.item() == 0
+    if hd == 128:
+        singles = [(0, (s, 260)) for s in range(65)]
+        times = [device_time(call(singles[:n])) for n in (65, 64)]
+        assert times[0] <= 1.7 * times[1], times
+
+
 @pytest.mark.parametrize("h_dt, w_dt", [(torch.float32, torch.float32), (torch.float32, torch.bfloat16)])
 @pytest.mark.parametrize("norm", [False, True])
 def test_router_topk(h_dt, w_dt, norm):
