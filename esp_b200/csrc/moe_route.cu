@@ -115,8 +115,8 @@ __device__ __forceinline__ float routing_weight(float my_p, float mass, int flag
     return my_p / denom * scale;
 }
 
-// One token's top-k by one warp.  ps[e]: its scores (left as they are when a correction or groups are given, else
-// the chosen entries are overwritten); cs: n_experts floats of scratch for the corrected scores.  The k experts with
+// One token's top-k by one warp.  ps[e]: its scores; cs: n_experts floats of scratch for the corrected scores.  What the two
+// hold afterwards is left open (of many experts the chosen entries are overwritten, of few they are not).  The k experts with
 // the largest (corrected, group-limited) score win, ties to the lower id; lane r keeps rank r: its expert in my_e and
 // that expert's uncorrected score in my_p.  Returns the sum of the chosen scores.
 __device__ __forceinline__ float choose_topk(float* ps, float* cs, int n_experts, int top_k, int lane, RouteChoice ch,

@@ -492,8 +492,8 @@ def test_route_small_equals_router_and_permutation(w_dt, n, e, k, norm):
 @pytest.mark.parametrize("e, k", [(1, 1), (31, 4), (32, 32), (33, 8), (128, 32), (129, 7)])
 @pytest.mark.parametrize("n", [5, 8, 9, 64])
 def test_route_small_chooses_in_order_with_ties_and_masked_scores(n, e, k):
-    """The raw logits as scores (chosen_softmax): negative ones, both zeros, many ties and -infinity, chosen in the order of
-    a stable sort; sizes around a warp's width and the limit of the experts that a warp keeps in registers."""
+    """The raw logits as scores (chosen_softmax): negative ones, both zeros, many ties and one near the lowest finite number, chosen
+    in the order of a stable sort; sizes around a warp's width and the limit of the experts that a warp keeps in registers."""
     rng = np.random.default_rng(n * 1000 + e)
     want = rng.choice([-3.5, -1.0, -0.0, 0.0, 0.5, 2.0], (n, e)).astype(np.float32)
     if e > k + 1:
@@ -513,6 +513,34 @@ def test_route_small_chooses_in_order_with_ties_and_masked_scores(n, e, k):
     chosen = np.take_along_axis(want.astype(np.float64), order, 1)
     ref = np.exp(chosen - chosen[:, :1])
     close(wt, torch.tensor(ref / ref.sum(1, keepdims=True), device=DEV), torch.float32, "routing weights")
+
+
+@pytest.mark.parametrize("e", [6, 33, 128, 129, 200])
+@pytest.mark.parametrize("fault", [None, "too few", "nan", "inf"])
+def test_route_small_of_infinite_scores(e, fault):
+    """Experts whose bias is -infinity are never chosen while top_k others remain (here exactly so many, or more); fewer, a NaN
+    or +infinity set the router's bit.  On both sides of the 128 experts that a warp keeps in registers."""
+    n, k = 9, 4
+    rng = np.random.default_rng(e)
+    lg = rng.choice([-3.5, -0.0, 0.0, 2.0], (n, e)).astype(np.float32)
+    masked = rng.permutation(e)[:e - k if e < 100 else e // 2]
+    bias = torch.zeros(e)
+    bias[masked] = -float("inf")
+    free = [i for i in range(e) if i not in set(masked.tolist())]
+    if fault == "too few":
+        bias[free[:len(free) - k + 1]] = -float("inf")
+    elif fault:
+        bias[free[1]] = float(fault)
+    w = torch.zeros(e, 64)
+    w[:, :n] = torch.tensor(lg).t()
+    i32, f32 = lambda *sh: torch.empty(*sh, dtype=torch.int32, device=DEV), lambda *sh: torch.empty(*sh, device=DEV)
+    ids, wt, st = i32(n, k), f32(n, k), status()
+    ops.route_small(torch.eye(n, 64, device=DEV), w.to(DEV), None, f32(n, e + 1), ids, wt, None, k, False, i32(e + 1), i32(n * k), f32(n * k),
+                    i32(n, k), st, bias=bias.to(DEV), chosen_softmax=True)
+    assert st.item() == (1 if fault else 0)
+    if fault is None:
+        scores = np.where(np.isin(np.arange(e), masked), -np.inf, lg.astype(np.float64)) + 0.0
+        assert np.array_equal(ids.cpu().numpy(), np.argsort(-scores, axis=1, kind="stable")[:, :k])
 
 
 def test_moe_permute_and_combine():
