@@ -387,8 +387,14 @@ ESP_API int esp_attn_simt(const void* q, const void* k_cache, const void* v_cach
     const uintptr_t ends = (uintptr_t)q | (uintptr_t)k_cache | (uintptr_t)v_cache | (uintptr_t)out;
     if (!is_bf16 && !out_is_bf16 && maps == 1 && hd % 4 == 0 && vd % 4 == 0 && hd <= 128 && vd <= 128 && ends % 16 == 0) {
         const int bytes = (TK * (hd + 4) + TK * vd + TQ * hd + TK * P_LD + TQ) * (int)sizeof(float);
-        static const cudaError_t raised = cudaFuncSetAttribute(attn_simt_tile_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, 96 * 1024);
-        if (raised != cudaSuccess) return (int)raised;
+        static bool raised[64] = {false};          // per device: the attribute belongs to the device's context
+        int device = 0;
+        if (cudaGetDevice(&device) != cudaSuccess || device < 0 || device >= 64) return (int)cudaErrorInvalidDevice;
+        if (!raised[device]) {
+            const cudaError_t e = cudaFuncSetAttribute(attn_simt_tile_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, 96 * 1024);
+            if (e != cudaSuccess) return (int)e;
+            raised[device] = true;
+        }
         // How many blocks share a window of 16 tokens: its runs are between one (a prompt) and 16 (a token of each sequence), which the
         // host does not know.  As many as it takes to fill the device four times over with two blocks an SM; those without a run
         // leave at once, and come last, as blockIdx.z varies slowest.

@@ -57,3 +57,12 @@ def test_every_source_file_belongs_to_one_library():
     listed = [f for files in LIBRARIES.values() for f in files]
     assert sorted(listed) == sorted(p.name for p in CSRC.glob("*.cu"))
     assert len(listed) == len(set(listed))
+
+
+def test_the_core_library_keeps_no_limit_for_all_devices_at_once():
+    """A kernel's raised shared-memory limit belongs to one device's context: it is raised at every launch or remembered per
+    device (an array), never once for the process, or a second device's launches are refused."""
+    for name in LIBRARIES["core"]:
+        text = (CSRC / name).read_text()
+        kept = re.findall(r"static\s+(?:const\s+)?(?:cudaError_t|bool)\s+\w+\s*=[^;]*;", text)
+        assert not kept, f"{name}: {kept}"
