@@ -109,9 +109,12 @@ constexpr int SCAN_UNROLL = ESP_SCAN_UNROLL;
 constexpr int CPT = ESP_SCAN_CPT;   // value columns a thread keeps: a token's q, k, d are read once for all of them
 constexpr int KT = 16;          // key channels a thread keeps
 constexpr int KTP = KT + 4;     // a slice's stride in shared memory: slices 80 bytes apart fall into different banks
-// Tokens staged at a time: 16, or 2 where the sequences bring one or two each.  Sixteen take 63 KB a block (K = V = 128), three
-// blocks an SM, and zeroing them was most of a decode step's time (8 sequences, 16 heads of 128 x 128, inside a step: 21 -> 7 us).
-constexpr int CHUNK_LONG = 16, CHUNK_SHORT = 2;
+// Tokens staged at a time.  More spread a chunk's barriers over more tokens, fewer leave room for more blocks an SM (16 take 63 KB
+// a block at K = V = 128, 8 half of that).  What the host knows is the number of rows and of sequences, so a run has at most
+// rows - sequences + 1.  Sixteen at a time where there are more than two rows a sequence on average; else eight, or two where no
+// run can have more than nine.  16 heads of 128 x 128, sixteen with all of both buffers zeroed (as it was) / two / eight:
+// 64 sequences of one 135 / 45 us; beside 400 of them a run of 400 1,097 / 593 / 563; 8 heads of 64 x 64 255 / 268 / 209.
+constexpr int CHUNK_LONG = 16, CHUNK_MIXED = 8, CHUNK_SHORT = 2;
 constexpr int MAX_K = 16 * KT;  // key channels of a head that the kernel takes
 
 enum : int {
@@ -177,8 +180,14 @@ gated_scan_kernel(const float* __restrict__ q, long long ldq, const float* __res
         c_lower[i] = in && lower && LOADS_D ? lower[h * K + i] : 0.f;
         c_bonus[i] = in && bonus ? bonus[h * K + i] : 1.f;
     }
-    // zero the padding of both buffers once (cp.async never writes it)
-    for (int i = tid; i < 2 * buf_floats; i += nthreads) smem[i] = 0.f;
+    // zero the padding once (cp.async never writes it): of the tokens that a chunk of this run has, and of the second buffer
+    // only where there is a second chunk
+    const int most = min(CHUNK, row1 - row0);
+    for (int buffer = 0; buffer < (row1 - row0 > CHUNK ? 2 : 1); buffer++) {
+        float* base = smem + buffer * buf_floats;
+        for (int i = tid; i < most * kp; i += nthreads) base[i] = base[CHUNK * kp + i] = base[2 * CHUNK * kp + i] = 0.f;
+        for (int i = tid; i < most * vt; i += nthreads) base[3 * CHUNK * kp + i] = 0.f;
+    }
     __syncthreads();
 
     pdl_wait();
@@ -777,15 +786,20 @@ ESP_API int esp_gated_scan(int mode, int ready, const float* q, long long ldq, c
     if ((long long)n_seqs * H * ((V + (threads / ks) * CPT - 1) / ((threads / ks) * CPT)) < 148 && ks <= 32 && V > (64 / ks) * CPT) threads = ESP_SCAN_SMALL_THREADS;
     const int vt = (threads / ks) * CPT;
     const int vtiles = (V + vt - 1) / vt;
-    const bool few = rows <= (long long)CHUNK_SHORT * n_seqs;      // a longer run among them still passes, two tokens at a time
-    const size_t smem = 2 * (size_t)(few ? CHUNK_SHORT : CHUNK_LONG) * (3 * ks * KTP + vt) * sizeof(float);
+    const int staged = rows > 2ll * n_seqs ? CHUNK_LONG : rows > n_seqs + 8ll ? CHUNK_MIXED : CHUNK_SHORT;
+    const size_t smem = 2 * (size_t)staged * (3 * ks * KTP + vt) * sizeof(float);
     dim3 grid(n_seqs, H, vtiles);
     if ((mode == GATE_EXP_EXP || mode == GATE_FIXED || ready) && !k) return (int)cudaErrorInvalidValue;
 #define ESP_SCAN(MODE_, READY_)                                                                                              \
     {                                                                                                                       \
-        auto kernel = few ? gated_scan_kernel<MODE_, READY_, CHUNK_SHORT> : gated_scan_kernel<MODE_, READY_, CHUNK_LONG>;    \
-        static bool set = false;                                                                                            \
-        if (!set && !few) { cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, 160 * 1024); set = true; } \
+        auto kernel = staged == CHUNK_SHORT   ? gated_scan_kernel<MODE_, READY_, CHUNK_SHORT>                                \
+                      : staged == CHUNK_MIXED ? gated_scan_kernel<MODE_, READY_, CHUNK_MIXED>                                \
+                                              : gated_scan_kernel<MODE_, READY_, CHUNK_LONG>;                                \
+        static bool set[2] = {false, false};                                                                                \
+        if (staged != CHUNK_SHORT && !set[staged == CHUNK_LONG]) {                                                          \
+            cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, 160 * 1024);                          \
+            set[staged == CHUNK_LONG] = true;                                                                               \
+        }                                                                                                                   \
         /* a step of many rows runs long and holds its shared memory: no early start beside its predecessor */             \
         esp_launch_pdl(READY_ ? 0 : ESP_PDL_SMALL, kernel, grid, dim3(threads), smem, stream, q, ldq, k, ldk, g, ldg, v, ldv, \
                        gate_bias, lower, bonus, state, state_stride, seq_start, seq_slot, out, H, K, V, ks, vt);            \
