@@ -33,7 +33,10 @@ constexpr float FIXED_ONE = 1099511627776.0f;   // 2^40
 constexpr unsigned ONE_BITS = 0x3F800000u;
 constexpr unsigned long long FIRST_MASS = 1ull << 40;      // of the first rank, whose weight is exp(0)
 constexpr int L1_BINS = 2048, LX_BINS = 512;    // a first-level bin is 2^18 steps of the weight's bits: 1,281 are used
-constexpr int KEPT_MAX = 24576;                 // weights that a block keeps in shared memory: 96 KB, two blocks to an SM
+// Weights that a block keeps in shared memory: 96 KB beside its 28 KB of bins.  Two blocks fit an SM up to about 21,900 of them
+// (175,000 ids), one from there on, which still draws faster than two that read the row anew in every pass (38 rows of 190,000
+// ids, three settings: 117 to 176 us against 128 to 205; greedy rows, 64 of them, lose by it: 34 against 23).
+constexpr int KEPT_MAX = 24576;
 
 typedef unsigned long long u64;
 
@@ -409,9 +412,12 @@ int launch_pick(const float* logits, int n_rows, int vocab, const float* tempera
 ESP_API int esp_pick_tokens(const float* logits, int n_rows, int vocab, const float* temperature, const float* top_p,
                             u64* rng_state, const int* row_slot, int* tokens, int* status, cudaStream_t stream) {
     if (n_rows <= 0) return 0;
-    // a block alone takes a vocabulary that its threads read in eight steps: no barrier of a cluster is worth it there
-    // (eight rows drawn from 8,192 ids by a block each 26 us, from 8,196 by clusters 37 us)
-    if (vocab <= 8192)
+    // A block alone takes a vocabulary that its threads read in eight steps: no barrier of a cluster is worth it there
+    // (eight rows drawn from 8,192 ids by a block each 26 us, from 8,196 by clusters 37 us), and up to what it keeps in shared
+    // memory where there are more than 32 rows, whose clusters no longer start at once (16,384 ids, 38 rows: greedy 8.4 us against
+    // 12.2, drawn 31 against 53; 64 rows 8.3 against 13.1, 31 against 68; 32 rows by clusters 9.9 and 39; 24,576 ids, eight rows:
+    // a block 38, a cluster 29).
+    if (vocab <= 8192 || (vocab <= KEPT_MAX && n_rows > 32))
         return launch_pick<1>(logits, n_rows, vocab, temperature, top_p, rng_state, row_slot, tokens, status, stream);
     return launch_pick<PICK_CLUSTER>(logits, n_rows, vocab, temperature, top_p, rng_state, row_slot, tokens, status, stream);
 }
