@@ -35,8 +35,8 @@ LIBRARIES = {
     "mixers": ["recurrent.cu", "latent.cu", "delta.cu", "selective.cu"],
     # bfloat16 only: loaded when a model runs in bfloat16
     "bf16": ["gemm_skinny.cu", "attn_decode.cu", "attn_prefill.cu", "attn_latent_mma.cu", "linear_attn.cu"],
-    # TMA + tcgen05/TMEM products for steps with many rows (bfloat16 prefill)
-    "tc05": ["gemm_tc05.cu", "attn_prefill_tc05.cu", "attn_diff_tc05.cu"],
+    # tcgen05/TMEM products: bfloat16 with many rows (prefill), 32-bit with any number of rows
+    "tc05": ["gemm_tc05.cu", "gemm_split.cu", "attn_prefill_tc05.cu", "attn_diff_tc05.cu"],
 }
 
 NVCC_FLAGS = ["-std=c++17", "-O3", "-gencode", "arch=compute_100a,code=sm_100a", "-lineinfo",

@@ -1,0 +1,541 @@
+// 32-bit matrix product on the 5th-generation tensor cores:
+//   C[m, n] = (sum_k A[row(m), k] * W[g][n, k] + bias[n]) * row_scale[m],   A, W, C float.
+//
+// A float is the sum of three bfloat16 numbers exactly (8 + 8 + 8 bits of mantissa, each piece rounded to nearest), and
+// the product of two bfloat16 numbers is exact in 32 bits.  So with x = x1 + x2 + x3 the product a * w is made of
+//   main = a1 w1,   c1 = a2 w1 + a1 w2,   c2 = a3 w1 + a2 w2 + a1 w3,
+// which are summed over k in three accumulators of their own in tensor memory; what is left out (a2 w3 and smaller) is below
+// 2^-26 of a product.  The tensor core cuts its sums off instead of rounding them, which would add up over a long sum: the
+// accumulators are read out every segment of k and their value main + (c1 + c2) is added to the running sum with an ordinary
+// rounded addition.  The order of everything depends on k alone, so a row's result has the same bits whatever other rows
+// are in the call, whatever the tile's width, whichever group the rows lie in and however many CTAs share a tile.
+// Error against 64 bits (2-norm, normal operands), this kernel / a chain of multiply-adds: K = 300 2.2e-7 / 3.1e-7, 512 2.4e-7 /
+// 4.1e-7, 1,024 4.7e-7 / 5.7e-7, 2,048 4.7e-7 / 8.1e-7, 5,632 4.8e-7 / 1.34e-6.  That is what sets the segments: with 512 k to a
+// segment K = 512 would be at 4.7e-7.
+//
+// Layout: the weights are the 128-row side of the MMA, up to NT token rows its N side; accumulator D[feature, token],
+// TMEM lane = feature, columns [main | c1 | c2] of n_tok each.  A ring of stages of 64 k: the weights come by TMA into shared
+// memory as they are; two groups of four warps take the stages in turn, split a stage and store its pieces as the A operand in
+// tensor memory (as shared-memory operands they would cost more of that memory's bandwidth than there is: the token rows' pieces
+// alone make the MMAs read 55 bytes a cycle).  Six warps load, split and store the token rows in shared memory (K-major,
+// 128-byte swizzle); a gather by a_rows costs nothing.  One thread issues the MMAs.  With the pieces of the token rows
+// [a1 | a2 | a3] one behind the other as N rows, one MMA multiplies w1 by all three, one w2 by the first two, one w3 by the
+// first.  Eight warps read the accumulators out.
+//
+// What bounds it (clock64 in each role, cycles a stage): many rows, the thread that issues the MMAs: 800 for the twelve MMAs, 340 for
+// the wait before and 190 for the commit behind them, 500 for the segment's accumulators; few rows, memory: 6 rows,
+// N = 151,936, K = 2,048 in 227 us (5.5 TB/s).  1,400 rows, N = 11,264, K = 2,048: 433 us, 149 TFLOP/s, where the multiply-add
+// tiles of gemm_simt.cu take 1,253 us.
+//
+// Persistent: a CTA per SM walks the tiles with the grid's stride; loads run ahead over the ends of tiles.  Every wait is
+// bounded: if one runs out the kernel raises ESP_STATUS_WAIT_EXPIRED, stops, frees its tensor memory and returns.
+//
+// Elements whose result is not finite (an infinity, a NaN or a number beyond bfloat16's range among the operands would
+// spread through the pieces) are made again with a chain of fused multiply-adds.
+#include "tc05.cuh"
+
+namespace {
+using namespace tc05;
+
+constexpr int BF = 128;                    // weight rows (features) of a tile
+constexpr int KS = 64;                     // k of a stage: four 16-wide MMA steps, 128 bytes of a token row's piece
+constexpr int A_COLS = 3 * KS / 2;         // TMEM columns of a stage of weights
+constexpr int RAW_BYTES = BF * KS * 4;     // the same as it comes: [4 steps][128 rows][16 k] float
+constexpr int MAX_PARTS = 12;              // segments of a tile that several CTAs share
+constexpr int SHORT_SEGMENT = 256, LONG_SEGMENT = 512, LONG_K = 1024;
+constexpr int W_WARPS = 8, E_WARPS = 8, T_WARPS = 6;     // with the one that issues the copies and the one that issues the MMAs: 24 warps
+constexpr int T_ROWS = T_WARPS * 4;        // token rows that the T_WARPS take at once, eight threads a row
+constexpr int THREADS = (W_WARPS + E_WARPS + T_WARPS + 2) * 32;
+
+struct SplitParams {
+    const float* A;
+    const int* a_rows;
+    const float* W;
+    const float* bias;
+    const float* row_scale;
+    float* C;
+    const int* group_offsets;
+    int groups, M, N, K;
+    long long lda, ldc;
+    int seg_stages, share;                 // stages of a segment; CTAs of a cluster that share a tile
+    int* status;
+};
+
+struct Tile {
+    int group, m0, rows, n_tok, f0;        // n_tok: rows rounded up to 16
+};
+
+// Walks the tiles of a CTA (or of the ``share`` CTAs of a cluster) in order.  A group's rows are cut evenly into ceil(rows / NT)
+// runs; its tiles are all runs of the first 128 features, then of the next (neighbours share their weights).
+template <int NT>
+struct Walk {
+    const SplitParams& p;
+    int feat_tiles, tile, step, group, begin, runs, width, rows;
+    int before;                            // tiles of the groups before
+    __device__ __forceinline__ Walk(const SplitParams& p_) : p(p_) {
+        feat_tiles = (p.N + BF - 1) / BF;
+        step = gridDim.x / p.share;
+        tile = (int)(blockIdx.x / p.share) - step;
+        group = -1;
+        before = 0;
+        runs = 0;
+    }
+    __device__ __forceinline__ bool next(Tile& t) {
+        tile += step;
+        while (group < 0 || tile >= before + runs * feat_tiles) {
+            if (group >= 0) before += runs * feat_tiles;
+            if (++group >= p.groups) {
+                group = p.groups - 1;      // stays behind the last one
+                before = 0, runs = 0;
+                return false;
+            }
+            int end = p.M;
+            begin = 0;
+            if (p.group_offsets) {
+                begin = p.group_offsets[group];
+                end = min(p.M, p.group_offsets[group + 1]);
+            }
+            rows = max(0, end - begin);
+            runs = (rows + NT - 1) / NT;
+            width = runs ? ((rows + runs - 1) / runs + 15) / 16 * 16 : 16;
+        }
+        const int at = tile - before;
+        const int run = at % runs;
+        t.group = group;
+        t.m0 = begin + run * width;
+        t.rows = min(width, rows - run * width);
+        t.n_tok = (t.rows + 15) / 16 * 16;
+        t.f0 = at / runs * BF;
+        return true;
+    }
+};
+
+// two floats, each rounded to bfloat16; the first in the low half
+__device__ __forceinline__ unsigned round2(float lo, float hi) {
+    unsigned r;
+    asm("cvt.rn.bf16x2.f32 %0, %1, %2;\n" : "=r"(r) : "f"(hi), "f"(lo));
+    return r;
+}
+// the next piece of two floats, packed; what is left of them stays
+__device__ __forceinline__ unsigned take2(float& x, float& y) {
+    const unsigned q = round2(x, y);
+    x -= __uint_as_float(q << 16), y -= __uint_as_float(q & 0xFFFF0000u);
+    return q;
+}
+// 16 lanes x 16 columns: of each run of 8 columns this thread's first two words go to lane t / 4, columns 2 (t % 4) and the
+// next, the other two eight lanes further
+__device__ __forceinline__ void tc_st_16x256(unsigned taddr, const unsigned (&a)[2], const unsigned (&b)[2], const unsigned (&c)[2],
+                                             const unsigned (&d)[2]) {
+    asm volatile("tcgen05.st.sync.aligned.16x256b.x2.b32 [%0], {%1, %2, %3, %4, %5, %6, %7, %8};\n"
+                 ::"r"(taddr), "r"(a[0]), "r"(a[1]), "r"(b[0]), "r"(b[1]), "r"(c[0]), "r"(c[1]), "r"(d[0]), "r"(d[1]) : "memory");
+}
+// two times 16 consecutive float columns of this thread's TMEM lane
+__device__ __forceinline__ void tc_ld16x2(unsigned ta, float (&a)[16], unsigned tb, float (&b)[16]) {
+    asm volatile(
+        "tcgen05.ld.sync.aligned.32x32b.x16.b32 {%0, %1, %2, %3, %4, %5, %6, %7, %8, %9, %10, %11, %12, %13, %14, %15}, [%32];\n"
+        "tcgen05.ld.sync.aligned.32x32b.x16.b32 {%16, %17, %18, %19, %20, %21, %22, %23, %24, %25, %26, %27, %28, %29, %30, %31}, [%33];\n"
+        "tcgen05.wait::ld.sync.aligned;\n"
+        : "=&f"(a[0]), "=&f"(a[1]), "=&f"(a[2]), "=&f"(a[3]), "=&f"(a[4]), "=&f"(a[5]), "=&f"(a[6]), "=&f"(a[7]), "=&f"(a[8]),
+          "=&f"(a[9]), "=&f"(a[10]), "=&f"(a[11]), "=&f"(a[12]), "=&f"(a[13]), "=&f"(a[14]), "=&f"(a[15]), "=&f"(b[0]), "=&f"(b[1]),
+          "=&f"(b[2]), "=&f"(b[3]), "=&f"(b[4]), "=&f"(b[5]), "=&f"(b[6]), "=&f"(b[7]), "=&f"(b[8]), "=&f"(b[9]), "=&f"(b[10]),
+          "=&f"(b[11]), "=&f"(b[12]), "=&f"(b[13]), "=&f"(b[14]), "=&f"(b[15])
+        : "r"(ta), "r"(tb) : "memory");
+}
+// bfloat16 x bfloat16 -> float, B K-major (A in tensor memory), M = 128, N = n
+__device__ __forceinline__ unsigned split_idesc(int n) {
+    return (1u << 4) | (1u << 7) | (1u << 10) | ((unsigned)(n >> 3) << 17) | ((unsigned)(BF >> 4) << 24);
+}
+__device__ __forceinline__ void cluster_sync() {
+    asm volatile("barrier.cluster.arrive.release.aligned;\n" ::: "memory");
+    asm volatile("barrier.cluster.wait.acquire.aligned;\n" ::: "memory");
+}
+// A value to the same place in the shared memory of another CTA of the cluster.
+__device__ __forceinline__ void st_cluster(float* p, unsigned rank, float v) {
+    unsigned there;
+    asm volatile("mapa.shared::cluster.u32 %0, %1, %2;\n" : "=r"(there) : "r"(smem_u32(p)), "r"(rank));
+    asm volatile("st.shared::cluster.f32 [%0], %1;\n" ::"r"(there), "f"(v) : "memory");
+}
+
+// One element as a chain of fused multiply-adds.
+__device__ __noinline__ float chain(const float* a, const float* w, int K) {
+    float s = 0.f;
+    for (int k = 0; k < K; k++) s = fmaf(a[k], w[k], s);
+    return s;
+}
+__device__ __forceinline__ void store(const SplitParams& p, const Tile& t, int row, int n, float v, float bias) {
+    const int m = t.m0 + row;
+    if (!(fabsf(v) <= 3.402823466e38f))
+        v = chain(p.A + (size_t)(p.a_rows ? p.a_rows[m] : m) * p.lda, p.W + ((size_t)t.group * p.N + n) * p.K, p.K);
+    if (p.bias) v += bias;
+    if (p.row_scale) v *= p.row_scale[m];
+    p.C[(size_t)m * p.ldc + n] = v;
+}
+
+// NT: token rows of a tile at most; ND: sets of accumulators, which the segments take in turn; NS: stages of the ring of split
+// operands, NR: of the ring of weights as they come.  SHARED: the CTAs of a cluster take a tile's segments in equal runs, and the
+// first of them adds the segments' sums in order.
+template <int NT, int ND, int NS, int NR, bool SHARED>
+__global__ void __launch_bounds__(THREADS, 1) gemm_split_kernel(const __grid_constant__ CUtensorMap map_w, SplitParams p) {
+    constexpr int D_COLS = ND * 3 * NT;
+    constexpr int T_BYTES = 3 * NT * KS * 2;
+    constexpr int RUNS = (NT / 16 + 1) / 2;                          // runs of 16 tokens that a warp reads out
+    static_assert(3 * NT <= 256 && D_COLS + NS * A_COLS <= 512, "tensor memory");
+    static_assert(!SHARED || NT == 16, "a shared tile is one run of 16 tokens");
+    extern __shared__ unsigned char smem_raw[];
+    unsigned char* smem = reinterpret_cast<unsigned char*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~(uintptr_t)1023);
+    unsigned char* raw = smem + NS * T_BYTES;
+    float* parts = reinterpret_cast<float*>(raw + NR * RAW_BYTES);   // SHARED, first CTA: [segment][16 rows][128 features]
+    __shared__ __align__(8) unsigned long long full[NS], empty[NS], raw_full[NR], raw_empty[NR], acc_full[ND], acc_empty[ND];
+    __shared__ unsigned tmem_slot;
+    __shared__ volatile int abort_flag;
+    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    if (threadIdx.x == 0) {
+        for (int i = 0; i < NS; i++) mbar_init(&full[i], W_WARPS / 2 + T_WARPS), mbar_init(&empty[i], 1);
+        for (int i = 0; i < NR; i++) mbar_init(&raw_full[i], 1), mbar_init(&raw_empty[i], W_WARPS / 2);
+        for (int i = 0; i < ND; i++) mbar_init(&acc_full[i], 1), mbar_init(&acc_empty[i], E_WARPS);
+        abort_flag = 0;
+        asm volatile("fence.mbarrier_init.release.cluster;\n" ::: "memory");
+    }
+    if (warp == W_WARPS + E_WARPS + T_WARPS + 1) {
+        asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;\n" ::"r"(smem_u32(&tmem_slot)), "r"(512));
+        asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;\n" ::);
+    }
+    tc_fence_before();
+    __syncthreads();
+    if (SHARED) cluster_sync();                                      // the first CTA runs before anything is written to its memory
+    tc_fence_after();
+    const unsigned tmem = tmem_slot;
+    const int all_stages = (p.K + KS - 1) / KS, segments = (all_stages + p.seg_stages - 1) / p.seg_stages;
+    const int rank = SHARED ? (int)(blockIdx.x % p.share) : 0;
+    const int seg0 = SHARED ? rank * segments / p.share : 0, seg1 = SHARED ? (rank + 1) * segments / p.share : segments;
+    const int stage0 = seg0 * p.seg_stages, stages = min(all_stages, seg1 * p.seg_stages) - stage0;      // of this CTA, of every tile
+    bool ok = true;
+
+    if (warp < W_WARPS) {
+        // weights into pieces.  A lane holds 4 k of rows 8 i + lane / 4 (i = 0..3) of two of the stage's four MMA steps at a time.
+        const int quad = warp & 3, half = warp >> 2;                 // TMEM lanes 32 quad .. + 31; the group
+        const unsigned lanes = tmem + ((unsigned)(quad * 32) << 16);
+        const int from = (quad * 32 + (lane >> 2)) * 64 + (lane & 3) * 16;    // byte of the stage: eight lanes read 128 bytes in a row
+        if (p.group_offsets) pdl_wait();
+        Walk<NT> walk(p);
+        Tile t;
+        int end = 0;                                                 // stages of the tiles seen so far
+        for (int it = half;; it += 2) {
+            bool more = it < end;
+            while (!more && walk.next(t)) more = it < (end += stages);
+            if (!more) break;
+            const int s = it % NS, r = it % NR;
+            ok = mbar_wait(&raw_full[r], (it / NR) & 1) && !abort_flag;
+            if (!ok) break;
+            const unsigned char* stage = raw + r * RAW_BYTES + from;
+            const unsigned at = lanes + D_COLS + s * A_COLS;
+#pragma unroll
+            for (int two = 0; two < 2; two++) {
+                float4 v[2][4];
+#pragma unroll
+                for (int j = 0; j < 2; j++)
+#pragma unroll
+                    for (int i = 0; i < 4; i++) v[j][i] = *reinterpret_cast<const float4*>(stage + (2 * two + j) * (BF * 64) + i * 512);
+                if (two == 0) {
+                    if (it >= NS) ok = mbar_wait(&empty[s], (it / NS - 1) & 1) && !abort_flag;     // its last contents have been multiplied
+                    tc_fence_after();
+                }
+                if (!ok) break;
+#pragma unroll
+                for (int piece = 0; piece < 3; piece++) {
+                    unsigned q[2][4][2];
+#pragma unroll
+                    for (int j = 0; j < 2; j++)
+#pragma unroll
+                        for (int i = 0; i < 4; i++) {
+                            q[j][i][0] = take2(v[j][i].x, v[j][i].y);
+                            q[j][i][1] = take2(v[j][i].z, v[j][i].w);
+                        }
+                    const unsigned to = at + piece * (KS / 2) + two * 16;
+                    tc_st_16x256(to, q[0][0], q[0][1], q[1][0], q[1][1]);
+                    tc_st_16x256(to + (16u << 16), q[0][2], q[0][3], q[1][2], q[1][3]);
+                }
+            }
+            if (!ok) break;
+            tc_wait_st();
+            tc_fence_before();
+            __syncwarp();
+            if (lane == 0) {
+                mbar_arrive(&full[s]);
+                mbar_arrive(&raw_empty[r]);
+            }
+        }
+    } else if (warp < W_WARPS + E_WARPS) {
+        // the accumulators: a warp has a quarter of the lanes and every second run of 16 tokens
+        const int quad = warp & 3, half = (warp - W_WARPS) >> 2;
+        const unsigned lanes = tmem + ((unsigned)(quad * 32) << 16);
+        pdl_wait();
+        Walk<NT> walk(p);
+        Tile o;
+        int count = 0;                                               // segments read out so far
+        while (ok && walk.next(o)) {
+            float total[RUNS][16];
+            for (int seg = seg0; seg < seg1; seg++, count++) {
+                ok = mbar_wait(&acc_full[count % ND], (count / ND) & 1) && !abort_flag;
+                if (!ok) break;
+                tc_fence_after();
+#pragma unroll
+                for (int r = 0; r < RUNS; r++) {
+                    const int c = (2 * r + half) * 16;
+                    if (c >= o.n_tok) continue;                      // the same for a whole warp
+                    const unsigned at = lanes + count % ND * 3 * NT + c;
+                    float sum[16], v[16];
+                    tc_ld16x2(at + o.n_tok, v, at + 2 * o.n_tok, sum);
+#pragma unroll
+                    for (int i = 0; i < 16; i++) sum[i] = v[i] + sum[i];
+                    tc_ld16(at, v);
+#pragma unroll
+                    for (int i = 0; i < 16; i++) {
+                        sum[i] = v[i] + sum[i];
+                        if (SHARED) st_cluster(parts + (seg * 16 + i) * BF + quad * 32 + lane, 0, sum[i]);
+                        else total[r][i] = seg == 0 ? sum[i] : total[r][i] + sum[i];
+                    }
+                }
+                tc_fence_before();
+                __syncwarp();
+                if (lane == 0) mbar_arrive(&acc_empty[count % ND]);
+            }
+            const int n = o.f0 + quad * 32 + lane;
+            if (SHARED || !ok || n >= p.N) continue;
+            const float b = p.bias ? p.bias[n] : 0.f;
+#pragma unroll
+            for (int r = 0; r < RUNS; r++) {
+                const int c = (2 * r + half) * 16;
+#pragma unroll
+                for (int i = 0; i < 16; i++)
+                    if (c + i < o.rows) store(p, o, c + i, n, total[r][i], b);
+            }
+        }
+    } else if (warp < W_WARPS + E_WARPS + T_WARPS) {
+        // token rows: eight threads to a row, each with eight k of it
+        const int tid = threadIdx.x - (W_WARPS + E_WARPS) * 32;
+        const int r0 = tid >> 3, part = tid & 7;
+        constexpr int PASSES = (NT + T_ROWS - 1) / T_ROWS;
+        pdl_wait();
+        Walk<NT> walk(p);
+        Tile t;
+        float4 next[PASSES][2];
+        const float* src[PASSES];
+        int n_tok = 0, n_next = 0, kb = stage0;
+        bool have = walk.next(t);
+        auto point = [&]() {
+#pragma unroll
+            for (int j = 0; j < PASSES; j++) {
+                const int r = r0 + T_ROWS * j;
+                src[j] = nullptr;
+                if (have && r < t.rows) src[j] = p.A + (size_t)(p.a_rows ? p.a_rows[t.m0 + r] : t.m0 + r) * p.lda + part * 8;
+            }
+            n_next = have ? t.n_tok : 0;
+        };
+        point();
+        auto load = [&]() {
+            const int k = kb * KS + part * 8;
+#pragma unroll
+            for (int j = 0; j < PASSES; j++) {
+                next[j][0] = next[j][1] = make_float4(0.f, 0.f, 0.f, 0.f);
+                if (src[j] && k < p.K) next[j][0] = *reinterpret_cast<const float4*>(src[j] + kb * KS);
+                if (src[j] && k + 4 < p.K) next[j][1] = *reinterpret_cast<const float4*>(src[j] + kb * KS + 4);
+            }
+            n_tok = n_next;
+            if (have && ++kb == stage0 + stages) {
+                kb = stage0;
+                have = walk.next(t);
+                point();
+            }
+        };
+        load();
+        for (int it = 0; n_tok > 0; it++) {
+            const int s = it % NS;
+            if (it >= NS) ok = mbar_wait(&empty[s], (it / NS - 1) & 1) && !abort_flag;
+            if (!ok) break;
+            const int n = n_tok;
+            unsigned char* base = smem + s * T_BYTES;
+#pragma unroll
+            for (int j = 0; j < PASSES; j++) {
+                const int r = r0 + T_ROWS * j;
+                if (r >= n) break;
+                uint4 q1, q2, q3;
+                auto take8 = [&](uint4& q) {
+                    q.x = take2(next[j][0].x, next[j][0].y), q.y = take2(next[j][0].z, next[j][0].w);
+                    q.z = take2(next[j][1].x, next[j][1].y), q.w = take2(next[j][1].z, next[j][1].w);
+                };
+                take8(q1), take8(q2), take8(q3);
+                unsigned char* at = base + r * 128 + ((part ^ (r & 7)) << 4);
+                *reinterpret_cast<uint4*>(at) = q1;
+                *reinterpret_cast<uint4*>(at + n * 128) = q2;
+                *reinterpret_cast<uint4*>(at + 2 * n * 128) = q3;
+            }
+            load();
+            fence_async_smem();
+            __syncwarp();
+            if (lane == 0) mbar_arrive(&full[s]);
+        }
+    } else if (warp == W_WARPS + E_WARPS + T_WARPS) {
+        // weights as they come: four boxes of 128 rows x 16 k a stage, a lane each
+        if (p.group_offsets) pdl_wait();                             // whose weights are read follows from the offsets; of a dense product they are never written
+        Walk<NT> walk(p);
+        Tile t;
+        int it = 0;
+        while (ok && walk.next(t)) {
+            for (int st = 0; st < stages && ok; st++, it++) {
+                const int r = it % NR, k = (stage0 + st) * KS + lane * 16;
+                if (it >= NR) ok = mbar_wait(&raw_empty[r], (it / NR - 1) & 1) && !abort_flag;
+                ok = __all_sync(0xffffffffu, ok);
+                if (!ok) break;
+                if (lane == 0) mbar_expect_tx(&raw_full[r], RAW_BYTES);
+                __syncwarp();
+                if (lane < 4) tma_load_3d(raw + r * RAW_BYTES + lane * (BF * 64), &map_w, k, t.f0, t.group, &raw_full[r]);
+            }
+        }
+        pdl_wait();
+    } else if (lane == 0) {
+        pdl_wait();
+        pdl_trigger();                                               // behind the wait: a dependent kernel may count on all before this one
+        Walk<NT> walk(p);
+        Tile t;
+        const unsigned long long desc0 = smem_desc(smem);
+        int it = 0, seg = 0;
+        while (ok && walk.next(t)) {
+            const int n = t.n_tok;
+            const unsigned d_three = split_idesc(3 * n), d_two = split_idesc(2 * n), d_one = split_idesc(n);
+            int in_seg = 0;
+            for (int st = 0; st < stages; st++, it++) {
+                const int s = it % NS;
+                if (in_seg == 0 && seg >= ND) ok = mbar_wait(&acc_empty[seg % ND], (seg / ND - 1) & 1);
+                if (ok) ok = mbar_wait(&full[s], (it / NS) & 1) && !abort_flag;
+                if (!ok) break;
+                tc_fence_after();
+                const unsigned d = tmem + seg % ND * 3 * NT, a0 = tmem + D_COLS + s * A_COLS;
+                const unsigned long long b0 = desc0 + (unsigned)((s * T_BYTES) >> 4);
+#pragma unroll
+                for (int j = 0; j < KS / 16; j++) {
+                    const unsigned a = a0 + 8 * j;
+                    const unsigned long long b = b0 + 2 * j;
+                    tc_mma_ta(d, a, b, d_three, in_seg == 0 && j == 0 ? 0u : 1u);             // main, c1, c2
+                    tc_mma_ta(d + n, a + KS / 2, b, d_two, 1u);                               // c1, c2
+                    tc_mma_ta(d + 2 * n, a + KS, b, d_one, 1u);                               // c2
+                }
+                tc_commit(&empty[s]);
+                if (++in_seg == p.seg_stages || st + 1 == stages) {
+                    tc_commit(&acc_full[seg % ND]);
+                    in_seg = 0;
+                    seg++;
+                }
+            }
+        }
+    }
+    if (!ok && lane == 0) {
+        atomicOr(p.status, ESP_STATUS_WAIT_EXPIRED);
+        abort_flag = 1;
+        for (int i = 0; i < 1000; i++) __nanosleep(1000);            // copies and MMAs in flight end before their memory is given up
+    }
+    tc_fence_before();
+    __syncthreads();
+    if (SHARED) {
+        // the segments' sums are with the first CTA, which adds them in order
+        cluster_sync();
+        if (rank == 0 && !abort_flag) {
+            Walk<NT> walk(p);
+            Tile o;
+            const bool have = walk.next(o);
+            for (int i = threadIdx.x; have && i < o.rows * BF; i += THREADS) {
+                const int n = o.f0 + i % BF;
+                if (n >= p.N) continue;
+                float v = parts[i];
+                for (int seg = 1; seg < segments; seg++) v += parts[seg * 16 * BF + i];
+                store(p, o, i / BF, n, v, p.bias ? p.bias[n] : 0.f);
+            }
+        }
+    }
+    if (warp == W_WARPS + E_WARPS + T_WARPS + 1) {
+        tc_fence_after();
+        asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;\n" ::"r"(tmem), "r"(512));
+    }
+}
+
+typedef CUresult (*EncodeTiledFn)(CUtensorMap*, CUtensorMapDataType, cuuint32_t, void*, const cuuint64_t*, const cuuint64_t*,
+                                  const cuuint32_t*, const cuuint32_t*, CUtensorMapInterleave, CUtensorMapSwizzle,
+                                  CUtensorMapL2promotion, CUtensorMapFloatOOBfill);
+
+// W as [groups][N][K] float, boxes of 128 rows x 16 k, zeros out of bounds
+int map_weights(CUtensorMap* map, const SplitParams& p) {
+    static EncodeTiledFn fn = nullptr;
+    if (!fn) {
+        void* ptr = nullptr;
+        cudaDriverEntryPointQueryResult found;
+        if (cudaGetDriverEntryPoint("cuTensorMapEncodeTiled", &ptr, cudaEnableDefault, &found) != cudaSuccess || found != cudaDriverEntryPointSuccess)
+            return (int)cudaErrorNotSupported;
+        fn = reinterpret_cast<EncodeTiledFn>(ptr);
+    }
+    const cuuint64_t dims[3] = {(cuuint64_t)p.K, (cuuint64_t)p.N, (cuuint64_t)p.groups};
+    const cuuint64_t strides[2] = {(cuuint64_t)p.K * 4, (cuuint64_t)p.K * p.N * 4};
+    const cuuint32_t box[3] = {16, BF, 1}, elem[3] = {1, 1, 1};
+    const CUresult r = fn(map, CU_TENSOR_MAP_DATA_TYPE_FLOAT32, 3, const_cast<float*>(p.W), dims, strides, box, elem,
+                          CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_NONE, CU_TENSOR_MAP_L2_PROMOTION_L2_256B,
+                          CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
+    return r == CUDA_SUCCESS ? 0 : (int)cudaErrorInvalidValue;
+}
+
+template <int NT, int ND, int NS, int NR, bool SHARED>
+int launch(SplitParams p, int sms, cudaStream_t stream) {
+    constexpr int SMEM = NS * 3 * NT * KS * 2 + NR * RAW_BYTES + (SHARED ? MAX_PARTS * 16 * BF * 4 : 0) + 1024;
+    static_assert(SMEM <= 231 * 1024 - 512, "shared memory");
+    CUtensorMap map;
+    const int rc = map_weights(&map, p);
+    if (rc) return rc;
+    const auto kernel = gemm_split_kernel<NT, ND, NS, NR, SHARED>;
+    const cudaError_t e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, SMEM);
+    if (e != cudaSuccess) return (int)e;
+    const long long runs = p.group_offsets ? p.M / NT + (p.groups < p.M ? p.groups : p.M) : (p.M + NT - 1) / NT;       // of groups: an upper bound
+    const long long tiles = runs * ((p.N + BF - 1) / BF);
+    if (tiles + sms > 0x3fffffffll) return (int)cudaErrorInvalidValue;
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = dim3((unsigned)(SHARED ? tiles * p.share : tiles < sms ? tiles : sms));
+    cfg.blockDim = dim3(THREADS);
+    cfg.dynamicSmemBytes = SMEM;
+    cfg.stream = stream;
+    cudaLaunchAttribute attr[2];
+    attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    attr[0].val.programmaticStreamSerializationAllowed = 1;
+    cfg.attrs = attr;
+    cfg.numAttrs = esp_pdl_enabled(ESP_PDL_DENSE) ? 1 : 0;
+    if (SHARED) {
+        cudaLaunchAttribute& cluster = attr[cfg.numAttrs++];
+        cluster.id = cudaLaunchAttributeClusterDimension;
+        cluster.val.clusterDim.x = p.share, cluster.val.clusterDim.y = 1, cluster.val.clusterDim.z = 1;
+    }
+    cudaLaunchKernelEx(&cfg, kernel, map, p);
+    return esp_launch_status();
+}
+}  // namespace
+
+// All float.  K, lda multiples of 4, A and W on 16 bytes.
+ESP_API int esp_gemm_split(const void* A, const int* a_rows, const void* W, const float* bias, const float* row_scale, void* C,
+                           const int* group_offsets, int groups, int M, int N, int K, long long lda, long long ldc, int* status,
+                           cudaStream_t stream) {
+    if (M <= 0 || N <= 0) return 0;
+    if (K <= 0 || K % 4 != 0 || lda % 4 != 0 || ((uintptr_t)A & 15) || ((uintptr_t)W & 15) || groups < 1) return (int)cudaErrorInvalidValue;
+    SplitParams p{(const float*)A, a_rows, (const float*)W, bias, row_scale, (float*)C, group_offsets, groups, M, N, K, lda, ldc,
+                  (K >= LONG_K ? LONG_SEGMENT : SHORT_SEGMENT) / KS, 1, status};
+    int dev = 0, sms = 0;
+    cudaError_t e = cudaGetDevice(&dev);
+    if (e == cudaSuccess) e = cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
+    if (e != cudaSuccess) return (int)e;
+    if (!group_offsets) {
+        // Few tiles of 16 rows: as many CTAs to each as there are SMs for (6 rows, K = 2,048: N = 2,048 31 us with a CTA a tile, 12 with
+        // four; N = 6,144 31 and 21 with two; K = 5,632, N = 2,048 76 and 38.  64 rows: N = 2,048 22 us, tiles of 64 rows 36)
+        const long long tiles = (long long)((M + 15) / 16) * ((N + BF - 1) / BF);
+        const int segments = ((K + KS - 1) / KS + p.seg_stages - 1) / p.seg_stages;
+        while (p.share < 8 && tiles * p.share * 2 <= sms && p.share * 2 <= segments) p.share *= 2;
+        if (segments > MAX_PARTS) p.share = 1;
+        if (p.share > 1) return launch<16, 2, 4, 3, true>(p, sms, stream);
+    }
+    // few rows, of a group four on average: a short tile leaves tensor memory for two sets of accumulators
+    if (M <= (group_offsets ? 4ll * groups : 16ll)) return launch<16, 2, 4, 6, false>(p, sms, stream);
+    return launch<64, 1, 3, 4, false>(p, sms, stream);
+}

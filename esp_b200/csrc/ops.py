@@ -47,6 +47,7 @@ _SIGNATURES = {
     "esp_finite_check": [P, c_int, c_longlong, P, c_int, P],
     "esp_normal_fill": [P, c_int, c_longlong, c_ulonglong, c_float, c_float, P],
     "esp_gemm_simt": [P, c_int, P, P, c_int, P, P, P, c_int, P, c_int, c_int, c_int, c_int, c_longlong, c_longlong, P],
+    "esp_gemm_split": [P, P, P, P, P, P, P, c_int, c_int, c_int, c_int, c_longlong, c_longlong, P, P],
     "esp_rope_kvwrite": [P, P, P, P, P, P, c_int, c_int, P, P, P, c_int, P, c_int, c_int, c_int, c_int, c_int, c_int,
                          c_int, c_int, P, P],
     "esp_attn_simt": [P, P, P, P, c_int, c_int, P, P, P, c_int, c_int, c_int, c_int, c_int, c_int, c_int, c_int, c_float, c_int, P,
@@ -229,6 +230,7 @@ def _ptr(t, dtype=None, what="tensor"):
 
 _F32, _BF16 = torch.float32, torch.bfloat16
 FLOATS = (_F32, _BF16)
+SPLIT_MIN_K, SPLIT_MIN_N = 256, 128
 
 
 def _is_bf16(t) -> int:
@@ -349,6 +351,37 @@ def gemm_simt(a, w, c, bias=None, row_scale=None, a_rows=None, group_offsets=Non
         _ptr(bias, torch.float32, "bias"), _ptr(row_scale, torch.float32, "row_scale"), c.data_ptr(), _is_bf16(c),
         _ptr(group_offsets, torch.int32, "group_offsets"), groups, m, n, k, a.stride(0), c.stride(0), _stream())
     _check(code, "gemm_simt")
+
+
+def gemm_split_fits(a, w) -> bool:
+    """Whether the 32-bit product ``a @ w.T`` (w [N, K] or [G, N, K]) is one for ``gemm_split``.  Asks for nothing that differs between
+    the rows of a model's calls, so that a row takes the same kernel in every call."""
+    k = w.shape[-1]
+    return (a.dtype is _F32 and w.dtype is _F32 and k >= SPLIT_MIN_K and w.shape[-2] >= SPLIT_MIN_N and k % 4 == 0
+            and a.stride(0) % 4 == 0 and a.data_ptr() % 16 == 0 and w.data_ptr() % 16 == 0)
+
+
+def gemm_split(a, w, c, status, bias=None, row_scale=None, a_rows=None, group_offsets=None, rows=None):
+    """``gemm_simt`` for float32 operands on the tensor cores: every operand as three bfloat16 pieces, their products summed
+    in 32 bits.  A row's bits do not depend on the other rows of the call."""
+    grouped = group_offsets is not None
+    if grouped:
+        groups, n, k = w.shape
+    else:
+        groups = 1
+        n, k = w.shape
+    m = c.shape[0] if rows is None else rows
+    if a.shape[-1] != k or c.shape[-1] != n:
+        raise Backend(f"gemm: shapes disagree: a {tuple(a.shape)}, w {tuple(w.shape)}, c {tuple(c.shape)}")
+    if a.stride(-1) != 1 or c.stride(-1) != 1 or not w.is_contiguous():
+        raise Backend("gemm: operands must be row-major")
+    if not (a.dtype is w.dtype is c.dtype is _F32):
+        raise Backend("gemm_split takes float32 operands")
+    code = _fn("tc05", "esp_gemm_split")(
+        a.data_ptr(), _ptr(a_rows, torch.int32, "a_rows"), w.data_ptr(), _ptr(bias, torch.float32, "bias"),
+        _ptr(row_scale, torch.float32, "row_scale"), c.data_ptr(), _ptr(group_offsets, torch.int32, "group_offsets"), groups, m, n, k,
+        a.stride(0), c.stride(0), _ptr(status, torch.int32), _stream())
+    _check(code, "gemm_split")
 
 
 def rope_kvwrite(qkv, bias, tok_seq, tok_pos, cos, sin, rot, q_out, k_cache, v_cache, block_table, page, nh, nkv, hd,

@@ -7,7 +7,7 @@ import torch
 from ..csrc import ops
 from ..errors import Unsupported
 from .base import ParamSpec, Part, register
-from .linear import grouped_linear, grouped_swiglu_linear, grouped_uses_tc05, linear, relu2_linear, swiglu_linear, xielu_linear
+from .linear import grouped_linear, grouped_swiglu_linear, grouped_uses_tc05, linear, product32, relu2_linear, swiglu_linear, xielu_linear
 
 
 class DeferredMoeCombine:
@@ -534,9 +534,9 @@ class ScaledInputMoe(Part):
                             max_rows=n, relu2=True)
             ops.gemm_skinny(act, self.w_down, out, group_offsets=offsets, rows=rows, max_rows=n)
         else:
-            ops.gemm_simt(h, self.w_up, z, a_rows=perm_token, row_scale=perm_weight, group_offsets=offsets, rows=rows)
+            product32(rt, h, self.w_up, z, a_rows=perm_token, row_scale=perm_weight, group_offsets=offsets, rows=rows)
             ops.relu2(z, act)
-            ops.gemm_simt(act, self.w_down, out, group_offsets=offsets, rows=rows)
+            product32(rt, act, self.w_down, out, group_offsets=offsets, rows=rows)
         if self.w_shared_up is not None:
             if beside:
                 rt.side_stream.join()

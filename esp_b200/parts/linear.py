@@ -1,8 +1,10 @@
 """Matrix products of the layers: ``out = a @ w.T``.
 
 Which kernel runs is decided here and nowhere else:
-* 32-bit engine, or a weight kept in 32-bit: the plain CUDA-core kernel with
-  true float32 multiply-adds and a fixed summation order;
+* 32-bit engine, or a weight kept in 32-bit: the tensor cores with every 32-bit
+  operand as three bfloat16 pieces where both operands are 32-bit and the
+  matrix is large enough, else the plain CUDA-core kernel with true float32
+  multiply-adds; both sum in an order that depends on K alone;
 * bfloat16 activations and weights, at most SKINNY_ROWS rows (decode): the
   weight-streaming tensor-core kernel of this library (grouped products: see
   ``grouped_uses_tc05``);
@@ -33,6 +35,14 @@ def _both_bf16(a, w) -> bool:
     return a.dtype == torch.bfloat16 and w.dtype == torch.bfloat16
 
 
+def product32(rt, a, w, out, **options):
+    """out = a @ w.T (``ops.gemm_simt``'s options) for operands that are not both bfloat16."""
+    if out.dtype == torch.float32 and ops.gemm_split_fits(a, w):
+        ops.gemm_split(a, w, out, rt.status, **options)
+    else:
+        ops.gemm_simt(a, w, out, **options)
+
+
 def linear(rt, a: torch.Tensor, w: torch.Tensor, out: torch.Tensor) -> torch.Tensor:
     """a [M,K] (activation dtype), w [N,K], out [M,N] float32."""
     if _both_bf16(a, w):
@@ -43,7 +53,7 @@ def linear(rt, a: torch.Tensor, w: torch.Tensor, out: torch.Tensor) -> torch.Ten
         else:
             torch.mm(a, w.t(), out_dtype=torch.float32, out=out)
     else:
-        ops.gemm_simt(a, w, out)
+        product32(rt, a, w, out)
     return out
 
 
@@ -123,7 +133,7 @@ def grouped_swiglu_linear(rt, a, w_gate_up, act, group_offsets, a_rows, rows, ma
         return act
     inter = w_gate_up.shape[1] // 2
     gu = rt.ws.get(tag + "_gu", (rows, 2 * inter), torch.float32)
-    ops.gemm_simt(a, w_gate_up, gu, a_rows=a_rows, group_offsets=group_offsets, rows=rows)
+    product32(rt, a, w_gate_up, gu, a_rows=a_rows, group_offsets=group_offsets, rows=rows)
     _gated_unit(gu, act, glu)
     return act
 
@@ -138,5 +148,5 @@ def grouped_linear(rt, a, w, out, group_offsets, row_scale, rows, max_rows, tile
         ops.gemm_skinny(a, w, out, row_scale=row_scale, group_offsets=group_offsets, rows=rows, max_rows=max_rows,
                         offsets_ready=offsets_ready)
     else:
-        ops.gemm_simt(a, w, out, row_scale=row_scale, group_offsets=group_offsets, rows=rows)
+        product32(rt, a, w, out, row_scale=row_scale, group_offsets=group_offsets, rows=rows)
     return out

@@ -1,0 +1,106 @@
+"""The 32-bit products on the tensor cores, every operand as three bfloat16 pieces."""
+import numpy as np
+import pytest
+import torch
+
+from esp_b200.csrc import ops
+
+pytestmark = pytest.mark.gpu
+DEV = "cuda:0"
+
+
+def rnd(*shape, seed=0):
+    return torch.randn(*shape, generator=torch.Generator().manual_seed(seed)).to(DEV)
+
+
+def check(c, a, w, what):
+    """Within rounding of the 64-bit product, element by element: every accumulation of 16 products, every segment and the three
+    accumulators' sum lose at most a unit in the last place of a partial sum, together less than K / 2 of them."""
+    exact = a.double() @ w.double().t()
+    bound = a.shape[1] * 2.0 ** -24 * (a.double().abs() @ w.double().abs().t())
+    assert torch.all((c.double() - exact).abs() <= bound), what
+    return exact
+
+
+@pytest.mark.parametrize("m, n, k", [
+    (1, 128, 256), (15, 300, 260),     # one run of 16 rows; features and k that end inside a tile and a stage
+    (16, 2048, 2048), (17, 130, 1028),  # tiles shared by clusters of four and two CTAs, two runs of rows
+    (33, 2048, 5632), (3, 640, 6660),  # by eight CTAs; more segments than are shared
+    (16, 19000, 512), (64, 9600, 300),  # a CTA a tile: short tiles, several a CTA; one full run of 64 rows
+    (65, 11264, 516), (200, 2304, 1100), (389, 1300, 256),   # uneven runs of rows
+])
+def test_dense(m, n, k):
+    a, w, status = rnd(m, k), rnd(n, k, seed=1), torch.zeros(1, dtype=torch.int32, device=DEV)
+    bias, scale = rnd(n, seed=2), rnd(m, seed=3)
+    c = torch.full((m + 1, n), 7.0, device=DEV)
+    ops.gemm_split(a, w, c, status, rows=m)
+    assert status.item() == 0 and torch.all(c[m] == 7.0)
+    exact = check(c[:m], a, w, "product")
+    # no further from the 64-bit product than the chain of multiply-adds
+    chain = torch.empty(m, n, device=DEV)
+    ops.gemm_simt(a, w, chain)
+    assert (c[:m].double() - exact).norm() <= 1.05 * (chain.double() - exact).norm()
+    # bias, then scale; rows of a wider matrix; a row alone has the same bits
+    wide, d = torch.zeros(m, k + 4, device=DEV), torch.empty(m, n, device=DEV)
+    wide[:, :k] = a
+    ops.gemm_split(wide[:, :k], w, d, status, bias=bias, row_scale=scale)
+    assert torch.equal(d, (c[:m] + bias) * scale[:, None])
+    one = torch.empty(1, n, device=DEV)
+    for r in {0, m // 2, m - 1}:
+        ops.gemm_split(a[r:r + 1], w, one, status)
+        assert torch.equal(one[0], c[r]), f"row {r}"
+    assert status.item() == 0
+
+
+@pytest.mark.parametrize("counts", [[3, 0, 66, 1, 0], [0] * 19 + [16] + [0] * 20, [1, 130, 0, 5], [64, 65, 63, 1, 200]])
+def test_grouped(counts):
+    n, k, rows = 300, 324, sum(counts)
+    groups = len(counts)
+    offsets = torch.tensor(np.concatenate([[0], np.cumsum(counts)]), dtype=torch.int32, device=DEV)
+    src, w, status = rnd(50, k), rnd(groups, n, k, seed=1), torch.zeros(1, dtype=torch.int32, device=DEV)
+    a_rows = torch.tensor(np.random.default_rng(0).integers(0, 50, rows), dtype=torch.int32, device=DEV)
+    scale, c = rnd(rows, seed=2), torch.full((rows + 3, n), 7.0, device=DEV)
+    ops.gemm_split(src, w, c, status, a_rows=a_rows, row_scale=scale, group_offsets=offsets, rows=rows)
+    assert status.item() == 0 and torch.all(c[rows:] == 7.0)
+    at, one = 0, torch.empty(1, n, device=DEV)
+    for g, count in enumerate(counts):
+        for r in range(at, at + count):
+            if r % 9 == 0 or r == at or r == at + count - 1:
+                row = a_rows[r].item()
+                ops.gemm_split(src[row:row + 1], w[g], one, status)
+                check(one, src[row:row + 1], w[g], f"row {r}")
+                assert torch.equal(one[0] * scale[r], c[r]), f"row {r}"
+        at += count
+
+
+def test_infinities_nans_and_the_largest_numbers():
+    """They would spread through the pieces: such elements are the chain's, the others stay as they were."""
+    m, n, k = 70, 260, 512
+    a, w, status = rnd(m, k), rnd(n, k, seed=1), torch.zeros(1, dtype=torch.int32, device=DEV)
+    plain = torch.empty(m, n, device=DEV)
+    ops.gemm_split(a, w, plain, status)
+    a[3, 5], a[4, 7], a[66, 500] = float("inf"), float("nan"), 3.4e38
+    a[5] = 0.0
+    w[9, 5], w[11, 100], w[255, 3] = 0.0, -float("inf"), 3.4e38
+    c, chain = torch.empty(m, n, device=DEV), torch.empty(m, n, device=DEV)
+    ops.gemm_split(a, w, c, status)
+    ops.gemm_simt(a, w, chain)
+    odd = torch.zeros(m, n, dtype=torch.bool, device=DEV)
+    odd[[3, 4, 66]], odd[:, [11, 255]] = True, True
+    odd[:, 9], odd[5] = True, True                                    # operands that changed
+    assert torch.equal(c[~odd], plain[~odd])
+    assert torch.equal(c.isnan(), chain.isnan()) and torch.equal(c.isinf(), chain.isinf())
+    odd = ~chain.isfinite() | ~c.isfinite()
+    assert torch.equal(c[odd & ~chain.isnan()], chain[odd & ~chain.isnan()])
+    assert c[3, 9].isnan() and c[3, 20].isinf() and (c[5, 20] == 0).item()
+
+
+def test_refusals():
+    status = torch.zeros(1, dtype=torch.int32, device=DEV)
+    c = torch.zeros(4, 128, device=DEV)
+    with pytest.raises(Exception, match="refused"):
+        ops.gemm_split(rnd(4, 258), rnd(128, 258), c, status)          # rows that do not start on 16 bytes
+    with pytest.raises(Exception, match="float32"):
+        ops.gemm_split(rnd(4, 256).bfloat16(), rnd(128, 256), c, status)
+    assert not ops.gemm_split_fits(rnd(4, 258), rnd(128, 258)) and ops.gemm_split_fits(rnd(4, 2048), rnd(2048, 2048))
+    assert torch.all(c == 0)
