@@ -156,6 +156,27 @@ __device__ __forceinline__ void st_cluster(float* p, unsigned rank, float v) {
     asm volatile("st.shared::cluster.f32 [%0], %1;\n" ::"r"(there), "f"(v) : "memory");
 }
 
+#ifndef SPLIT_SPIN
+#define SPLIT_SPIN 1
+#endif
+// A bounded wait that asks without being put to sleep at first.
+__device__ __forceinline__ bool wait_now(void* bar, unsigned parity) {
+    if (SPLIT_SPIN >= 1) {
+        const unsigned addr = smem_u32(bar);
+        for (int i = 0; i < 256; i++) {
+            unsigned done;
+            asm volatile(
+                "{\n.reg .pred p;\n"
+                "mbarrier.test_wait.parity.shared::cta.b64 p, [%1], %2;\n"
+                "selp.u32 %0, 1, 0, p;\n}\n"
+                : "=r"(done) : "r"(addr), "r"(parity) : "memory");
+            if (done) return true;
+        }
+    }
+    return mbar_wait(bar, parity);
+}
+__device__ __forceinline__ bool wait_soon(void* bar, unsigned parity) { return SPLIT_SPIN >= 2 ? wait_now(bar, parity) : mbar_wait(bar, parity); }
+
 // One element as a chain of fused multiply-adds.
 __device__ __noinline__ float chain(const float* a, const float* w, int K) {
     float s = 0.f;
@@ -225,7 +246,10 @@ __global__ void __launch_bounds__(THREADS, 1) gemm_split_kernel(const __grid_con
             while (!more && walk.next(t)) more = it < (end += stages);
             if (!more) break;
             const int s = it % NS, r = it % NR;
-            ok = mbar_wait(&raw_full[r], (it / NR) & 1) && !abort_flag;
+            // With an odd ring the groups take a slot in turn: a wait for this use of it means something only once the other group's
+            // use before has completed (a parity says no more than which of two neighbouring phases is over).
+            if (NR % 2 && it >= NR) ok = wait_soon(&raw_full[r], (it / NR - 1) & 1);
+            if (ok) ok = wait_soon(&raw_full[r], (it / NR) & 1) && !abort_flag;
             if (!ok) break;
             const unsigned char* stage = raw + r * RAW_BYTES + from;
             const unsigned at = lanes + D_COLS + s * A_COLS;
@@ -237,7 +261,7 @@ __global__ void __launch_bounds__(THREADS, 1) gemm_split_kernel(const __grid_con
 #pragma unroll
                     for (int i = 0; i < 4; i++) v[j][i] = *reinterpret_cast<const float4*>(stage + (2 * two + j) * (BF * 64) + i * 512);
                 if (two == 0) {
-                    if (it >= NS) ok = mbar_wait(&empty[s], (it / NS - 1) & 1) && !abort_flag;     // its last contents have been multiplied
+                    if (it >= NS) ok = wait_soon(&empty[s], (it / NS - 1) & 1) && !abort_flag;     // its last contents have been multiplied
                     tc_fence_after();
                 }
                 if (!ok) break;
@@ -351,7 +375,7 @@ __global__ void __launch_bounds__(THREADS, 1) gemm_split_kernel(const __grid_con
         load();
         for (int it = 0; n_tok > 0; it++) {
             const int s = it % NS;
-            if (it >= NS) ok = mbar_wait(&empty[s], (it / NS - 1) & 1) && !abort_flag;
+            if (it >= NS) ok = wait_soon(&empty[s], (it / NS - 1) & 1) && !abort_flag;
             if (!ok) break;
             const int n = n_tok;
             unsigned char* base = smem + s * T_BYTES;
@@ -406,8 +430,8 @@ __global__ void __launch_bounds__(THREADS, 1) gemm_split_kernel(const __grid_con
             int in_seg = 0;
             for (int st = 0; st < stages; st++, it++) {
                 const int s = it % NS;
-                if (in_seg == 0 && seg >= ND) ok = mbar_wait(&acc_empty[seg % ND], (seg / ND - 1) & 1);
-                if (ok) ok = mbar_wait(&full[s], (it / NS) & 1) && !abort_flag;
+                if (in_seg == 0 && seg >= ND) ok = wait_now(&acc_empty[seg % ND], (seg / ND - 1) & 1);
+                if (ok) ok = wait_now(&full[s], (it / NS) & 1) && !abort_flag;
                 if (!ok) break;
                 tc_fence_after();
                 const unsigned d = tmem + seg % ND * 3 * NT, a0 = tmem + D_COLS + s * A_COLS;

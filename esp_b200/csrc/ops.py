@@ -230,7 +230,7 @@ def _ptr(t, dtype=None, what="tensor"):
 
 _F32, _BF16 = torch.float32, torch.bfloat16
 FLOATS = (_F32, _BF16)
-SPLIT_MIN_K, SPLIT_MIN_N = 256, 128
+SPLIT_MIN_K, SPLIT_MIN_ELEMENTS = 1024, 2 << 20
 
 
 def _is_bf16(t) -> int:
@@ -357,7 +357,7 @@ def gemm_split_fits(a, w) -> bool:
     """Whether the 32-bit product ``a @ w.T`` (w [N, K] or [G, N, K]) is one for ``gemm_split``.  Asks for nothing that differs between
     the rows of a model's calls, so that a row takes the same kernel in every call."""
     k = w.shape[-1]
-    return (a.dtype is _F32 and w.dtype is _F32 and k >= SPLIT_MIN_K and w.shape[-2] >= SPLIT_MIN_N and k % 4 == 0
+    return (a.dtype is _F32 and w.dtype is _F32 and k >= SPLIT_MIN_K and w.shape[-2] * k >= SPLIT_MIN_ELEMENTS and k % 4 == 0
             and a.stride(0) % 4 == 0 and a.data_ptr() % 16 == 0 and w.data_ptr() % 16 == 0)
 
 
