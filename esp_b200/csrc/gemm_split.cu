@@ -10,8 +10,8 @@
 // rounded addition.  The order of everything depends on k alone, so a row's result has the same bits whatever other rows
 // are in the call, whatever the tile's width, whichever group the rows lie in and however many CTAs share a tile.
 // Error against 64 bits (2-norm, normal operands), this kernel / a chain of multiply-adds: K = 300 2.2e-7 / 3.1e-7, 512 2.4e-7 /
-// 4.1e-7, 1,024 4.7e-7 / 5.7e-7, 2,048 4.7e-7 / 8.1e-7, 5,632 4.8e-7 / 1.34e-6.  That is what sets the segments: with 512 k to a
-// segment K = 512 would be at 4.7e-7.
+// 4.1e-7, 1,024 4.7e-7 / 5.7e-7, 2,048 4.7e-7 / 8.1e-7.  That is what sets the segments: with 512 k to a segment K = 512 would be at
+// 4.7e-7; K = 5,632 4.8e-7 / 1.34e-6 with 512 k to a segment, twice that with 1,024.
 //
 // Layout: the weights are the 128-row side of the MMA, up to NT token rows its N side; accumulator D[feature, token],
 // TMEM lane = feature, columns [main | c1 | c2] of n_tok each.  A ring of stages of 64 k: the weights come by TMA into shared
@@ -41,8 +41,9 @@ constexpr int BF = 128;                    // weight rows (features) of a tile
 constexpr int KS = 64;                     // k of a stage: four 16-wide MMA steps, 128 bytes of a token row's piece
 constexpr int A_COLS = 3 * KS / 2;         // TMEM columns of a stage of weights
 constexpr int RAW_BYTES = BF * KS * 4;     // the same as it comes: [4 steps][128 rows][16 k] float
-constexpr int MAX_PARTS = 12;              // segments of a tile that several CTAs share
-constexpr int SHORT_SEGMENT = 256, LONG_SEGMENT = 512, LONG_K = 1024;
+constexpr int MAX_PARTS = 9;               // segments of a tile that several CTAs share
+// k of a segment: 256, from K = 1,024 on 512, from K = 4,096 on 1,024
+__host__ __device__ constexpr int segment_of(int K) { return K >= 4096 ? 1024 : K >= 1024 ? 512 : 256; }
 constexpr int W_WARPS = 8, E_WARPS = 8, T_WARPS = 6;     // with the one that issues the copies and the one that issues the MMAs: 24 warps
 constexpr int T_ROWS = T_WARPS * 4;        // token rows that the T_WARPS take at once, eight threads a row
 constexpr int THREADS = (W_WARPS + E_WARPS + T_WARPS + 2) * 32;
@@ -201,6 +202,9 @@ __global__ void __launch_bounds__(THREADS, 1) gemm_split_kernel(const __grid_con
     constexpr int T_BYTES = 3 * NT * KS * 2;
     constexpr int RUNS = (NT / 16 + 1) / 2;                          // runs of 16 tokens that a warp reads out
     static_assert(3 * NT <= 256 && D_COLS + NS * A_COLS <= 512, "tensor memory");
+    // A group waits for every second stage.  A wait tells a phase from its neighbours only, so each group must have waited for the use of
+    // the slot before this one, which an even ring gives.
+    static_assert(NR % 2 == 0, "each slot belongs to one group");
     static_assert(!SHARED || NT == 16, "a shared tile is one run of 16 tokens");
     extern __shared__ unsigned char smem_raw[];
     unsigned char* smem = reinterpret_cast<unsigned char*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~(uintptr_t)1023);
@@ -246,10 +250,7 @@ __global__ void __launch_bounds__(THREADS, 1) gemm_split_kernel(const __grid_con
             while (!more && walk.next(t)) more = it < (end += stages);
             if (!more) break;
             const int s = it % NS, r = it % NR;
-            // With an odd ring the groups take a slot in turn: a wait for this use of it means something only once the other group's
-            // use before has completed (a parity says no more than which of two neighbouring phases is over).
-            if (NR % 2 && it >= NR) ok = wait_soon(&raw_full[r], (it / NR - 1) & 1);
-            if (ok) ok = wait_soon(&raw_full[r], (it / NR) & 1) && !abort_flag;
+            ok = wait_soon(&raw_full[r], (it / NR) & 1) && !abort_flag;
             if (!ok) break;
             const unsigned char* stage = raw + r * RAW_BYTES + from;
             const unsigned at = lanes + D_COLS + s * A_COLS;
@@ -545,19 +546,22 @@ ESP_API int esp_gemm_split(const void* A, const int* a_rows, const void* W, cons
     if (M <= 0 || N <= 0) return 0;
     if (K <= 0 || K % 4 != 0 || lda % 4 != 0 || ((uintptr_t)A & 15) || ((uintptr_t)W & 15) || groups < 1) return (int)cudaErrorInvalidValue;
     SplitParams p{(const float*)A, a_rows, (const float*)W, bias, row_scale, (float*)C, group_offsets, groups, M, N, K, lda, ldc,
-                  (K >= LONG_K ? LONG_SEGMENT : SHORT_SEGMENT) / KS, 1, status};
+                  segment_of(K) / KS, 1, status};
     int dev = 0, sms = 0;
     cudaError_t e = cudaGetDevice(&dev);
     if (e == cudaSuccess) e = cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
     if (e != cudaSuccess) return (int)e;
     if (!group_offsets) {
         // Few tiles of 16 rows: as many CTAs to each as there are SMs for (6 rows, K = 2,048: N = 2,048 31 us with a CTA a tile, 12 with
-        // four; N = 6,144 31 and 21 with two; K = 5,632, N = 2,048 76 and 38.  64 rows: N = 2,048 22 us, tiles of 64 rows 36)
+        // four; N = 6,144 31 and 21 with two.  64 rows: N = 2,048 22 us, tiles of 64 rows 36).  Clusters of eight did not all find room at once
         const long long tiles = (long long)((M + 15) / 16) * ((N + BF - 1) / BF);
         const int segments = ((K + KS - 1) / KS + p.seg_stages - 1) / p.seg_stages;
-        while (p.share < 8 && tiles * p.share * 2 <= sms && p.share * 2 <= segments) p.share *= 2;
-        if (segments > MAX_PARTS) p.share = 1;
-        if (p.share > 1) return launch<16, 2, 4, 3, true>(p, sms, stream);
+        const long long most = segments > MAX_PARTS ? 1 : min(min(6ll, (long long)segments), sms / tiles);
+        if (most > 1) {
+            const int each = (segments + (int)most - 1) / (int)most;     // segments of a CTA at most
+            p.share = (segments + each - 1) / each;
+        }
+        if (p.share > 1) return launch<16, 2, 3, 4, true>(p, sms, stream);
     }
     // few rows, of a group four on average: a short tile leaves tensor memory for two sets of accumulators
     if (M <= (group_offsets ? 4ll * groups : 16ll)) return launch<16, 2, 4, 6, false>(p, sms, stream);

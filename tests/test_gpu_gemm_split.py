@@ -24,8 +24,8 @@ def check(c, a, w, what):
 
 @pytest.mark.parametrize("m, n, k", [
     (1, 128, 256), (15, 300, 260),     # one run of 16 rows; features and k that end inside a tile and a stage
-    (16, 2048, 2048), (17, 130, 1028),  # tiles shared by clusters of four and two CTAs, two runs of rows
-    (33, 2048, 5632), (3, 640, 6660),  # by eight CTAs; more segments than are shared
+    (16, 2048, 2048), (17, 130, 1028), (6, 6144, 2048),  # tiles shared by clusters of four, three and two CTAs, two runs of rows
+    (33, 2048, 5632), (3, 640, 9300), (2, 200, 4100),   # of three; more segments than are shared; of five
     (16, 19000, 512), (64, 9600, 300),  # a CTA a tile: short tiles, several a CTA; one full run of 64 rows
     (65, 11264, 516), (200, 2304, 1100), (389, 1300, 256),   # uneven runs of rows
 ])
