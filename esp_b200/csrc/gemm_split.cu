@@ -157,27 +157,6 @@ __device__ __forceinline__ void st_cluster(float* p, unsigned rank, float v) {
     asm volatile("st.shared::cluster.f32 [%0], %1;\n" ::"r"(there), "f"(v) : "memory");
 }
 
-#ifndef SPLIT_SPIN
-#define SPLIT_SPIN 1
-#endif
-// A bounded wait that asks without being put to sleep at first.
-__device__ __forceinline__ bool wait_now(void* bar, unsigned parity) {
-    if (SPLIT_SPIN >= 1) {
-        const unsigned addr = smem_u32(bar);
-        for (int i = 0; i < 256; i++) {
-            unsigned done;
-            asm volatile(
-                "{\n.reg .pred p;\n"
-                "mbarrier.test_wait.parity.shared::cta.b64 p, [%1], %2;\n"
-                "selp.u32 %0, 1, 0, p;\n}\n"
-                : "=r"(done) : "r"(addr), "r"(parity) : "memory");
-            if (done) return true;
-        }
-    }
-    return mbar_wait(bar, parity);
-}
-__device__ __forceinline__ bool wait_soon(void* bar, unsigned parity) { return SPLIT_SPIN >= 2 ? wait_now(bar, parity) : mbar_wait(bar, parity); }
-
 // One element as a chain of fused multiply-adds.
 __device__ __noinline__ float chain(const float* a, const float* w, int K) {
     float s = 0.f;
@@ -196,10 +175,13 @@ __device__ __forceinline__ void store(const SplitParams& p, const Tile& t, int r
 // NT: token rows of a tile at most; ND: sets of accumulators, which the segments take in turn; NS: stages of the ring of split
 // operands, NR: of the ring of weights as they come.  SHARED: the CTAs of a cluster take a tile's segments in equal runs, and the
 // first of them adds the segments' sums in order.
-template <int NT, int ND, int NS, int NR, bool SHARED>
+template <int NT, int ND, int NS, int NR, int G, bool SHARED>
 __global__ void __launch_bounds__(THREADS, 1) gemm_split_kernel(const __grid_constant__ CUtensorMap map_w, SplitParams p) {
     constexpr int D_COLS = ND * 3 * NT;
     constexpr int T_BYTES = 3 * NT * KS * 2;
+    // G stages share their mbarriers.  A tile then has a whole number of them; stages behind K are zeros.
+    constexpr int SLOTS = NS / G;
+    static_assert(NS % G == 0, "whole slots");
     constexpr int RUNS = (NT / 16 + 1) / 2;                          // runs of 16 tokens that a warp reads out
     static_assert(3 * NT <= 256 && D_COLS + NS * A_COLS <= 512, "tensor memory");
     // A group waits for every second stage.  A wait tells a phase from its neighbours only, so each group must have waited for the use of
@@ -210,12 +192,12 @@ __global__ void __launch_bounds__(THREADS, 1) gemm_split_kernel(const __grid_con
     unsigned char* smem = reinterpret_cast<unsigned char*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~(uintptr_t)1023);
     unsigned char* raw = smem + NS * T_BYTES;
     float* parts = reinterpret_cast<float*>(raw + NR * RAW_BYTES);   // SHARED, first CTA: [segment][16 rows][128 features]
-    __shared__ __align__(8) unsigned long long full[NS], empty[NS], raw_full[NR], raw_empty[NR], acc_full[ND], acc_empty[ND];
+    __shared__ __align__(8) unsigned long long full[SLOTS], empty[SLOTS], raw_full[NR], raw_empty[NR], acc_full[ND], acc_empty[ND];
     __shared__ unsigned tmem_slot;
     __shared__ volatile int abort_flag;
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     if (threadIdx.x == 0) {
-        for (int i = 0; i < NS; i++) mbar_init(&full[i], W_WARPS / 2 + T_WARPS), mbar_init(&empty[i], 1);
+        for (int i = 0; i < SLOTS; i++) mbar_init(&full[i], G * (W_WARPS / 2 + T_WARPS)), mbar_init(&empty[i], 1);
         for (int i = 0; i < NR; i++) mbar_init(&raw_full[i], 1), mbar_init(&raw_empty[i], W_WARPS / 2);
         for (int i = 0; i < ND; i++) mbar_init(&acc_full[i], 1), mbar_init(&acc_empty[i], E_WARPS);
         abort_flag = 0;
@@ -230,7 +212,7 @@ __global__ void __launch_bounds__(THREADS, 1) gemm_split_kernel(const __grid_con
     if (SHARED) cluster_sync();                                      // the first CTA runs before anything is written to its memory
     tc_fence_after();
     const unsigned tmem = tmem_slot;
-    const int all_stages = (p.K + KS - 1) / KS, segments = (all_stages + p.seg_stages - 1) / p.seg_stages;
+    const int all_stages = (p.K + G * KS - 1) / (G * KS) * G, segments = (all_stages + p.seg_stages - 1) / p.seg_stages;
     const int rank = SHARED ? (int)(blockIdx.x % p.share) : 0;
     const int seg0 = SHARED ? rank * segments / p.share : 0, seg1 = SHARED ? (rank + 1) * segments / p.share : segments;
     const int stage0 = seg0 * p.seg_stages, stages = min(all_stages, seg1 * p.seg_stages) - stage0;      // of this CTA, of every tile
@@ -249,8 +231,8 @@ __global__ void __launch_bounds__(THREADS, 1) gemm_split_kernel(const __grid_con
             bool more = it < end;
             while (!more && walk.next(t)) more = it < (end += stages);
             if (!more) break;
-            const int s = it % NS, r = it % NR;
-            ok = wait_soon(&raw_full[r], (it / NR) & 1) && !abort_flag;
+            const int s = it % NS, use = it / G / SLOTS, slot = it / G % SLOTS, r = it % NR;
+            ok = mbar_wait(&raw_full[r], (it / NR) & 1) && !abort_flag;
             if (!ok) break;
             const unsigned char* stage = raw + r * RAW_BYTES + from;
             const unsigned at = lanes + D_COLS + s * A_COLS;
@@ -262,7 +244,7 @@ __global__ void __launch_bounds__(THREADS, 1) gemm_split_kernel(const __grid_con
 #pragma unroll
                     for (int i = 0; i < 4; i++) v[j][i] = *reinterpret_cast<const float4*>(stage + (2 * two + j) * (BF * 64) + i * 512);
                 if (two == 0) {
-                    if (it >= NS) ok = wait_soon(&empty[s], (it / NS - 1) & 1) && !abort_flag;     // its last contents have been multiplied
+                    if (use > 0) ok = mbar_wait(&empty[slot], (use - 1) & 1) && !abort_flag;     // its last contents have been multiplied
                     tc_fence_after();
                 }
                 if (!ok) break;
@@ -286,7 +268,7 @@ __global__ void __launch_bounds__(THREADS, 1) gemm_split_kernel(const __grid_con
             tc_fence_before();
             __syncwarp();
             if (lane == 0) {
-                mbar_arrive(&full[s]);
+                mbar_arrive(&full[slot]);
                 mbar_arrive(&raw_empty[r]);
             }
         }
@@ -375,8 +357,8 @@ __global__ void __launch_bounds__(THREADS, 1) gemm_split_kernel(const __grid_con
         };
         load();
         for (int it = 0; n_tok > 0; it++) {
-            const int s = it % NS;
-            if (it >= NS) ok = wait_soon(&empty[s], (it / NS - 1) & 1) && !abort_flag;
+            const int s = it % NS, use = it / G / SLOTS, slot = it / G % SLOTS;
+            if (it % G == 0 && use > 0) ok = mbar_wait(&empty[slot], (use - 1) & 1) && !abort_flag;
             if (!ok) break;
             const int n = n_tok;
             unsigned char* base = smem + s * T_BYTES;
@@ -398,7 +380,7 @@ __global__ void __launch_bounds__(THREADS, 1) gemm_split_kernel(const __grid_con
             load();
             fence_async_smem();
             __syncwarp();
-            if (lane == 0) mbar_arrive(&full[s]);
+            if (lane == 0) mbar_arrive(&full[slot]);
         }
     } else if (warp == W_WARPS + E_WARPS + T_WARPS) {
         // weights as they come: four boxes of 128 rows x 16 k a stage, a lane each
@@ -429,24 +411,29 @@ __global__ void __launch_bounds__(THREADS, 1) gemm_split_kernel(const __grid_con
             const int n = t.n_tok;
             const unsigned d_three = split_idesc(3 * n), d_two = split_idesc(2 * n), d_one = split_idesc(n);
             int in_seg = 0;
-            for (int st = 0; st < stages; st++, it++) {
-                const int s = it % NS;
-                if (in_seg == 0 && seg >= ND) ok = wait_now(&acc_empty[seg % ND], (seg / ND - 1) & 1);
-                if (ok) ok = wait_now(&full[s], (it / NS) & 1) && !abort_flag;
+            for (int st = 0; st < stages; st += G, it += G) {
+                const int use = it / G / SLOTS, slot = it / G % SLOTS;
+                if (in_seg == 0 && seg >= ND) ok = mbar_wait(&acc_empty[seg % ND], (seg / ND - 1) & 1);
+                if (ok) ok = mbar_wait(&full[slot], use & 1) && !abort_flag;
                 if (!ok) break;
                 tc_fence_after();
-                const unsigned d = tmem + seg % ND * 3 * NT, a0 = tmem + D_COLS + s * A_COLS;
-                const unsigned long long b0 = desc0 + (unsigned)((s * T_BYTES) >> 4);
+                const unsigned d = tmem + seg % ND * 3 * NT;
 #pragma unroll
-                for (int j = 0; j < KS / 16; j++) {
-                    const unsigned a = a0 + 8 * j;
-                    const unsigned long long b = b0 + 2 * j;
-                    tc_mma_ta(d, a, b, d_three, in_seg == 0 && j == 0 ? 0u : 1u);             // main, c1, c2
-                    tc_mma_ta(d + n, a + KS / 2, b, d_two, 1u);                               // c1, c2
-                    tc_mma_ta(d + 2 * n, a + KS, b, d_one, 1u);                               // c2
+                for (int g = 0; g < G; g++) {
+                    const unsigned a0 = tmem + D_COLS + (slot * G + g) * A_COLS;
+                    const unsigned long long b0 = desc0 + (unsigned)(((slot * G + g) * T_BYTES) >> 4);
+#pragma unroll
+                    for (int j = 0; j < KS / 16; j++) {
+                        const unsigned a = a0 + 8 * j;
+                        const unsigned long long b = b0 + 2 * j;
+                        tc_mma_ta(d, a, b, d_three, in_seg == 0 && g == 0 && j == 0 ? 0u : 1u);   // main, c1, c2
+                        tc_mma_ta(d + n, a + KS / 2, b, d_two, 1u);                               // c1, c2
+                        tc_mma_ta(d + 2 * n, a + KS, b, d_one, 1u);                               // c2
+                    }
                 }
-                tc_commit(&empty[s]);
-                if (++in_seg == p.seg_stages || st + 1 == stages) {
+                tc_commit(&empty[slot]);
+                in_seg += G;
+                if (in_seg == p.seg_stages || st + G == stages) {
                     tc_commit(&acc_full[seg % ND]);
                     in_seg = 0;
                     seg++;
@@ -506,18 +493,22 @@ int map_weights(CUtensorMap* map, const SplitParams& p) {
     return r == CUDA_SUCCESS ? 0 : (int)cudaErrorInvalidValue;
 }
 
-template <int NT, int ND, int NS, int NR, bool SHARED>
+// runs of at most ``nt`` rows; of groups an upper bound
+long long row_runs(const SplitParams& p, int nt) {
+    return p.group_offsets ? p.M / nt + (p.groups < p.M ? p.groups : p.M) : (p.M + nt - 1) / nt;
+}
+
+template <int NT, int ND, int NS, int NR, int G, bool SHARED>
 int launch(SplitParams p, int sms, cudaStream_t stream) {
     constexpr int SMEM = NS * 3 * NT * KS * 2 + NR * RAW_BYTES + (SHARED ? MAX_PARTS * 16 * BF * 4 : 0) + 1024;
     static_assert(SMEM <= 231 * 1024 - 512, "shared memory");
     CUtensorMap map;
     const int rc = map_weights(&map, p);
     if (rc) return rc;
-    const auto kernel = gemm_split_kernel<NT, ND, NS, NR, SHARED>;
+    const auto kernel = gemm_split_kernel<NT, ND, NS, NR, G, SHARED>;
     const cudaError_t e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, SMEM);
     if (e != cudaSuccess) return (int)e;
-    const long long runs = p.group_offsets ? p.M / NT + (p.groups < p.M ? p.groups : p.M) : (p.M + NT - 1) / NT;       // of groups: an upper bound
-    const long long tiles = runs * ((p.N + BF - 1) / BF);
+    const long long tiles = row_runs(p, NT) * ((p.N + BF - 1) / BF);
     if (tiles + sms > 0x3fffffffll) return (int)cudaErrorInvalidValue;
     cudaLaunchConfig_t cfg = {};
     cfg.gridDim = dim3((unsigned)(SHARED ? tiles * p.share : tiles < sms ? tiles : sms));
@@ -551,19 +542,25 @@ ESP_API int esp_gemm_split(const void* A, const int* a_rows, const void* W, cons
     cudaError_t e = cudaGetDevice(&dev);
     if (e == cudaSuccess) e = cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
     if (e != cudaSuccess) return (int)e;
-    if (!group_offsets) {
+    {
         // Few tiles of 16 rows: as many CTAs to each as there are SMs for (6 rows, K = 2,048: N = 2,048 31 us with a CTA a tile, 12 with
         // four; N = 6,144 31 and 21 with two.  64 rows: N = 2,048 22 us, tiles of 64 rows 36).  Clusters of eight did not all find room at once
-        const long long tiles = (long long)((M + 15) / 16) * ((N + BF - 1) / BF);
+        const long long tiles = row_runs(p, 16) * ((N + BF - 1) / BF);
         const int segments = ((K + KS - 1) / KS + p.seg_stages - 1) / p.seg_stages;
         const long long most = segments > MAX_PARTS ? 1 : min(min(6ll, (long long)segments), sms / tiles);
         if (most > 1) {
             const int each = (segments + (int)most - 1) / (int)most;     // segments of a CTA at most
             p.share = (segments + each - 1) / each;
         }
-        if (p.share > 1) return launch<16, 2, 3, 4, true>(p, sms, stream);
+        if (p.share > 1) return launch<16, 2, 4, 4, 1, true>(p, sms, stream);
     }
-    // few rows, of a group four on average: a short tile leaves tensor memory for two sets of accumulators
-    if (M <= (group_offsets ? 4ll * groups : 16ll)) return launch<16, 2, 4, 6, false>(p, sms, stream);
-    return launch<64, 1, 3, 4, false>(p, sms, stream);
+    // Few rows, of a group four on average: a short tile leaves tensor memory for two sets of accumulators.  A wait and a commit keep
+    // the issuing thread 300 and 90 cycles, a third of its time where the MMAs are short: groups, and a tile a CTA, have two stages behind
+    // one of each (100 rows over 60 groups, N = 2,816: 223 -> 192 us; one row, N = 11,264 29.7 -> 26.7).  Many tiles a CTA of one matrix,
+    // which memory bounds, are better off with the finer ring (6 rows, N = 151,936: 230 us against 245).
+    if (M <= (group_offsets ? 4ll * groups : 16ll)) {
+        if (group_offsets || (N + BF - 1) / BF <= sms) return launch<16, 2, 4, 6, 2, false>(p, sms, stream);
+        return launch<16, 2, 4, 6, 1, false>(p, sms, stream);
+    }
+    return launch<64, 1, 3, 4, 1, false>(p, sms, stream);
 }
