@@ -41,7 +41,8 @@ constexpr int BF = 128;                    // weight rows (features) of a tile
 constexpr int KS = 64;                     // k of a stage: four 16-wide MMA steps, 128 bytes of a token row's piece
 constexpr int A_COLS = 3 * KS / 2;         // TMEM columns of a stage of weights
 constexpr int RAW_BYTES = BF * KS * 4;     // the same as it comes: [4 steps][128 rows][16 k] float
-constexpr int MAX_PARTS = 9;               // segments of a tile that several CTAs share
+constexpr int MAX_GROUPS = 256;
+constexpr int MAX_PARTS = 8;               // segments of a tile that several CTAs share
 // k of a segment: 256, from K = 1,024 on 512, from K = 4,096 on 1,024
 __host__ __device__ constexpr int segment_of(int K) { return K >= 4096 ? 1024 : K >= 1024 ? 512 : 256; }
 constexpr int W_WARPS = 8, E_WARPS = 8, T_WARPS = 6;     // with the one that issues the copies and the one that issues the MMAs: 24 warps
@@ -66,48 +67,74 @@ struct Tile {
     int group, m0, rows, n_tok, f0;        // n_tok: rows rounded up to 16
 };
 
+// A group that has rows, and the number of tiles of the groups before it.
+struct Group {
+    int group, begin, rows, before;
+};
+template <int NT> __device__ __forceinline__ int runs_of(int rows) { return (rows + NT - 1) / NT; }
+
+// Lists the groups that have rows in shared memory (one warp).  Every role of a CTA walks this list, some several times: looked up in
+// the offsets one by one, 60 groups took a role 2 us at the start of its first tile and again behind its last one.
+template <int NT>
+__device__ __forceinline__ void list_groups(const SplitParams& p, Group* list, int* count) {
+    const int lane = threadIdx.x & 31, feat_tiles = (p.N + BF - 1) / BF;
+    if (!p.group_offsets) {
+        if (lane == 0) list[0] = Group{0, 0, p.M, 0}, *count = 1;
+        return;
+    }
+    int at = 0, before = 0;
+    for (int g0 = 0; g0 < p.groups; g0 += 128) {
+        int begin[4], rows[4];
+#pragma unroll
+        for (int r = 0; r < 4; r++) {
+            const int g = g0 + 32 * r + lane;
+            begin[r] = g < p.groups ? p.group_offsets[g] : 0;
+            rows[r] = g < p.groups ? min(p.M, p.group_offsets[g + 1]) - begin[r] : 0;
+        }
+#pragma unroll
+        for (int r = 0; r < 4; r++) {
+            const unsigned some = __ballot_sync(0xffffffffu, rows[r] > 0);
+            const int tiles = rows[r] > 0 ? runs_of<NT>(rows[r]) * feat_tiles : 0;
+            int upto = tiles;
+#pragma unroll
+            for (int o = 1; o < 32; o <<= 1) {
+                const int v = __shfl_up_sync(0xffffffffu, upto, o);
+                if (lane >= o) upto += v;
+            }
+            if (rows[r] > 0) list[at + __popc(some & ((1u << lane) - 1))] = Group{g0 + 32 * r + lane, begin[r], rows[r], before + upto - tiles};
+            at += __popc(some);
+            before += __shfl_sync(0xffffffffu, upto, 31);
+        }
+    }
+    if (lane == 0) *count = at;
+}
+
 // Walks the tiles of a CTA (or of the ``share`` CTAs of a cluster) in order.  A group's rows are cut evenly into ceil(rows / NT)
 // runs; its tiles are all runs of the first 128 features, then of the next (neighbours share their weights).
 template <int NT>
 struct Walk {
-    const SplitParams& p;
-    int feat_tiles, tile, step, group, begin, runs, width, rows;
-    int before;                            // tiles of the groups before
-    __device__ __forceinline__ Walk(const SplitParams& p_) : p(p_) {
+    const Group* list;
+    int count, feat_tiles, tile, step, at;
+    __device__ __forceinline__ Walk(const SplitParams& p, const Group* list_, int count_) : list(list_), count(count_), at(0) {
         feat_tiles = (p.N + BF - 1) / BF;
         step = gridDim.x / p.share;
         tile = (int)(blockIdx.x / p.share) - step;
-        group = -1;
-        before = 0;
-        runs = 0;
     }
     __device__ __forceinline__ bool next(Tile& t) {
         tile += step;
-        while (group < 0 || tile >= before + runs * feat_tiles) {
-            if (group >= 0) before += runs * feat_tiles;
-            if (++group >= p.groups) {
-                group = p.groups - 1;      // stays behind the last one
-                before = 0, runs = 0;
-                return false;
-            }
-            int end = p.M;
-            begin = 0;
-            if (p.group_offsets) {
-                begin = p.group_offsets[group];
-                end = min(p.M, p.group_offsets[group + 1]);
-            }
-            rows = max(0, end - begin);
-            runs = (rows + NT - 1) / NT;
-            width = runs ? ((rows + runs - 1) / runs + 15) / 16 * 16 : 16;
+        for (; at < count; at++) {
+            const Group g = list[at];
+            const int runs = runs_of<NT>(g.rows), i = tile - g.before;
+            if (i >= runs * feat_tiles) continue;
+            const int width = ((g.rows + runs - 1) / runs + 15) / 16 * 16, run = i % runs;
+            t.group = g.group;
+            t.m0 = g.begin + run * width;
+            t.rows = min(width, g.rows - run * width);
+            t.n_tok = (t.rows + 15) / 16 * 16;
+            t.f0 = i / runs * BF;
+            return true;
         }
-        const int at = tile - before;
-        const int run = at % runs;
-        t.group = group;
-        t.m0 = begin + run * width;
-        t.rows = min(width, rows - run * width);
-        t.n_tok = (t.rows + 15) / 16 * 16;
-        t.f0 = at / runs * BF;
-        return true;
+        return false;
     }
 };
 
@@ -194,6 +221,8 @@ __global__ void __launch_bounds__(THREADS, 1) gemm_split_kernel(const __grid_con
     float* parts = reinterpret_cast<float*>(raw + NR * RAW_BYTES);   // SHARED, first CTA: [segment][16 rows][128 features]
     __shared__ __align__(8) unsigned long long full[SLOTS], empty[SLOTS], raw_full[NR], raw_empty[NR], acc_full[ND], acc_empty[ND];
     __shared__ unsigned tmem_slot;
+    __shared__ __align__(16) Group groups[MAX_GROUPS];
+    __shared__ int group_count;
     __shared__ volatile int abort_flag;
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     if (threadIdx.x == 0) {
@@ -207,8 +236,13 @@ __global__ void __launch_bounds__(THREADS, 1) gemm_split_kernel(const __grid_con
         asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;\n" ::"r"(smem_u32(&tmem_slot)), "r"(512));
         asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;\n" ::);
     }
+    if (warp == 0) {
+        if (p.group_offsets) pdl_wait();
+        list_groups<NT>(p, groups, &group_count);
+    }
     tc_fence_before();
     __syncthreads();
+    const int n_groups = group_count;
     if (SHARED) cluster_sync();                                      // the first CTA runs before anything is written to its memory
     tc_fence_after();
     const unsigned tmem = tmem_slot;
@@ -224,7 +258,7 @@ __global__ void __launch_bounds__(THREADS, 1) gemm_split_kernel(const __grid_con
         const unsigned lanes = tmem + ((unsigned)(quad * 32) << 16);
         const int from = (quad * 32 + (lane >> 2)) * 64 + (lane & 3) * 16;    // byte of the stage: eight lanes read 128 bytes in a row
         if (p.group_offsets) pdl_wait();
-        Walk<NT> walk(p);
+        Walk<NT> walk(p, groups, n_groups);
         Tile t;
         int end = 0;                                                 // stages of the tiles seen so far
         for (int it = half;; it += 2) {
@@ -277,7 +311,7 @@ __global__ void __launch_bounds__(THREADS, 1) gemm_split_kernel(const __grid_con
         const int quad = warp & 3, half = (warp - W_WARPS) >> 2;
         const unsigned lanes = tmem + ((unsigned)(quad * 32) << 16);
         pdl_wait();
-        Walk<NT> walk(p);
+        Walk<NT> walk(p, groups, n_groups);
         Tile o;
         int count = 0;                                               // segments read out so far
         while (ok && walk.next(o)) {
@@ -324,7 +358,7 @@ __global__ void __launch_bounds__(THREADS, 1) gemm_split_kernel(const __grid_con
         const int r0 = tid >> 3, part = tid & 7;
         constexpr int PASSES = (NT + T_ROWS - 1) / T_ROWS;
         pdl_wait();
-        Walk<NT> walk(p);
+        Walk<NT> walk(p, groups, n_groups);
         Tile t;
         float4 next[PASSES][2];
         const float* src[PASSES];
@@ -385,7 +419,7 @@ __global__ void __launch_bounds__(THREADS, 1) gemm_split_kernel(const __grid_con
     } else if (warp == W_WARPS + E_WARPS + T_WARPS) {
         // weights as they come: four boxes of 128 rows x 16 k a stage, a lane each
         if (p.group_offsets) pdl_wait();                             // whose weights are read follows from the offsets; of a dense product they are never written
-        Walk<NT> walk(p);
+        Walk<NT> walk(p, groups, n_groups);
         Tile t;
         int it = 0;
         while (ok && walk.next(t)) {
@@ -403,7 +437,7 @@ __global__ void __launch_bounds__(THREADS, 1) gemm_split_kernel(const __grid_con
     } else if (lane == 0) {
         pdl_wait();
         pdl_trigger();                                               // behind the wait: a dependent kernel may count on all before this one
-        Walk<NT> walk(p);
+        Walk<NT> walk(p, groups, n_groups);
         Tile t;
         const unsigned long long desc0 = smem_desc(smem);
         int it = 0, seg = 0;
@@ -452,7 +486,7 @@ __global__ void __launch_bounds__(THREADS, 1) gemm_split_kernel(const __grid_con
         // the segments' sums are with the first CTA, which adds them in order
         cluster_sync();
         if (rank == 0 && !abort_flag) {
-            Walk<NT> walk(p);
+            Walk<NT> walk(p, groups, n_groups);
             Tile o;
             const bool have = walk.next(o);
             for (int i = threadIdx.x; have && i < o.rows * BF; i += THREADS) {
@@ -501,7 +535,7 @@ long long row_runs(const SplitParams& p, int nt) {
 template <int NT, int ND, int NS, int NR, int G, bool SHARED>
 int launch(SplitParams p, int sms, cudaStream_t stream) {
     constexpr int SMEM = NS * 3 * NT * KS * 2 + NR * RAW_BYTES + (SHARED ? MAX_PARTS * 16 * BF * 4 : 0) + 1024;
-    static_assert(SMEM <= 231 * 1024 - 512, "shared memory");
+    static_assert(SMEM + 4096 + 512 <= 227 * 1024, "shared memory");
     CUtensorMap map;
     const int rc = map_weights(&map, p);
     if (rc) return rc;
@@ -530,12 +564,13 @@ int launch(SplitParams p, int sms, cudaStream_t stream) {
 }
 }  // namespace
 
-// All float.  K, lda multiples of 4, A and W on 16 bytes.
+// All float.  K, lda multiples of 4, A and W on 16 bytes, at most 256 groups.
 ESP_API int esp_gemm_split(const void* A, const int* a_rows, const void* W, const float* bias, const float* row_scale, void* C,
                            const int* group_offsets, int groups, int M, int N, int K, long long lda, long long ldc, int* status,
                            cudaStream_t stream) {
     if (M <= 0 || N <= 0) return 0;
-    if (K <= 0 || K % 4 != 0 || lda % 4 != 0 || ((uintptr_t)A & 15) || ((uintptr_t)W & 15) || groups < 1) return (int)cudaErrorInvalidValue;
+    if (K <= 0 || K % 4 != 0 || lda % 4 != 0 || ((uintptr_t)A & 15) || ((uintptr_t)W & 15) || groups < 1 || groups > MAX_GROUPS)
+        return (int)cudaErrorInvalidValue;
     SplitParams p{(const float*)A, a_rows, (const float*)W, bias, row_scale, (float*)C, group_offsets, groups, M, N, K, lda, ldc,
                   segment_of(K) / KS, 1, status};
     int dev = 0, sms = 0;

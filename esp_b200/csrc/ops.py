@@ -230,7 +230,7 @@ def _ptr(t, dtype=None, what="tensor"):
 
 _F32, _BF16 = torch.float32, torch.bfloat16
 FLOATS = (_F32, _BF16)
-SPLIT_MIN_K, SPLIT_MIN_ELEMENTS = 1024, 2 << 20
+SPLIT_MIN_K, SPLIT_MIN_ELEMENTS, SPLIT_MAX_GROUPS = 1024, 2 << 20, 256
 
 
 def _is_bf16(t) -> int:
@@ -358,7 +358,7 @@ def gemm_split_fits(a, w) -> bool:
     the rows of a model's calls, so that a row takes the same kernel in every call."""
     k = w.shape[-1]
     return (a.dtype is _F32 and w.dtype is _F32 and k >= SPLIT_MIN_K and w.shape[-2] * k >= SPLIT_MIN_ELEMENTS and k % 4 == 0
-            and a.stride(0) % 4 == 0 and a.data_ptr() % 16 == 0 and w.data_ptr() % 16 == 0)
+            and (w.dim() == 2 or w.shape[0] <= SPLIT_MAX_GROUPS) and a.stride(0) % 4 == 0 and a.data_ptr() % 16 == 0 and w.data_ptr() % 16 == 0)
 
 
 def gemm_split(a, w, c, status, bias=None, row_scale=None, a_rows=None, group_offsets=None, rows=None):

@@ -52,7 +52,7 @@ def test_dense(m, n, k):
     assert status.item() == 0
 
 
-@pytest.mark.parametrize("counts", [[3, 0, 66, 1, 0], [0] * 19 + [16] + [0] * 20, [1, 130, 0, 5], [64, 65, 63, 1, 200]])
+@pytest.mark.parametrize("counts", [[3, 0, 66, 1, 0], [0] * 19 + [16] + [0] * 20, [1, 130, 0, 5], [64, 65, 63, 1, 200], [0, 2] * 128, [1] + [0] * 140 + [17, 0, 3]])
 def test_grouped(counts):
     n, k, rows = 300, 324, sum(counts)
     groups = len(counts)
