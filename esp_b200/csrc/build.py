@@ -163,5 +163,71 @@ def load_library(name: str) -> ctypes.CDLL:
         return lib
 
 
+# ctypes type -> the letter of a signature and the C++ type (entry.cpp)
+_LETTERS = {ctypes.c_void_p: ("P", "void*"), ctypes.c_int: ("i", "int"), ctypes.c_longlong: ("q", "long long"),
+            ctypes.c_ulonglong: ("Q", "unsigned long long"), ctypes.c_float: ("f", "float")}
+
+
+def signature_letters(argtypes) -> str:
+    return "".join(_LETTERS[t][0] for t in argtypes)
+
+
+def build_entry(signatures: dict, verbose: bool = True) -> Path:
+    """Compiles ``entry.cpp``, the Python module that calls the entry points, with a typed call for every signature among
+    ``signatures`` (entry point -> ctypes argument types)."""
+    import sysconfig
+
+    import torch
+    out_dir = build_dir()
+    so = out_dir / "esp_b200_entry.so"
+    lines = sorted({f'{{"{signature_letters(a)}", call<{", ".join(_LETTERS[t][1] for t in a)}>}},' for a in map(tuple, signatures.values())})
+    torch_dir = Path(torch.__file__).resolve().parent
+    cmd = ["-std=c++17", "-O2", "-fPIC", "-shared", "-fvisibility=hidden", f"-D_GLIBCXX_USE_CXX11_ABI={int(torch._C._GLIBCXX_USE_CXX11_ABI)}"]
+    h = hashlib.sha256()
+    for part in (" ".join(cmd), torch.__version__, sys.version, *lines, (CSRC / "entry.cpp").read_text()):
+        h.update(part.encode())
+    want = h.hexdigest()
+    stamp_file = out_dir / "entry.stamp"
+    with open(out_dir / "entry.lock", "w") as lock:
+        fcntl.flock(lock, fcntl.LOCK_EX)
+        if so.is_file() and stamp_file.is_file() and stamp_file.read_text() == want:
+            return so
+        gxx = shutil.which("g++")
+        if gxx is None:
+            raise Backend("g++ was not found; the module that calls the kernels cannot be compiled")
+        if verbose:
+            _say(f"compiling the entry module into {out_dir}")
+        (out_dir / "entry_signatures.inc").write_text("\n".join(lines) + "\n")
+        tmp = out_dir / f"esp_b200_entry.{os.getpid()}.tmp.so"
+        lib = torch_dir / "lib"
+        proc = subprocess.run([gxx, *cmd, "-I", str(out_dir), "-isystem", str(torch_dir / "include"), "-isystem", sysconfig.get_paths()["include"],
+                               str(CSRC / "entry.cpp"), "-o", str(tmp), "-L", str(lib), f"-Wl,-rpath,{lib}", "-lc10", "-ltorch_cpu",
+                               "-ltorch_python"], capture_output=True, text=True)
+        if proc.returncode != 0:
+            raise Backend(f"g++ failed on entry.cpp:\n{proc.stderr[-4000:]}")
+        os.replace(tmp, so)
+        stamp_file.write_text(want)
+        return so
+
+
+def load_entry(signatures: dict):
+    """The compiled entry module, built first if needed."""
+    import importlib.machinery
+    import importlib.util
+    with _lock:
+        module = _loaded.get("entry")
+        if module is None:
+            path = build_entry(signatures)
+            loader = importlib.machinery.ExtensionFileLoader("esp_b200_entry", str(path))
+            try:
+                module = importlib.util.module_from_spec(importlib.util.spec_from_loader("esp_b200_entry", loader))
+                loader.exec_module(module)
+            except ImportError as e:
+                raise Backend(f"cannot load {path}: {e}") from None
+            _loaded["entry"] = module
+        return module
+
+
 def build_all(verbose: bool = True) -> list:
-    return [build_library(name, verbose) for name in LIBRARIES]
+    from .ops import _SIGNATURES
+    return [build_library(name, verbose) for name in LIBRARIES] + [build_entry(_SIGNATURES, verbose)]

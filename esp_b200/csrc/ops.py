@@ -15,7 +15,7 @@ from ctypes import c_float, c_int, c_longlong, c_ulonglong, c_void_p
 import torch
 
 from ..errors import Backend
-from .build import load_library
+from .build import load_entry, load_library, signature_letters
 
 P = c_void_p
 
@@ -117,13 +117,17 @@ _bound: dict = {}
 def _fn(library: str, name: str):
     f = _bound.get(name)
     if f is None:
+        global _ptr
         lib = load_library(library)
         try:
-            f = getattr(lib, name)
+            address = ctypes.cast(getattr(lib, name), c_void_p).value
         except AttributeError:
             raise Backend(f"the compiled library '{library}' has no entry point {name}") from None
-        f.argtypes = _SIGNATURES[name]
-        f.restype = c_int
+        entry = load_entry(_SIGNATURES)
+        if _ptr is _careful_ptr:
+            entry.set_careful_ptr(_careful_ptr)
+            _ptr = entry.ptr
+        f = entry.bind(address, signature_letters(_SIGNATURES[name]))
         _bound[name] = f
     return f
 
@@ -211,14 +215,11 @@ def _check(code: int, what: str) -> None:
                       f"(invalid value means a size this kernel does not take)")
 
 
-def _ptr(t, dtype=None, what="tensor"):
+def _careful_ptr(t, dtype=None, what="tensor"):
+    """A tensor's address, or what is wrong with it.  The entry module's ``ptr`` does the same and takes this place once it is
+    loaded; it comes here for what is not in order."""
     if t is None:
         return None
-    # a launch asks for six of these on average: what is in order leaves by the short way
-    if t.is_cuda and t.is_contiguous():
-        have = t.dtype
-        if have is dtype or dtype is None or (dtype is FLOATS and (have is _F32 or have is _BF16)):
-            return t.data_ptr()
     if not t.is_cuda:
         raise Backend(f"{what} must live on the GPU; this library has no CPU path")
     if not t.is_contiguous():
@@ -226,6 +227,9 @@ def _ptr(t, dtype=None, what="tensor"):
     if dtype is not None and t.dtype not in (dtype if isinstance(dtype, tuple) else (dtype,)):
         raise Backend(f"{what} has dtype {t.dtype}, expected {dtype}")
     return t.data_ptr()
+
+
+_ptr = _careful_ptr
 
 
 _F32, _BF16 = torch.float32, torch.bfloat16
