@@ -183,6 +183,8 @@ attn_prefill_tc05_kernel(const __grid_constant__ CUtensorMap map_q, const __grid
     __syncthreads();
     tc_fence_after();
     const unsigned tmem_base = *tmem_slot;
+    pdl_wait();                                                        // set up while the kernel before it ends
+    pdl_trigger();
     const unsigned tm_s = tmem_base, tm_o = tmem_base + 256;           // S of the groups at columns 0 and 128, O at 256 and 384
 
     if (warp == 0 || warp == V_WARP) {
@@ -545,7 +547,8 @@ int launch(const CUtensorMap& mq, const CUtensorMap& mk, const CUtensorMap& mv, 
     const long long grid = items < sm_count ? items : sm_count;
     AttnParams pp = p;
     pp.smem_bytes = (int)smem;
-    attn_prefill_tc05_kernel<HD, ROWT><<<(int)grid, 96 + GROUPS * ROWT * 128, smem, stream>>>(mq, mk, mv, pp);
+    esp_launch_pdl(ESP_PDL_MANY_ROWS, attn_prefill_tc05_kernel<HD, ROWT>, dim3((unsigned)grid), dim3(96 + GROUPS * ROWT * 128), smem, stream, mq, mk,
+                   mv, pp);
     return esp_launch_status();
 }
 }  // namespace

@@ -142,12 +142,13 @@ template <typename T> __device__ __forceinline__ T* behind_wait(T* p) {
     return p;
 }
 
-#define ESP_PDL_DEFAULT_MASK 61
+#define ESP_PDL_DEFAULT_MASK 125
 // classes of kernels, so that the attribute can be tried class by class: ESP_B200_PDL is a bit mask.  GROUPED: every
 // grouped product (off: it holds SM room while it waits for the routing); GROUPED_AFTER: a second grouped product
-// whose offsets were complete before the first one started; GROUPED_FITS: a short grouped product (gemm_skinny.cu).
+// whose offsets were complete before the first one started; GROUPED_FITS: a short grouped product (gemm_skinny.cu); MANY_ROWS: the
+// products, attention and routing of steps with many rows.
 enum : int { ESP_PDL_DENSE = 1, ESP_PDL_GROUPED = 2, ESP_PDL_ATTENTION = 4, ESP_PDL_SMALL = 8, ESP_PDL_GROUPED_AFTER = 16,
-              ESP_PDL_GROUPED_FITS = 32 };
+              ESP_PDL_GROUPED_FITS = 32, ESP_PDL_MANY_ROWS = 64 };
 static inline bool esp_pdl_enabled(int kind) {
     static int mask = -1;
     if (mask < 0) {

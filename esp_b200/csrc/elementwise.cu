@@ -227,10 +227,14 @@ ESP_API int esp_swiglu(const float* gu, void* act, int act_is_bf16, long long ro
 // out[r, :] = src[rows[r], :] for bfloat16 rows whose width is a multiple of 8 (16-byte pieces).
 __global__ void gather_rows_kernel(const bf16* __restrict__ src, const int* __restrict__ rows, bf16* __restrict__ out,
                                    int n_rows, int pieces) {
+    pdl_wait();
+    pdl_trigger();
+    const int* rows_now = behind_wait(rows);
+    const uint4* src_now = behind_wait(reinterpret_cast<const uint4*>(src));
     const long long total = (long long)n_rows * pieces;
     for (long long idx = blockIdx.x * (long long)blockDim.x + threadIdx.x; idx < total; idx += (long long)gridDim.x * blockDim.x) {
         const int r = (int)(idx / pieces), q = (int)(idx - (long long)r * pieces);
-        reinterpret_cast<uint4*>(out)[idx] = reinterpret_cast<const uint4*>(src)[(size_t)rows[r] * pieces + q];
+        reinterpret_cast<uint4*>(out)[idx] = src_now[(size_t)rows_now[r] * pieces + q];
     }
 }
 
@@ -240,7 +244,8 @@ ESP_API int esp_gather_rows(const void* src, const int* rows, void* out, int n_r
     const long long total = (long long)n_rows * (width / 8);
     long long blocks = (total + 255) / 256;
     if (blocks > 148 * 16) blocks = 148 * 16;
-    gather_rows_kernel<<<(int)blocks, 256, 0, stream>>>((const bf16*)src, rows, (bf16*)out, n_rows, width / 8);
+    esp_launch_pdl(ESP_PDL_MANY_ROWS, gather_rows_kernel, dim3((unsigned)blocks), dim3(256), 0, stream, (const bf16*)src, rows, (bf16*)out, n_rows,
+                   width / 8);
     return esp_launch_status();
 }
 

@@ -185,9 +185,6 @@ gemm_tc05_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constan
     const int unit = PAIR ? blockIdx.x >> 1 : blockIdx.x;            // the CTA (or pair) among those of the grid
     const int n_units = PAIR ? gridDim.x >> 1 : gridDim.x;
     const int feat_tiles = PAIR ? ((p.N + FEATS - 1) / FEATS + 1) / 2 : (p.N + FEATS - 1) / FEATS;
-    const int token_tiles = p.tile_group ? *p.n_tiles : (p.M + MAX_TOK - 1) / MAX_TOK;
-    const int total_tiles = token_tiles * feat_tiles;
-    if (unit >= total_tiles) return;                                 // the whole CTA (pair) leaves before any barrier exists
     const int k_iters = (p.K + BK - 1) / BK;
 
     if (threadIdx.x == 0) {
@@ -216,8 +213,15 @@ gemm_tc05_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constan
     if (PAIR) cluster_sync_all();                                    // the peer's barriers exist before anything reaches them
     tc_fence_after();
     const unsigned tmem_base = *tmem_slot;
+    // The kernel is set up while the one before it ends; from here on it reads what that one wrote.  The signal is given behind the
+    // wait: a dependent kernel may count on everything before this one.
+    pdl_wait();
+    pdl_trigger();
+    const int token_tiles = p.tile_group ? *behind_wait(p.n_tiles) : (p.M + MAX_TOK - 1) / MAX_TOK;
+    const int total_tiles = token_tiles * feat_tiles;
 
-    if (warp == 0 || warp == 6) {
+    if (unit >= total_tiles) {                                       // nothing for this CTA (pair)
+    } else if (warp == 0 || warp == 6) {
         // Producer warps: warp 0 takes the even k steps of the CTA's run of tiles, warp 6 the odd ones.  Lane 0
         // waits for the stage and announces its bytes; then the lanes issue one box each in one instruction:
         // lane 0 the weight rows (PLAIN: 128 rows; SWIGLU: the 64 gate rows), lane 1 the 64 up rows, lanes 2..
@@ -618,18 +622,21 @@ ESP_API int esp_gemm_tc05(const void* A, long long rows_total, const void* W, in
     cfg.blockDim = dim3(THREADS);
     cfg.dynamicSmemBytes = smem;
     cfg.stream = stream;
-    cudaLaunchAttribute attr[1];
+    cudaLaunchAttribute attr[2];
+    attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    attr[0].val.programmaticStreamSerializationAllowed = 1;
+    cfg.attrs = attr;
+    cfg.numAttrs = esp_pdl_enabled(ESP_PDL_MANY_ROWS) ? 1 : 0;
     if (pair) {
         // two CTAs of a cluster share a token tile: the grid is a whole number of pairs, one pair per two SMs
         const long long pair_tiles = (long long)token_tiles * (((N + feats - 1) / feats + 1) / 2);
         const long long pairs = pair_tiles < ctas / 2 ? pair_tiles : ctas / 2;
         cfg.gridDim = dim3((unsigned)(2 * pairs));
-        attr[0].id = cudaLaunchAttributeClusterDimension;
-        attr[0].val.clusterDim.x = 2;
-        attr[0].val.clusterDim.y = 1;
-        attr[0].val.clusterDim.z = 1;
-        cfg.attrs = attr;
-        cfg.numAttrs = 1;
+        cudaLaunchAttribute& cluster = attr[cfg.numAttrs++];
+        cluster.id = cudaLaunchAttributeClusterDimension;
+        cluster.val.clusterDim.x = 2;
+        cluster.val.clusterDim.y = 1;
+        cluster.val.clusterDim.z = 1;
     } else {
         cfg.gridDim = dim3((unsigned)(tiles_bound < ctas ? tiles_bound : ctas));
     }

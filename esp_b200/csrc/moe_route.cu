@@ -371,12 +371,15 @@ __device__ __forceinline__ void mma_16816(float (&d)[4], unsigned a0, unsigned a
 
 template <int NT, int KW>                                        // KW: warps that share the columns
 __global__ void __launch_bounds__(KW * 32)
-router_logits_mma_kernel(const float* __restrict__ h, const bf16* __restrict__ w_router, const bf16* __restrict__ w_gate,
+router_logits_mma_kernel(const float* h, const bf16* __restrict__ w_router, const bf16* __restrict__ w_gate,
                          float* __restrict__ logits, int n_tokens, int width, int n_experts) {
     __shared__ float part[KW - 1][16][NT * 8 + 1];               // the partial sums of warps 1..
     const int n0 = blockIdx.x * 16, warp = threadIdx.x >> 5, lane = threadIdx.x & 31, g = lane >> 2, tg = lane & 3;
     const int rows = n_experts + (w_gate ? 1 : 0);
     const int row_a = min(n0 + g, n_tokens - 1), row_b = min(n0 + g + 8, n_tokens - 1);
+    pdl_wait();
+    pdl_trigger();
+    h = behind_wait(h);
     const float* xa = h + (size_t)row_a * width;
     const float* xb = h + (size_t)row_b * width;
     // this lane's weight row in every column tile (rows beyond the last read the last one; never stored)
@@ -440,13 +443,16 @@ router_logits_mma_kernel(const float* __restrict__ h, const bf16* __restrict__ w
 
 // softmax, top-k and weights of a token from its logits [n, E + 1]: one warp per token
 __global__ void __launch_bounds__(256)
-router_select_kernel(const float* __restrict__ logits, int* __restrict__ topk_ids, float* __restrict__ topk_w,
+router_select_kernel(const float* logits, int* __restrict__ topk_ids, float* __restrict__ topk_w,
                      float* __restrict__ gate, float* __restrict__ probs_out, int n_tokens, int n_experts, int top_k,
                      int norm_topk, int has_gate, RouteChoice choice, int* __restrict__ status) {
     extern __shared__ float sel_ps[];                               // [8 warps][2 * n_experts]: scores, corrected scores
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
     const int n = blockIdx.x * 8 + warp;
+    pdl_wait();
+    pdl_trigger();
     if (n >= n_tokens) return;
+    logits = behind_wait(logits);
     float* ps = sel_ps + warp * 2 * n_experts;
     const float* lg = logits + (size_t)n * (n_experts + 1);
     scores_from_logits(lg, ps, n_experts, lane, norm_topk, choice.bias, probs_out ? probs_out + (size_t)n * n_experts : nullptr);
@@ -599,7 +605,7 @@ __device__ __forceinline__ bool e_bad(int e, int n_ids) { return e < 0 || e >= n
 // the warps gives every warp its first row in every expert's range, and the warp places its pairs there.
 // shared memory: [32 warps][n_experts] counts, then [n_experts + 1] offsets.
 __global__ void __launch_bounds__(1024)
-moe_permute_wide_kernel(const int* __restrict__ topk_ids, const float* __restrict__ topk_w, int n_pairs, int n_experts,
+moe_permute_wide_kernel(const int* topk_ids, const float* topk_w, int n_pairs, int n_experts,
                         int* __restrict__ offsets, int* __restrict__ perm_token, float* __restrict__ perm_weight,
                         int* __restrict__ inverse, int top_k, int* __restrict__ tile_group, int* __restrict__ tile_row0,
                         int* __restrict__ tile_count, int* __restrict__ n_tiles, int tile_rows, int max_tiles,
@@ -609,6 +615,10 @@ moe_permute_wide_kernel(const int* __restrict__ topk_ids, const float* __restric
     int* offs = sm + 32 * n_experts;                 // [n_experts + 1]
     const int tid = threadIdx.x, warp = tid >> 5;
     for (int i = tid; i < 32 * n_experts; i += 1024) hist[i] = 0;
+    pdl_wait();
+    pdl_trigger();
+    topk_ids = behind_wait(topk_ids);
+    topk_w = behind_wait(topk_w);
     __syncthreads();
     int* mine = hist + warp * n_experts;
     // pair i belongs to warp (i / 32) % 32 in both passes.  A thread's first PER pairs stay in registers: their loads
@@ -985,8 +995,8 @@ ESP_API int esp_router_topk(const void* h, int h_is_bf16, const void* w_router, 
         (reinterpret_cast<uintptr_t>(w_router) & 7) == 0 && (!w_gate || (reinterpret_cast<uintptr_t>(w_gate) & 7) == 0)) {
         const int blocks = (n_tokens + 15) / 16;
 #define ESP_ROUTER_MMA(NT, KW)                                                                                         \
-    router_logits_mma_kernel<NT, KW><<<blocks, KW * 32, 0, stream>>>((const float*)h, (const bf16*)w_router,            \
-                                                                      (const bf16*)w_gate, logits, n_tokens, width, n_experts)
+    esp_launch_pdl(ESP_PDL_MANY_ROWS, router_logits_mma_kernel<NT, KW>, dim3(blocks), dim3(KW * 32), 0, stream, (const float*)h,      \
+                   (const bf16*)w_router, (const bf16*)w_gate, logits, n_tokens, width, n_experts)
         if (width % 256 == 0) {
             if (rows <= 64) ESP_ROUTER_MMA(8, 8);
             else ESP_ROUTER_MMA(9, 8);
@@ -995,7 +1005,7 @@ ESP_API int esp_router_topk(const void* h, int h_is_bf16, const void* w_router, 
             else ESP_ROUTER_MMA(9, 4);
         }
 #undef ESP_ROUTER_MMA
-        router_select_kernel<<<(n_tokens + 7) / 8, 256, (size_t)16 * n_experts * sizeof(float), stream>>>(
+        esp_launch_pdl(ESP_PDL_MANY_ROWS, router_select_kernel, dim3((n_tokens + 7) / 8), dim3(256), (size_t)16 * n_experts * sizeof(float), stream,
             logits, topk_ids, topk_w, gate, probs_out, n_tokens, n_experts, top_k, norm_topk, w_gate ? 1 : 0, choice, status);
         return esp_launch_status();
     }
@@ -1086,7 +1096,7 @@ ESP_API int esp_moe_permute(const int* topk_ids, const float* topk_w, int n_toke
     if (smem > 48 * 1024) return (int)cudaErrorInvalidValue;
     const size_t smem_wide = (size_t)(33 * n_experts + 1) * sizeof(int);
     if (n_tokens * top_k >= 2048 && smem_wide <= 48 * 1024) {
-        moe_permute_wide_kernel<<<1, 1024, smem_wide, stream>>>(topk_ids, topk_w, n_tokens * top_k, n_experts, offsets,
+        esp_launch_pdl(ESP_PDL_MANY_ROWS, moe_permute_wide_kernel, dim3(1), dim3(1024), smem_wide, stream, topk_ids, topk_w, n_tokens * top_k, n_experts, offsets,
                                                                 perm_token, perm_weight, inverse, top_k, tile_group, tile_row0,
                                                                 tile_count, n_tiles, tile_rows, max_tiles, status, distinct, n_ids);
         return esp_launch_status();
