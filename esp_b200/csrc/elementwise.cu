@@ -167,6 +167,15 @@ add_rmsnorm_rows_kernel(float* __restrict__ x, const float* __restrict__ y, cons
     }
 }
 
+// Threads of a block that holds a row of ``width`` channels in pieces of four.
+static int row_threads(int width, int n_rows, int h_is_bf16) {
+    // one piece per thread while a block can hold them: a row's sum then has the same order whatever else is in
+    // the step (the 32-bit path relies on it).  Many rows rounded to bfloat16: four pieces per thread, smaller
+    // blocks, more rows in flight per SM.
+    if (width / 4 <= 1024 && !(h_is_bf16 && n_rows >= 256)) return (width / 4 + 31) / 32 * 32;
+    return ((width / 4 + 3) / 4 + 31) / 32 * 32;                  // up to four pieces per thread
+}
+
 // ``beta`` (may be null): the layer norm with this bias instead of the RMS norm.
 ESP_API int esp_add_rmsnorm(float* x, const float* y, const float* yscale, const float* gamma, const float* beta, const int* rows,
                             void* h, int h_is_bf16, float* h32, int n_rows, int width, float eps, int write_x, cudaStream_t stream) {
@@ -182,11 +191,7 @@ ESP_API int esp_add_rmsnorm(float* x, const float* y, const float* yscale, const
         else ESP_ADD_NORM(KERNEL, float, false);                 \
     } while (0)
     if (width % 4 == 0 && width <= 16384) {
-        int threads = ((width / 4 + 3) / 4 + 31) / 32 * 32;       // up to four pieces per thread
-        // one piece per thread while a block can hold them: a row's sum then has the same order whatever else is in
-        // the step (the 32-bit path relies on it).  Many rows rounded to bfloat16: four pieces per thread, smaller
-        // blocks, more rows in flight per SM.
-        if (width / 4 <= 1024 && !(h_is_bf16 && n_rows >= 256)) threads = (width / 4 + 31) / 32 * 32;
+        const int threads = row_threads(width, n_rows, h_is_bf16);
         ESP_ADD_NORM_T(add_rmsnorm_rows_kernel);
         return esp_launch_status();
     }
@@ -365,6 +370,78 @@ __global__ void depth_mix_kernel(float* __restrict__ x, const float* __restrict_
         for (int j = 0; j <= index; j++) acc = fmaf(weights[j], history[(size_t)j * count + i], acc);
         x[i] = fmaf(weights[index + 1], v, acc);
     }
+}
+
+// The same, then h = rmsnorm(x) * gamma as add_rmsnorm_rows_kernel has it (the same operations in the same order: equal bits): a row
+// a block, which holds it in registers.  A decode step of a model that averages over depth is a chain of short kernels; this is
+// one link less a layer.
+template <typename TH>
+__global__ void __launch_bounds__(1024)
+depth_mix_rmsnorm_kernel(float* __restrict__ x, const float* __restrict__ y, const float* __restrict__ yscale, float* __restrict__ history,
+                         const float* __restrict__ weights, int index, const float* __restrict__ gamma, TH* __restrict__ h, int width, float eps) {
+    pdl_trigger();
+    pdl_wait();
+    __shared__ float scratch[33];
+    const int r = blockIdx.x, pieces = width / 4;
+    const size_t layer = (size_t)gridDim.x * pieces, row = (size_t)r * pieces;       // in pieces
+    float4* xr = reinterpret_cast<float4*>(x) + row;
+    const float4* yr = y ? reinterpret_cast<const float4*>(y) + row : nullptr;
+    float4* hist = reinterpret_cast<float4*>(history) + row;
+    float4 v[4];
+    float ss = 0.f;
+#pragma unroll
+    for (int i = 0; i < 4; i++) {
+        const int q = threadIdx.x + i * blockDim.x;
+        if (q >= pieces) continue;
+        float4 t = xr[q];
+        if (yr) {
+            float4 a = yr[q];
+            if (yscale) {                                          // one rounding for both, as in depth_mix_kernel
+                const float4 sc = reinterpret_cast<const float4*>(yscale)[q];
+                t.x = fmaf(a.x, sc.x, t.x), t.y = fmaf(a.y, sc.y, t.y), t.z = fmaf(a.z, sc.z, t.z), t.w = fmaf(a.w, sc.w, t.w);
+            } else {
+                t.x += a.x, t.y += a.y, t.z += a.z, t.w += a.w;
+            }
+        }
+        hist[(index + 1) * layer + q] = t;
+        float4 acc = make_float4(0.f, 0.f, 0.f, 0.f);
+#pragma unroll 4
+        for (int j = 0; j <= index; j++) {
+            const float w = weights[j];
+            const float4 p = hist[j * layer + q];
+            acc.x = fmaf(w, p.x, acc.x), acc.y = fmaf(w, p.y, acc.y), acc.z = fmaf(w, p.z, acc.z), acc.w = fmaf(w, p.w, acc.w);
+        }
+        const float w = weights[index + 1];
+        v[i] = make_float4(fmaf(w, t.x, acc.x), fmaf(w, t.y, acc.y), fmaf(w, t.z, acc.z), fmaf(w, t.w, acc.w));
+        xr[q] = v[i];
+        ss = fmaf(v[i].x, v[i].x, ss);
+        ss = fmaf(v[i].y, v[i].y, ss);
+        ss = fmaf(v[i].z, v[i].z, ss);
+        ss = fmaf(v[i].w, v[i].w, ss);
+    }
+    const float inv = 1.0f / sqrtf(block_sum(ss, scratch) / (float)width + eps);
+#pragma unroll
+    for (int i = 0; i < 4; i++) {
+        const int q = threadIdx.x + i * blockDim.x;
+        if (q >= pieces) continue;
+        const float4 gm = reinterpret_cast<const float4*>(gamma)[q];
+        Vec4<TH>::store(h + (size_t)r * width + 4 * q, v[i].x * inv * gm.x, v[i].y * inv * gm.y, v[i].z * inv * gm.z, v[i].w * inv * gm.w);
+    }
+}
+
+// Rows of a multiple of 4 channels, at most 16,384.
+ESP_API int esp_depth_mix_rmsnorm(float* x, const float* y, const float* yscale, float* history, const float* weights, int index,
+                                  const float* gamma, void* h, int h_is_bf16, int n_rows, int width, float eps, cudaStream_t stream) {
+    if (n_rows <= 0) return 0;
+    if (width % 4 != 0 || width > 16384) return (int)cudaErrorInvalidValue;
+    const dim3 grid(n_rows), block(row_threads(width, n_rows, h_is_bf16));
+    if (h_is_bf16)
+        esp_launch_pdl(ESP_PDL_SMALL, depth_mix_rmsnorm_kernel<bf16>, grid, block, 0, stream, x, y, yscale, history, weights, index, gamma, (bf16*)h,
+                       width, eps);
+    else
+        esp_launch_pdl(ESP_PDL_SMALL, depth_mix_rmsnorm_kernel<float>, grid, block, 0, stream, x, y, yscale, history, weights, index, gamma, (float*)h,
+                       width, eps);
+    return esp_launch_status();
 }
 
 ESP_API int esp_depth_mix(float* x, const float* y, const float* yscale, float* history, const float* weights, int index,

@@ -25,6 +25,7 @@ _SIGNATURES = {
     "esp_feed_tokens": [P, P, P, c_int, P],
     "esp_add_rmsnorm": [P, P, P, P, P, P, P, c_int, P, c_int, c_int, c_float, c_int, P],
     "esp_depth_mix": [P, P, P, P, P, c_int, c_int, c_int, P],
+    "esp_depth_mix_rmsnorm": [P, P, P, P, P, c_int, P, P, c_int, c_int, c_int, c_float, P],
     "esp_xielu": [P, P, P, c_int, c_longlong, P],
     "esp_tanh": [P, P, c_int, c_longlong, P],
     "esp_token_shift_mix": [P, c_int, P, c_longlong, P, P, P, P, P, c_int, c_int, c_int, P],
@@ -298,6 +299,23 @@ def depth_mix(x, y, yscale, history, weights, index: int):
         _ptr(x, torch.float32, "x"), _ptr(y, torch.float32, "y"), _ptr(yscale, torch.float32, "yscale"),
         _ptr(history, torch.float32, "history"), _ptr(weights, torch.float32, "weights"), int(index), n, width, _stream()),
         "depth_mix")
+
+
+def depth_mix_rmsnorm_fits(width: int) -> bool:
+    return width % 4 == 0 and width <= 16384
+
+
+def depth_mix_rmsnorm(x, y, yscale, history, weights, index: int, gamma, h, eps):
+    """``depth_mix``, then h = rmsnorm(x) * gamma (h float32 or bfloat16, a row for every row of x)."""
+    n, width = x.shape
+    if history.shape[0] < index + 2 or tuple(history.shape[1:]) != (n, width) or weights.shape[0] < index + 2:
+        raise Backend("depth_mix: the history or the weights are too short for this layer")
+    if tuple(h.shape) != (n, width) or gamma.shape[0] != width:
+        raise Backend("depth_mix: the normed rows' shape disagrees")
+    _check(_fn("core", "esp_depth_mix_rmsnorm")(
+        _ptr(x, torch.float32, "x"), _ptr(y, torch.float32, "y"), _ptr(yscale, torch.float32, "yscale"),
+        _ptr(history, torch.float32, "history"), _ptr(weights, torch.float32, "weights"), int(index), _ptr(gamma, torch.float32, "gamma"),
+        _ptr(h, FLOATS, "h"), _is_bf16(h), n, width, float(eps), _stream()), "depth_mix_rmsnorm")
 
 
 def xielu(z, pq, act):

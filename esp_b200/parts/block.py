@@ -40,18 +40,37 @@ class PreNormResidualBlock(Part):
             self.ffn_norm.forward(x, plain_delta(self.ffn_norm, delta), h, h32=h32)
             delta = self.ffn.forward(h, ctx, h32=h32)
         if "residual_trace" in ctx.aux:
-            # debugging aid (see ScaledDepthMixBlock._trace): the add is done here so that x is the layer's result
+            # debugging aid (see ScaledDepthMixBlock._end): the add is done here so that x is the layer's result
             x.add_(plain_delta(None, delta))
             ctx.aux["residual_trace"].append(x.clone())
             return None
         return delta
 
 
+class DeferredDepthMix:
+    """The end of a ``ScaledDepthMixBlock``, left to the norm that reads its result: one launch for both.  It adds nothing to
+    the residual stream itself (``materialize()`` is None): x is the weighted sum once it has run."""
+
+    def __init__(self, x, delta, scale, history, weights, index):
+        self.x, self.delta, self.scale, self.history, self.weights, self.index = x, delta, scale, history, weights, index
+
+    def materialize(self):
+        ops.depth_mix(self.x, self.delta, self.scale, self.history, self.weights, self.index)
+        return None
+
+    def fused_add_rmsnorm(self, x, gamma, h, eps, rows, write_x, h32):
+        if rows is None and write_x and h32 is None and x is self.x and ops.depth_mix_rmsnorm_fits(x.shape[1]):
+            ops.depth_mix_rmsnorm(x, self.delta, self.scale, self.history, self.weights, self.index, gamma, h, eps)
+        else:
+            self.materialize()
+            ops.add_rmsnorm(x, None, gamma, h, eps, rows=rows, write_x=write_x, h32=h32)
+
+
 class ScaledDepthMixBlock(Part):
     """x <- x + m s1 * mixer(norm1(x)); x <- x + m s2 * ffn(norm2(x)) with s1, s2 a scale per channel and m the
     residual multiplier; the result X_(i+1) of layer i is kept, and what the next layer (or the model's end) reads is
     sum_j w[j] X_j over the embedding output X_0 and every result so far.  The first add is folded into the second
-    norm; the second add, the bookkeeping of X and the weighted sum are one kernel.  A layer without a feed-forward
+    norm; the second add, the bookkeeping of X and the weighted sum are one kernel, which the next layer's norm takes along (``DeferredDepthMix``).  A layer without a feed-forward
     has no second norm and no second scale."""
 
     graph_safe = True
@@ -103,21 +122,20 @@ class ScaledDepthMixBlock(Part):
             history[0].copy_(x)                   # X_0: what the embedding (and anything before this stack) left
         delta = self.mixer.forward(h, ctx, layer)
         if self.ffn is None:
-            ops.depth_mix(x, delta, self.scale1, history, self.weights, s.index)
-            self._trace(x, ctx)
-            return None
+            return self._end(DeferredDepthMix(x, plain_delta(None, delta), self.scale1, history, self.weights, s.index), ctx)
         self.ffn_norm.forward(x, delta, h, delta_scale=self.scale1)
         delta = self.ffn.forward(h, ctx)
-        ops.depth_mix(x, plain_delta(None, delta), self.scale2, history, self.weights, s.index)
-        self._trace(x, ctx)
-        return None
+        return self._end(DeferredDepthMix(x, plain_delta(None, delta), self.scale2, history, self.weights, s.index), ctx)
 
     @staticmethod
-    def _trace(x, ctx):
+    def _end(mix, ctx):
         """Debugging aid: a caller that passes ``aux={"residual_trace": []}`` to the step gets a copy of the
         residual stream behind every layer (such a step is never replayed from a captured graph)."""
-        if "residual_trace" in ctx.aux:
-            ctx.aux["residual_trace"].append(x.clone())
+        if "residual_trace" not in ctx.aux:
+            return mix
+        mix.materialize()
+        ctx.aux["residual_trace"].append(mix.x.clone())
+        return None
 
 
 class SandwichBlock(Part):
@@ -152,7 +170,7 @@ class SandwichBlock(Part):
             self.ffn_norm.forward(x, plain_delta(self.ffn_norm, pending), h, h32=h32)
             pending = DeferredPostNorm(rt, plain_delta(None, self.ffn.forward(h, ctx, h32=h32)), self.ffn_post)
         if "residual_trace" in ctx.aux:
-            # debugging aid (see ScaledDepthMixBlock._trace): the add is done here so that x is the layer's result
+            # debugging aid (see ScaledDepthMixBlock._end): the add is done here so that x is the layer's result
             pending.add_to(x)
             ctx.aux["residual_trace"].append(x.clone())
             return None
@@ -201,7 +219,7 @@ class OutputNormBlock(Part):
             h32 = x if getattr(self.ffn, "wants_f32_input", False) and h is not x else None
             pending = DeferredPostNorm(rt, self.ffn.forward(h, ctx, h32=h32), self.ffn_post)
         if "residual_trace" in ctx.aux:
-            # debugging aid (see ScaledDepthMixBlock._trace): the add is done here so that x is the layer's result
+            # debugging aid (see ScaledDepthMixBlock._end): the add is done here so that x is the layer's result
             pending.add_to(x)
             ctx.aux["residual_trace"].append(x.clone())
             return None
@@ -255,7 +273,7 @@ class ParallelResidualBlock(Part):
             if not getattr(pending, "take_along", lambda rows: False)(mixed):
                 pending = plain_delta(None, pending).add_(mixed)
         if "residual_trace" in ctx.aux:
-            # debugging aid (see ScaledDepthMixBlock._trace): the add is done here so that x is the layer's result
+            # debugging aid (see ScaledDepthMixBlock._end): the add is done here so that x is the layer's result
             x.add_(plain_delta(None, pending))
             ctx.aux["residual_trace"].append(x.clone())
             return None
@@ -359,7 +377,7 @@ class HyperConnectionBlock(Part):
             last = w2
         pending = DeferredStreamWrite(rt, streams, x, y, last["mix"], last["write"])
         if "residual_trace" in ctx.aux:
-            # debugging aid (see ScaledDepthMixBlock._trace): the write is done here so that x is the layer's result
+            # debugging aid (see ScaledDepthMixBlock._end): the write is done here so that x is the layer's result
             pending.materialize()
             ctx.aux["residual_trace"].append(x.clone())
             return None
