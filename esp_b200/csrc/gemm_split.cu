@@ -22,10 +22,11 @@
 // [a1 | a2 | a3] one behind the other as N rows, one MMA multiplies w1 by all three, one w2 by the first two, one w3 by the
 // first.  Eight warps read the accumulators out.
 //
-// What bounds it (clock64 in each role, cycles a stage): many rows, the thread that issues the MMAs: 800 for the twelve MMAs, 340 for
-// the wait before and 190 for the commit behind them, 500 for the segment's accumulators; few rows, memory: 6 rows,
-// N = 151,936, K = 2,048 in 227 us (5.5 TB/s).  1,400 rows, N = 11,264, K = 2,048: 433 us, 149 TFLOP/s, where the multiply-add
-// tiles of gemm_simt.cu take 1,253 us.
+// What bounds it (clock64 in each role, cycles a stage of 64 k): many rows, the thread that issues the MMAs: 800 for the twelve MMAs
+// (896 is what they take at 64 token rows), 320 for the wait before and 195 for the commits behind them, 520 for the read-out of a
+// segment; few rows, memory (6 rows, N = 151,936, K = 2,048 in 228 us, 5.5 TB/s) or, with few tiles, the same chain.  1,400 rows, N =
+// 11,264, K = 2,048: 418 us, 154 TFLOP/s, where the multiply-add tiles of gemm_simt.cu take 1,267 us; one row 26 us where they take 19.
+// Tiles of 48 rows, which leave room for a second set of accumulators, were slower (491 us: every MMA takes as long as for 64 rows).
 //
 // Persistent: a CTA per SM walks the tiles with the grid's stride; loads run ahead over the ends of tiles.  Every wait is
 // bounded: if one runs out the kernel raises ESP_STATUS_WAIT_EXPIRED, stops, frees its tensor memory and returns.
