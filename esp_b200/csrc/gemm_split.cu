@@ -29,7 +29,8 @@
 // Tiles of 48 rows, which leave room for a second set of accumulators, were slower (491 us: every MMA takes as long as for 64 rows).
 //
 // Persistent: a CTA per SM walks the tiles with the grid's stride; loads run ahead over the ends of tiles.  Every wait is
-// bounded: if one runs out the kernel raises ESP_STATUS_WAIT_EXPIRED, stops, frees its tensor memory and returns.
+// bounded: if one runs out the kernel raises ESP_STATUS_WAIT_EXPIRED, stops, waits for its own copies and MMAs, frees its tensor
+// memory and returns.  The lanes of a warp leave a role together: tcgen05.ld and .st and the barriers behind them want whole warps.
 //
 // Elements whose result is not finite (an infinity, a NaN or a number beyond bfloat16's range among the operands would
 // spread through the pieces) are made again with a chain of fused multiply-adds.
@@ -61,6 +62,7 @@ struct SplitParams {
     int groups, M, N, K;
     long long lda, ldc;
     int seg_stages, share;                 // stages of a segment; CTAs of a cluster that share a tile
+    unsigned polls;                        // of a wait, at most
     int* status;
 };
 
@@ -220,7 +222,7 @@ __global__ void __launch_bounds__(THREADS, 1) gemm_split_kernel(const __grid_con
     unsigned char* smem = reinterpret_cast<unsigned char*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~(uintptr_t)1023);
     unsigned char* raw = smem + NS * T_BYTES;
     float* parts = reinterpret_cast<float*>(raw + NR * RAW_BYTES);   // SHARED, first CTA: [segment][16 rows][128 features]
-    __shared__ __align__(8) unsigned long long full[SLOTS], empty[SLOTS], raw_full[NR], raw_empty[NR], acc_full[ND], acc_empty[ND];
+    __shared__ __align__(8) unsigned long long full[SLOTS], empty[SLOTS], raw_full[NR], raw_empty[NR], acc_full[ND], acc_empty[ND], drained;
     __shared__ unsigned tmem_slot;
     __shared__ __align__(16) Group groups[MAX_GROUPS];
     __shared__ int group_count;
@@ -230,6 +232,7 @@ __global__ void __launch_bounds__(THREADS, 1) gemm_split_kernel(const __grid_con
         for (int i = 0; i < SLOTS; i++) mbar_init(&full[i], G * (W_WARPS / 2 + T_WARPS)), mbar_init(&empty[i], 1);
         for (int i = 0; i < NR; i++) mbar_init(&raw_full[i], 1), mbar_init(&raw_empty[i], W_WARPS / 2);
         for (int i = 0; i < ND; i++) mbar_init(&acc_full[i], 1), mbar_init(&acc_empty[i], E_WARPS);
+        mbar_init(&drained, 1);
         abort_flag = 0;
         asm volatile("fence.mbarrier_init.release.cluster;\n" ::: "memory");
     }
@@ -252,6 +255,8 @@ __global__ void __launch_bounds__(THREADS, 1) gemm_split_kernel(const __grid_con
     const int seg0 = SHARED ? rank * segments / p.share : 0, seg1 = SHARED ? (rank + 1) * segments / p.share : segments;
     const int stage0 = seg0 * p.seg_stages, stages = min(all_stages, seg1 * p.seg_stages) - stage0;      // of this CTA, of every tile
     bool ok = true;
+    // for all lanes of a warp alike
+    auto warp_wait = [&](void* bar, unsigned parity) { return __all_sync(0xffffffffu, mbar_wait_limited(bar, parity, p.polls) && !abort_flag) != 0; };
 
     if (warp < W_WARPS) {
         // weights into pieces.  A lane holds 4 k of rows 8 i + lane / 4 (i = 0..3) of two of the stage's four MMA steps at a time.
@@ -267,7 +272,7 @@ __global__ void __launch_bounds__(THREADS, 1) gemm_split_kernel(const __grid_con
             while (!more && walk.next(t)) more = it < (end += stages);
             if (!more) break;
             const int s = it % NS, use = it / G / SLOTS, slot = it / G % SLOTS, r = it % NR;
-            ok = mbar_wait(&raw_full[r], (it / NR) & 1) && !abort_flag;
+            ok = warp_wait(&raw_full[r], (it / NR) & 1);
             if (!ok) break;
             const unsigned char* stage = raw + r * RAW_BYTES + from;
             const unsigned at = lanes + D_COLS + s * A_COLS;
@@ -279,7 +284,7 @@ __global__ void __launch_bounds__(THREADS, 1) gemm_split_kernel(const __grid_con
 #pragma unroll
                     for (int i = 0; i < 4; i++) v[j][i] = *reinterpret_cast<const float4*>(stage + (2 * two + j) * (BF * 64) + i * 512);
                 if (two == 0) {
-                    if (use > 0) ok = mbar_wait(&empty[slot], (use - 1) & 1) && !abort_flag;     // its last contents have been multiplied
+                    if (use > 0) ok = warp_wait(&empty[slot], (use - 1) & 1);     // its last contents have been multiplied
                     tc_fence_after();
                 }
                 if (!ok) break;
@@ -318,7 +323,7 @@ __global__ void __launch_bounds__(THREADS, 1) gemm_split_kernel(const __grid_con
         while (ok && walk.next(o)) {
             float total[RUNS][16];
             for (int seg = seg0; seg < seg1; seg++, count++) {
-                ok = mbar_wait(&acc_full[count % ND], (count / ND) & 1) && !abort_flag;
+                ok = warp_wait(&acc_full[count % ND], (count / ND) & 1);
                 if (!ok) break;
                 tc_fence_after();
 #pragma unroll
@@ -393,7 +398,7 @@ __global__ void __launch_bounds__(THREADS, 1) gemm_split_kernel(const __grid_con
         load();
         for (int it = 0; n_tok > 0; it++) {
             const int s = it % NS, use = it / G / SLOTS, slot = it / G % SLOTS;
-            if (it % G == 0 && use > 0) ok = mbar_wait(&empty[slot], (use - 1) & 1) && !abort_flag;
+            if (it % G == 0 && use > 0) ok = warp_wait(&empty[slot], (use - 1) & 1);
             if (!ok) break;
             const int n = n_tok;
             unsigned char* base = smem + s * T_BYTES;
@@ -426,14 +431,15 @@ __global__ void __launch_bounds__(THREADS, 1) gemm_split_kernel(const __grid_con
         while (ok && walk.next(t)) {
             for (int st = 0; st < stages && ok; st++, it++) {
                 const int r = it % NR, k = (stage0 + st) * KS + lane * 16;
-                if (it >= NR) ok = mbar_wait(&raw_empty[r], (it / NR - 1) & 1) && !abort_flag;
-                ok = __all_sync(0xffffffffu, ok);
+                if (it >= NR) ok = warp_wait(&raw_empty[r], (it / NR - 1) & 1);
                 if (!ok) break;
                 if (lane == 0) mbar_expect_tx(&raw_full[r], RAW_BYTES);
                 __syncwarp();
                 if (lane < 4) tma_load_3d(raw + r * RAW_BYTES + lane * (BF * 64), &map_w, k, t.f0, t.group, &raw_full[r]);
             }
         }
+        // its copies land before the shared memory is given up, whoever has stopped reading them
+        for (int i = it > NR ? it - NR : 0; i < it; i++) mbar_wait(&raw_full[i % NR], (i / NR) & 1);
         pdl_wait();
     } else if (lane == 0) {
         pdl_wait();
@@ -448,8 +454,8 @@ __global__ void __launch_bounds__(THREADS, 1) gemm_split_kernel(const __grid_con
             int in_seg = 0;
             for (int st = 0; st < stages; st += G, it += G) {
                 const int use = it / G / SLOTS, slot = it / G % SLOTS;
-                if (in_seg == 0 && seg >= ND) ok = mbar_wait(&acc_empty[seg % ND], (seg / ND - 1) & 1);
-                if (ok) ok = mbar_wait(&full[slot], use & 1) && !abort_flag;
+                if (in_seg == 0 && seg >= ND) ok = mbar_wait_limited(&acc_empty[seg % ND], (seg / ND - 1) & 1, p.polls);
+                if (ok) ok = mbar_wait_limited(&full[slot], use & 1, p.polls) && !abort_flag;
                 if (!ok) break;
                 tc_fence_after();
                 const unsigned d = tmem + seg % ND * 3 * NT;
@@ -475,12 +481,14 @@ __global__ void __launch_bounds__(THREADS, 1) gemm_split_kernel(const __grid_con
                 }
             }
         }
+        tc_commit(&drained);                                         // the MMAs end before their memory is given up
+        mbar_wait(&drained, 0);
     }
     if (!ok && lane == 0) {
         atomicOr(p.status, ESP_STATUS_WAIT_EXPIRED);
         abort_flag = 1;
-        for (int i = 0; i < 1000; i++) __nanosleep(1000);            // copies and MMAs in flight end before their memory is given up
     }
+    __syncwarp();
     tc_fence_before();
     __syncthreads();
     if (SHARED) {
@@ -567,13 +575,13 @@ int launch(SplitParams p, int sms, cudaStream_t stream) {
 
 // All float.  K, lda multiples of 4, A and W on 16 bytes, at most 256 groups.
 ESP_API int esp_gemm_split(const void* A, const int* a_rows, const void* W, const float* bias, const float* row_scale, void* C,
-                           const int* group_offsets, int groups, int M, int N, int K, long long lda, long long ldc, int* status,
+                           const int* group_offsets, int groups, int M, int N, int K, long long lda, long long ldc, int polls, int* status,
                            cudaStream_t stream) {
     if (M <= 0 || N <= 0) return 0;
-    if (K <= 0 || K % 4 != 0 || lda % 4 != 0 || ((uintptr_t)A & 15) || ((uintptr_t)W & 15) || groups < 1 || groups > MAX_GROUPS)
+    if (K <= 0 || K % 4 != 0 || lda % 4 != 0 || ((uintptr_t)A & 15) || ((uintptr_t)W & 15) || groups < 1 || groups > MAX_GROUPS || polls < 0)
         return (int)cudaErrorInvalidValue;
     SplitParams p{(const float*)A, a_rows, (const float*)W, bias, row_scale, (float*)C, group_offsets, groups, M, N, K, lda, ldc,
-                  segment_of(K) / KS, 1, status};
+                  segment_of(K) / KS, 1, (unsigned)polls, status};
     int dev = 0, sms = 0;
     cudaError_t e = cudaGetDevice(&dev);
     if (e == cudaSuccess) e = cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);

@@ -48,7 +48,7 @@ _SIGNATURES = {
     "esp_finite_check": [P, c_int, c_longlong, P, c_int, P],
     "esp_normal_fill": [P, c_int, c_longlong, c_ulonglong, c_float, c_float, P],
     "esp_gemm_simt": [P, c_int, P, P, c_int, P, P, P, c_int, P, c_int, c_int, c_int, c_int, c_longlong, c_longlong, P],
-    "esp_gemm_split": [P, P, P, P, P, P, P, c_int, c_int, c_int, c_int, c_longlong, c_longlong, P, P],
+    "esp_gemm_split": [P, P, P, P, P, P, P, c_int, c_int, c_int, c_int, c_longlong, c_longlong, c_int, P, P],
     "esp_rope_kvwrite": [P, P, P, P, P, P, c_int, c_int, P, P, P, c_int, P, c_int, c_int, c_int, c_int, c_int, c_int,
                          c_int, c_int, P, P],
     "esp_attn_simt": [P, P, P, P, c_int, c_int, P, P, P, c_int, c_int, c_int, c_int, c_int, c_int, c_int, c_int, c_float, c_int, P,
@@ -386,9 +386,10 @@ def gemm_split_fits(a, w) -> bool:
             and (w.dim() == 2 or w.shape[0] <= SPLIT_MAX_GROUPS) and a.stride(0) % 4 == 0 and a.data_ptr() % 16 == 0 and w.data_ptr() % 16 == 0)
 
 
-def gemm_split(a, w, c, status, bias=None, row_scale=None, a_rows=None, group_offsets=None, rows=None):
+def gemm_split(a, w, c, status, bias=None, row_scale=None, a_rows=None, group_offsets=None, rows=None, polls=1 << 22):
     """``gemm_simt`` for float32 operands on the tensor cores: every operand as three bfloat16 pieces, their products summed
-    in 32 bits.  A row's bits do not depend on the other rows of the call."""
+    in 32 bits.  A row's bits do not depend on the other rows of the call.  ``polls``: how often a wait inside the kernel asks before it
+    gives up and the status says so."""
     grouped = group_offsets is not None
     if grouped:
         groups, n, k = w.shape
@@ -405,7 +406,7 @@ def gemm_split(a, w, c, status, bias=None, row_scale=None, a_rows=None, group_of
     code = _fn("tc05", "esp_gemm_split")(
         a.data_ptr(), _ptr(a_rows, torch.int32, "a_rows"), w.data_ptr(), _ptr(bias, torch.float32, "bias"),
         _ptr(row_scale, torch.float32, "row_scale"), c.data_ptr(), _ptr(group_offsets, torch.int32, "group_offsets"), groups, m, n, k,
-        a.stride(0), c.stride(0), _ptr(status, torch.int32), _stream())
+        a.stride(0), c.stride(0), int(polls), _ptr(status, torch.int32), _stream())
     _check(code, "gemm_split")
 
 

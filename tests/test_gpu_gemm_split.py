@@ -104,3 +104,27 @@ def test_refusals():
         ops.gemm_split(rnd(4, 256).bfloat16(), rnd(128, 256), c, status)
     assert not ops.gemm_split_fits(rnd(4, 258), rnd(128, 258)) and ops.gemm_split_fits(rnd(4, 2048), rnd(2048, 2048))
     assert torch.all(c == 0)
+
+
+@pytest.mark.parametrize("m, n, k, groups", [(6, 2048, 2048, 0), (16, 19000, 512, 0), (16, 19100, 512, 0), (200, 2304, 1100, 0), (100, 300, 2048, 30)])
+def test_a_wait_that_runs_out_ends_the_kernel_in_an_orderly_way(m, n, k, groups):
+    """With no polls at all every wait gives up; with few some do, and each role may be anywhere by then.  The status says so, rows behind
+    the last are left alone, and the next call is right."""
+    a, w, status = rnd(m, k), rnd(*([groups] if groups else []), n, k, seed=1), torch.zeros(1, dtype=torch.int32, device=DEV)
+    options = {}
+    if groups:
+        options["group_offsets"] = torch.linspace(0, m, groups + 1, device=DEV).int()
+    want, c = torch.empty(m, n, device=DEV), torch.full((m + 1, n), 7.0, device=DEV)
+    ops.gemm_split(a, w, want, status, **options)
+    assert status.item() == 0
+    for polls in (0, 0, 1, 2, 3, 4, 6, 8, 16, 32, 64):
+        ops.gemm_split(a, w, c, status, rows=m, polls=polls, **options)
+        expired = status.item()
+        assert expired == 4 if polls == 0 else expired in (0, 4)
+        assert expired or torch.equal(c[:m], want)
+        status.zero_()
+        c[:m] = 7.0
+        ops.gemm_split(a, w, c, status, rows=m, **options)
+        assert status.item() == 0 and torch.equal(c[:m], want) and torch.all(c[m] == 7.0)
+    with pytest.raises(Exception, match="refused"):
+        ops.gemm_split(a, w, c, status, rows=m, polls=-1, **options)
