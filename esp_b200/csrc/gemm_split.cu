@@ -29,7 +29,8 @@
 // Tiles of 48 rows, which leave room for a second set of accumulators, were slower (491 us: every MMA takes as long as for 64 rows).
 //
 // Persistent: a CTA per SM walks the tiles with the grid's stride; loads run ahead over the ends of tiles.  Every wait is
-// bounded: if one runs out the kernel raises ESP_STATUS_WAIT_EXPIRED, stops, waits for its own copies and MMAs, frees its tensor
+// bounded, and begun behind pdl_wait() where it hangs on the token rows, so that it times this kernel and not those before it (one
+// may start beside a scan of many milliseconds, two launches back): if one runs out the kernel raises ESP_STATUS_WAIT_EXPIRED, stops, waits for its own copies and MMAs, frees its tensor
 // memory and returns.  The lanes of a warp leave a role together: tcgen05.ld and .st and the barriers behind them want whole warps.
 //
 // Elements whose result is not finite (an infinity, a NaN or a number beyond bfloat16's range among the operands would
@@ -217,6 +218,7 @@ __global__ void __launch_bounds__(THREADS, 1) gemm_split_kernel(const __grid_con
     // A group waits for every second stage.  A wait tells a phase from its neighbours only, so each group must have waited for the use of
     // the slot before this one, which an even ring gives.
     static_assert(NR % 2 == 0, "each slot belongs to one group");
+    static_assert(NS <= NR, "the first stages are split before the weights' ring waits for its readers");
     static_assert(!SHARED || NT == 16, "a shared tile is one run of 16 tokens");
     extern __shared__ unsigned char smem_raw[];
     unsigned char* smem = reinterpret_cast<unsigned char*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~(uintptr_t)1023);
@@ -272,6 +274,7 @@ __global__ void __launch_bounds__(THREADS, 1) gemm_split_kernel(const __grid_con
             while (!more && walk.next(t)) more = it < (end += stages);
             if (!more) break;
             const int s = it % NS, use = it / G / SLOTS, slot = it / G % SLOTS, r = it % NR;
+            if (it >= NS && it < NS + 2) pdl_wait();                 // once a group: from here on its waits hang on the MMAs
             ok = warp_wait(&raw_full[r], (it / NR) & 1);
             if (!ok) break;
             const unsigned char* stage = raw + r * RAW_BYTES + from;
@@ -431,6 +434,7 @@ __global__ void __launch_bounds__(THREADS, 1) gemm_split_kernel(const __grid_con
         while (ok && walk.next(t)) {
             for (int st = 0; st < stages && ok; st++, it++) {
                 const int r = it % NR, k = (stage0 + st) * KS + lane * 16;
+                if (it == NR) pdl_wait();                            // its reader may be waiting for MMAs, these for the token rows
                 if (it >= NR) ok = warp_wait(&raw_empty[r], (it / NR - 1) & 1);
                 if (!ok) break;
                 if (lane == 0) mbar_expect_tx(&raw_full[r], RAW_BYTES);

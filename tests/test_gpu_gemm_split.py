@@ -128,3 +128,37 @@ def test_a_wait_that_runs_out_ends_the_kernel_in_an_orderly_way(m, n, k, groups)
         assert status.item() == 0 and torch.equal(c[:m], want) and torch.all(c[m] == 7.0)
     with pytest.raises(Exception, match="refused"):
         ops.gemm_split(a, w, c, status, rows=m, polls=-1, **options)
+
+
+@pytest.mark.parametrize("m, n, k", [(200, 2304, 1100), (16, 19100, 512), (6, 2048, 2048)])
+def test_waits_do_not_count_the_kernel_before(m, n, k):
+    """The product starts beside a scan of many milliseconds that lets the next kernel in at once.  Its waits get a few times the polls
+    that it needs by itself."""
+    a, w, status = rnd(m, k), rnd(n, k, seed=1), torch.zeros(1, dtype=torch.int32, device=DEV)
+    want, c = torch.empty(m, n, device=DEV), torch.empty(m, n, device=DEV)
+    ops.gemm_split(a, w, want, status)
+    tokens, channels = 400_000, 32
+    gates, gate = torch.zeros(tokens, 1, 2, channels, device=DEV), torch.ones(tokens, channels, device=DEV)
+    out, state = torch.empty_like(gate), torch.zeros(1, channels, device=DEV)
+    zeros, start, slot = torch.zeros(channels, device=DEV), torch.tensor([0, tokens], dtype=torch.int32, device=DEV), torch.zeros(1, dtype=torch.int32, device=DEV)
+
+    def scan():
+        ops.diag_scan(gates, zeros, zeros, zeros, 8.0, gate, gate, state, start, slot, out, 1, channels, 1)
+
+    scan()                                                            # loads its library
+    torch.cuda.synchronize()
+    polls = 1
+    while polls < 1 << 16:
+        for _ in range(3):
+            ops.gemm_split(a, w, c, status, polls=polls)
+        if status.item() == 0:
+            break
+        status.zero_()
+        polls *= 2
+    began, ended = torch.cuda.Event(enable_timing=True), torch.cuda.Event(enable_timing=True)
+    began.record()
+    scan()
+    ops.gemm_split(a, w, c, status, polls=8 * polls)
+    ended.record()
+    assert status.item() == 0 and torch.equal(c, want), f"{polls} polls are enough for the product alone"
+    assert began.elapsed_time(ended) > 2.0
