@@ -1,12 +1,13 @@
 // 32-bit matrix product on the 5th-generation tensor cores:
 //   C[m, n] = (sum_k A[row(m), k] * W[g][n, k] + bias[n]) * row_scale[m],   A, W, C float.
 //
-// A float is the sum of three bfloat16 numbers exactly (8 + 8 + 8 bits of mantissa, each piece rounded to nearest), and
-// the product of two bfloat16 numbers is exact in 32 bits.  So with x = x1 + x2 + x3 the product a * w is made of
-//   main = a1 w1,   c1 = a2 w1 + a1 w2,   c2 = a3 w1 + a2 w2 + a1 w3,
-// which are summed over k in three accumulators of their own in tensor memory; what is left out (a2 w3 and smaller) is below
-// 2^-26 of a product.  The tensor core cuts its sums off instead of rounding them, which would add up over a long sum: the
-// accumulators are read out every segment of k and their value main + (c1 + c2) is added to the running sum with an ordinary
+// A float is the sum of three bfloat16 numbers exactly (8 + 8 + 8 bits of mantissa, each piece rounded to nearest; numbers below
+// 2^-110, 1e-33, lose what is below 2^-133, bfloat16's smallest), and the product of two bfloat16 numbers is exact in 32 bits.  So
+// with x = x1 + x2 + x3 the product a * w is made of
+//   main = a1 w1,   c1 = a2 w1 + a1 w2 + a1 w3,   c2 = a3 w1 + a2 w2 + a2 w3,
+// which are summed over k in three accumulators of their own in tensor memory; what is left out (a3 w2, a3 w3) is at most 2^-25 of a
+// product (|a3| <= 2^-17 and |w2| <= 2^-8 of the powers of two that a and w start with).  The tensor core cuts its sums off instead of rounding them, which would add up over a long sum:
+// the accumulators are read out every segment of k and their value main + (c1 + c2) is added to the running sum with an ordinary
 // rounded addition.  The order of everything depends on k alone, so a row's result has the same bits whatever other rows
 // are in the call, whatever the tile's width, whichever group the rows lie in and however many CTAs share a tile.
 // Error against 64 bits (2-norm, normal operands), this kernel / a chain of multiply-adds: K = 300 2.2e-7 / 3.1e-7, 512 2.4e-7 /
@@ -18,9 +19,11 @@
 // memory as they are; two groups of four warps take the stages in turn, split a stage and store its pieces as the A operand in
 // tensor memory (as shared-memory operands they would cost more of that memory's bandwidth than there is: the token rows' pieces
 // alone make the MMAs read 55 bytes a cycle).  Six warps load, split and store the token rows in shared memory (K-major,
-// 128-byte swizzle); a gather by a_rows costs nothing.  One thread issues the MMAs.  With the pieces of the token rows
-// [a1 | a2 | a3] one behind the other as N rows, one MMA multiplies w1 by all three, one w2 by the first two, one w3 by the
-// first.  Eight warps read the accumulators out.
+// 128-byte swizzle); a gather by a_rows costs nothing.  One thread issues the MMAs.  The pieces of the token rows lie
+// one behind the other as N rows [a1 | a2 | a3]: one MMA of n columns multiplies w1 by a1, and three of 2 n columns, into [c1 | c2], w1 by
+// [a2 | a3], w2 and w3 by [a1 | a2].  MMAs keep their order where accumulator and shape are the same, and here those that share an
+// accumulator have one shape.  (Three MMAs of 3 n, 2 n and n columns into overlapping accumulators would be an eighth less work, but
+// nothing says that the second adds to what the first has written.)  Eight warps read the accumulators out.
 //
 // What bounds it (clock64 in each role, cycles a stage of 64 k): many rows, the thread that issues the MMAs: 800 for the twelve MMAs
 // (896 is what they take at 64 token rows), 320 for the wait before and 195 for the commits behind them, 520 for the read-out of a
@@ -454,7 +457,7 @@ __global__ void __launch_bounds__(THREADS, 1) gemm_split_kernel(const __grid_con
         int it = 0, seg = 0;
         while (ok && walk.next(t)) {
             const int n = t.n_tok;
-            const unsigned d_three = split_idesc(3 * n), d_two = split_idesc(2 * n), d_one = split_idesc(n);
+            const unsigned d_two = split_idesc(2 * n), d_one = split_idesc(n);
             int in_seg = 0;
             for (int st = 0; st < stages; st += G, it += G) {
                 const int use = it / G / SLOTS, slot = it / G % SLOTS;
@@ -471,9 +474,11 @@ __global__ void __launch_bounds__(THREADS, 1) gemm_split_kernel(const __grid_con
                     for (int j = 0; j < KS / 16; j++) {
                         const unsigned a = a0 + 8 * j;
                         const unsigned long long b = b0 + 2 * j;
-                        tc_mma_ta(d, a, b, d_three, in_seg == 0 && g == 0 && j == 0 ? 0u : 1u);   // main, c1, c2
-                        tc_mma_ta(d + n, a + KS / 2, b, d_two, 1u);                               // c1, c2
-                        tc_mma_ta(d + 2 * n, a + KS, b, d_one, 1u);                               // c2
+                        const unsigned add = in_seg == 0 && g == 0 && j == 0 ? 0u : 1u;
+                        tc_mma_ta(d, a, b, d_one, add);                                           // w1 a1
+                        tc_mma_ta(d + n, a, b + n * (KS * 2 >> 4), d_two, add);                   // w1 a2 | w1 a3
+                        tc_mma_ta(d + n, a + KS / 2, b, d_two, 1u);                               // w2 a1 | w2 a2
+                        tc_mma_ta(d + n, a + KS, b, d_two, 1u);                                   // w3 a1 | w3 a2
                     }
                 }
                 tc_commit(&empty[slot]);

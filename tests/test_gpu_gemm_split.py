@@ -52,6 +52,21 @@ def test_dense(m, n, k):
     assert status.item() == 0
 
 
+def test_single_products():
+    """One product an element, mantissas next to the ones whose pieces leave most behind (1.0038986 squared) among them: what is left out is at
+    most 2^-25 of it, the sum of the accumulators rounds once."""
+    m, n, k = 64, 3000, 64
+    a, w, status = torch.zeros(m, k, device=DEV), 1 + rnd(n, k).abs().remainder(1.0), torch.zeros(1, dtype=torch.int32, device=DEV)
+    w[::3] = 1.0038986 + 1e-6 * rnd(1000, k, seed=1)
+    diagonal = 1 + rnd(m, seed=2).abs().remainder(1.0)
+    diagonal[::2] = 1.0038986 + 1e-6 * rnd(m // 2, seed=3)
+    a[torch.arange(m), torch.arange(m)] = diagonal
+    c = torch.empty(m, n, device=DEV)
+    ops.gemm_split(a, w, c, status)
+    exact = a.double() @ w.double().t()
+    assert ((c.double() - exact).abs() / exact).max() <= 1.55 * 2.0 ** -24
+
+
 @pytest.mark.parametrize("counts", [[3, 0, 66, 1, 0], [0] * 19 + [16] + [0] * 20, [1, 130, 0, 5], [64, 65, 63, 1, 200], [0, 2] * 128, [1] + [0] * 140 + [17, 0, 3]])
 def test_grouped(counts):
     n, k, rows = 300, 324, sum(counts)
