@@ -6,16 +6,19 @@
 // with x = x1 + x2 + x3 the product a * w is made of
 //   main = a1 w1,   c1 = a2 w1 + a1 w2 + a1 w3,   c2 = a3 w1 + a2 w2 + a2 w3,
 // which are summed over k in three accumulators of their own in tensor memory; what is left out (a3 w2, a3 w3) is at most 2^-25 of a
-// product (|a3| <= 2^-17 and |w2| <= 2^-8 of the powers of two that a and w start with).  The tensor core cuts its sums off instead of rounding them, which would add up over a long sum:
-// the accumulators are read out every segment of k and their value main + (c1 + c2) is added to the running sum with an ordinary
-// rounded addition.  The order of everything depends on k alone, so a row's result has the same bits whatever other rows
-// are in the call, whatever the tile's width, whichever group the rows lie in and however many CTAs share a tile.
-// Error against 64 bits (2-norm, normal operands), this kernel / a chain of multiply-adds: K = 300 2.2e-7 / 3.1e-7, 512 2.4e-7 /
-// 4.1e-7, 1,024 4.7e-7 / 5.7e-7, 2,048 4.7e-7 / 8.1e-7.  That is what sets the segments: with 512 k to a segment K = 512 would be at
-// 4.7e-7; K = 5,632 4.8e-7 / 1.34e-6 with 512 k to a segment, twice that with 1,024.
+// product (|a3| <= 2^-17 and |w2| <= 2^-8 of the powers of two that a and w start with).  The tensor core cuts its sums off instead of rounding them.  That
+// error has one sign, so it grows with the number of additions and not with its root, most where one product or a growing sum outweighs what
+// is added.  So main is read out every SUB stages, 128 k, and added up with ordinary rounded additions.  c1 and c2 are 2^-8 of main and
+// are read out a segment (256 to 1,024 k), whose value main + (c1 + c2) is added to the running sum.  The order of everything depends on
+// k alone, so a row's result has the same bits whatever other rows are in the call, whatever the tile's width, whichever group the
+// rows lie in and however many CTAs share a tile.
+// Error against 64 bits (2-norm), this kernel / a chain of multiply-adds, K = 1,024, 2,048, 5,632: normal operands 1.3e-7 / 5.8e-7,
+// 1.3e-7 / 8.1e-7, 1.4e-7 / 1.35e-6; positive ones 1.7e-7 / 4.9e-7, 1.7e-7 / 7.0e-7, 1.7e-7 / 1.06e-6; one channel of the rows 300 times
+// the others 2.9e-7 / 5.8 to 8.0e-7, 2.9e-7 / 0.8 to 1.2e-6, 2.9e-7 / 1.4 to 1.9e-6 by its place.  With main read out once a segment the last
+// two were 9.0e-7, 9.0e-7, 2.1e-6 and 1.07e-6, 1.06e-6, 2.1e-6.
 //
 // Layout: the weights are the 128-row side of the MMA, up to NT token rows its N side; accumulator D[feature, token],
-// TMEM lane = feature, columns [main | c1 | c2] of n_tok each.  A ring of stages of 64 k: the weights come by TMA into shared
+// TMEM lane = feature, columns of n_tok each.  A ring of stages of 64 k: the weights come by TMA into shared
 // memory as they are; two groups of four warps take the stages in turn, split a stage and store its pieces as the A operand in
 // tensor memory (as shared-memory operands they would cost more of that memory's bandwidth than there is: the token rows' pieces
 // alone make the MMAs read 55 bytes a cycle).  Six warps load, split and store the token rows in shared memory (K-major,
@@ -25,11 +28,8 @@
 // accumulator have one shape.  (Three MMAs of 3 n, 2 n and n columns into overlapping accumulators would be an eighth less work, but
 // nothing says that the second adds to what the first has written.)  Eight warps read the accumulators out.
 //
-// What bounds it (clock64 in each role, cycles a stage of 64 k): many rows, the thread that issues the MMAs: 800 for the twelve MMAs
-// (896 is what they take at 64 token rows), 320 for the wait before and 195 for the commits behind them, 520 for the read-out of a
-// segment; few rows, memory (6 rows, N = 151,936, K = 2,048 in 228 us, 5.5 TB/s) or, with few tiles, the same chain.  1,400 rows, N =
-// 11,264, K = 2,048: 418 us, 154 TFLOP/s, where the multiply-add tiles of gemm_simt.cu take 1,267 us; one row 26 us where they take 19.
-// Tiles of 48 rows, which leave room for a second set of accumulators, were slower (491 us: every MMA takes as long as for 64 rows).
+// Main has two sets of columns, so that its read-out runs beside the next MMAs; 64 token rows leave room for two stages of split weights
+// then (2 x 64 + 128 + 2 x 96 of 512 columns).
 //
 // Persistent: a CTA per SM walks the tiles with the grid's stride; loads run ahead over the ends of tiles.  Every wait is
 // bounded, and begun behind pdl_wait() where it hangs on the token rows, so that it times this kernel and not those before it (one
@@ -49,7 +49,8 @@ constexpr int A_COLS = 3 * KS / 2;         // TMEM columns of a stage of weights
 constexpr int RAW_BYTES = BF * KS * 4;     // the same as it comes: [4 steps][128 rows][16 k] float
 constexpr int MAX_GROUPS = 256;
 constexpr int MAX_PARTS = 8;               // segments of a tile that several CTAs share
-// k of a segment: 256, from K = 1,024 on 512, from K = 4,096 on 1,024
+constexpr int SUB = 2;                     // stages whose main products are summed in the tensor core
+// k of a segment, a multiple of SUB stages: 256, from K = 1,024 on 512, from K = 4,096 on 1,024
 __host__ __device__ constexpr int segment_of(int K) { return K >= 4096 ? 1024 : K >= 1024 ? 512 : 256; }
 constexpr int W_WARPS = 8, E_WARPS = 8, T_WARPS = 6;     // with the one that issues the copies and the one that issues the MMAs: 24 warps
 constexpr int T_ROWS = T_WARPS * 4;        // token rows that the T_WARPS take at once, eight threads a row
@@ -176,6 +177,21 @@ __device__ __forceinline__ void tc_ld16x2(unsigned ta, float (&a)[16], unsigned 
           "=&f"(b[11]), "=&f"(b[12]), "=&f"(b[13]), "=&f"(b[14]), "=&f"(b[15])
         : "r"(ta), "r"(tb) : "memory");
 }
+// one lane of a whole warp, always the same
+__device__ __forceinline__ bool elect_one() {
+    unsigned r;
+    asm volatile("{\n.reg .pred p;\nelect.sync _|p, 0xffffffff;\nselp.u32 %0, 1, 0, p;\n}\n" : "=r"(r));
+    return r != 0;
+}
+// tc_mma_ta with the operand descriptor given as its two words
+__device__ __forceinline__ void tc_mma_ta_lo(unsigned tmem_d, unsigned tmem_a, unsigned b_lo, unsigned b_hi, unsigned idesc, unsigned accumulate) {
+    asm volatile(
+        "{\n.reg .pred p;\n.reg .b64 db;\n"
+        "setp.ne.b32 p, %5, 0;\n"
+        "mov.b64 db, {%2, %3};\n"
+        "tcgen05.mma.cta_group::1.kind::f16 [%0], [%1], db, %4, p;\n}\n"
+        ::"r"(tmem_d), "r"(tmem_a), "r"(b_lo), "r"(b_hi), "r"(idesc), "r"(accumulate) : "memory");
+}
 // bfloat16 x bfloat16 -> float, B K-major (A in tensor memory), M = 128, N = n
 __device__ __forceinline__ unsigned split_idesc(int n) {
     return (1u << 4) | (1u << 7) | (1u << 10) | ((unsigned)(n >> 3) << 17) | ((unsigned)(BF >> 4) << 24);
@@ -206,28 +222,30 @@ __device__ __forceinline__ void store(const SplitParams& p, const Tile& t, int r
     p.C[(size_t)m * p.ldc + n] = v;
 }
 
-// NT: token rows of a tile at most; ND: sets of accumulators, which the segments take in turn; NS: stages of the ring of split
-// operands, NR: of the ring of weights as they come.  SHARED: the CTAs of a cluster take a tile's segments in equal runs, and the
-// first of them adds the segments' sums in order.
-template <int NT, int ND, int NS, int NR, int G, bool SHARED>
+// NT: token rows of a tile at most; MD: sets of accumulators of main products, which the SUB stages take in turn, CD: of the corrections,
+// which the segments take in turn; NS: stages of the ring of split operands, NR: of the ring of weights as they come.  SHARED: the
+// CTAs of a cluster take a tile's segments in equal runs, and the first of them adds the segments' sums in order.
+template <int NT, int MD, int CD, int NS, int NR, int G, bool SHARED>
 __global__ void __launch_bounds__(THREADS, 1) gemm_split_kernel(const __grid_constant__ CUtensorMap map_w, SplitParams p) {
-    constexpr int D_COLS = ND * 3 * NT;
+    constexpr int C_COL = MD * NT, A_COL = C_COL + CD * 2 * NT;      // columns: [main sets][correction sets][stages of weights]
     constexpr int T_BYTES = 3 * NT * KS * 2;
     // G stages share their mbarriers.  A tile then has a whole number of them; stages behind K are zeros.
     constexpr int SLOTS = NS / G;
     static_assert(NS % G == 0, "whole slots");
     constexpr int RUNS = (NT / 16 + 1) / 2;                          // runs of 16 tokens that a warp reads out
-    static_assert(3 * NT <= 256 && D_COLS + NS * A_COLS <= 512, "tensor memory");
+    static_assert(2 * NT <= 256 && A_COL + NS * A_COLS <= 512, "tensor memory");
+    static_assert(SUB % G == 0, "whole slots");
     // A group waits for every second stage.  A wait tells a phase from its neighbours only, so each group must have waited for the use of
     // the slot before this one, which an even ring gives.
-    static_assert(NR % 2 == 0, "each slot belongs to one group");
+    static_assert(NR % 2 == 0 && (G > 1 || NS % 2 == 0), "each slot belongs to one group, or to both");
     static_assert(NS <= NR, "the first stages are split before the weights' ring waits for its readers");
     static_assert(!SHARED || NT == 16, "a shared tile is one run of 16 tokens");
     extern __shared__ unsigned char smem_raw[];
     unsigned char* smem = reinterpret_cast<unsigned char*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~(uintptr_t)1023);
     unsigned char* raw = smem + NS * T_BYTES;
-    float* parts = reinterpret_cast<float*>(raw + NR * RAW_BYTES);   // SHARED, first CTA: [segment][16 rows][128 features]
-    __shared__ __align__(8) unsigned long long full[SLOTS], empty[SLOTS], raw_full[NR], raw_empty[NR], acc_full[ND], acc_empty[ND], drained;
+    // SHARED, first CTA: [segment][16 rows][128 features].  More than a run of tokens a warp: the running sums, [NT rows][128 features]
+    float* parts = reinterpret_cast<float*>(raw + NR * RAW_BYTES);
+    __shared__ __align__(8) unsigned long long full[SLOTS], empty[SLOTS], raw_full[NR], raw_empty[NR], main_full[MD], main_empty[MD], corr_empty[CD], drained;
     __shared__ unsigned tmem_slot;
     __shared__ __align__(16) Group groups[MAX_GROUPS];
     __shared__ int group_count;
@@ -236,7 +254,8 @@ __global__ void __launch_bounds__(THREADS, 1) gemm_split_kernel(const __grid_con
     if (threadIdx.x == 0) {
         for (int i = 0; i < SLOTS; i++) mbar_init(&full[i], G * (W_WARPS / 2 + T_WARPS)), mbar_init(&empty[i], 1);
         for (int i = 0; i < NR; i++) mbar_init(&raw_full[i], 1), mbar_init(&raw_empty[i], W_WARPS / 2);
-        for (int i = 0; i < ND; i++) mbar_init(&acc_full[i], 1), mbar_init(&acc_empty[i], E_WARPS);
+        for (int i = 0; i < MD; i++) mbar_init(&main_full[i], 1), mbar_init(&main_empty[i], E_WARPS);
+        for (int i = 0; i < CD; i++) mbar_init(&corr_empty[i], E_WARPS);
         mbar_init(&drained, 1);
         abort_flag = 0;
         asm volatile("fence.mbarrier_init.release.cluster;\n" ::: "memory");
@@ -281,7 +300,7 @@ __global__ void __launch_bounds__(THREADS, 1) gemm_split_kernel(const __grid_con
             ok = warp_wait(&raw_full[r], (it / NR) & 1);
             if (!ok) break;
             const unsigned char* stage = raw + r * RAW_BYTES + from;
-            const unsigned at = lanes + D_COLS + s * A_COLS;
+            const unsigned at = lanes + A_COL + s * A_COLS;
 #pragma unroll
             for (int two = 0; two < 2; two++) {
                 float4 v[2][4];
@@ -325,33 +344,55 @@ __global__ void __launch_bounds__(THREADS, 1) gemm_split_kernel(const __grid_con
         pdl_wait();
         Walk<NT> walk(p, groups, n_groups);
         Tile o;
-        int count = 0;                                               // segments read out so far
+        int subs = 0, count = 0;                                     // SUB stages and segments read out so far
+        float* mine = parts + quad * 32 + lane;
         while (ok && walk.next(o)) {
-            float total[RUNS][16];
+            float sum[RUNS][16], total[RUNS][16];
             for (int seg = seg0; seg < seg1; seg++, count++) {
-                ok = warp_wait(&acc_full[count % ND], (count / ND) & 1);
+                const int n_subs = (min(p.seg_stages, all_stages - seg * p.seg_stages) + SUB - 1) / SUB;
+                for (int u = 0; u < n_subs; u++, subs++) {
+                    ok = warp_wait(&main_full[subs % MD], (subs / MD) & 1);
+                    if (!ok) break;
+                    tc_fence_after();
+                    if (u == n_subs - 1) {                           // the corrections of the segment, before its last main sum
+                        const unsigned at = lanes + C_COL + count % CD * 2 * NT;
+#pragma unroll
+                        for (int r = 0; r < RUNS; r++) {
+                            const int c = (2 * r + half) * 16;
+                            if (c >= o.n_tok) continue;              // the same for a whole warp
+                            float c1[16], c2[16];
+                            tc_ld16x2(at + c, c1, at + o.n_tok + c, c2);
+#pragma unroll
+                            for (int i = 0; i < 16; i++) sum[r][i] = u == 0 ? c1[i] + c2[i] : sum[r][i] + (c1[i] + c2[i]);
+                        }
+                        tc_fence_before();
+                        __syncwarp();
+                        if (lane == 0) mbar_arrive(&corr_empty[count % CD]);
+                    }
+                    const unsigned at = lanes + subs % MD * NT + half * 16;
+                    float v[RUNS][16];
+                    if (RUNS == 2) tc_ld16x2(at, v[0], at + 32, v[RUNS - 1]);    // (columns behind n_tok are read and not used)
+                    else tc_ld16(at, v[0]);
+                    tc_fence_before();
+                    __syncwarp();
+                    if (lane == 0) mbar_arrive(&main_empty[subs % MD]);
+#pragma unroll
+                    for (int r = 0; r < RUNS; r++)
+#pragma unroll
+                        for (int i = 0; i < 16; i++) sum[r][i] = u == 0 && n_subs > 1 ? v[r][i] : sum[r][i] + v[r][i];
+                }
                 if (!ok) break;
-                tc_fence_after();
 #pragma unroll
                 for (int r = 0; r < RUNS; r++) {
                     const int c = (2 * r + half) * 16;
-                    if (c >= o.n_tok) continue;                      // the same for a whole warp
-                    const unsigned at = lanes + count % ND * 3 * NT + c;
-                    float sum[16], v[16];
-                    tc_ld16x2(at + o.n_tok, v, at + 2 * o.n_tok, sum);
-#pragma unroll
-                    for (int i = 0; i < 16; i++) sum[i] = v[i] + sum[i];
-                    tc_ld16(at, v);
+                    if (c >= o.n_tok) continue;
 #pragma unroll
                     for (int i = 0; i < 16; i++) {
-                        sum[i] = v[i] + sum[i];
-                        if (SHARED) st_cluster(parts + (seg * 16 + i) * BF + quad * 32 + lane, 0, sum[i]);
-                        else total[r][i] = seg == 0 ? sum[i] : total[r][i] + sum[i];
+                        if (SHARED) st_cluster(mine + (seg * 16 + i) * BF, 0, sum[r][i]);
+                        else if (RUNS > 1) mine[(c + i) * BF] = seg == 0 ? sum[r][i] : mine[(c + i) * BF] + sum[r][i];
+                        else total[r][i] = seg == 0 ? sum[r][i] : total[r][i] + sum[r][i];
                     }
                 }
-                tc_fence_before();
-                __syncwarp();
-                if (lane == 0) mbar_arrive(&acc_empty[count % ND]);
             }
             const int n = o.f0 + quad * 32 + lane;
             if (SHARED || !ok || n >= p.N) continue;
@@ -361,7 +402,7 @@ __global__ void __launch_bounds__(THREADS, 1) gemm_split_kernel(const __grid_con
                 const int c = (2 * r + half) * 16;
 #pragma unroll
                 for (int i = 0; i < 16; i++)
-                    if (c + i < o.rows) store(p, o, c + i, n, total[r][i], b);
+                    if (c + i < o.rows) store(p, o, c + i, n, RUNS > 1 ? mine[(c + i) * BF] : total[r][i], b);
             }
         }
     } else if (warp < W_WARPS + E_WARPS + T_WARPS) {
@@ -448,49 +489,60 @@ __global__ void __launch_bounds__(THREADS, 1) gemm_split_kernel(const __grid_con
         // its copies land before the shared memory is given up, whoever has stopped reading them
         for (int i = it > NR ? it - NR : 0; i < it; i++) mbar_wait(&raw_full[i % NR], (i / NR) & 1);
         pdl_wait();
-    } else if (lane == 0) {
+    } else {
+        // The MMAs.  The whole warp walks along, so that what an MMA is given is the same in all lanes and known to be; one lane issues.
         pdl_wait();
-        pdl_trigger();                                               // behind the wait: a dependent kernel may count on all before this one
+        if (lane == 0) pdl_trigger();                                // behind the wait: a dependent kernel may count on all before this one
         Walk<NT> walk(p, groups, n_groups);
         Tile t;
+        const unsigned cols = __shfl_sync(0xffffffffu, tmem, 0);
         const unsigned long long desc0 = smem_desc(smem);
-        int it = 0, seg = 0;
+        const unsigned desc_hi = (unsigned)(desc0 >> 32), desc_lo = __shfl_sync(0xffffffffu, (unsigned)desc0, 0);
+        int it = 0, subs = 0, count = 0;                             // subs, count: of the SUB stages and segments begun
         while (ok && walk.next(t)) {
-            const int n = t.n_tok;
-            const unsigned d_two = split_idesc(2 * n), d_one = split_idesc(n);
+            const int n = __shfl_sync(0xffffffffu, t.n_tok, 0);
+            const unsigned d_two = split_idesc(2 * n), d_one = split_idesc(n), off = n * (KS * 2 >> 4);
             int in_seg = 0;
             for (int st = 0; st < stages; st += G, it += G) {
                 const int use = it / G / SLOTS, slot = it / G % SLOTS;
-                if (in_seg == 0 && seg >= ND) ok = mbar_wait_limited(&acc_empty[seg % ND], (seg / ND - 1) & 1, p.polls);
-                if (ok) ok = mbar_wait_limited(&full[slot], use & 1, p.polls) && !abort_flag;
+                const bool new_sub = st % SUB == 0, new_seg = in_seg == 0;
+                if (new_sub && subs >= MD) ok = warp_wait(&main_empty[subs % MD], (subs / MD - 1) & 1);
+                if (ok) ok = warp_wait(&full[slot], use & 1);
                 if (!ok) break;
                 tc_fence_after();
-                const unsigned d = tmem + seg % ND * 3 * NT;
+                const unsigned main = cols + (subs - !new_sub) % MD * NT, corr = cols + C_COL + (count - !new_seg) % CD * 2 * NT;
+                const unsigned a0 = cols + A_COL + slot * G * A_COLS, b0 = desc_lo + ((slot * G * T_BYTES) >> 4);
+                subs += new_sub;
+                const bool wait_corr = new_seg && count >= CD;
+                count += new_seg;
+                in_seg = in_seg + G == p.seg_stages ? 0 : in_seg + G;
+                if (elect_one()) {
 #pragma unroll
-                for (int g = 0; g < G; g++) {
-                    const unsigned a0 = tmem + D_COLS + (slot * G + g) * A_COLS;
-                    const unsigned long long b0 = desc0 + (unsigned)(((slot * G + g) * T_BYTES) >> 4);
-#pragma unroll
-                    for (int j = 0; j < KS / 16; j++) {
-                        const unsigned a = a0 + 8 * j;
-                        const unsigned long long b = b0 + 2 * j;
-                        const unsigned add = in_seg == 0 && g == 0 && j == 0 ? 0u : 1u;
-                        tc_mma_ta(d, a, b, d_one, add);                                           // w1 a1
-                        tc_mma_ta(d + n, a, b + n * (KS * 2 >> 4), d_two, add);                   // w1 a2 | w1 a3
-                        tc_mma_ta(d + n, a + KS / 2, b, d_two, 1u);                               // w2 a1 | w2 a2
-                        tc_mma_ta(d + n, a + KS, b, d_two, 1u);                                   // w3 a1 | w3 a2
+                    for (int i = 0; i < G * KS / 16; i++) {
+                        const int g = i / (KS / 16), j = i % (KS / 16);
+                        tc_mma_ta_lo(main, a0 + g * A_COLS + 8 * j, b0 + ((g * T_BYTES) >> 4) + 2 * j, desc_hi, d_one, i == 0 && new_sub ? 0u : 1u);      // w1 a1
                     }
                 }
-                tc_commit(&empty[slot]);
-                in_seg += G;
-                if (in_seg == p.seg_stages || st + G == stages) {
-                    tc_commit(&acc_full[seg % ND]);
-                    in_seg = 0;
-                    seg++;
+                if (wait_corr) {
+                    ok = warp_wait(&corr_empty[(count - 1) % CD], ((count - 1) / CD - 1) & 1);
+                    if (!ok) break;
+                    tc_fence_after();
+                }
+                if (elect_one()) {
+#pragma unroll
+                    for (int i = 0; i < G * KS / 16; i++) {
+                        const int g = i / (KS / 16), j = i % (KS / 16);
+                        const unsigned a = a0 + g * A_COLS + 8 * j, b = b0 + ((g * T_BYTES) >> 4) + 2 * j;
+                        tc_mma_ta_lo(corr, a, b + off, desc_hi, d_two, i == 0 && new_seg ? 0u : 1u);      // w1 a2 | w1 a3
+                        tc_mma_ta_lo(corr, a + KS / 2, b, desc_hi, d_two, 1u);                            // w2 a1 | w2 a2
+                        tc_mma_ta_lo(corr, a + KS, b, desc_hi, d_two, 1u);                                // w3 a1 | w3 a2
+                    }
+                    tc_commit(&empty[slot]);
+                    if ((st + G) % SUB == 0 || st + G >= stages) tc_commit(&main_full[(subs - 1) % MD]);
                 }
             }
         }
-        tc_commit(&drained);                                         // the MMAs end before their memory is given up
+        if (elect_one()) tc_commit(&drained);                        // the MMAs end before their memory is given up
         mbar_wait(&drained, 0);
     }
     if (!ok && lane == 0) {
@@ -550,14 +602,14 @@ long long row_runs(const SplitParams& p, int nt) {
     return p.group_offsets ? p.M / nt + (p.groups < p.M ? p.groups : p.M) : (p.M + nt - 1) / nt;
 }
 
-template <int NT, int ND, int NS, int NR, int G, bool SHARED>
+template <int NT, int MD, int CD, int NS, int NR, int G, bool SHARED>
 int launch(SplitParams p, int sms, cudaStream_t stream) {
-    constexpr int SMEM = NS * 3 * NT * KS * 2 + NR * RAW_BYTES + (SHARED ? MAX_PARTS * 16 * BF * 4 : 0) + 1024;
+    constexpr int SMEM = NS * 3 * NT * KS * 2 + NR * RAW_BYTES + (SHARED ? MAX_PARTS * 16 * BF * 4 : NT > 32 ? NT * BF * 4 : 0) + 1024;
     static_assert(SMEM + 4096 + 512 <= 227 * 1024, "shared memory");
     CUtensorMap map;
     const int rc = map_weights(&map, p);
     if (rc) return rc;
-    const auto kernel = gemm_split_kernel<NT, ND, NS, NR, G, SHARED>;
+    const auto kernel = gemm_split_kernel<NT, MD, CD, NS, NR, G, SHARED>;
     const cudaError_t e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, SMEM);
     if (e != cudaSuccess) return (int)e;
     const long long tiles = row_runs(p, NT) * ((p.N + BF - 1) / BF);
@@ -605,15 +657,15 @@ ESP_API int esp_gemm_split(const void* A, const int* a_rows, const void* W, cons
             const int each = (segments + (int)most - 1) / (int)most;     // segments of a CTA at most
             p.share = (segments + each - 1) / each;
         }
-        if (p.share > 1) return launch<16, 2, 4, 4, 1, true>(p, sms, stream);
+        if (p.share > 1) return launch<16, 2, 2, 4, 4, 1, true>(p, sms, stream);
     }
     // Few rows, of a group four on average: a short tile leaves tensor memory for two sets of accumulators.  A wait and a commit keep
     // the issuing thread 300 and 90 cycles, a third of its time where the MMAs are short: groups, and a tile a CTA, have two stages behind
     // one of each (100 rows over 60 groups, N = 2,816: 223 -> 192 us; one row, N = 11,264 29.7 -> 26.7).  Many tiles a CTA of one matrix,
     // which memory bounds, are better off with the finer ring (6 rows, N = 151,936: 230 us against 245).
     if (M <= (group_offsets ? 4ll * groups : 16ll)) {
-        if (group_offsets || (N + BF - 1) / BF <= sms) return launch<16, 2, 4, 6, 2, false>(p, sms, stream);
-        return launch<16, 2, 4, 6, 1, false>(p, sms, stream);
+        if (group_offsets || (N + BF - 1) / BF <= sms) return launch<16, 2, 2, 4, 6, 2, false>(p, sms, stream);
+        return launch<16, 2, 2, 4, 6, 1, false>(p, sms, stream);
     }
-    return launch<64, 1, 3, 4, 1, false>(p, sms, stream);
+    return launch<64, 2, 1, 2, 4, 1, false>(p, sms, stream);
 }

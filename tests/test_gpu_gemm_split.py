@@ -14,8 +14,8 @@ def rnd(*shape, seed=0):
 
 
 def check(c, a, w, what):
-    """Within rounding of the 64-bit product, element by element: every accumulation of 16 products, every segment and the three
-    accumulators' sum lose at most a unit in the last place of a partial sum, together less than K / 2 of them."""
+    """Within rounding of the 64-bit product, element by element: every accumulation of 16 products, every addition to the running sum
+    and the accumulators' sum lose at most a unit in the last place of a partial sum, together less than K / 2 of them."""
     exact = a.double() @ w.double().t()
     bound = a.shape[1] * 2.0 ** -24 * (a.double().abs() @ w.double().abs().t())
     assert torch.all((c.double() - exact).abs() <= bound), what
@@ -50,6 +50,30 @@ def test_dense(m, n, k):
         ops.gemm_split(a[r:r + 1], w, one, status)
         assert torch.equal(one[0], c[r]), f"row {r}"
     assert status.item() == 0
+
+
+@pytest.mark.parametrize("k", [324, 1024, 1408, 2048, 4096, 5632])
+@pytest.mark.parametrize("kind", ["normal", "positive", "first", "behind the middle", "last third", "several"])
+def test_no_further_from_64_bits_than_the_chain_of_multiply_adds(kind, k):
+    """Also where the running sum outweighs what is added to it: all of one sign, or a channel of the rows 300 times the others.  (The tensor
+    core cuts its sums off, always towards zero.)  ``normal`` and ``positive`` sums lose at most a third of what the chain does from
+    K = 1,024 on: a chain's error grows with the root of K, theirs is that of 128 k."""
+    m, n = 64, 640
+    status = torch.zeros(1, dtype=torch.int32, device=DEV)
+    ours = chain = 0.0
+    for seed in range(2):
+        a, w = rnd(m, k, seed=2 * seed), rnd(n, k, seed=2 * seed + 1)
+        if kind == "positive":
+            a, w = a.abs(), w.abs()
+        elif kind != "normal":
+            a[:, {"first": [0], "behind the middle": [k // 2], "last third": [2 * k // 3], "several": [5, k // 4, k // 2 + 9]}[kind]] *= 300.0
+        exact = a.double() @ w.double().t()
+        c, d = torch.empty(m, n, device=DEV), torch.empty(m, n, device=DEV)
+        ops.gemm_split(a, w, c, status)
+        ops.gemm_simt(a, w, d)
+        ours += ((c.double() - exact).norm() / exact.norm()).item()
+        chain += ((d.double() - exact).norm() / exact.norm()).item()
+    assert status.item() == 0 and ours <= chain * (0.4 if kind in ("normal", "positive") and k >= 1024 else 1.0), (ours, chain)
 
 
 def test_single_products():
