@@ -36,8 +36,10 @@
 // may start beside a scan of many milliseconds, two launches back): if one runs out the kernel raises ESP_STATUS_WAIT_EXPIRED, stops, waits for its own copies and MMAs, frees its tensor
 // memory and returns.  The lanes of a warp leave a role together: tcgen05.ld and .st and the barriers behind them want whole warps.
 //
-// Elements whose result is not finite (an infinity, a NaN or a number beyond bfloat16's range among the operands would
-// spread through the pieces) are made again with a chain of fused multiply-adds.
+// Elements whose result is not finite (an infinity or a number beyond bfloat16's range among the operands would spread through the
+// pieces) are made again with a chain of fused multiply-adds, by all warps of a CTA when its tiles are done: in the read-out, where
+// others wait for its warps, one such row of six took 4.3 times the whole product (N = 40,000, K = 2,048).  A row of A with a NaN is
+// NaN as it is.
 #include "tc05.cuh"
 
 namespace {
@@ -207,19 +209,46 @@ __device__ __forceinline__ void st_cluster(float* p, unsigned rank, float v) {
     asm volatile("st.shared::cluster.f32 [%0], %1;\n" ::"r"(there), "f"(v) : "memory");
 }
 
-// One element as a chain of fused multiply-adds.
-__device__ __noinline__ float chain(const float* a, const float* w, int K) {
-    float s = 0.f;
-    for (int k = 0; k < K; k++) s = fmaf(a[k], w[k], s);
-    return s;
-}
-__device__ __forceinline__ void store(const SplitParams& p, const Tile& t, int row, int n, float v, float bias) {
-    const int m = t.m0 + row;
-    if (!(fabsf(v) <= 3.402823466e38f))
-        v = chain(p.A + (size_t)(p.a_rows ? p.a_rows[m] : m) * p.lda, p.W + ((size_t)t.group * p.N + n) * p.K, p.K);
-    if (p.bias) v += bias;
+__device__ __forceinline__ bool finite(float v) { return fabsf(v) <= 3.402823466e38f; }
+__device__ __forceinline__ const float* a_row(const SplitParams& p, int m) { return p.A + (size_t)(p.a_rows ? p.a_rows[m] : m) * p.lda; }
+// The element of row m (of the whole product) and feature n from its sum.
+__device__ __forceinline__ void store(const SplitParams& p, int m, int n, float v) {
+    if (p.bias) v += p.bias[n];
     if (p.row_scale) v *= p.row_scale[m];
     p.C[(size_t)m * p.ldc + n] = v;
+}
+
+// Makes the elements of a tile that are not finite again, each as a chain of fused multiply-adds.  A warp to a row; whole CTA.
+__device__ __forceinline__ void chains(const SplitParams& p, const Tile& t) {
+    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    for (int r = warp; r < t.rows; r += THREADS / 32) {
+        const int m = t.m0 + r;
+        const float* a = a_row(p, m);
+        unsigned odd = 0;
+        for (int j = 0; j < BF / 32; j++) {
+            const int n = t.f0 + 32 * j + lane;
+            if (n < p.N && !finite(p.C[(size_t)m * p.ldc + n])) odd |= 1u << j;
+        }
+        if (!__any_sync(0xffffffffu, odd != 0)) continue;
+        bool nan = false;
+        for (int k = lane * 4; k < p.K; k += 128) {
+            const float4 v = *reinterpret_cast<const float4*>(a + k);
+            nan |= isnan(v.x) || isnan(v.y) || isnan(v.z) || isnan(v.w);
+        }
+        if (__any_sync(0xffffffffu, nan)) continue;
+        for (int j = 0; j < BF / 32; j++) {
+            if (!(odd >> j & 1)) continue;
+            const int n = t.f0 + 32 * j + lane;
+            const float* w = p.W + ((size_t)t.group * p.N + n) * p.K;
+            float s = 0.f;
+#pragma unroll 4
+            for (int k = 0; k < p.K; k += 4) {
+                const float4 x = *reinterpret_cast<const float4*>(a + k), y = *reinterpret_cast<const float4*>(w + k);
+                s = fmaf(x.w, y.w, fmaf(x.z, y.z, fmaf(x.y, y.y, fmaf(x.x, y.x, s))));
+            }
+            store(p, m, n, s);
+        }
+    }
 }
 
 // NT: token rows of a tile at most; MD: sets of accumulators of main products, which the SUB stages take in turn, CD: of the corrections,
@@ -249,7 +278,7 @@ __global__ void __launch_bounds__(THREADS, 1) gemm_split_kernel(const __grid_con
     __shared__ unsigned tmem_slot;
     __shared__ __align__(16) Group groups[MAX_GROUPS];
     __shared__ int group_count;
-    __shared__ volatile int abort_flag;
+    __shared__ volatile int abort_flag, odd_flag;                    // odd_flag: some element is not finite
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     if (threadIdx.x == 0) {
         for (int i = 0; i < SLOTS; i++) mbar_init(&full[i], G * (W_WARPS / 2 + T_WARPS)), mbar_init(&empty[i], 1);
@@ -257,7 +286,7 @@ __global__ void __launch_bounds__(THREADS, 1) gemm_split_kernel(const __grid_con
         for (int i = 0; i < MD; i++) mbar_init(&main_full[i], 1), mbar_init(&main_empty[i], E_WARPS);
         for (int i = 0; i < CD; i++) mbar_init(&corr_empty[i], E_WARPS);
         mbar_init(&drained, 1);
-        abort_flag = 0;
+        abort_flag = 0, odd_flag = 0;
         asm volatile("fence.mbarrier_init.release.cluster;\n" ::: "memory");
     }
     if (warp == W_WARPS + E_WARPS + T_WARPS + 1) {
@@ -397,13 +426,29 @@ __global__ void __launch_bounds__(THREADS, 1) gemm_split_kernel(const __grid_con
             const int n = o.f0 + quad * 32 + lane;
             if (SHARED || !ok || n >= p.N) continue;
             const float b = p.bias ? p.bias[n] : 0.f;
+            bool odd = false;
 #pragma unroll
             for (int r = 0; r < RUNS; r++) {
-                const int c = (2 * r + half) * 16;
+                const int c = (2 * r + half) * 16, m = o.m0 + c;
+                float* to = p.C + (size_t)m * p.ldc + n;
+                auto put = [&](int i, float v) {
+                    odd |= !finite(v);
+                    if (p.bias) v += b;
+                    if (p.row_scale) v *= p.row_scale[m + i];
+                    *to = v;
+                    to += p.ldc;
+                };
+                if (RUNS > 1) {
+                    const int count = min(16, o.rows - c);
+#pragma unroll 4
+                    for (int i = 0; i < count; i++) put(i, mine[(c + i) * BF]);
+                } else {
 #pragma unroll
-                for (int i = 0; i < 16; i++)
-                    if (c + i < o.rows) store(p, o, c + i, n, RUNS > 1 ? mine[(c + i) * BF] : total[r][i], b);
+                    for (int i = 0; i < 16; i++)
+                        if (c + i < o.rows) put(i, total[r][i]);
+                }
             }
+            if (odd) odd_flag = 1;
         }
     } else if (warp < W_WARPS + E_WARPS + T_WARPS) {
         // token rows: eight threads to a row, each with eight k of it
@@ -422,7 +467,7 @@ __global__ void __launch_bounds__(THREADS, 1) gemm_split_kernel(const __grid_con
             for (int j = 0; j < PASSES; j++) {
                 const int r = r0 + T_ROWS * j;
                 src[j] = nullptr;
-                if (have && r < t.rows) src[j] = p.A + (size_t)(p.a_rows ? p.a_rows[t.m0 + r] : t.m0 + r) * p.lda + part * 8;
+                if (have && r < t.rows) src[j] = a_row(p, t.m0 + r) + part * 8;
             }
             n_next = have ? t.n_tok : 0;
         };
@@ -564,9 +609,16 @@ __global__ void __launch_bounds__(THREADS, 1) gemm_split_kernel(const __grid_con
                 if (n >= p.N) continue;
                 float v = parts[i];
                 for (int seg = 1; seg < segments; seg++) v += parts[seg * 16 * BF + i];
-                store(p, o, i / BF, n, v, p.bias ? p.bias[n] : 0.f);
+                if (!finite(v)) odd_flag = 1;
+                store(p, o.m0 + i / BF, n, v);
             }
         }
+        __syncthreads();
+    }
+    if (odd_flag && rank == 0 && !abort_flag) {
+        Walk<NT> walk(p, groups, n_groups);
+        Tile o;
+        while (walk.next(o)) chains(p, o);
     }
     if (warp == W_WARPS + E_WARPS + T_WARPS + 1) {
         tc_fence_after();

@@ -134,6 +134,47 @@ def test_infinities_nans_and_the_largest_numbers():
     assert c[3, 9].isnan() and c[3, 20].isinf() and (c[5, 20] == 0).item()
 
 
+@pytest.mark.parametrize("m, n, k", [(6, 40000, 2048), (6, 2048, 2048), (300, 2304, 2048)])
+def test_rows_with_a_nan_take_no_longer(m, n, k):
+    """One row with a NaN, then all: their elements are not made again one by one."""
+    a, w, status, c = rnd(m, k), rnd(n, k, seed=1), torch.zeros(1, dtype=torch.int32, device=DEV), torch.empty(m, n, device=DEV)
+
+    def milliseconds():
+        times = []
+        for _ in range(5):
+            began, ended = torch.cuda.Event(enable_timing=True), torch.cuda.Event(enable_timing=True)
+            began.record()
+            for _ in range(4):
+                ops.gemm_split(a, w, c, status)
+            ended.record()
+            torch.cuda.synchronize()
+            times.append(began.elapsed_time(ended))
+        return min(times)
+
+    milliseconds()
+    plain = milliseconds()
+    a[m // 2, 9] = float("nan")
+    assert milliseconds() < 2.5 * plain and c[m // 2].isnan().all() and c.isfinite().sum() == (m - 1) * n
+    a[:, 11] = float("nan")
+    assert milliseconds() < 2.5 * plain and c.isnan().all() and status.item() == 0
+
+
+def test_infinities_in_every_form():
+    """The chains of a shared tile, of a short one and of groups, with bias and scale behind them."""
+    for m, n, k, groups in ((6, 2048, 2048, 0), (16, 19100, 512, 0), (5, 300, 1028, 3)):
+        a, w, status = rnd(m, k), rnd(*([groups] if groups else []), n, k, seed=1), torch.zeros(1, dtype=torch.int32, device=DEV)
+        a[1, 9], a[3, k - 1], a[4, 7] = float("inf"), -3.4e38, float("nan")
+        bias, scale = rnd(n, seed=2), rnd(m, seed=3)
+        options = {"group_offsets": torch.tensor([0, 2, 2, m], dtype=torch.int32, device=DEV)} if groups else {}
+        c, chain = torch.empty(m, n, device=DEV), torch.empty(m, n, device=DEV)
+        ops.gemm_split(a, w, c, status, bias=bias, row_scale=scale, **options)
+        ops.gemm_simt(a, w, chain, bias=bias, row_scale=scale, **options)
+        odd = ~chain.isfinite()
+        assert odd[1].all() and odd[4].all() and status.item() == 0
+        assert torch.equal(c.isnan(), chain.isnan()) and torch.equal(c[odd & ~chain.isnan()], chain[odd & ~chain.isnan()])
+        assert torch.equal(c[3], chain[3])
+
+
 def test_refusals():
     status = torch.zeros(1, dtype=torch.int32, device=DEV)
     c = torch.zeros(4, 128, device=DEV)
