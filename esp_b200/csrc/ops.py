@@ -10,6 +10,7 @@ from __future__ import annotations
 import ctypes
 import functools
 import os
+import warnings
 from ctypes import c_float, c_int, c_longlong, c_ulonglong, c_void_p
 
 import torch
@@ -113,22 +114,37 @@ _SIGNATURES = {
 }
 
 _bound: dict = {}
+_entry = None                            # the module that calls the entry points; False where it cannot be compiled
+
+
+def _entry_module():
+    global _entry, _ptr
+    if _entry is None:
+        try:
+            _entry = load_entry(_SIGNATURES)
+        except Backend as e:
+            warnings.warn(f"the kernels are called through ctypes, some microseconds a launch slower: {e}", RuntimeWarning, stacklevel=4)
+            _entry = False
+        else:
+            _entry.set_careful_ptr(_careful_ptr)
+            _ptr = _entry.ptr
+    return _entry
 
 
 def _fn(library: str, name: str):
     f = _bound.get(name)
     if f is None:
-        global _ptr
         lib = load_library(library)
         try:
-            address = ctypes.cast(getattr(lib, name), c_void_p).value
+            f = getattr(lib, name)
         except AttributeError:
             raise Backend(f"the compiled library '{library}' has no entry point {name}") from None
-        entry = load_entry(_SIGNATURES)
-        if _ptr is _careful_ptr:
-            entry.set_careful_ptr(_careful_ptr)
-            _ptr = entry.ptr
-        f = entry.bind(address, signature_letters(_SIGNATURES[name]))
+        entry = _entry_module()
+        if entry:
+            f = entry.bind(ctypes.cast(f, c_void_p).value, signature_letters(_SIGNATURES[name]))
+        else:
+            f.argtypes = _SIGNATURES[name]
+            f.restype = c_int
         _bound[name] = f
     return f
 

@@ -51,6 +51,31 @@ def test_addresses_are_given_for_what_is_in_order_only(entry):
         entry.ptr(3.5)
 
 
+def test_without_the_module_the_kernels_are_called_through_ctypes(monkeypatch):
+    """Where it cannot be compiled (no g++, no headers) the entry points are reached as they were before there was a module."""
+    got = []
+    types = ops._SIGNATURES["esp_softcap"]
+    back = ctypes.CFUNCTYPE(ctypes.c_int, *types)(lambda *a: got.append(a) or -3)
+
+    def fails(signatures):
+        raise Backend("g++ was not found")
+
+    class Library:
+        esp_softcap = back
+
+    monkeypatch.setattr(ops, "load_entry", fails)
+    monkeypatch.setattr(ops, "load_library", lambda name: Library)
+    monkeypatch.setattr(ops, "_bound", {})
+    monkeypatch.setattr(ops, "_entry", None)
+    monkeypatch.setattr(ops, "_ptr", ops._careful_ptr)
+    with pytest.warns(RuntimeWarning, match="g\\+\\+ was not found"):
+        f = ops._fn("core", "esp_softcap")
+    assert f(None, 1, 3.0, 1 << 40) == -3 and got == [(None, 1, 3.0, 1 << 40)]
+    assert ops._fn("core", "esp_softcap") is f and ops._ptr is ops._careful_ptr
+    with pytest.raises(Backend, match="no entry point"):
+        ops._fn("core", "esp_depth_mix")
+
+
 @pytest.mark.gpu
 def test_addresses_of_tensors_on_the_device(entry):
     t = torch.ones(4, 6, device="cuda:0")
