@@ -10,6 +10,7 @@ __global__ void embed_gather_kernel(const TW* __restrict__ table, const int* __r
                                     int n_tokens, int width, int vocab, float scale, int* __restrict__ status) {
     pdl_trigger();
     pdl_wait();
+    ids = behind_wait(ids);
     const int n = blockIdx.x;
     if (n >= n_tokens) return;
     int id = ids[n];
@@ -40,6 +41,7 @@ ESP_API int esp_embed_gather(const void* table, int table_is_bf16, const int* id
 __global__ void feed_tokens_kernel(int* __restrict__ ids, const int* __restrict__ picks, const int* __restrict__ src, int n) {
     pdl_trigger();
     pdl_wait();
+    picks = behind_wait(picks), src = behind_wait(src);
     const int j = blockIdx.x * blockDim.x + threadIdx.x;
     if (j < n && src[j] >= 0) ids[j] = picks[src[j]];
 }
@@ -67,6 +69,7 @@ __global__ void add_rmsnorm_kernel(float* __restrict__ x, const float* __restric
                                    float eps, int write_x) {
     pdl_trigger();
     pdl_wait();
+    y = behind_wait(y), rows = behind_wait(rows);
     __shared__ float scratch[33];
     const int r = blockIdx.x;
     const size_t s = rows ? (size_t)rows[r] : (size_t)r;
@@ -115,6 +118,7 @@ add_rmsnorm_rows_kernel(float* __restrict__ x, const float* __restrict__ y, cons
                         int write_x) {
     pdl_trigger();
     pdl_wait();
+    y = behind_wait(y), rows = behind_wait(rows);
     __shared__ float scratch[33];
     const int r = blockIdx.x;
     const size_t s = rows ? (size_t)rows[r] : (size_t)r;
@@ -261,6 +265,7 @@ template <typename T>
 __global__ void finite_check_kernel(const T* __restrict__ v, long long count, int* __restrict__ status, int bit) {
     pdl_trigger();
     pdl_wait();
+    v = behind_wait(v);
     bool bad = false;
     for (long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x; i < count; i += (long long)gridDim.x * blockDim.x)
         bad |= !isfinite(to_f32(v[i]));
@@ -362,6 +367,7 @@ __global__ void depth_mix_kernel(float* __restrict__ x, const float* __restrict_
                                  long long count, int width) {
     pdl_trigger();
     pdl_wait();
+    y = behind_wait(y);
     for (long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x; i < count; i += (long long)gridDim.x * blockDim.x) {
         float v = x[i];
         if (y) v += yscale ? y[i] * yscale[i % width] : y[i];
@@ -381,6 +387,7 @@ depth_mix_rmsnorm_kernel(float* __restrict__ x, const float* __restrict__ y, con
                          const float* __restrict__ weights, int index, const float* __restrict__ gamma, TH* __restrict__ h, int width, float eps) {
     pdl_trigger();
     pdl_wait();
+    y = behind_wait(y);
     __shared__ float scratch[33];
     const int r = blockIdx.x, pieces = width / 4;
     const size_t layer = (size_t)gridDim.x * pieces, row = (size_t)r * pieces;       // in pieces
@@ -464,6 +471,7 @@ template <typename TO>
 __global__ void xielu_kernel(const float* __restrict__ z, const float* __restrict__ pq, TO* __restrict__ act, long long count) {
     pdl_trigger();
     pdl_wait();
+    z = behind_wait(z);
     const float ap = softplus_f(pq[0]), an = 0.5f + softplus_f(pq[1]);
     auto f = [&](float v) { return v > 0.f ? fmaf(ap * v, v, 0.5f * v) : fmaf(an, expm1f(v) - v, 0.5f * v); };
     if (count % 4 == 0 && ((size_t)z % 16) == 0 && ((size_t)act % 16) == 0) {       // four values a piece
@@ -494,6 +502,7 @@ template <typename TO>
 __global__ void tanh_kernel(const float* __restrict__ z, TO* __restrict__ out, long long count) {
     pdl_trigger();
     pdl_wait();
+    z = behind_wait(z);
     for (long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x; i < count; i += (long long)gridDim.x * blockDim.x)
         out[i] = from_f32<TO>(tanhf(z[i]));
 }
@@ -523,6 +532,7 @@ __global__ void embed_sum_kernel(const TW* __restrict__ table, const TW* __restr
                                  long long mul_prev, long long mul_cur, float scale, int* __restrict__ status) {
     pdl_trigger();
     pdl_wait();
+    ids = behind_wait(ids);
     const int n = blockIdx.x;
     int id = ids[n];
     if (id < 0 || id >= vocab) {
@@ -595,6 +605,7 @@ __global__ void norm_add_rmsnorm_kernel(float* __restrict__ x, const float* __re
                                         TH* __restrict__ h, float* __restrict__ h32, int width, float eps, int write_x) {
     pdl_trigger();
     pdl_wait();
+    rows = behind_wait(rows);
     y = behind_wait(y);
     __shared__ float scratch[33];
     const int r = blockIdx.x;
@@ -636,6 +647,7 @@ norm_add_rmsnorm_rows_kernel(float* __restrict__ x, const float* __restrict__ y,
                              TH* __restrict__ h, float* __restrict__ h32, int width, float eps, int write_x) {
     pdl_trigger();
     pdl_wait();
+    rows = behind_wait(rows);
     y = behind_wait(y);
     __shared__ float scratch[33];
     const int r = blockIdx.x;
@@ -731,6 +743,7 @@ __global__ void relu2_kernel(const float* __restrict__ z, const float* __restric
                              long long rows, int width) {
     pdl_trigger();
     pdl_wait();
+    z = behind_wait(z), row_scale = behind_wait(row_scale);
     const long long total = rows * width;
     for (long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x; i < total; i += (long long)gridDim.x * blockDim.x) {
         float v = z[i];
@@ -782,6 +795,7 @@ __global__ void hc_step_kernel(float* __restrict__ streams, const float* __restr
     }
     __syncthreads();
     pdl_wait();
+    x0 = behind_wait(x0), y = behind_wait(y), rows = behind_wait(rows);
     const int i = blockIdx.x;
     const size_t r = rows ? (size_t)rows[i] : (size_t)i;
     const float* yrow = y ? y + r * width : nullptr;
@@ -852,6 +866,7 @@ hc_step_vec_kernel(float* __restrict__ streams, const float* __restrict__ x0, co
         rw[s] = read_w ? read_w[s] : 1.f;
     }
     pdl_wait();
+    x0 = behind_wait(x0), y = behind_wait(y), rows = behind_wait(rows);
     const int i = blockIdx.x, tid = threadIdx.x;
     const size_t r = rows ? (size_t)rows[i] : (size_t)i;
     const float* yrow = y ? y + r * width : nullptr;
@@ -976,6 +991,7 @@ __global__ void glu_clamped_kernel(const float* __restrict__ gu, TO* __restrict_
                                    float alpha, float shift) {
     pdl_trigger();
     pdl_wait();
+    gu = behind_wait(gu);
     const long long total = rows * inter;
     for (long long idx = blockIdx.x * (long long)blockDim.x + threadIdx.x; idx < total;
          idx += (long long)gridDim.x * blockDim.x) {
@@ -995,6 +1011,7 @@ glu_clamped_vec_kernel(const float* __restrict__ gu, TO* __restrict__ act, long 
                        float alpha, float shift) {
     pdl_trigger();
     pdl_wait();
+    gu = behind_wait(gu);
     const int quads = inter / 4;
     const long long total = rows * quads;
     for (long long idx = blockIdx.x * (long long)blockDim.x + threadIdx.x; idx < total;
@@ -1043,6 +1060,7 @@ __global__ void weighted_sum_kernel(float* __restrict__ out, const float* __rest
                                     float sd, long long count) {
     pdl_trigger();
     pdl_wait();
+    a = behind_wait(a), b = behind_wait(b), c = behind_wait(c), d = behind_wait(d);
     for (long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x; i < count; i += (long long)gridDim.x * blockDim.x) {
         float v = sa * a[i];
         if (b) v = fmaf(sb, b[i], v);
@@ -1059,6 +1077,7 @@ weighted_sum_vec_kernel(float4* __restrict__ out, const float4* __restrict__ a, 
                         long long quads) {
     pdl_trigger();
     pdl_wait();
+    a = behind_wait(a), b = behind_wait(b), c = behind_wait(c), d = behind_wait(d);
     for (long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x; i < quads; i += (long long)gridDim.x * blockDim.x) {
         const float4 x = a[i];
         float4 v = make_float4(sa * x.x, sa * x.y, sa * x.z, sa * x.w);
@@ -1092,6 +1111,7 @@ template <typename TO>
 __global__ void cast_cols_kernel(const float* __restrict__ src, long long ld, TO* __restrict__ dst, long long rows, int width) {
     pdl_trigger();
     pdl_wait();
+    src = behind_wait(src);
     const long long total = rows * width;
     for (long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x; i < total; i += (long long)gridDim.x * blockDim.x) {
         const long long r = i / width;
@@ -1144,6 +1164,7 @@ diff_combine_kernel(const float* __restrict__ a, float lambda, float eps, float 
                     long long ldg, T* __restrict__ y, long long pairs, int H, int V) {
     pdl_trigger();
     pdl_wait();
+    gate = behind_wait(gate);
     const int lane = threadIdx.x & 31;
     const long long pair = (long long)blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5);
     if (pair >= pairs) return;

@@ -35,6 +35,37 @@ def test_equals_the_two_kernels(dtype, rows, width, index, parts):
     assert (h2.double() - normed).norm() <= 2 * bound * normed.norm()
 
 
+@pytest.mark.parametrize("rows, width", [(8, 2048), (400, 2048), (5, 16384)])
+def test_reads_what_the_kernel_before_has_written(rows, width):
+    """The kernel before (tanh) lets the next one in at once and writes what that one reads: nothing may be asked for ahead of the
+    wait.  Over and over in one stream, each time with other numbers in the place of the last ones."""
+    gamma, weights, scale = rnd(width, seed=1), rnd(2, seed=2), rnd(width, seed=4)
+    z, y = rnd(12, rows, width, seed=5), torch.zeros(rows, width, device=DEV)
+    x = rnd(rows, width)
+    history = torch.zeros(2, rows, width, device=DEV)
+    wanted = []
+    for i in range(12):
+        ops.tanh(z[i], y)
+        torch.cuda.synchronize()
+        x1, h = x.clone(), torch.empty(rows, width, device=DEV)
+        torch.cuda.synchronize()
+        if i % 2:
+            ops.depth_mix_rmsnorm(x1, y, scale, history, weights, 0, gamma, h, 1e-5)
+        else:
+            ops.add_rmsnorm(x1, y, gamma, h, 1e-5)
+        wanted.append((x1, h))
+    copies = [(x.clone(), torch.empty(rows, width, device=DEV)) for _ in range(12)]
+    torch.cuda.synchronize()
+    for i, (x1, h) in enumerate(copies):
+        ops.tanh(z[i], y)
+        if i % 2:
+            ops.depth_mix_rmsnorm(x1, y, scale, history, weights, 0, gamma, h, 1e-5)
+        else:
+            ops.add_rmsnorm(x1, y, gamma, h, 1e-5)
+    for (a, b), (c, d) in zip(wanted, copies):
+        assert torch.equal(a, c) and torch.equal(b, d)
+
+
 def test_refusals():
     x, h = rnd(2, 8), torch.empty(2, 8, device=DEV)
     with pytest.raises(Exception, match="too short"):
