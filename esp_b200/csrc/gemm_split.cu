@@ -154,10 +154,11 @@ __device__ __forceinline__ unsigned round2(float lo, float hi) {
     asm("cvt.rn.bf16x2.f32 %0, %1, %2;\n" : "=r"(r) : "f"(hi), "f"(lo));
     return r;
 }
-// the next piece of two floats, packed; what is left of them stays
+// the next piece of two floats, packed; what is left of them stays (one subtraction for both)
 __device__ __forceinline__ unsigned take2(float& x, float& y) {
     const unsigned q = round2(x, y);
-    x -= __uint_as_float(q << 16), y -= __uint_as_float(q & 0xFFFF0000u);
+    asm("{\n.reg .b64 a, b;\nmov.b64 a, {%0, %1};\nmov.b64 b, {%2, %3};\nsub.rn.f32x2 a, a, b;\nmov.b64 {%0, %1}, a;\n}\n"
+        : "+f"(x), "+f"(y) : "f"(__uint_as_float(q << 16)), "f"(__uint_as_float(q & 0xFFFF0000u)));
     return q;
 }
 // 16 lanes x 16 columns: of each run of 8 columns this thread's first two words go to lane t / 4, columns 2 (t % 4) and the
@@ -375,6 +376,7 @@ __global__ void __launch_bounds__(THREADS, 1) gemm_split_kernel(const __grid_con
         Tile o;
         int subs = 0, count = 0;                                     // SUB stages and segments read out so far
         float* mine = parts + quad * 32 + lane;
+        const bool wide = p.ldc % 4 == 0 && (reinterpret_cast<uintptr_t>(p.C) & 15) == 0;      // a row's features start on 16 bytes
         while (ok && walk.next(o)) {
             float sum[RUNS][16], total[RUNS][16];
             for (int seg = seg0; seg < seg1; seg++, count++) {
@@ -440,8 +442,31 @@ __global__ void __launch_bounds__(THREADS, 1) gemm_split_kernel(const __grid_con
                 };
                 if (RUNS > 1) {
                     const int count = min(16, o.rows - c);
+                    if (wide && o.f0 + BF <= p.N) {
+                        // four rows at a time, eight lanes to the 32 features of one
+                        __syncwarp();
+                        const float* from = parts + c * BF + quad * 32 + (lane & 7) * 4;
+                        const int n4 = o.f0 + quad * 32 + (lane & 7) * 4;
+                        float4 b4 = make_float4(0.f, 0.f, 0.f, 0.f);
+                        if (p.bias) b4 = make_float4(p.bias[n4], p.bias[n4 + 1], p.bias[n4 + 2], p.bias[n4 + 3]);
+#pragma unroll
+                        for (int i0 = 0; i0 < 16; i0 += 4) {
+                            const int i = i0 + (lane >> 3);
+                            if (i >= count) continue;
+                            float4 v = *reinterpret_cast<const float4*>(from + i * BF);
+                            odd |= !finite(v.x) || !finite(v.y) || !finite(v.z) || !finite(v.w);
+                            if (p.bias) v.x += b4.x, v.y += b4.y, v.z += b4.z, v.w += b4.w;
+                            if (p.row_scale) {
+                                const float f = p.row_scale[m + i];
+                                v.x *= f, v.y *= f, v.z *= f, v.w *= f;
+                            }
+                            *reinterpret_cast<float4*>(p.C + (size_t)(m + i) * p.ldc + n4) = v;
+                        }
+                        __syncwarp();
+                    } else {
 #pragma unroll 4
-                    for (int i = 0; i < count; i++) put(i, mine[(c + i) * BF]);
+                        for (int i = 0; i < count; i++) put(i, mine[(c + i) * BF]);
+                    }
                 } else {
 #pragma unroll
                     for (int i = 0; i < 16; i++)
