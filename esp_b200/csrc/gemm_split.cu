@@ -6,16 +6,18 @@
 // with x = x1 + x2 + x3 the product a * w is made of
 //   main = a1 w1,   c1 = a2 w1 + a1 w2 + a1 w3,   c2 = a3 w1 + a2 w2 + a2 w3,
 // which are summed over k in three accumulators of their own in tensor memory; what is left out (a3 w2, a3 w3) is at most 2^-25 of a
-// product (|a3| <= 2^-17 and |w2| <= 2^-8 of the powers of two that a and w start with).  The tensor core cuts its sums off instead of rounding them.  That
-// error has one sign, so it grows with the number of additions and not with its root, most where one product or a growing sum outweighs what
-// is added.  So main is read out every SUB stages, 128 k, and added up with ordinary rounded additions.  c1 and c2 are 2^-8 of main and
-// are read out a segment (256 to 1,024 k), whose value main + (c1 + c2) is added to the running sum.  The order of everything depends on
+// product (|a3| <= 2^-17 and |w2| <= 2^-8 of the powers of two that a and w start with).  The tensor core cuts its sums off instead of
+// rounding them.  That error has one sign, so it grows with the number of additions and not with its root, most where one product or a
+// growing sum outweighs what is added.  So main is read out every SUB stages, 128 k, and added up with ordinary rounded additions.  c1
+// and c2 are 2^-8 of main and are read out a segment (256 to 1,024 k), whose value main + (c1 + c2) is added to the running sum.  The order of everything depends on
 // k alone, so a row's result has the same bits whatever other rows are in the call, whatever the tile's width, whichever group the
 // rows lie in and however many CTAs share a tile.
 // Error against 64 bits (2-norm), this kernel / a chain of multiply-adds, K = 1,024, 2,048, 5,632: normal operands 1.3e-7 / 5.8e-7,
 // 1.3e-7 / 8.1e-7, 1.4e-7 / 1.35e-6; positive ones 1.7e-7 / 4.9e-7, 1.7e-7 / 7.0e-7, 1.7e-7 / 1.06e-6; one channel of the rows 300 times
-// the others 2.9e-7 / 5.8 to 8.0e-7, 2.9e-7 / 0.8 to 1.2e-6, 2.9e-7 / 1.4 to 1.9e-6 by its place.  With main read out once a segment the last
-// two were 9.0e-7, 9.0e-7, 2.1e-6 and 1.07e-6, 1.06e-6, 2.1e-6.
+// the others 2.9e-7 / 5.8 to 8.0e-7, 2.9e-7 / 0.8 to 1.2e-6, 2.9e-7 / 1.4 to 1.9e-6 where it stands in the first half.  That channel sets
+// SUB: 128 k before the row's end, the place where a chain has least to add behind it, they are 2.8e-7 / 2.95e-7, and SUB twice as
+// long doubles ours.  With main read out once a segment the three were 4.7e-7, 4.7e-7, 9.7e-7, 9.0e-7, 9.0e-7, 2.1e-6 and 1.07e-6, 1.06e-6,
+// 2.1e-6 (1,400 rows of 11,264 x 2,048 489 us then, 520 now; SUB = 4 502).
 //
 // Layout: the weights are the 128-row side of the MMA, up to NT token rows its N side; accumulator D[feature, token],
 // TMEM lane = feature, columns of n_tok each.  A ring of stages of 64 k: the weights come by TMA into shared
@@ -25,16 +27,24 @@
 // 128-byte swizzle); a gather by a_rows costs nothing.  One thread issues the MMAs.  The pieces of the token rows lie
 // one behind the other as N rows [a1 | a2 | a3]: one MMA of n columns multiplies w1 by a1, and three of 2 n columns, into [c1 | c2], w1 by
 // [a2 | a3], w2 and w3 by [a1 | a2].  MMAs keep their order where accumulator and shape are the same, and here those that share an
-// accumulator have one shape.  (Three MMAs of 3 n, 2 n and n columns into overlapping accumulators would be an eighth less work, but
+// accumulator have one shape.  (Three MMAs of 3 n, 2 n and n columns into overlapping accumulators would be a seventh less work, but
 // nothing says that the second adds to what the first has written.)  Eight warps read the accumulators out.
 //
 // Main has two sets of columns, so that its read-out runs beside the next MMAs; 64 token rows leave room for two stages of split weights
 // then (2 x 64 + 128 + 2 x 96 of 512 columns).
 //
+// What bounds it, 64 token rows (1,400 rows, N = 11,264, K = 2,048: 520 us, 124 TFLOP/s, multiply-adds 1,251): a stage takes 1,900
+// cycles, of which the tensor core works 840 to 900.  The warp that issues (clock64) spends 711 of them issuing, 366 waiting for a stage,
+// 333 for accumulators to be read out and 282 on commits; the warps that split are busy most of the time as well (0.61 of the SM's issue
+// slots), so that neither twice the warps for the token rows (539), pieces made before their slot is free (623) nor all eight weight warps
+// on each stage (673) helped.  Short tiles: 1,200 to 1,500 cycles a stage; six rows, N = 151,936 in 238 us, 5.2 TB/s; one row,
+// N = 11,264 / 6,144 / 2,048 27 / 18 / 10 us where multiply-adds take 21 / 17 / 14, K = 5,632, N = 2,048 17 and 34.
+//
 // Persistent: a CTA per SM walks the tiles with the grid's stride; loads run ahead over the ends of tiles.  Every wait is
 // bounded, and begun behind pdl_wait() where it hangs on the token rows, so that it times this kernel and not those before it (one
-// may start beside a scan of many milliseconds, two launches back): if one runs out the kernel raises ESP_STATUS_WAIT_EXPIRED, stops, waits for its own copies and MMAs, frees its tensor
-// memory and returns.  The lanes of a warp leave a role together: tcgen05.ld and .st and the barriers behind them want whole warps.
+// may start beside a scan of many milliseconds, two launches back): if one runs out the kernel raises ESP_STATUS_WAIT_EXPIRED, stops,
+// waits for its own copies and MMAs, frees its tensor memory and returns.  The lanes of a warp leave a role together: tcgen05.ld and
+// .st and the barriers behind them want whole warps.
 //
 // Elements whose result is not finite (an infinity or a number beyond bfloat16's range among the operands would spread through the
 // pieces) are made again with a chain of fused multiply-adds, by all warps of a CTA when its tiles are done: in the read-out, where

@@ -91,9 +91,13 @@ def test_single_products():
     assert ((c.double() - exact).abs() / exact).max() <= 1.55 * 2.0 ** -24
 
 
-@pytest.mark.parametrize("counts", [[3, 0, 66, 1, 0], [0] * 19 + [16] + [0] * 20, [1, 130, 0, 5], [64, 65, 63, 1, 200], [0, 2] * 128, [1] + [0] * 140 + [17, 0, 3]])
-def test_grouped(counts):
-    n, k, rows = 300, 324, sum(counts)
+@pytest.mark.parametrize("counts, k", [
+    ([3, 0, 66, 1, 0], 324), ([0] * 19 + [16] + [0] * 20, 324), ([1, 130, 0, 5], 324), ([64, 65, 63, 1, 200], 324), ([0, 2] * 128, 324),
+    ([1] + [0] * 140 + [17, 0, 3], 324),
+    ([3, 0, 66, 1], 1100), ([1, 0, 9, 0, 70], 2052), ([2, 1, 0, 1], 5632), ([0, 65, 3], 9300),      # several segments: of 512 k, of 1,024
+])
+def test_grouped(counts, k):
+    n, rows = 300, sum(counts)
     groups = len(counts)
     offsets = torch.tensor(np.concatenate([[0], np.cumsum(counts)]), dtype=torch.int32, device=DEV)
     src, w, status = rnd(50, k), rnd(groups, n, k, seed=1), torch.zeros(1, dtype=torch.int32, device=DEV)
