@@ -76,6 +76,7 @@ attn_latent_mma_kernel(const bf16* __restrict__ qx, const bf16* __restrict__ poo
     const int pieces = hdk / 8;
 
     pdl_wait();
+    qx = behind_wait(qx), pool = behind_wait(pool);
     // ---- the tile's queries -> shared memory (rows beyond the tile's tokens or the heads are zero)
     for (int idx = tid; idx < ROWS * pieces; idx += THREADS) {
         const int r = idx / pieces, p = idx - r * pieces;
@@ -282,6 +283,7 @@ attn_latent_combine_kernel(const float* __restrict__ part_o, const float* __rest
                            int n_splits, int hdv) {
     pdl_trigger();
     pdl_wait();
+    part_o = behind_wait(part_o), part_ml = behind_wait(part_ml);
     extern __shared__ float wts[];                  // [n_splits] weights of the splits, then their sum
     const int row = blockIdx.x, tid = threadIdx.x;
     const float* ml = part_ml + (size_t)row * n_splits * 2;

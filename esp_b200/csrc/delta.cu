@@ -171,6 +171,7 @@ __global__ void delta_prepare_kernel(float* __restrict__ qk, long long ldqk, int
                                      float* __restrict__ beta, int H) {
     pdl_trigger();
     pdl_wait();
+    raw = behind_wait(raw), b_raw = behind_wait(b_raw);
     const size_t n = blockIdx.x;
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, nwarp = blockDim.x >> 5;
     for (int job = warp; job < 2 * G; job += nwarp) {
@@ -196,6 +197,7 @@ __global__ void channel_decay_prepare_kernel(float* __restrict__ z, const float*
                                              float* __restrict__ q_out, long long rows, int width) {
     pdl_trigger();
     pdl_wait();
+    q = behind_wait(q);
     const long long total = rows * width;
     for (long long idx = blockIdx.x * (long long)blockDim.x + threadIdx.x; idx < total; idx += (long long)gridDim.x * blockDim.x) {
         const long long r = idx / width;
@@ -216,6 +218,7 @@ __global__ void causal_conv_kernel(const float* __restrict__ x, long long ldx, c
                                    const int* __restrict__ seq_slot, float* __restrict__ y, int C, int taps, int act) {
     pdl_trigger();
     pdl_wait();
+    x = behind_wait(x), conv_state = behind_wait(conv_state);
     const int n = blockIdx.x;
     const int seq = tok_seq[n];
     const int in_run = n - seq_start[seq];
@@ -259,6 +262,7 @@ causal_conv_tile_kernel(const float* __restrict__ x, long long ldx, const float*
         for (int e = 0; e < 4; e++) bs[e] = bias[c + e];
     }
     pdl_wait();
+    conv_state = behind_wait(conv_state);
     const int first = blockIdx.x * CONV_TILE_ROWS;
     const int last = min(first + CONV_TILE_ROWS, n_rows);
     float4 own[CONV_TILE_ROWS];                         // the tile's own inputs, all loads in flight together
@@ -322,6 +326,7 @@ __global__ void causal_conv_keep_kernel(const float* __restrict__ x, long long l
                                         const int* __restrict__ seq_slot, int C, int taps) {
     pdl_trigger();
     pdl_wait();
+    x = behind_wait(x);
     const int b = blockIdx.x;
     const int row0 = seq_start[b], run = seq_start[b + 1] - row0;
     if (run <= 0) return;

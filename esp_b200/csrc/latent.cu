@@ -31,6 +31,7 @@ __global__ void latent_kv_store_kernel(const float* __restrict__ d, const float*
                                        T* __restrict__ pool, int rank, int rot, float eps, int* __restrict__ status) {
     pdl_trigger();
     pdl_wait();
+    d = behind_wait(d);
     __shared__ float scratch[33];
     const int n = blockIdx.x, width = rank + rot;
     const float* src = d + (size_t)n * width;
@@ -72,6 +73,7 @@ __global__ void latent_q_rotate_kernel(const float* __restrict__ q, const float*
                                        int rot, int rank) {
     pdl_trigger();
     pdl_wait();
+    q = behind_wait(q);
     const int n = blockIdx.x;
     const float pos = (float)tok_pos[n];
     const int half = rot_dims / 2;
@@ -248,6 +250,7 @@ per_head_mma_kernel(const TA* __restrict__ a, long long lda, int a_head, const b
                     long long ldo, int o_head, int n_rows, int kin, int nout) {
     pdl_trigger();
     pdl_wait();
+    a = behind_wait(a);
     __shared__ __align__(16) bf16 as[PHM_T * PHM_LD];
     __shared__ __align__(16) bf16 ws[PHM_T * PHM_LD];
     const int n0 = blockIdx.x * PHM_T, h = blockIdx.y, j0 = blockIdx.z * PHM_T;
@@ -349,6 +352,7 @@ attn_latent_kernel(const T* __restrict__ qx, const T* __restrict__ pool, T* __re
                    int* __restrict__ status) {
     pdl_trigger();
     pdl_wait();
+    qx = behind_wait(qx), pool = behind_wait(pool);
     extern __shared__ float sm[];
     const int stride = hdk + 1;                    // rows of the chunk one bank apart
     float* rows = sm;                              // [LA_CHUNK][stride]
@@ -489,6 +493,7 @@ __global__ void head_scalar_gate_kernel(const TI* __restrict__ o, const float* _
                                         T* __restrict__ y, long long total, int H, int V) {
     pdl_trigger();
     pdl_wait();
+    o = behind_wait(o), gate = behind_wait(gate);
     const long long step = (long long)gridDim.x * blockDim.x;
     if (VEC) {
         const long long pieces = total / 4;
@@ -524,6 +529,7 @@ __global__ void heads_to_pages_kernel(const float* __restrict__ k, long long ldk
                                       int* __restrict__ status) {
     pdl_trigger();
     pdl_wait();
+    k = behind_wait(k), v = behind_wait(v);
     const int n = blockIdx.x;
     const int seq = tok_seq[n], pos = tok_pos[n];
     const int pg = table[(size_t)seq * table_stride + pos / page];

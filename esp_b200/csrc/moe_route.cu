@@ -823,6 +823,7 @@ __global__ void moe_combine_kernel(const float* __restrict__ expert_out, const i
                                    const float* __restrict__ topk_w, const float* __restrict__ ident, int n_real) {
     pdl_trigger();
     pdl_wait();
+    topk_ids = behind_wait(topk_ids), inverse = behind_wait(inverse), gate = behind_wait(gate), topk_w = behind_wait(topk_w);
     expert_out = behind_wait(expert_out);
     shared = behind_wait(shared);
     __shared__ int src[MAX_TOPK];

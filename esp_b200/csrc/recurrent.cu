@@ -30,6 +30,7 @@ __global__ void token_shift_mix_kernel(const T* __restrict__ h, const float* __r
                                        int n_mix, int n_rows, int width) {
     pdl_trigger();
     pdl_wait();
+    h = behind_wait(h), prev_state = behind_wait(prev_state);
     const int n = blockIdx.x;
     const int seq = tok_seq[n];
     const bool first = n == seq_start[seq];
@@ -84,6 +85,7 @@ __global__ void token_shift_keep_kernel(const T* __restrict__ h, float* __restri
                                         const int* __restrict__ seq_start, const int* __restrict__ seq_slot, int width) {
     pdl_trigger();
     pdl_wait();
+    h = behind_wait(h);
     const int b = blockIdx.x;
     const int last = seq_start[b + 1] - 1;
     if (last < seq_start[b]) return;
@@ -348,6 +350,7 @@ __global__ void gate_prepare_kernel(const float* __restrict__ q, long long ldq, 
                                     long long rows, int width) {
     pdl_trigger();
     pdl_wait();
+    q = behind_wait(q), g = behind_wait(g);
     const long long total = rows * width;
     for (long long idx = blockIdx.x * (long long)blockDim.x + threadIdx.x; idx < total; idx += (long long)gridDim.x * blockDim.x) {
         const long long r = idx / width;
@@ -374,6 +377,7 @@ __global__ void head_rmsnorm_gate_kernel(const float* __restrict__ o, const floa
                                          int H, int V, float eps, int gate_sigmoid) {
     pdl_trigger();
     pdl_wait();
+    o = behind_wait(o), gate = behind_wait(gate);
     const int warp = (blockIdx.x * blockDim.x + threadIdx.x) >> 5, lane = threadIdx.x & 31;
     if (warp >= n_rows * H) return;
     const int n = warp / H, h = warp - n * H;
@@ -424,6 +428,7 @@ row_rmsnorm_gate_kernel(const float* __restrict__ o, const float* __restrict__ w
                         int gate_sigmoid) {
     pdl_trigger();
     pdl_wait();
+    gate = behind_wait(gate);
     __shared__ float scratch[33];
     const int n = blockIdx.x / H, h = blockIdx.x - n * H, pieces = V / 4;
     const float4* src = reinterpret_cast<const float4*>(behind_wait(o) + ((size_t)n * H + h) * V);
@@ -474,6 +479,7 @@ matrix_memory_gates_kernel(const float* __restrict__ gi, const float* __restrict
                            float* __restrict__ m_out, int H) {
     pdl_trigger();
     pdl_wait();
+    gi = behind_wait(gi), gf = behind_wait(gf);
     __shared__ float s_i[MM_CHUNK], s_f[MM_CHUNK], s_carried[MM_CHUNK], s_new[MM_CHUNK];
     __shared__ float s_m;
     const int b = blockIdx.x, h = blockIdx.y, tid = threadIdx.x;
@@ -519,6 +525,7 @@ __global__ void matrix_memory_expand_kernel(const float* __restrict__ v, long lo
                                             float* __restrict__ v_out, int H, int V, int V1) {
     pdl_trigger();
     pdl_wait();
+    v = behind_wait(v), take = behind_wait(take);
     const size_t r = blockIdx.x;
     const int vw = H * V1;
     for (int c = threadIdx.x; c < vw; c += blockDim.x) {
@@ -538,6 +545,7 @@ __global__ void matrix_memory_finish_kernel(const float* __restrict__ o, const f
                                             float floor_eps, float q_scale) {
     pdl_trigger();
     pdl_wait();
+    o = behind_wait(o), m = behind_wait(m), gate = behind_wait(gate);
     const int warp = (blockIdx.x * blockDim.x + threadIdx.x) >> 5, lane = threadIdx.x & 31;
     if (warp >= n_rows * H) return;
     const int n = warp / H, h = warp - n * H;
@@ -600,6 +608,7 @@ __global__ void conv_branches_kernel(const float* __restrict__ proj, const float
                                      int taps) {
     pdl_trigger();
     pdl_wait();
+    proj = behind_wait(proj), conv_state = behind_wait(conv_state);
     const int n = blockIdx.x;
     const int seq = tok_seq[n];
     const int in_run = n - seq_start[seq];
@@ -628,6 +637,7 @@ __global__ void conv_state_keep_kernel(const float* __restrict__ proj, const flo
                                        const int* __restrict__ seq_start, const int* __restrict__ seq_slot, int C, int taps) {
     pdl_trigger();
     pdl_wait();
+    proj = behind_wait(proj);
     const int b = blockIdx.x;
     const int row0 = seq_start[b], run = seq_start[b + 1] - row0;
     if (run <= 0) return;
@@ -660,6 +670,7 @@ __global__ void diag_coefficients_kernel(float* __restrict__ gates, const float*
                                          const float* __restrict__ u, int C, int cb) {
     pdl_trigger();
     pdl_wait();
+    u = behind_wait(u);
     const size_t r = blockIdx.x;
     for (int c = threadIdx.x; c < C; c += blockDim.x) {
         const int blk = c / cb, j = c - blk * cb;

@@ -35,6 +35,7 @@ __global__ void rope_kvwrite_kernel(const float* __restrict__ qkv, const float* 
                                     int heads_per_block, int* __restrict__ status) {
     pdl_trigger();
     pdl_wait();
+    qkv = behind_wait(qkv);
     const int n = blockIdx.x;
     const int pos = tok_pos[n];
     const int seq = tok_seq[n];
@@ -94,6 +95,7 @@ rope_kvwrite_vec_kernel(const float* __restrict__ qkv, const float* __restrict__
                         int hd, int write_kv, int heads_per_block, int* __restrict__ status) {
     pdl_trigger();
     pdl_wait();
+    qkv = behind_wait(qkv);
     const int n = blockIdx.x;
     const int pos = tok_pos[n], seq = tok_seq[n];
     const int half = hd / 2, quads = half / 4, heads = nh + 2 * nkv;
@@ -203,6 +205,7 @@ __global__ void qknorm_kvwrite_kernel(const float* __restrict__ qkv, const float
                                       int* __restrict__ status) {
     pdl_trigger();
     pdl_wait();
+    qkv = behind_wait(qkv);
     const int n = blockIdx.x;
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, nwarp = blockDim.x >> 5;
     const int pos = tok_pos[n], seq = tok_seq[n];
@@ -292,6 +295,7 @@ __global__ void widenorm_rope_kvwrite_kernel(const float* __restrict__ qkv, cons
                                              int* __restrict__ status) {
     pdl_trigger();
     pdl_wait();
+    qkv = behind_wait(qkv);
     __shared__ float scratch[33];
     const int n = blockIdx.x, tid = threadIdx.x;
     const int pos = tok_pos[n], seq = tok_seq[n];
@@ -642,6 +646,7 @@ __global__ void pair_rope_unitnorm_kvwrite_kernel(const float* __restrict__ qkv,
                                                   int* __restrict__ status) {
     pdl_trigger();
     pdl_wait();
+    qkv = behind_wait(qkv);
     extern __shared__ float rope_cs[];                    // [rot / 2] cosines, then [rot / 2] sines of this row's angles
     const int n = blockIdx.x;
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, nwarp = blockDim.x >> 5;

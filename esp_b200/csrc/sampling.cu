@@ -204,6 +204,7 @@ pick_tokens_kernel(const float* __restrict__ logits, int vocab, int per_block, i
                    const int* __restrict__ row_slot, int* __restrict__ tokens, int* __restrict__ status) {
     pdl_trigger();
     pdl_wait();
+    logits = behind_wait(logits);
     extern __shared__ __align__(16) unsigned char smem_raw[];
     PickShared<CS>& s = *reinterpret_cast<PickShared<CS>*>(smem_raw);
     float* weights = reinterpret_cast<float*>(smem_raw + (sizeof(PickShared<CS>) + 15) / 16 * 16);     // [per_block] if keep

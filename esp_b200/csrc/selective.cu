@@ -95,6 +95,7 @@ selective_scan_kernel(const float* __restrict__ x, long long ldx, const float* _
     }
     const float dsk = live ? d_skip[c] : 0.f;
     pdl_wait();
+    dt_raw = behind_wait(dt_raw), bc = behind_wait(bc);
     const int seq = blockIdx.y;
     const int row0 = seq_start[seq], row1 = seq_start[seq + 1];
     if (row0 >= row1) return;
