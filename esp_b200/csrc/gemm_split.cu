@@ -9,9 +9,9 @@
 // product (|a3| <= 2^-17 and |w2| <= 2^-8 of the powers of two that a and w start with).  The tensor core cuts its sums off instead of
 // rounding them.  That error has one sign, so it grows with the number of additions and not with its root, most where one product or a
 // growing sum outweighs what is added.  So main is read out every SUB stages, 128 k, and added up with ordinary rounded additions.  c1
-// and c2 are 2^-8 of main and are read out a segment (256 to 1,024 k), whose value main + (c1 + c2) is added to the running sum.  The order of everything depends on
-// k alone, so a row's result has the same bits whatever other rows are in the call, whatever the tile's width, whichever group the
-// rows lie in and however many CTAs share a tile.
+// and c2 are 2^-8 of main and are read out a segment (256 to 1,024 k), whose value main + (c1 + c2) is added to the running sum.
+// The order of everything depends on k alone, so a row's result has the same bits whatever other rows are in the call, whatever the
+// tile's width, whichever group the rows lie in and however many CTAs share a tile.
 // Error against 64 bits (2-norm), this kernel / a chain of multiply-adds, K = 1,024, 2,048, 5,632: normal operands 1.3e-7 / 5.8e-7,
 // 1.3e-7 / 8.1e-7, 1.4e-7 / 1.35e-6; positive ones 1.7e-7 / 4.9e-7, 1.7e-7 / 7.0e-7, 1.7e-7 / 1.06e-6; one channel of the rows 300 times
 // the others 2.9e-7 / 5.8 to 8.0e-7, 2.9e-7 / 0.8 to 1.2e-6, 2.9e-7 / 1.4 to 1.9e-6 where it stands in the first half.  That channel sets
@@ -33,9 +33,9 @@
 // Main has two sets of columns, so that its read-out runs beside the next MMAs; 64 token rows leave room for two stages of split weights
 // then (2 x 64 + 128 + 2 x 96 of 512 columns).
 //
-// What bounds it, 64 token rows (1,400 rows, N = 11,264, K = 2,048: 520 us, 124 TFLOP/s, multiply-adds 1,251): a stage takes 1,900
-// cycles, of which the tensor core works 840 to 900.  The warp that issues (clock64) spends 711 of them issuing, 366 waiting for a stage,
-// 333 for accumulators to be read out and 282 on commits; the warps that split are busy most of the time as well (0.61 of the SM's issue
+// What bounds it, 64 token rows (1,400 rows, N = 11,264, K = 2,048: 520 us, 124 TFLOP/s, multiply-adds 1,251): a stage takes 1,750
+// cycles, of which the tensor core works 840 to 900.  The warp that issues (clock64; 1,900 with it) spends 711 of them issuing, 366
+// waiting for a stage, 333 for accumulators to be read out and 282 on commits; the warps that split are busy most of the time as well (0.66 of the SM's issue
 // slots), so that neither twice the warps for the token rows (539), pieces made before their slot is free (623) nor all eight weight warps
 // on each stage (673) helped.  Short tiles: 1,200 to 1,500 cycles a stage; six rows, N = 151,936 in 238 us, 5.2 TB/s; one row,
 // N = 11,264 / 6,144 / 2,048 27 / 18 / 10 us where multiply-adds take 21 / 17 / 14, K = 5,632, N = 2,048 17 and 34.
@@ -735,8 +735,8 @@ ESP_API int esp_gemm_split(const void* A, const int* a_rows, const void* W, cons
     if (e == cudaSuccess) e = cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
     if (e != cudaSuccess) return (int)e;
     {
-        // Few tiles of 16 rows: as many CTAs to each as there are SMs for (6 rows, K = 2,048: N = 2,048 31 us with a CTA a tile, 12 with
-        // four; N = 6,144 31 and 21 with two.  64 rows: N = 2,048 22 us, tiles of 64 rows 36).  Clusters of eight did not all find room at once
+        // Few tiles of 16 rows: as many CTAs to each as there are SMs for (6 rows, K = 2,048: N = 2,048 24.5 us with a CTA a tile, 9.6 with
+        // four; N = 6,144 24.8 and 17.5 with two.  64 rows: N = 2,048 18.5 us, tiles of 64 rows 35.8).  Clusters of eight did not all find room at once
         const long long tiles = row_runs(p, 16) * ((N + BF - 1) / BF);
         const int segments = ((K + KS - 1) / KS + p.seg_stages - 1) / p.seg_stages;
         const long long most = segments > MAX_PARTS ? 1 : min(min(6ll, (long long)segments), sms / tiles);
@@ -747,9 +747,10 @@ ESP_API int esp_gemm_split(const void* A, const int* a_rows, const void* W, cons
         if (p.share > 1) return launch<16, 2, 2, 4, 4, 1, true>(p, sms, stream);
     }
     // Few rows, of a group four on average: a short tile leaves tensor memory for two sets of accumulators.  A wait and a commit keep
-    // the issuing thread 300 and 90 cycles, a third of its time where the MMAs are short: groups, and a tile a CTA, have two stages behind
-    // one of each (100 rows over 60 groups, N = 2,816: 223 -> 192 us; one row, N = 11,264 29.7 -> 26.7).  Many tiles a CTA of one matrix,
-    // which memory bounds, are better off with the finer ring (6 rows, N = 151,936: 230 us against 245).
+    // the issuing warp some 300 and 90 cycles, a third of its time where the MMAs are short: groups, and a tile a CTA, have two stages
+    // behind one of each (200 rows over 60 groups, N = 2,816, K = 2,048 255 -> 243 us, 16 rows, N = 2,048, K = 1,408 44.8 -> 40.9; one row,
+    // N = 11,264 27.2 -> 25.6).  Many tiles a CTA of one matrix, which memory bounds, are better off with the finer ring (6 rows, N = 151,936:
+    // 234 us against 242).
     if (M <= (group_offsets ? 4ll * groups : 16ll)) {
         if (group_offsets || (N + BF - 1) / BF <= sms) return launch<16, 2, 2, 4, 6, 2, false>(p, sms, stream);
         return launch<16, 2, 2, 4, 6, 1, false>(p, sms, stream);

@@ -251,9 +251,10 @@ _ptr = _careful_ptr
 
 _F32, _BF16 = torch.float32, torch.bfloat16
 FLOATS = (_F32, _BF16)
-# From which size on 32-bit products go to the tensor cores, for any number of rows.  A launch there takes 6 us before its first sum: one
-# row / 200 rows, microseconds against the multiply-add kernels: N = 1,024, K = 512 6.9 / 14.0 against 4.3 / 18.2, K = 1,024 10.2 / 20.6
-# against 7.6 / 34, K = 2,048 10.4 / 34.6 against 13.5 / 64.5; 1,400 rows of 11,264 x 2,048 418 against 1,251.
+# From which size on 32-bit products go to the tensor cores, for any number of rows (a row's bits depend on its kernel).  A launch there
+# takes 6 us before its first sum: one row / 200 rows, microseconds against the multiply-add kernels: N = 1,024, K = 512 5.9 / 13.1
+# against 4.3 / 17.8, K = 1,024 9.0 / 20.5 against 7.7 / 34, K = 2,048 9.2 / 35.9 against 13.7 / 64.7; N = 2,048, K = 1,024 9.2 / 20.9
+# against 8.2 / 49.6; 1,400 rows of 11,264 x 2,048 520 against 1,252.
 SPLIT_MIN_K, SPLIT_MIN_ELEMENTS, SPLIT_MAX_GROUPS = 1024, 2 << 20, 256
 
 
