@@ -35,10 +35,11 @@
 //
 // What bounds it, 64 token rows (1,400 rows, N = 11,264, K = 2,048: 520 us, 124 TFLOP/s, multiply-adds 1,251): a stage takes 1,750
 // cycles, of which the tensor core works 840 to 900.  The warp that issues (clock64; 1,900 with it) spends 711 of them issuing, 366
-// waiting for a stage, 333 for accumulators to be read out and 282 on commits; the warps that split are busy most of the time as well (0.66 of the SM's issue
-// slots), so that neither twice the warps for the token rows (539), pieces made before their slot is free (623) nor all eight weight warps
-// on each stage (673) helped.  Short tiles: 1,200 to 1,500 cycles a stage; six rows, N = 151,936 in 238 us, 5.2 TB/s; one row,
-// N = 11,264 / 6,144 / 2,048 27 / 18 / 10 us where multiply-adds take 21 / 17 / 14, K = 5,632, N = 2,048 17 and 34.
+// waiting for a stage, 333 for accumulators to be read out and 282 on commits; the warps that split are busy most of the time as well
+// (0.66 of the SM's issue slots), so that neither eight warps for the token rows (539 us) nor pieces made before their slot is free
+// (623) nor all eight weight warps on each stage (673) helped.  Short tiles: 1,200 to 1,500 cycles a stage; six rows, N = 151,936 in
+// 234 us, 5.3 TB/s; one row, N = 11,264 / 6,144 / 2,048 26 to 30 / 18 / 10 us where multiply-adds take 21 / 17 / 14, K = 5,632, N = 2,048
+// 17 and 34.
 //
 // Persistent: a CTA per SM walks the tiles with the grid's stride; loads run ahead over the ends of tiles.  Every wait is
 // bounded, and begun behind pdl_wait() where it hangs on the token rows, so that it times this kernel and not those before it (one
